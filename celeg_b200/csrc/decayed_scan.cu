@@ -22,17 +22,14 @@
 //             q_i / P(i+1..4), k_j P(j+1..4) or k_j / P(5..j): at most four decays are divided by, and as a decay below
 //             1e-8 counts as 1e-8 (the old state's share is then below float32's rounding) that stays within range. The
 //             sums are one small product; between two blocks it has one more factor a channel, a product of decays.
-//   states    sum_j (k_j P(j+1..n)) v_j^T of every chunk, a 64 x 64 tile a block
-//   carry     the states at the chunks' starts, one element a thread, and the span's state after its last token
-//   outputs   both terms of o, a tile of 64 tokens x 64 columns a block
+// What follows is shared with other recurrences (chunk_scan.cuh): the states before the chunks and the span's last one, then
+// both terms of o; of the scalar form the sums of q.k too.
 //
 // Decoding is one launch: a block a (token, head) reads, updates and writes the state once.
-#include "common.cuh"
+#include "chunk_scan.cuh"
 
 namespace celeg_b200 {
 
-constexpr int kChunk = 64;
-constexpr int kPitch = kChunk + 4;           // floats of a row of a tile in shared memory: 16-byte rows, banks spread
 constexpr int kDecayMaxDim = 256;            // key size of the channel form
 
 __device__ __forceinline__ float softplus_of(float x) { return fmaxf(x, 0.0f) + log1pf(expf(-fabsf(x))); }
@@ -55,11 +52,6 @@ __global__ void chunk_plan_kernel(const int* span_begin, int spans, int chunk, i
 }
 
 // ------------------------------------------------------------------------------------------------- prepare, scalar
-__device__ __forceinline__ float2 two_floats(double x) {
-    const float high = (float)x;
-    return make_float2(high, (float)(x - (double)high));
-}
-
 // cum[t, h]: the sum of the decays' logarithms from the chunk's first token through t, a float and what it leaves of the double
 // that is summed in; dt[t, h]. A block takes 8 heads of a chunk: a warp a head, two neighbouring tokens a lane, the running
 // sum by shuffles.
@@ -102,84 +94,6 @@ __global__ void __launch_bounds__(256) scalar_decay_kernel(const float* raw, int
         cum[(size_t)(begin + t) * heads + h0 + h] = cum_s[t][h];
         dt[(size_t)(begin + t) * heads + h0 + h] = dt_s[t][h];
     }
-}
-
-// exp of the difference of two such sums
-__device__ __forceinline__ float decay_between(const float2& later, const float2& earlier) {
-    return expf((later.x - earlier.x) + (later.y - earlier.y));
-}
-
-// A tile of 64 x 64 floats into shared memory: rows r < rows of `src` (`stride` apart) times scale(r), columns c < columns;
-// zeros beyond. 256 threads, four neighbours a load where `four` says the rows allow it.
-template <typename Scale>
-__device__ __forceinline__ void load_tile(float (*dst)[kPitch], const float* src, long long stride, int rows, int columns,
-                                          bool four, Scale scale) {
-    if (four) {
-        float4 x[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int r = (threadIdx.x >> 4) + 16 * u, c = (threadIdx.x & 15) * 4;
-            x[u] = r < rows && c < columns ? *reinterpret_cast<const float4*>(src + r * stride + c)
-                                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int r = (threadIdx.x >> 4) + 16 * u, c = (threadIdx.x & 15) * 4;
-            const float f = scale(r);
-            *reinterpret_cast<float4*>(&dst[r][c]) = make_float4(x[u].x * f, x[u].y * f, x[u].z * f, x[u].w * f);
-        }
-        return;
-    }
-    for (int i = threadIdx.x; i < kChunk * kChunk; i += 256) {
-        const int r = i >> 6, c = i & 63;
-        dst[r][c] = r < rows && c < columns ? src[r * stride + c] * scale(r) : 0.0f;
-    }
-}
-struct NoScale { __device__ __forceinline__ float operator()(int) const { return 1.0f; } };
-// rows that begin at multiples of four floats (every offset in them is one of `sizes`, a sum of multiples where those are)
-__device__ __forceinline__ bool by_fours(const float* p, long long stride, int sizes) {
-    return ((((unsigned long long)p >> 2) | (unsigned long long)stride | (unsigned)sizes) & 3) == 0;
-}
-
-// products[chunk, group, i, j] = q_i . k_j, 64 x 64 a block
-__global__ void __launch_bounds__(256) chunk_products_kernel(const float* q, int q_stride, const float* k, int k_stride,
-                                                             const int* chunk_begin, float* products, int groups, int dim) {
-    __shared__ __align__(16) float q_s[kChunk][kPitch];
-    __shared__ __align__(16) float k_s[kChunk][kPitch];
-    chain_release();
-    chain_wait();
-    const int chunk = blockIdx.y, group = blockIdx.x;
-    const int begin = chunk_begin[chunk], count = chunk_begin[chunk + 1] - begin;
-    if (count <= 0) return;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    for (int e0 = 0; e0 < dim; e0 += kChunk) {
-        if (e0 > 0) __syncthreads();
-        load_tile(q_s, q + (size_t)begin * q_stride + (size_t)group * dim + e0, q_stride, count, dim - e0,
-                  by_fours(q, q_stride, dim), NoScale());
-        load_tile(k_s, k + (size_t)begin * k_stride + (size_t)group * dim + e0, k_stride, count, dim - e0,
-                  by_fours(k, k_stride, dim), NoScale());
-        __syncthreads();
-        const int width = min(kChunk, (dim - e0 + 3) & ~3);
-#pragma unroll 1
-        for (int e = 0; e < width; e += 4) {
-            float4 a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(&q_s[ty * 4 + i][e]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(&k_s[tx + 16 * j][e]);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[i][j] = fmaf(a[i].x, b[j].x, fmaf(a[i].y, b[j].y, fmaf(a[i].z, b[j].z, fmaf(a[i].w, b[j].w, acc[i][j]))));
-        }
-    }
-    float* dst = products + ((size_t)chunk * groups + group) * kChunk * kChunk;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dst[(ty * 4 + i) * kChunk + tx + 16 * j] = acc[i][j];
 }
 
 // ------------------------------------------------------------------------------------------------ prepare, channel
@@ -320,238 +234,6 @@ static int launch_channel_prepare(const ChannelPrepareArgs& args, int chunks, cu
     }
     launch_chained(channel_prepare_kernel<D>, dim3(args.heads, chunks), 256, smem, stream, args);
     return check_launch("channel_prepare");
-}
-
-// --------------------------------------------------------------------------------------------- states, carry, outputs
-struct ChunkArgs {
-    const float* q; int q_stride; const float* k; int k_stride;        // channel: prepared; scalar: as projected, shared
-    const float* v; int v_stride;
-    const float2* cum; const float* dt;      // scalar: [tokens, heads]
-    const float* total;                      // channel: [chunks, heads * dim]
-    const float* products;                   // channel: per head; scalar: per group of heads
-    const float* direct;                     // scalar: [heads], the values' share of the read-out, or null
-    const int* chunk_begin;
-    float* states;                           // [chunks, heads, dim, vdim]
-    float* out;                              // [tokens, heads * vdim]
-    int heads, groups, dim, vdim;
-};
-
-// sum_t k_t v_t^T over a chunk's tokens, k taken to the chunk's end
-template <bool CHANNEL>
-__global__ void __launch_bounds__(256) chunk_states_kernel(const ChunkArgs p) {
-    __shared__ __align__(16) float k_s[kChunk][kPitch];
-    __shared__ __align__(16) float v_s[kChunk][kPitch];
-    __shared__ float w_s[kChunk];
-    chain_release();
-    chain_wait();
-    const int chunk = blockIdx.z, head = blockIdx.y;
-    const int begin = p.chunk_begin[chunk], count = p.chunk_begin[chunk + 1] - begin;
-    if (count <= 0) return;
-    const int v_tiles = (p.vdim + kChunk - 1) / kChunk;
-    const int e0 = (blockIdx.x / v_tiles) * kChunk, c0 = (blockIdx.x % v_tiles) * kChunk;
-    const int k_at = (CHANNEL ? head : head / (p.heads / p.groups)) * p.dim + e0;
-    if (!CHANNEL) {
-        if (threadIdx.x < count) {
-            const size_t t = (size_t)(begin + threadIdx.x) * p.heads + head;
-            w_s[threadIdx.x] = p.dt[t] * decay_between(p.cum[(size_t)(begin + count - 1) * p.heads + head], p.cum[t]);
-        }
-        __syncthreads();
-    }
-    const float* k_src = p.k + (size_t)begin * p.k_stride + k_at;
-    if (CHANNEL) load_tile(k_s, k_src, p.k_stride, count, p.dim - e0, by_fours(p.k, p.k_stride, p.dim), NoScale());
-    else load_tile(k_s, k_src, p.k_stride, count, p.dim - e0, by_fours(p.k, p.k_stride, p.dim),
-                   [&](int r) { return r < count ? w_s[r] : 0.0f; });
-    load_tile(v_s, p.v + (size_t)begin * p.v_stride + (size_t)head * p.vdim + c0, p.v_stride, count, p.vdim - c0,
-              by_fours(p.v, p.v_stride, p.vdim), NoScale());
-    __syncthreads();
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-#pragma unroll 8
-    for (int t = 0; t < count; ++t) {
-        const float4 a = *reinterpret_cast<const float4*>(&k_s[t][ty * 4]);
-        const float4 b = *reinterpret_cast<const float4*>(&v_s[t][tx * 4]);
-        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-    float* dst = p.states + ((size_t)chunk * p.heads + head) * p.dim * p.vdim;
-    const bool four = (p.vdim & 3) == 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int e = e0 + ty * 4 + i;
-        if (e >= p.dim) continue;
-        if (four) {
-            if (c0 + tx * 4 < p.vdim)
-                *reinterpret_cast<float4*>(dst + (size_t)e * p.vdim + c0 + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-            continue;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = c0 + tx * 4 + j;
-            if (c < p.vdim) dst[(size_t)e * p.vdim + c] = acc[i][j];
-        }
-    }
-}
-
-// a thread V neighbouring elements of the state: a chunk's own sum is replaced by the state before the chunk
-template <bool CHANNEL, int V>
-__global__ void __launch_bounds__(128) chunk_carry_kernel(const ChunkArgs p, float* state, long long slot_stride,
-                                                          const int* span_slot, const int* span_first) {
-    chain_release();
-    chain_wait();
-    const int elements = p.heads * p.dim * p.vdim;
-    const int e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
-    if (e >= elements) return;
-    const int span = blockIdx.y;
-    const int first = span_first[span], last = span_first[span + 1];
-    if (first == last) return;
-    const int row = e / p.vdim, head = row / p.dim;                    // row: head * dim + key channel (V divides vdim)
-    float* cell = state + (long long)span_slot[span] * slot_stride + e;
-    float s[V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) s[i] = cell[i];
-    constexpr int kAhead = 8;
-    for (int c0 = first; c0 < last; c0 += kAhead) {
-        float own[kAhead][V], keep[kAhead];
-        int ends[kAhead];
-#pragma unroll
-        for (int i = 0; i < kAhead; ++i) {
-            const int c = c0 + i;
-            if (c >= last) continue;
-            ends[i] = CHANNEL ? 0 : p.chunk_begin[c + 1] - 1;
-            const float* src = p.states + (size_t)c * elements + e;
-            if (V == 4) {
-                const float4 x = *reinterpret_cast<const float4*>(src);
-                own[i][0] = x.x; own[i][1 % V] = x.y; own[i][2 % V] = x.z; own[i][3 % V] = x.w;
-            } else {
-                own[i][0] = *src;
-            }
-            if (CHANNEL) keep[i] = p.total[(size_t)c * p.heads * p.dim + row];
-        }
-        if (!CHANNEL) {
-#pragma unroll
-            for (int i = 0; i < kAhead; ++i)
-                if (c0 + i < last) keep[i] = p.cum[(size_t)ends[i] * p.heads + head].x;
-        }
-#pragma unroll
-        for (int i = 0; i < kAhead; ++i) {
-            const int c = c0 + i;
-            if (c >= last) continue;
-            float* dst = p.states + (size_t)c * elements + e;
-            if (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(s[0], s[1 % V], s[2 % V], s[3 % V]);
-            else *dst = s[0];
-            const float f = CHANNEL ? keep[i] : expf(keep[i]);
-#pragma unroll
-            for (int j = 0; j < V; ++j) s[j] = fmaf(f, s[j], own[i][j]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < V; ++i) cell[i] = s[i];
-}
-
-__device__ __forceinline__ void tile_product(const float (*a_s)[kPitch], const float (*b_s)[kPitch], int depth, int tx, int ty,
-                                             float (&acc)[4][4]) {
-#pragma unroll 1
-    for (int k = 0; k < depth; k += 4) {
-        float4 a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(&a_s[ty * 4 + i][k]);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) b[u] = *reinterpret_cast<const float4*>(&b_s[k + u][tx * 4]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float av[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                acc[i][0] = fmaf(av[u], b[u].x, acc[i][0]);
-                acc[i][1] = fmaf(av[u], b[u].y, acc[i][1]);
-                acc[i][2] = fmaf(av[u], b[u].z, acc[i][2]);
-                acc[i][3] = fmaf(av[u], b[u].w, acc[i][3]);
-            }
-        }
-    }
-}
-
-template <bool CHANNEL>
-__global__ void __launch_bounds__(256, 4) chunk_outputs_kernel(const ChunkArgs p) {
-    __shared__ __align__(16) float a_s[kChunk][kPitch];
-    __shared__ __align__(16) float b_s[kChunk][kPitch];
-    __shared__ float2 cum_s[kChunk];
-    __shared__ float dt_s[kChunk];
-    chain_release();
-    chain_wait();
-    const int chunk = blockIdx.z, head = blockIdx.y, c0 = blockIdx.x * kChunk;
-    const int begin = p.chunk_begin[chunk], count = p.chunk_begin[chunk + 1] - begin;
-    if (count <= 0) return;
-    const int group = CHANNEL ? head : head / (p.heads / p.groups);
-    if (!CHANNEL) {
-        if (threadIdx.x < kChunk) {
-            const size_t t = (size_t)(begin + threadIdx.x) * p.heads + head;
-            cum_s[threadIdx.x] = threadIdx.x < count ? p.cum[t] : make_float2(0.0f, 0.0f);
-            dt_s[threadIdx.x] = threadIdx.x < count ? p.dt[t] : 0.0f;
-        }
-        __syncthreads();
-    }
-    // the chunk's own tokens
-    const float* m = p.products + ((size_t)chunk * (CHANNEL ? p.heads : p.groups) + group) * kChunk * kChunk;
-    load_tile(b_s, p.v + (size_t)begin * p.v_stride + (size_t)head * p.vdim + c0, p.v_stride, count, p.vdim - c0,
-              by_fours(p.v, p.v_stride, p.vdim), NoScale());
-    {
-        float4 x[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) x[u] = reinterpret_cast<const float4*>(m)[threadIdx.x + 256 * u];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int r = (threadIdx.x >> 4) + 16 * u, c = (threadIdx.x & 15) * 4;
-            float v[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const bool seen = c + i <= r && r < count;
-                if (CHANNEL) v[i] = seen ? v[i] : 0.0f;
-                else v[i] = seen ? v[i] * decay_between(cum_s[r], cum_s[c + i]) * dt_s[c + i] : 0.0f;
-            }
-            *reinterpret_cast<float4*>(&a_s[r][c]) = make_float4(v[0], v[1], v[2], v[3]);
-        }
-    }
-    __syncthreads();
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    tile_product(a_s, b_s, min(kChunk, ty * 4 + 4), tx, ty, acc);      // (zeros beyond the diagonal)
-    if (!CHANNEL && p.direct) {
-        const float d = p.direct[head];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(d, b_s[ty * 4 + i][tx * 4 + j], acc[i][j]);
-    }
-    // the state before the chunk
-    const float* state = p.states + ((size_t)chunk * p.heads + head) * p.dim * p.vdim;
-    for (int e0 = 0; e0 < p.dim; e0 += kChunk) {
-        __syncthreads();
-        const float* q_src = p.q + (size_t)begin * p.q_stride + (size_t)group * p.dim + e0;
-        if (CHANNEL) load_tile(a_s, q_src, p.q_stride, count, p.dim - e0, by_fours(p.q, p.q_stride, p.dim), NoScale());
-        else load_tile(a_s, q_src, p.q_stride, count, p.dim - e0, by_fours(p.q, p.q_stride, p.dim),
-                       [&](int r) { return expf(cum_s[r].x); });
-        load_tile(b_s, state + (size_t)e0 * p.vdim + c0, p.vdim, p.dim - e0, p.vdim - c0, by_fours(p.states, p.vdim, p.dim * p.vdim),
-                  NoScale());
-        __syncthreads();
-        tile_product(a_s, b_s, min(kChunk, (p.dim - e0 + 3) & ~3), tx, ty, acc);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = ty * 4 + i;
-        if (r >= count) continue;
-        float* dst = p.out + (size_t)(begin + r) * p.heads * p.vdim + (size_t)head * p.vdim + c0;
-        if ((p.vdim & 3) == 0) {
-            if (c0 + tx * 4 < p.vdim) *reinterpret_cast<float4*>(dst + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-            continue;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (c0 + tx * 4 + j < p.vdim) dst[tx * 4 + j] = acc[i][j];
-    }
 }
 
 // ---------------------------------------------------------------------------------------------------- decoding
@@ -699,26 +381,6 @@ static int launch_decay_decode(const DecayDecodeArgs& p, int tokens, cudaStream_
     return check_launch("decay_decode");
 }
 
-template <bool CHANNEL>
-static int launch_chunks(const ChunkArgs& p, float* state, long long slot_stride, const int* span_slot, const int* span_first,
-                         int spans, int chunks, cudaStream_t stream) {
-    const int v_tiles = (p.vdim + kChunk - 1) / kChunk, e_tiles = (p.dim + kChunk - 1) / kChunk;
-    launch_chained(chunk_states_kernel<CHANNEL>, dim3(v_tiles * e_tiles, p.heads, chunks), 256, 0, stream, p);
-    int status = check_launch("chunk_states");
-    if (status != 0) return status;
-    const long long elements = (long long)p.heads * p.dim * p.vdim;
-    if (p.vdim % 4 == 0)                     // (scratch and slots are laid out for 16-byte accesses)
-        launch_chained(chunk_carry_kernel<CHANNEL, 4>, dim3((unsigned)((elements / 4 + 127) / 128), spans), 128, 0, stream, p, state,
-                       slot_stride, span_slot, span_first);
-    else
-        launch_chained(chunk_carry_kernel<CHANNEL, 1>, dim3((unsigned)((elements + 127) / 128), spans), 128, 0, stream, p, state,
-                       slot_stride, span_slot, span_first);
-    status = check_launch("chunk_carry");
-    if (status != 0) return status;
-    launch_chained(chunk_outputs_kernel<CHANNEL>, dim3(v_tiles, p.heads, chunks), 256, 0, stream, p);
-    return check_launch("chunk_outputs");
-}
-
 }  // namespace celeg_b200
 
 using namespace celeg_b200;
@@ -754,9 +416,13 @@ CELEG_API int celeg_channel_decay_scan(const float* q, int q_stride, const float
                      : dim <= 128 ? launch_channel_prepare<128>(first, chunks, stream)
                                   : launch_channel_prepare<256>(first, chunks, stream);
     if (status != 0) return status;
-    const ChunkArgs p = {q_out, heads * dim, k_out, heads * dim, v, v_stride, nullptr, nullptr, total, products, nullptr, plan,
-                         states, out, heads, heads, dim, vdim};
-    return launch_chunks<true>(p, state, slot_stride, span_slot, span_first, spans, chunks, stream);
+    ChunkArgs p = {};
+    p.q = q_out; p.q_stride = heads * dim; p.k = k_out; p.k_stride = heads * dim; p.v = v; p.v_stride = v_stride;
+    p.total = total; p.products = products;
+    p.chunk_begin = plan; p.pieces = 1; p.span_first = span_first; p.spans = spans;
+    p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = states; p.out = out;
+    p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = vdim;
+    return launch_chunk_scan<kChunkChannel>(p, chunks, stream);
 }
 
 // The scalar form: q and k have `groups` heads of dim that heads / groups heads of v share; raw: the steps before bias and
@@ -775,14 +441,15 @@ CELEG_API int celeg_scalar_decay_scan(const float* q, int q_stride, const float*
     const int* span_first = plan + max_chunks + 1;
     launch_chained(scalar_decay_kernel, dim3((heads + 7) / 8, chunks), 256, 0, stream, raw, raw_stride, dt_bias, a_log, plan,
                    cum, dt, heads);
-    int status = check_launch("scalar_decay");
+    const int status = check_launch("scalar_decay");
     if (status != 0) return status;
-    launch_chained(chunk_products_kernel, dim3(groups, chunks), 256, 0, stream, q, q_stride, k, k_stride, plan, products, groups, dim);
-    status = check_launch("chunk_products");
-    if (status != 0) return status;
-    const ChunkArgs p = {q, q_stride, k, k_stride, v, v_stride, cum, dt, nullptr, products, direct, plan, states, out, heads,
-                         groups, dim, vdim};
-    return launch_chunks<false>(p, state, slot_stride, span_slot, span_first, spans, chunks, stream);
+    ChunkArgs p = {};
+    p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = v; p.v_stride = v_stride;
+    p.cum = cum; p.dt = dt; p.direct = direct;
+    p.chunk_begin = plan; p.pieces = 1; p.span_first = span_first; p.spans = spans;
+    p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = states; p.out = out;
+    p.heads = heads; p.groups = groups; p.dim = dim; p.vdim = vdim;
+    return launch_chunk_scan<kChunkScalar>(p, chunks, stream);
 }
 
 // A token a request (row i of the inputs is request i's token, its slot span_slot[i]): state update, read-out, and for the

@@ -22,7 +22,7 @@
 //
 // Beside the scans: the gates of both mixers from their projections, the delta rule's short convolutions with
 // their carried inputs, unit norms and decay, and the per-head norm with the output gate.
-#include "common.cuh"
+#include "chunk_scan.cuh"
 
 namespace celeg_b200 {
 
@@ -50,10 +50,6 @@ struct ScanParams {
 __device__ __forceinline__ void cp_async_4(void* smem, const void* global) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(global));
-}
-__device__ __forceinline__ void cp_async_16(void* smem, const void* global) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(global));
 }
 __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() {
@@ -240,6 +236,54 @@ __global__ void mlstm_gates_kernel(const float* pre_i, const float* pre_f, int s
     const float gf = fminf(z, 0.0f) - log1pf(expf(-fabsf(z)));
     gates[(size_t)t * 2 * heads + h] = gi;
     gates[(size_t)t * 2 * heads + heads + h] = gf;
+}
+
+// What the mLSTM's chunked scan needs of a chunk's gates, each as two floats: with F_t the sum of the log forget gates from the
+// chunk's first token through t, F_t, i_t - F_t and the largest i_s - F_s of s <= t. The running maximum after token t is
+// then F_t + max(the one before the chunk, that), and F cancels in every weight: exp((i_s - F_s) - max(..)). A block takes 8
+// heads of a chunk: a warp a head, two neighbouring tokens a lane, sums and maxima by shuffles.
+__global__ void __launch_bounds__(256) mlstm_chunk_gates_kernel(const float* pre_i, const float* pre_f, int stride,
+                                                                const float* bias_i, const float* bias_f, float cap,
+                                                                const int* chunk_begin, float2* gates, int heads) {
+    chain_release();
+    chain_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.x * 8 + warp;
+    const int begin = chunk_begin[blockIdx.y], count = chunk_begin[blockIdx.y + 1] - begin;
+    if (h >= heads || count <= 0) return;
+    double gi[2], gf[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int t = min(2 * lane + u, count - 1);
+        gi[u] = cap * tanhf((pre_i[(size_t)(begin + t) * stride + h] + bias_i[h]) / cap);
+        const float z = cap * tanhf((pre_f[(size_t)(begin + t) * stride + h] + bias_f[h]) / cap);
+        gf[u] = fminf(z, 0.0f) - log1pf(expf(-fabsf(z)));              // logsigmoid(z)
+    }
+    double sum = gf[0] + gf[1];
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+        const double below = __shfl_up_sync(0xffffffffu, sum, offset);
+        if (lane >= offset) sum += below;
+    }
+    const double up = __shfl_up_sync(0xffffffffu, sum, 1);
+    const double first = (lane > 0 ? up : 0.0) + gf[0], second = first + gf[1];
+    const double own = gi[0] - first, next = gi[1] - second;
+    double high = fmax(own, next);
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+        const double below = __shfl_up_sync(0xffffffffu, high, offset);
+        if (lane >= offset) high = fmax(high, below);
+    }
+    const double below = __shfl_up_sync(0xffffffffu, high, 1);
+    const double high_first = lane > 0 ? fmax(below, own) : own;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int t = 2 * lane + u;
+        if (t >= count) continue;
+        float2* dst = gates + (size_t)(begin + t) * 3 * heads + h;
+        dst[0] = two_floats(u ? second : first);
+        dst[heads] = two_floats(u ? next : own);
+        dst[2 * heads] = two_floats(u ? high : high_first);
+    }
 }
 
 struct DeltaPrepareArgs {
@@ -776,7 +820,8 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Retention over long spans, cut into segments. With a constant decay d the state after token t of a segment
+// Retention over long spans, cut into segments: of up to 128 tokens by the kernels of chunk_scan.cuh, a state every 64 tokens;
+// longer ones, for which the caller's scratch holds no such states, by the kernels here. With a constant decay d the state after token t of a segment
 // that begins at token b is S_t = d^(t-b+1) S_(b-1) + L_t, L_t the state the segment's own tokens would have built
 // from zero. So the segments of all spans are scanned side by side from zero states (the scan kernel above, one
 // "span" a segment), which also gives the segment's final L and the local read-outs L_t^T q_t; the states at the
@@ -1236,15 +1281,27 @@ CELEG_API int celeg_retention_segmented(const float* q, int q_stride, const floa
                   "retention_segmented: %d segments do not hold %d tokens in %d spans (or exceed one launch)", max_segments,
                   tokens, spans);
     if (spans == 0 || tokens == 0) return 0;
-    const long long elements = (long long)heads * dim * vdim;
-    float* local = float_scratch;
-    float* carried = float_scratch + (size_t)max_segments * elements;
     int* seg_begin = int_scratch;                          // [max_segments + 1]
     int* span_first = int_scratch + max_segments + 1;      // [spans + 1]
-    cudaMemsetAsync(local, 0, (size_t)max_segments * elements * sizeof(float), stream);
+    const int pieces = segment / 64;
+    CELEG_REQUIRE((long long)max_segments * pieces <= 65535, "retention_segmented: %d segments of %d pieces exceed one launch",
+                  max_segments, pieces);
     launch_chained(retention_plan_kernel, 1, 32, 0, stream, span_begin, spans, segment, max_segments, seg_begin, span_first);
     int status = check_launch("retention_plan");
     if (status != 0) return status;
+    if (pieces <= 2) {         // the scratch holds a state for every 64 tokens
+        ChunkArgs p = {};
+        p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = v; p.v_stride = v_stride;
+        p.decay = decay; p.q_scale = q_scale;
+        p.chunk_begin = seg_begin; p.pieces = pieces; p.span_first = span_first; p.spans = spans;
+        p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = float_scratch; p.out = out;
+        p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = vdim;
+        return launch_chunk_scan<kChunkConstant>(p, max_segments * pieces, stream);
+    }
+    const long long elements = (long long)heads * dim * vdim;
+    float* local = float_scratch;
+    float* carried = float_scratch + (size_t)max_segments * elements;
+    cudaMemsetAsync(local, 0, (size_t)max_segments * elements * sizeof(float), stream);
     const int vector_copies = dim % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && (((size_t)q | (size_t)k) & 15) == 0;
     const ScanParams p = {q, k, v, q_stride, k_stride, v_stride, decay, out, local, elements, seg_begin, identity,
                           heads, heads, dim, vdim, q_scale, vector_copies};
@@ -1255,11 +1312,38 @@ CELEG_API int celeg_retention_segmented(const float* q, int q_stride, const floa
                                                             carried, decay, (int)elements, dim * vdim);
     status = check_launch("retention_carry");
     if (status != 0) return status;
-    const int pieces = segment / 64;
     dim3 add_grid((vdim + 63) / 64, heads, max_segments * pieces);
-    CELEG_REQUIRE((long long)max_segments * pieces <= 65535, "retention_segmented: %d segments of %d pieces exceed one launch",
-                  max_segments, pieces);
     retention_add_carried_kernel<<<add_grid, 256, 0, stream>>>(q, q_stride, carried, seg_begin, decay, out, heads, dim, vdim,
                                                                 pieces);
     return check_launch("retention_add_carried");
+}
+
+// The mLSTM over the step's spans in chunks of 64 tokens, from the projection's rows to the read-outs. plan: of
+// celeg_chunk_plan with the same max_chunks (>= what the spans make; `chunks` bounds it). Scratch: gates (two floats each)
+// [tokens, 3, heads], peaks (doubles) [chunks, heads], norms [chunks, heads, dim], states [chunks, heads, dim, vdim]. The slots
+// hold what celeg_recurrent_scan's do. Same result as the gates' kernel and mode 1 of that scan but for rounding.
+CELEG_API int celeg_mlstm_chunk_scan(const float* q, int q_stride, const float* k, int k_stride, const float* v, int v_stride,
+                                     const float* pre_i, const float* pre_f, int pre_stride, const float* bias_i,
+                                     const float* bias_f, float cap, float2* gates, double* peaks, float* norms, float* states,
+                                     float* out, float* state, long long slot_stride, const int* span_slot, const int* plan,
+                                     int max_chunks, int spans, int chunks, int heads, int dim, int vdim, float q_scale,
+                                     cudaStream_t stream) {
+    CELEG_REQUIRE(spans >= 0 && chunks >= 0 && heads > 0 && dim > 0 && vdim > 0 && cap > 0.0f,
+                  "mlstm_chunk_scan: invalid sizes spans=%d chunks=%d heads=%d dim=%d vdim=%d cap=%g", spans, chunks, heads, dim,
+                  vdim, cap);
+    CELEG_REQUIRE(dim <= kScanMaxDim, "mlstm_chunk_scan: a key size of %d exceeds %d", dim, kScanMaxDim);
+    CELEG_REQUIRE(chunks <= max_chunks && chunks <= 65535 && spans <= 65535 && heads <= 65535,
+                  "mlstm_chunk_scan: %d chunks of %d, %d spans or %d heads exceed one launch", chunks, max_chunks, spans, heads);
+    if (spans == 0 || chunks == 0) return 0;
+    launch_chained(mlstm_chunk_gates_kernel, dim3((heads + 7) / 8, chunks), 256, 0, stream, pre_i, pre_f, pre_stride, bias_i,
+                   bias_f, cap, plan, gates, heads);
+    const int status = check_launch("mlstm_chunk_gates");
+    if (status != 0) return status;
+    ChunkArgs p = {};
+    p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = v; p.v_stride = v_stride;
+    p.gates = gates; p.peaks = peaks; p.norms = norms; p.q_scale = q_scale;
+    p.chunk_begin = plan; p.pieces = 1; p.span_first = plan + max_chunks + 1; p.spans = spans;
+    p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = states; p.out = out;
+    p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = vdim;
+    return launch_chunk_scan<kChunkStable>(p, chunks, stream);
 }

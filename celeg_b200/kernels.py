@@ -179,6 +179,9 @@ _SIGNATURES = {
     "celeg_channel_decay_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    "celeg_mlstm_chunk_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
+                               c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
+                               c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
     "celeg_scalar_decay_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
@@ -914,6 +917,28 @@ def recurrent_scan(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
                                           _ptr(span_slot), spans, heads, kv_heads, dim, vdim, q_scale, _stream()))
 
 
+def mlstm_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, pre_i: torch.Tensor, pre_f: torch.Tensor,
+                     bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float, gates: torch.Tensor, peaks: torch.Tensor,
+                     norms: torch.Tensor, states: torch.Tensor, out: torch.Tensor, state: torch.Tensor, slot_stride: int,
+                     span_slot: torch.Tensor, plan: torch.Tensor, max_chunks: int, spans: int, chunks: int, heads: int,
+                     dim: int, vdim: int, q_scale: float) -> None:
+    """The mLSTM (:func:`mlstm_gates`, then mode SCAN_MLSTM of :func:`recurrent_scan`) over the step's spans in chunks of
+    64 tokens (csrc/chunk_scan.cuh), from a plan of :func:`chunk_plan`. Scratch: float32 ``gates`` [tokens, 6 heads],
+    float64 ``peaks`` [chunks * heads], float32 ``norms`` [chunks * heads * dim], ``states`` [chunks * heads * dim * vdim]."""
+    for tensor in (q, k, v, pre_i, pre_f, bias_i, bias_f, gates, norms, states, out, state):
+        assert tensor.dtype == torch.float32 and tensor.stride(-1) == 1
+    assert gates.is_contiguous() and gates.shape[1] == 6 * heads and pre_i.stride(0) == pre_f.stride(0)
+    assert out.is_contiguous() and out.shape[1] == heads * vdim
+    assert peaks.dtype == torch.float64 and peaks.numel() >= chunks * heads
+    assert norms.numel() >= chunks * heads * dim and states.numel() >= chunks * heads * dim * vdim
+    _check(library().celeg_mlstm_chunk_scan(
+        _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(pre_i), _ptr(pre_f), pre_i.stride(0),
+        _ptr(bias_i), _ptr(bias_f), cap, _ptr(gates), _ptr(peaks), _ptr(norms), _ptr(states), _ptr(out), _ptr(state), slot_stride,
+        _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, dim, vdim, q_scale, _stream()))
+    global LAUNCHES
+    LAUNCHES += 2          # the gates, the states (one launch or two), the read-outs
+
+
 def retention_segmented(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
                         state: torch.Tensor, slot_stride: int, span_begin: torch.Tensor, span_slot: torch.Tensor, spans: int,
                         tokens: int, heads: int, dim: int, vdim: int, q_scale: float, segment: int, max_segments: int,
@@ -932,7 +957,7 @@ def retention_segmented(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay
                                                tokens, heads, dim, vdim, q_scale, segment, max_segments,
                                                _ptr(float_scratch), _ptr(int_scratch), _ptr(identity), _stream()))
     global LAUNCHES
-    LAUNCHES += 4          # the plan, the scan, the carried states, their share of the read-outs (and a memset)
+    LAUNCHES += 2 if segment <= 128 else 3     # the plan, the states, the read-outs; or scan, carried states and their share
 
 
 def recurrent_decode(mode: int, proj: torch.Tensor, offsets: Tuple[int, int, int, int, int, int],
@@ -1377,7 +1402,7 @@ def channel_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: tor
         _ptr(q_out), _ptr(k_out), _ptr(total), _ptr(products), _ptr(states), _ptr(out), _ptr(state), slot_stride,
         _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, dim, vdim, _stream()))
     global LAUNCHES
-    LAUNCHES += 3          # the chunks' own products, their states, the carried states, the read-outs
+    LAUNCHES += 2          # the chunks' own products, the states (one launch or two), the read-outs
 
 
 def scalar_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: torch.Tensor, dt_bias: torch.Tensor,
@@ -1398,7 +1423,7 @@ def scalar_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: to
         _ptr(direct), _ptr(cum), _ptr(dt), _ptr(products), _ptr(states), _ptr(out), _ptr(state), slot_stride, _ptr(span_slot),
         _ptr(plan), max_chunks, spans, chunks, heads, groups, dim, vdim, _stream()))
     global LAUNCHES
-    LAUNCHES += 4          # the decays, the products, then as above
+    LAUNCHES += 2          # the decays, then as above
 
 
 def channel_decay_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_scale: float, low: torch.Tensor,

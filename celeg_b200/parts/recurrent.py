@@ -24,6 +24,7 @@ import torch
 
 from .. import kernels
 from ..cache.manager import StateNeed
+from .decayed import ChunkedSpans
 from .mixers import StateBinding
 from .registry import register_part
 from .runtime import Runtime, StepContext
@@ -61,6 +62,17 @@ class MlstmMixer:
         self.gates = rt.scratch("recurrent.gates", 2 * self.heads, torch.float32)
         self.read = rt.scratch("recurrent.read", self.v_width, torch.float32)
         self.gated = rt.scratch("recurrent.gated", self.v_width)
+        self.spans = ChunkedSpans(rt)
+        chunks = self.spans.max_chunks
+        self.chunk_gates = rt.scratch("recurrent.chunk_gates", 6 * self.heads, torch.float32)
+        self.peaks = rt.flat_scratch("recurrent.peaks", chunks * self.heads, torch.float64)
+        self.norms = rt.flat_scratch("recurrent.norms", chunks * self.qk_width, torch.float32)
+        self.states = rt.flat_scratch("recurrent.states", chunks * self.qk_width * self.vdim, torch.float32)
+
+    # Steps whose longest portion has at least this many tokens are scanned in chunks. Measured for one portion at 16 heads of
+    # 64 x 128, the mixer between its projections included: 128 tokens 53 us in chunks, 51 token by token; 192: 57 and 70;
+    # 2,048: 163 and 564.
+    CHUNKED_FROM = 144
 
     def cache_need(self):
         return StateNeed(elements=self.heads * self.dim * self.vdim + self.heads * self.dim + self.heads)
@@ -92,10 +104,20 @@ class MlstmMixer:
                                      self.gated)
             rt.linear(self.gated, self.w_out, out, t)
             return
-        kernels.mlstm_gates(pre_i, pre_f, self.bias_i, self.bias_f, self.cap, self.gates, t, self.heads)
-        kernels.recurrent_scan(kernels.SCAN_MLSTM, q, k, v, self.gates, self.read, b.state, b.slot_stride,
-                               step.span_begin, step.span_slot, step.spans, self.heads, self.heads, self.dim,
-                               self.vdim, self.dim ** -0.5)
+        # long portions in chunks; what lies before them (single tokens), and steps of short spans, token by token
+        one_by_one = step.leading_single_tokens if step.max_span >= self.CHUNKED_FROM else t
+        if one_by_one:
+            spans = step.spans if one_by_one == t else one_by_one
+            kernels.mlstm_gates(pre_i, pre_f, self.bias_i, self.bias_f, self.cap, self.gates, one_by_one, self.heads)
+            kernels.recurrent_scan(kernels.SCAN_MLSTM, q, k, v, self.gates, self.read, b.state, b.slot_stride,
+                                   step.span_begin, step.span_slot, spans, self.heads, self.heads, self.dim,
+                                   self.vdim, self.dim ** -0.5)
+        if one_by_one < t:
+            plan, spans, chunks = self.spans.of(step, one_by_one)
+            kernels.mlstm_chunk_scan(q, k, v, pre_i, pre_f, self.bias_i, self.bias_f, self.cap, self.chunk_gates, self.peaks,
+                                     self.norms, self.states, self.read, b.state, b.slot_stride, step.span_slot[one_by_one:],
+                                     plan, self.spans.max_chunks, spans, chunks, self.heads, self.dim, self.vdim,
+                                     self.dim ** -0.5)
         kernels.gated_head_norm(self.read, gate, self.norm, True, self.gated, t, self.heads, self.vdim, self.eps,
                                 kernels.GATE_SIGMOID)
         rt.linear(self.gated, self.w_out, out, t)
@@ -223,8 +245,8 @@ class RetentionMixer:
         self.projected = rt.scratch("recurrent.proj", self.proj_width, torch.float32)
         self.read = rt.scratch("recurrent.read", self.v_width, torch.float32)
         self.gated = rt.scratch("recurrent.gated", self.v_width)
-        # long prompts: segments of SEGMENT tokens scanned side by side (the decay is a constant, so a segment's
-        # state and read-outs from a zero state are corrected afterwards by what was carried into it)
+        # long prompts: segments of SEGMENT tokens side by side (the decay is a constant, so what a segment's tokens leave
+        # in the state does not depend on what was carried into it)
         self.max_segments = rt.max_tokens // self.SEGMENT + rt.max_requests + 16
         elements = self.heads * self.dim * self.vdim
         self.segment_states = rt.flat_scratch("retention.segments", 2 * self.max_segments * elements, torch.float32)
@@ -232,7 +254,29 @@ class RetentionMixer:
         self.segment_numbers = torch.arange(self.max_segments, dtype=torch.int32, device=rt.device)
 
     SEGMENT = 128               # tokens a segment
-    SEGMENTED_FROM = 384        # steps of at least this many tokens are scanned in segments
+    # Steps of at least this many tokens are scanned in segments. Measured for one portion at 16 heads of 64 x 128, the mixer
+    # between its projections included: 128 tokens 39 us in segments, 41 token by token; 192: 43 and 53; 384: 51 and 91.
+    SEGMENTED_FROM = 160
+
+    def _scan(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, step: StepContext, scale: float) -> None:
+        """The recurrence over the step's spans into ``read``: single tokens at the step's head token by token, long
+        portions behind them in segments."""
+        b, t = self.binding, step.tokens
+        single = step.leading_single_tokens
+        spans = step.spans - single
+        segments = (t - single) // self.SEGMENT + spans
+        if not (t - single >= self.SEGMENTED_FROM and segments <= self.max_segments
+                and segments + spans + 2 <= self.segment_plan.numel()):
+            single, spans = t, step.spans
+        if single:
+            kernels.recurrent_scan(kernels.SCAN_RETENTION, q, k, v, self.decay, self.read, b.state, b.slot_stride,
+                                   step.span_begin, step.span_slot, spans if single == t else single, self.heads, self.heads,
+                                   self.dim, self.vdim, scale)
+        if single < t:
+            # (span_begin counts the step's tokens: the rows stay where they are)
+            kernels.retention_segmented(q, k, v, self.decay, self.read, b.state, b.slot_stride, step.span_begin[single:],
+                                        step.span_slot[single:], spans, t - single, self.heads, self.dim, self.vdim, scale,
+                                        self.SEGMENT, segments, self.segment_states, self.segment_plan, self.segment_numbers)
 
     def cache_need(self):
         return StateNeed(elements=self.heads * self.dim * self.vdim)
@@ -260,15 +304,7 @@ class RetentionMixer:
         k = rows[:, width:2 * width]
         v = rows[:, 2 * width:2 * width + self.v_width]
         gate = rows[:, 2 * width + self.v_width:]
-        segments = t // self.SEGMENT + step.spans
-        if t >= self.SEGMENTED_FROM and segments <= self.max_segments and segments + step.spans + 2 <= self.segment_plan.numel():
-            kernels.retention_segmented(q, k, v, self.decay, self.read, b.state, b.slot_stride, step.span_begin,
-                                        step.span_slot, step.spans, t, self.heads, self.dim, self.vdim, self.dim ** -0.5,
-                                        self.SEGMENT, segments, self.segment_states, self.segment_plan, self.segment_numbers)
-        else:
-            kernels.recurrent_scan(kernels.SCAN_RETENTION, q, k, v, self.decay, self.read, b.state, b.slot_stride,
-                                   step.span_begin, step.span_slot, step.spans, self.heads, self.heads, self.dim,
-                                   self.vdim, self.dim ** -0.5)
+        self._scan(q, k, v, step, self.dim ** -0.5)
         kernels.gated_head_norm(self.read, gate, None, False, self.gated, t, self.heads, self.vdim, self.eps,
                                 kernels.GATE_SILU)
         rt.linear(self.gated, self.w_out, out, t)
@@ -307,17 +343,7 @@ class LightningAttentionMixer(RetentionMixer):
             q = rows[:, :width]
             k = rows[:, width:2 * width]
             v = rows[:, 2 * width:2 * width + self.v_width]
-            segments = t // self.SEGMENT + step.spans
-            if (t >= self.SEGMENTED_FROM and segments <= self.max_segments
-                    and segments + step.spans + 2 <= self.segment_plan.numel()):
-                kernels.retention_segmented(q, k, v, self.decay, self.read, b.state, b.slot_stride, step.span_begin,
-                                            step.span_slot, step.spans, t, self.heads, self.dim, self.vdim, 1.0,
-                                            self.SEGMENT, segments, self.segment_states, self.segment_plan,
-                                            self.segment_numbers)
-            else:
-                kernels.recurrent_scan(kernels.SCAN_RETENTION, q, k, v, self.decay, self.read, b.state, b.slot_stride,
-                                       step.span_begin, step.span_slot, step.spans, self.heads, self.heads, self.dim,
-                                       self.vdim, 1.0)
+            self._scan(q, k, v, step, 1.0)
         # one norm over all heads: a single "head" as wide as all of them
         kernels.gated_head_norm(self.read, gate, self.norm, True, self.gated, t, 1, self.v_width, self.eps,
                                 kernels.GATE_SIGMOID)
