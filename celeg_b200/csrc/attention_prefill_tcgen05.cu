@@ -1,19 +1,17 @@
 // Paged causal grouped-query attention for prompt portions on Blackwell's fifth-generation tensor
-// cores, for a head size of 64 (bfloat16):
+// cores, for head sizes D of 64 and 128 (bfloat16):
 //
 //   grid = (query heads, query tiles); a query tile is up to 128 consecutive tokens of one span; tiles with
 //   many keys come first in launch order, so that the grid drains with short ones.
-//   Six warps. Warp 0 brings Q (one box of 128 rows x 64) and, per block of 64 keys, the K and V
-//   rows page by page through the request's block table into a four-stage ring by TMA (128-byte
-//   swizzle; a page is one box of page_tokens rows x 64): lane 0 waits for the stage, then lane 2 pg brings
-//   page pg of K and lane 2 pg + 1 that of V, each looked up one block ahead (one thread issuing a block's
-//   up to 16 copies in turn took longer than the block's softmax). Warp 1 issues the MMAs:
-//       S[128 x 64] = Q K^T           (tcgen05.mma M128 N64 K16 x 4, both operands K-major)
-//       O[128 x 64] += P V            (M128 N64 K16 x 4, P from tensor memory as the A operand, V as it lies
+//   Six warps. Warp 0 brings Q (boxes of 128 rows x 64) and, per block of 64 keys, the K and V
+//   rows page by page through the request's block table into a ring each by TMA (128-byte
+//   swizzle; a page is D / 64 boxes of page_tokens rows x 64, a lane each; K a block ahead of V). Warp 1 issues the MMAs:
+//       S[128 x 64] = Q K^T           (tcgen05.mma M128 N64 K16 x D / 16, both operands K-major)
+//       O[128 x D] += P V             (M128 N64 K16 x 4 D / 64, P from tensor memory as the A operand, V as it lies
 //                                      in the cache, keys x 64: the MN-major form of the B operand)
 //   with S, P and O in tensor memory. S and P exist twice (even and odd blocks of keys): the scores of block
 //   j+1 are being multiplied while the softmax threads work on block j, and P V of block j runs while they
-//   work on block j+1. 256 columns of tensor memory and 81 KiB of shared memory a block: two blocks per SM.
+//   work on block j+1. 256 columns of tensor memory and 81 or 97 KiB of shared memory a block: two blocks per SM.
 //   Warps 2-5 are the softmax: a thread owns one query row (its TMEM lane), reads S with tcgen05.ld, masks
 //   (causal, window, rows past the span; blocks that every row sees whole skip the mask), takes the maximum,
 //   writes P = exp2(scaled S - maximum) as bfloat16 pairs into tensor memory with tcgen05.st and adds to its
@@ -26,7 +24,12 @@
 //   Every wait on an mbarrier is bounded (tcgen05.cuh); a role that gives up records a code, and the
 //   block leaves through the common exit (tensor memory released).
 //
-// Head sizes other than 64, pages that are no multiple of 8 tokens or do not divide 64, and float32
+// What bounds it: the softmax's chain a block (read S, maximum, 64 exponentials a thread, write P), of which two blocks an SM
+// hide one another's; at 32 heads of 64 and 8,192 tokens 433 us, 635 TFLOP/s. A head size of 128 has twice the products
+// behind the same chain: prompts of 889 and 3,112 tokens in one launch, 16 heads on 4, 71 us (605 TFLOP/s) against 248 us of
+// the mma.sync kernel; 128 tokens after 16,000: 309 us with the projections, 762 before.
+//
+// Other head sizes, pages that are no multiple of 8 tokens or do not divide 64, and float32
 // go to attention_prefill.cu (mma.sync) or attention_generic.cu.
 //
 // Counterparts in celeg: see attention_prefill.cu.
@@ -37,18 +40,32 @@ namespace celeg_b200 {
 constexpr int kFaThreads = 192;
 constexpr int kFaM = 128;                 // query rows per tile
 constexpr int kFaN = 64;                  // keys per block
-constexpr int kFaD = 64;
-constexpr unsigned kFaQBytes = kFaM * kFaD * 2;         // 16 KiB
-constexpr unsigned kFaKvBytes = kFaN * kFaD * 2;        // 8 KiB each for K and V
-constexpr int kFaStages = 4;
-constexpr unsigned kFaSmemBytes = kFaQBytes + kFaStages * 2 * kFaKvBytes + 1024;
-// Tensor memory: S of even and odd blocks at columns 0..63 and 64..127, O at 128..191, P (bfloat16, two keys a
-// column) of even and odd blocks at 192..223 and 224..255
+// D: the head size, 64 or 128. Rows of 128 lie in shared memory as two halves of 64 (a swizzled row is 128 bytes). Four stages
+// of a block's K and V together, or, where two are all that two blocks per SM leave room for, K and V on their own: a block's
+// K is free when its scores are done, a whole block before its V. (Four stages of K and V on their own cost a head size of 64
+// a tenth: one more wait a block for the copying warp and for the thread that issues the products.)
+template <int D>
+struct FaLayout {
+    static constexpr int kHalves = D / 64;
+    static constexpr bool kTogether = D == 64;
+    static constexpr int kStages = kTogether ? 4 : 2;
+    static constexpr unsigned kQHalf = kFaM * 128, kKvHalf = kFaN * 128;
+    static constexpr unsigned kQBytes = kHalves * kQHalf;       // 16 or 32 KiB
+    static constexpr unsigned kKvBytes = kHalves * kKvHalf;     // 8 or 16 KiB each for a block's K and V
+    static constexpr unsigned kSmemBytes = kQBytes + kStages * 2 * kKvBytes + 1024;      // 81 or 97 KiB
+    // Tensor memory: S of even and odd blocks at columns 0..63 and 64..127, O from 128 on. P (bfloat16, two keys a column) of
+    // even and odd blocks at 192..223 and 224..255; at a head size of 128, where O takes those, over the scores it is made
+    // of, and a block's scores then wait until P V of the block before the last has read its P.
+    static constexpr unsigned kOColumn = 2 * kFaN;
+    static constexpr bool kOverScores = D == 128;
+    static __device__ __forceinline__ unsigned p_column(int i) {
+        return kOverScores ? (unsigned)((i & 1) * kFaN) : 2 * kFaN + D + (unsigned)((i & 1) * (kFaN / 2));
+    }
+};
 constexpr unsigned kFaTmemColumns = 256;
-constexpr unsigned kFaOColumn = 2 * kFaN, kFaPColumn = 2 * kFaN + kFaD;
 
 struct FaParams {
-    __nv_bfloat16* out;            // [tokens, q_heads * 64]
+    __nv_bfloat16* out;            // [tokens, q_heads * D]
     const int* positions;          // [tokens]
     const int* span_begin;         // [spans + 1]
     const int* block_table;        // [spans, table_stride]
@@ -78,12 +95,15 @@ __host__ __device__ constexpr unsigned instruction_descriptor_b_mn(int m, int n)
     return instruction_descriptor(m, n) | (1u << 16);
 }
 
+template <int D>
 __global__ void __launch_bounds__(kFaThreads)
 attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                  const __grid_constant__ CUtensorMap map_v, const FaParams p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long q_full, kv_full[kFaStages], kv_empty[kFaStages], s_full[2], p_full[2],
-        o_full[2];
+    using L = FaLayout<D>;
+    constexpr int kStages = L::kStages;
+    __shared__ __align__(8) unsigned long long q_full, k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages],
+        s_full[2], p_full[2], o_full[2];
     __shared__ unsigned tmem_base_slot;
     __shared__ int tile_span, tile_first;
 
@@ -105,9 +125,11 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         tile_span = found;
         tile_first = first;
         mbar_init(smem_u32(&q_full), 1);
-        for (int s = 0; s < kFaStages; ++s) {
-            mbar_init(smem_u32(&kv_full[s]), 1);
-            mbar_init(smem_u32(&kv_empty[s]), 1);
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(smem_u32(&k_full[s]), 1);
+            mbar_init(smem_u32(&k_empty[s]), 1);
+            mbar_init(smem_u32(&v_full[s]), 1);
+            mbar_init(smem_u32(&v_empty[s]), 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&s_full[b]), 1);
@@ -125,7 +147,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 
     const unsigned smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const unsigned q_addr = smem_base;
-    const unsigned kv_addr = q_addr + kFaQBytes;                       // stage s: K at +s*2*kv, V behind it
+    const unsigned k_addr = q_addr + L::kQBytes, v_addr = k_addr + kStages * L::kKvBytes;
 
     int error = 0;
     if (span >= 0) {
@@ -142,19 +164,19 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 
         if (warp == 0) {
             // ------------------------------------------------------------------ producer
-            // Lane 0 waits for the stage; then lane 2 pg brings page pg of K and lane 2 pg + 1 that of V: one
-            // thread issuing the up to 16 copies of a block one after the other took longer than the softmax
-            // of a block. Every lane looks its page up one block ahead.
+            // Lane 0 waits for the stage; then every lane of the first pages x pieces brings a piece of its page: one
+            // thread issuing the up to 16 copies of a block one after the other took longer than the softmax of a block.
+            // Every lane looks its page up one block ahead. On its own, K goes one block ahead of V.
             const int* table = p.block_table + (size_t)span * p.table_stride;
             if (lane == 0) {
-                mbar_expect_tx(smem_u32(&q_full), kFaQBytes);
-                tma_load_2d(q_addr, &map_q, smem_u32(&q_full), h * kFaD, t0);
+                mbar_expect_tx(smem_u32(&q_full), L::kQBytes);
+#pragma unroll
+                for (int half = 0; half < L::kHalves; ++half)
+                    tma_load_2d(q_addr + half * L::kQHalf, &map_q, smem_u32(&q_full), h * D + half * 64, t0);
             }
             const int pages_per_block = kFaN / p.page_tokens;          // 1 to 8
-            const unsigned page_bytes = (unsigned)p.page_tokens * kFaD * 2;
-            const int pg = lane >> 1;
+            const int pg = lane / 2, part = lane % 2;                  // (part: V instead of K, or the second half of a row)
             const bool copies = pg < pages_per_block;
-            const CUtensorMap* map = (lane & 1) ? &map_v : &map_k;
             auto lookup = [&](int kb) -> int {
                 const int key0 = kb * kFaN + pg * p.page_tokens;
                 // (keys nobody may see: any page of finite numbers will do)
@@ -162,49 +184,73 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                     return table[key0 / p.page_tokens];
                 return 0;
             };
-            int page_next = lookup(block_begin);
-            for (int kb = block_begin; kb < block_end; ++kb) {
-                const int i = kb - block_begin;
-                const int s = i % kFaStages;
-                int page = page_next;
-                page_next = lookup(kb + 1);
-                const unsigned bar = smem_u32(&kv_full[s]);
+            // the lane's piece of block i, `bytes` in all, from column x of its page to `to` in the block's stage
+            auto bring = [&](const CUtensorMap* map, unsigned full, unsigned empty, unsigned bytes, unsigned to, int x, int i,
+                             int page) -> bool {
+                const int s = i % kStages;
+                const unsigned bar = full + 8u * s;
                 int ok = 1;
                 if (lane == 0) {
-                    if (i >= kFaStages && !mbar_wait_suspended(smem_u32(&kv_empty[s]), ((i / kFaStages) - 1) & 1)) ok = 0;
-                    if (ok) mbar_expect_tx(bar, 2 * kFaKvBytes);
+                    if (i >= kStages && !mbar_wait_suspended(empty + 8u * s, ((i / kStages) - 1) & 1)) ok = 0;
+                    if (ok) mbar_expect_tx(bar, bytes);
                 }
                 ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) {
-                    error = lane == 0 ? 61 : 0;
-                    break;
-                }
-                if (copies) {
+                if (ok && copies) {
                     if (page < 0) {                       // the host never builds such a table
                         atomicExch(p.error_flag, 2);
                         page = 0;
                     }
                     const int row = (page * p.kv_heads + kvh) * p.page_tokens;
-                    const unsigned dst = kv_addr + s * 2 * kFaKvBytes + ((lane & 1) ? kFaKvBytes : 0u) + pg * page_bytes;
-                    tma_load_2d(dst, map, bar, 0, row);
+                    tma_load_2d(to + s * L::kKvBytes + pg * (unsigned)p.page_tokens * 128u, map, bar, x, row);
+                }
+                return ok;
+            };
+            const unsigned kf = smem_u32(k_full), ke = smem_u32(k_empty), vf = smem_u32(v_full), ve = smem_u32(v_empty);
+            const int blocks = block_end - block_begin;
+            int page = lookup(block_begin), page_next = lookup(block_begin + 1);
+            bool ok = true;
+            if (L::kTogether) {
+                for (int i = 0; i < blocks && ok; ++i) {
+                    const int mine = page;
+                    page = page_next;
+                    page_next = lookup(block_begin + i + 2);
+                    ok = bring(part ? &map_v : &map_k, kf, ke, 2 * L::kKvBytes, part ? v_addr : k_addr, 0, i, mine);
+                }
+            } else {
+                const unsigned half = part * L::kKvHalf;
+                ok = bring(&map_k, kf, ke, L::kKvBytes, k_addr + half, part * 64, 0, page);
+                for (int i = 0; i < blocks && ok; ++i) {
+                    const int page_v = page;
+                    if (i + 1 < blocks) {
+                        page = page_next;
+                        page_next = lookup(block_begin + i + 2);
+                        ok = bring(&map_k, kf, ke, L::kKvBytes, k_addr + half, part * 64, i + 1, page);
+                    }
+                    ok = ok && bring(&map_v, vf, ve, L::kKvBytes, v_addr + half, part * 64, i, page_v);
                 }
             }
+            if (!ok && lane == 0) error = 61;
         } else if (warp == 1 && lane == 0) {
             // ---------------------------------------------------------------- MMA issuer
             constexpr unsigned idesc_s = instruction_descriptor(kFaM, kFaN);
-            constexpr unsigned idesc_o = instruction_descriptor_b_mn(kFaM, kFaD);
+            constexpr unsigned idesc_o = instruction_descriptor_b_mn(kFaM, 64);      // (64 columns of O at a time)
             const int blocks = block_end - block_begin;
             const unsigned long long desc_q = smem_descriptor(q_addr);
             // S of block i into its buffer, as soon as its keys are there
             auto scores = [&](int i) -> bool {
-                const int s = i % kFaStages;
-                if (!mbar_wait_suspended(smem_u32(&kv_full[s]), (i / kFaStages) & 1)) return false;
+                const int s = i % kStages;
+                if (!mbar_wait_suspended(smem_u32(&k_full[s]), (i / kStages) & 1)) return false;
+                if (L::kOverScores && i >= 2 && !mbar_wait_suspended(smem_u32(&o_full[i & 1]), ((i - 2) >> 1) & 1)) return false;
                 tcgen05_fence_after();
-                const unsigned long long desc_k = smem_descriptor(kv_addr + s * 2 * kFaKvBytes);
+                const unsigned long long desc_k = smem_descriptor(k_addr + s * L::kKvBytes);
 #pragma unroll
-                for (int kk = 0; kk < kFaD / kUmmaK; ++kk)
-                    umma_bf16(tmem_base + (unsigned)((i & 1) * kFaN), desc_q + 2 * kk, desc_k + 2 * kk, idesc_s, kk > 0 ? 1u : 0u);
+                for (int kk = 0; kk < D / kUmmaK; ++kk) {
+                    const unsigned long long half = kk >> 2, part = 2 * (kk & 3);
+                    umma_bf16(tmem_base + (unsigned)((i & 1) * kFaN), desc_q + half * (L::kQHalf >> 4) + part,
+                              desc_k + half * (L::kKvHalf >> 4) + part, idesc_s, kk > 0 ? 1u : 0u);
+                }
                 umma_commit(smem_u32(&s_full[i & 1]));
+                if (!L::kTogether) umma_commit(smem_u32(&k_empty[s]));
                 return true;
             };
             if (!mbar_wait_suspended(smem_u32(&q_full), 0)) error = 62;
@@ -216,20 +262,25 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                     error = 63;
                     break;
                 }
-                if (!mbar_wait_suspended(smem_u32(&p_full[i & 1]), (i >> 1) & 1)) {
+                const int s = i % kStages;
+                if (!mbar_wait_suspended(smem_u32(&p_full[i & 1]), (i >> 1) & 1) ||
+                    (!L::kTogether && !mbar_wait_suspended(smem_u32(&v_full[s]), (i / kStages) & 1))) {
                     error = 64;
                     break;
                 }
                 tcgen05_fence_after();
-                const int s = i % kFaStages;
-                const unsigned long long desc_v = smem_descriptor(kv_addr + s * 2 * kFaKvBytes + kFaKvBytes);
+                const unsigned long long desc_v = smem_descriptor(v_addr + s * L::kKvBytes);
 #pragma unroll
                 for (int kk = 0; kk < kFaN / kUmmaK; ++kk) {
-                    // P: 16 keys = 8 columns of tensor memory; V: 16 keys further = 16 rows of 128 bytes = 2 KiB
-                    umma_bf16_a_tmem(tmem_base + kFaOColumn, tmem_base + kFaPColumn + (unsigned)((i & 1) * (kFaN / 2) + kk * 8),
-                                     desc_v + (unsigned long long)(kk * 128), idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
+#pragma unroll
+                    for (int half = 0; half < L::kHalves; ++half) {
+                        // P: 16 keys = 8 columns of tensor memory; V: 16 keys further = 16 rows of 128 bytes = 2 KiB
+                        umma_bf16_a_tmem(tmem_base + L::kOColumn + half * 64, tmem_base + L::p_column(i) + (unsigned)(kk * 8),
+                                         desc_v + (unsigned long long)(half * (L::kKvHalf >> 4) + kk * 128), idesc_o,
+                                         (i > 0 || kk > 0) ? 1u : 0u);
+                    }
                 }
-                umma_commit(smem_u32(&kv_empty[s]));
+                umma_commit(smem_u32(L::kTogether ? &k_empty[s] : &v_empty[s]));
                 umma_commit(smem_u32(&o_full[i & 1]));
             }
         } else if (warp >= 2) {
@@ -247,7 +298,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             float used_max = -INFINITY, run_sum = 0.0f;
             bool ok = true;
             const int blocks = block_end - block_begin;
-            const unsigned o_taddr = lane_base + kFaOColumn;
+            const unsigned o_taddr = lane_base + L::kOColumn;
             const unsigned long long scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
             for (int i = 0; i < blocks; ++i) {
                 // (S of block i complete also means: P V of block i-2 is complete, its P buffer is free)
@@ -358,9 +409,9 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                         const float factor = !grown ? 1.0f : (used_max == -INFINITY ? 0.0f : exp2f(used_max - new_max));
                         const unsigned long long factor2 = pack_f32x2(factor, factor);
 #pragma unroll
-                        for (int half = 0; half < 2; ++half) {
+                        for (int c0 = 0; c0 < D; c0 += 32) {
                             unsigned part[32];
-                            tmem_load_32_issue(o_taddr + (unsigned)(half * 32), part);
+                            tmem_load_32_issue(o_taddr + (unsigned)c0, part);
                             tmem_load_wait();
 #pragma unroll
                             for (int j = 0; j < 32; j += 2) {
@@ -369,7 +420,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                                 part[j] = __float_as_uint(a);
                                 part[j + 1] = __float_as_uint(b);
                             }
-                            tmem_store_32(o_taddr + (unsigned)(half * 32), part);
+                            tmem_store_32(o_taddr + (unsigned)c0, part);
                         }
                         tmem_store_wait();
                         run_sum *= factor;
@@ -390,7 +441,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                     const __nv_bfloat162 pair = __floats2bfloat162_rn(a, b);          // key 2 j2 in the lower half
                     p_packed[j2] = *reinterpret_cast<const unsigned*>(&pair);
                 }
-                tmem_store_32(lane_base + kFaPColumn + (unsigned)((i & 1) * (kFaN / 2)), p_packed);
+                tmem_store_32(lane_base + L::p_column(i), p_packed);
                 tmem_store_wait();
                 {
                     float s0, s1;
@@ -401,43 +452,40 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                 mbar_arrive_one(smem_u32(&p_full[i & 1]));
             }
             // the output: O of the last block complete, divided by the denominator
-            float o[kFaD];
             if (ok && blocks > 0) {
                 ok = mbar_wait(smem_u32(&o_full[(blocks - 1) & 1]), ((blocks - 1) >> 1) & 1);
                 ok = __all_sync(0xffffffffu, ok);
-                if (ok) {
-                    tcgen05_fence_after();
-                    unsigned lo[32], hi[32];
-                    tmem_load_32_issue(o_taddr, lo);
-                    tmem_load_32_issue(o_taddr + 32u, hi);
-                    tmem_load_wait();
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        o[j] = __uint_as_float(lo[j]);
-                        o[32 + j] = __uint_as_float(hi[j]);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < kFaD; ++j) o[j] = 0.0f;
+                if (ok) tcgen05_fence_after();
             }
             if (!ok) {
                 if (lane == 0) atomicExch(p.error_flag, 65);
-            } else if (live) {
+            } else {
                 // a sink joins the denominator relative to the maximum the sum is relative to (a row without a
                 // key in reach has none and no output either)
                 const float sink_part = (p.sinks && run_sum > 0.0f)
                                             ? exp2f(p.sinks[h] * 1.4426950408889634f - used_max) : 0.0f;
                 const float inv = run_sum > 0.0f ? 1.0f / (run_sum + sink_part) : 0.0f;
-                __nv_bfloat16* dst = p.out + ((size_t)(t0 + row) * p.q_heads + h) * kFaD;
+                __nv_bfloat16* dst = p.out + ((size_t)(t0 + row) * p.q_heads + h) * D;
 #pragma unroll
-                for (int c0 = 0; c0 < kFaD; c0 += 8) {
-                    uint4 packed;
-                    __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&packed);
+                for (int c0 = 0; c0 < D; c0 += 32) {
+                    unsigned o[32];
+                    if (blocks > 0) {
+                        tmem_load_32_issue(o_taddr + (unsigned)c0, o);
+                        tmem_load_wait();
+                    } else {
 #pragma unroll
-                    for (int e2 = 0; e2 < 4; ++e2)
-                        h2[e2] = __floats2bfloat162_rn(o[c0 + 2 * e2] * inv, o[c0 + 2 * e2 + 1] * inv);
-                    *reinterpret_cast<uint4*>(dst + c0) = packed;
+                        for (int j = 0; j < 32; ++j) o[j] = 0u;
+                    }
+                    if (!live) continue;
+#pragma unroll
+                    for (int c = 0; c < 32; c += 8) {
+                        uint4 packed;
+                        __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+                        for (int e2 = 0; e2 < 4; ++e2)
+                            h2[e2] = __floats2bfloat162_rn(__uint_as_float(o[c + 2 * e2]) * inv, __uint_as_float(o[c + 2 * e2 + 1]) * inv);
+                        *reinterpret_cast<uint4*>(dst + c0 + c) = packed;
+                    }
                 }
             }
         }
@@ -454,12 +502,12 @@ using namespace celeg_b200;
 
 // Whether the shapes fit this kernel (the caller then uses celeg_attention_prefill or the general kernel).
 CELEG_API int celeg_attention_prefill_tcgen05_supported(int q_heads, int kv_heads, int head_dim, int page_tokens) {
-    return head_dim == kFaD && kv_heads > 0 && q_heads % kv_heads == 0 && page_tokens >= 8 && page_tokens % 8 == 0 &&
+    return (head_dim == 64 || head_dim == 128) && kv_heads > 0 && q_heads % kv_heads == 0 && page_tokens >= 8 && page_tokens % 8 == 0 &&
            kFaN % page_tokens == 0;
 }
 
-// q: [q_rows, q_row_stride] bfloat16 with head h at column h * 64 (q_rows: rows of the buffer that may be
-// read, at least `tokens`); caches [pages, kv_heads, page_tokens, 64]. tile_count = sum over spans of
+// q: [q_rows, q_row_stride] bfloat16 with head h at column h * head_dim (q_rows: rows of the buffer that may be
+// read, at least `tokens`); caches [pages, kv_heads, page_tokens, head_dim]. tile_count = sum over spans of
 // ceil(length / 128), computed by the caller, who knows the lengths.
 CELEG_API int celeg_attention_prefill_tcgen05(const void* q, int q_row_stride, int q_rows, void* out, const void* k_cache,
                                               const void* v_cache, int pages, const int* positions,
@@ -482,8 +530,8 @@ CELEG_API int celeg_attention_prefill_tcgen05(const void* q, int q_row_stride, i
     CUtensorMap map_q, map_k, map_v;
     if (!tensor_map_for(q, q_rows, q_row_stride, q_row_stride, kFaM, &map_q)) return -2;
     const long long cache_rows = (long long)pages * kv_heads * page_tokens;
-    if (!tensor_map_for(k_cache, cache_rows, kFaD, kFaD, page_tokens, &map_k)) return -2;
-    if (!tensor_map_for(v_cache, cache_rows, kFaD, kFaD, page_tokens, &map_v)) return -2;
+    if (!tensor_map_for(k_cache, cache_rows, head_dim, head_dim, page_tokens, &map_k)) return -2;
+    if (!tensor_map_for(v_cache, cache_rows, head_dim, head_dim, page_tokens, &map_v)) return -2;
     FaParams p;
     p.out = (__nv_bfloat16*)out;
     p.positions = positions;
@@ -503,12 +551,13 @@ CELEG_API int celeg_attention_prefill_tcgen05(const void* q, int q_row_stride, i
     p.cap_in = softcap > 0.0f ? scale / softcap : 0.0f;
     p.cap_out = softcap > 0.0f ? softcap / scale : 0.0f;
     p.error_flag = error_flag;
-    const cudaError_t status = cudaFuncSetAttribute(attention_prefill_tcgen05_kernel,
-                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFaSmemBytes);
+    auto kernel = head_dim == 64 ? attention_prefill_tcgen05_kernel<64> : attention_prefill_tcgen05_kernel<128>;
+    const unsigned smem = head_dim == 64 ? FaLayout<64>::kSmemBytes : FaLayout<128>::kSmemBytes;
+    const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (status != cudaSuccess) {
         set_error("attention_prefill_tcgen05: %s", cudaGetErrorString(status));
         return -2;
     }
-    attention_prefill_tcgen05_kernel<<<dim3(q_heads, tile_count), kFaThreads, kFaSmemBytes, stream>>>(map_q, map_k, map_v, p);
+    kernel<<<dim3(q_heads, tile_count), kFaThreads, smem, stream>>>(map_q, map_k, map_v, p);
     return check_launch("attention_prefill_tcgen05");
 }

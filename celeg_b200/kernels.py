@@ -612,8 +612,8 @@ def attention_prefill(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_c
 
 def attention_prefill_tcgen05_supported(q_heads: int, kv_heads: int, head_dim: int, page_tokens: int,
                                         dtype: torch.dtype) -> bool:
-    """Shapes the tcgen05 kernel for prompt portions takes: head size 64, pages of 8, 16, 32 or 64 tokens."""
-    return (dtype == torch.bfloat16 and head_dim == 64 and kv_heads > 0 and q_heads % kv_heads == 0
+    """Shapes the tcgen05 kernel for prompt portions takes: head sizes 64 and 128, pages of 8, 16, 32 or 64 tokens."""
+    return (dtype == torch.bfloat16 and head_dim in (64, 128) and kv_heads > 0 and q_heads % kv_heads == 0
             and page_tokens >= 8 and page_tokens % 8 == 0 and 64 % page_tokens == 0)
 
 

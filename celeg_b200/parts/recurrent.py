@@ -71,7 +71,7 @@ class MlstmMixer:
 
     # Steps whose longest portion has at least this many tokens are scanned in chunks. Measured for one portion at 16 heads of
     # 64 x 128, the mixer between its projections included: 128 tokens 53 us in chunks, 51 token by token; 192: 57 and 70;
-    # 2,048: 163 and 564.
+    # 2,048: 171 and 564.
     CHUNKED_FROM = 144
 
     def cache_need(self):
