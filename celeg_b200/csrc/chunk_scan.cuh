@@ -37,11 +37,11 @@ enum ChunkMode : int {
 struct ChunkArgs {
     const float* q; int q_stride; const float* k; int k_stride;        // head (or group) h at h * dim
     const float* v; int v_stride;
-    const float2* cum; const float* dt;      // scalar: [tokens, heads]: sums of the decays' logarithms, steps
+    const float2* cum; const float* dt;      // scalar: [tokens, heads]: sums of the decays' logarithms, steps (null: ones)
     const float* total;                      // channel: [chunks, heads * dim], the chunk's product of decays
     const float* products;                   // channel: [chunks, heads, 64, 64], zero above the diagonal
     const float* direct;                     // scalar: [heads], the values' share of the read-out, or null
-    const float* decay; float q_scale;       // constant: [heads], and the keys' factor; stable: the queries' factor
+    const float* decay; float q_scale;       // constant: [heads], and the keys' factor; stable, scalar: the queries' factor
     const float2* gates;                     // stable: [tokens, 3, heads]: forget sum F, i - F, the largest i - F so far
     double* peaks;                           // stable: [chunks, heads], the running maximum before the chunk
     float* norms;                            // stable: [chunks, heads, dim], the normaliser before the chunk
@@ -101,13 +101,13 @@ __device__ __forceinline__ void mma_split(float (*acc)[4], const unsigned (&a)[3
 
 // ----------------------------------------------------------------------------------------------- tiles in shared memory
 // Three planes (hi, mid, lo) of ROWS x COLUMNS bfloat16 numbers; the 16-byte pieces of a row are permuted so that eight rows'
-// pieces of one column lie in eight different bank groups (COLUMNS 32: two rows fill the 128 bytes of all banks).
+// pieces of one column lie in eight different bank groups (COLUMNS 32: two rows fill the 128 bytes of all banks; 16: four).
 template <int ROWS, int COLUMNS>
 struct SplitTile {
     static constexpr int kPlane = ROWS * COLUMNS;
     static constexpr int kElements = 3 * kPlane;
     static __device__ __forceinline__ int at(int row, int piece) {
-        return row * COLUMNS + ((COLUMNS == 32 ? piece ^ ((row >> 1) & 3) : piece ^ (row & 7)) << 3);
+        return row * COLUMNS + ((piece ^ (COLUMNS == 16 ? (row >> 2) & 1 : COLUMNS == 32 ? (row >> 1) & 3 : row & 7)) << 3);
     }
 };
 
@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
         const size_t t = begin + min(tid, count - 1), head = head0 + h;
         if (MODE == kChunkScalar) {
             next_cum = p.cum[t * p.heads + head];
-            next_step = p.dt[t * p.heads + head];
+            next_step = p.q_scale * (p.dt ? p.dt[t * p.heads + head] : 1.0f);
         } else if (MODE == kChunkStable) {
             before = p.peaks[(size_t)chunk * p.heads + head];
             next_forget = p.gates[(t * 3) * p.heads + head];
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
         if constexpr (MODE == kChunkScalar) {
             if (tid < kChunk) {
                 gates.cum[tid] = next_cum;
-                gates.from_start[tid] = expf(next_cum.x);
+                gates.from_start[tid] = p.q_scale * expf(next_cum.x);
                 gates.step[tid] = tid < count ? next_step : 0.0f;
             }
             ask_gates(h + 1);
@@ -978,15 +978,8 @@ inline int launch_read(const ChunkArgs& p, int chunks, int heads_a_block, cudaSt
     return check_launch("chunk_read");
 }
 
-// `chunks` bounds the chunks of all spans; p.chunk_begin has chunks / p.pieces + 1 entries
 template <int MODE>
-inline int launch_chunk_scan(const ChunkArgs& p, int chunks, cudaStream_t stream) {
-    // The walk moves a third of the bytes but needs a block and a half an SM to keep them busy: at 64 heads of 128 x 64 (256
-    // blocks) a span of 2,048 tokens takes 88 us, sums and carry 107 (62 + 45); at 16 heads of 64 x 128 (64 blocks) 46 us and
-    // 26 (17 + 9; the mLSTM's carry, with its maxima, 21).
-    const long long blocks = (long long)((p.vdim + kWalkColumns - 1) / kWalkColumns) * ((p.dim + 63) / 64) * p.heads * p.spans;
-    const int status = blocks >= 222 ? launch_walk<MODE>(p, stream) : launch_sums<MODE>(p, chunks, stream);
-    if (status != 0) return status;
+inline int launch_reads(const ChunkArgs& p, int chunks, cudaStream_t stream) {
     // heads that share queries and keys share a block's products of them, as long as the blocks fill the GPU
     int heads_a_block = 1;
     if (MODE == kChunkScalar)
@@ -995,6 +988,17 @@ inline int launch_chunk_scan(const ChunkArgs& p, int chunks, cudaStream_t stream
             heads_a_block *= 2;
     return p.dim <= 64 ? launch_read<MODE, 64>(p, chunks, heads_a_block, stream)
                        : launch_read<MODE, 128>(p, chunks, heads_a_block, stream);
+}
+
+// `chunks` bounds the chunks of all spans; p.chunk_begin has chunks / p.pieces + 1 entries
+template <int MODE>
+inline int launch_chunk_scan(const ChunkArgs& p, int chunks, cudaStream_t stream) {
+    // The walk moves a third of the bytes but needs a block and a half an SM to keep them busy: at 64 heads of 128 x 64 (256
+    // blocks) a span of 2,048 tokens takes 88 us, sums and carry 107 (62 + 45); at 16 heads of 64 x 128 (64 blocks) 46 us and
+    // 26 (17 + 9; the mLSTM's carry, with its maxima, 21).
+    const long long blocks = (long long)((p.vdim + kWalkColumns - 1) / kWalkColumns) * ((p.dim + 63) / 64) * p.heads * p.spans;
+    const int status = blocks >= 222 ? launch_walk<MODE>(p, stream) : launch_sums<MODE>(p, chunks, stream);
+    return status != 0 ? status : launch_reads<MODE>(p, chunks, stream);
 }
 
 }  // namespace celeg_b200

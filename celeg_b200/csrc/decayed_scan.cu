@@ -394,6 +394,16 @@ CELEG_API int celeg_chunk_plan(const int* span_begin, int spans, int max_chunks,
     return check_launch("chunk_plan");
 }
 
+// The running sums alone (of decays exp(-exp(a_log) softplus(raw + bias))), for another recurrence over the same chunks.
+CELEG_API int celeg_decay_sums(const float* raw, int raw_stride, const float* bias, const float* a_log, float2* cum, float* dt,
+                               const int* plan, int chunks, int heads, cudaStream_t stream) {
+    CELEG_REQUIRE(chunks >= 0 && chunks <= 65535 && heads > 0, "decay_sums: invalid sizes chunks=%d heads=%d", chunks, heads);
+    if (chunks == 0) return 0;
+    launch_chained(scalar_decay_kernel, dim3((heads + 7) / 8, chunks), 256, 0, stream, raw, raw_stride, bias, a_log, plan, cum, dt,
+                   heads);
+    return check_launch("decay_sums");
+}
+
 // The channel form over the step's spans. q, k: float32 rows, head h at h * dim; z: the decay before its bias; scratch:
 // q_out, k_out [tokens, heads * dim], total [chunks, heads * dim], products [chunks, heads, 64, 64], states [chunks, heads,
 // dim, vdim]. plan: of celeg_chunk_plan with the same max_chunks (>= what the spans make).
@@ -445,7 +455,7 @@ CELEG_API int celeg_scalar_decay_scan(const float* q, int q_stride, const float*
     if (status != 0) return status;
     ChunkArgs p = {};
     p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = v; p.v_stride = v_stride;
-    p.cum = cum; p.dt = dt; p.direct = direct;
+    p.cum = cum; p.dt = dt; p.direct = direct; p.q_scale = 1.0f;
     p.chunk_begin = plan; p.pieces = 1; p.span_first = span_first; p.spans = spans;
     p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = states; p.out = out;
     p.heads = heads; p.groups = groups; p.dim = dim; p.vdim = vdim;

@@ -1,0 +1,518 @@
+// The gated delta rule over prompts in chunks of 64 tokens (recurrent_scan.cu has it token by token, and says what it is):
+//
+//   S~ = g S;  u = beta (v - S~^T k);  S' = S~ + k u^T;  o = q_scale S'^T q
+//
+// With G(i, j) = g_(j+1) .. g_i over the chunk's tokens (G(i) from its first) and S_0 the state before it, the u of the chunk
+// are the solution of a unit lower triangular system (the compact form of a product of such updates: Bischof and Van Loan,
+// "The WY Representation for Products of Householder Matrices", 1987; Yang et al., "Parallelizing Linear Transformers with the
+// Delta Rule over Sequence Length", 2024):
+//
+//   u_i + sum_(j<i) beta_i G(i, j) (k_i . k_j) u_j = beta_i v_i - beta_i G(i) S_0^T k_i
+//
+// so u = U_0 - W S_0 with U_0, W the solutions for the right sides beta v and beta G k, and then
+//
+//   o_i = q_scale [ G(i) S_0^T q_i + sum_(j<=i) G(i, j) (q_i . k_j) u_j ]         S_n = G(n) S_0 + sum_j G(n, j) k_j u_j^T
+//
+//   decays    the running sums of the decays' logarithms (decayed_scan.cu)
+//   solve     a block a (chunk, head): k.k, the system's inverse, its products with the right sides; leaves U_0 in float32,
+//             and -W and G(n, j) k_j split for the tensor cores, as they will lie in shared memory
+//   walk      a block a (span, head, run of columns) goes through the chunks: u = U_0 - W S, then S, two products a chunk, the
+//             next chunk's operands under way as one bulk copy each; leaves u and the states before the chunks
+//   read-outs those of the other chunked scans (chunk_scan.cuh) with u in the place of v
+//
+// Products and their precision: chunk_scan.cuh.
+#include "chunk_scan.cuh"
+#include "tcgen05.cuh"
+
+namespace celeg_b200 {
+
+struct DeltaChunkArgs {
+    const float* k; int k_stride;            // [tokens, kv_heads * dim], unit vectors
+    const float* v; int v_stride;            // [tokens, heads * vdim]
+    const float* gates;                      // [tokens, 2 * heads]: beta in the first half
+    const float2* cum;                       // [tokens, heads]
+    const int* chunk_begin; const int* span_first;
+    __nv_bfloat16* operands;                 // [chunks, heads, 2]: -W, G(n, .) k, a SplitTile<64, WIDTH> each
+    float* u;                                // [tokens, heads * vdim]: U_0, then u
+    float* states;                           // [chunks, heads, dim, vdim]
+    float* state; long long slot_stride; const int* span_slot;
+    int heads, kv_heads, dim, vdim;
+    int* error_flag;
+};
+
+// ------------------------------------------------------------------------------------------------------------- solve
+// The system's matrix is inverted, T = (1 + L)^-1: its four diagonal blocks of 16 by substitution, a warp a block and a lane a
+// column; then two blocks of 16 and at last two of 32 are joined, T_21 = -T_22 L_21 T_11; and W and U_0 are products of T, its
+// columns scaled, with k and v as they lie. (Substitution over whole right sides, a thread two columns, was one chain of 64
+// steps a block: 138 us for 32 heads of 64 and 2,048 tokens, 69 us like this.)
+constexpr int kSolveThreads = 128;
+constexpr int kSolvePitch = kChunk + 4;
+template <int WIDTH> constexpr int solve_bytes() {
+    return (SplitTile<kChunk, WIDTH>::kElements + SplitTile<kChunk, 64>::kElements) * 2 + kChunk * kSolvePitch * 4;
+}
+static_assert(SplitTile<kChunk, 64>::kElements * 2 >= kChunk * kSolvePitch * 4, "L lies where T's planes will");
+
+// out = sign a b of N x N blocks of matrices with kSolvePitch floats a row, 128 / (N * N / 4) of them side by side; a thread four
+// neighbours of a row. `a`, `b`, `out`: of the thread's block.
+template <int N>
+__device__ __forceinline__ void join_product(const float* a, const float* b, float* out, float sign, int slot) {
+    const int r = slot / (N / 4), c = (slot % (N / 4)) * 4;
+    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
+    for (int k = 0; k < N; ++k) {
+        const float x = a[r * kSolvePitch + k];
+        const float4 y = *reinterpret_cast<const float4*>(b + k * kSolvePitch + c);
+        sum.x = fmaf(x, y.x, sum.x); sum.y = fmaf(x, y.y, sum.y); sum.z = fmaf(x, y.z, sum.z); sum.w = fmaf(x, y.w, sum.w);
+    }
+    *reinterpret_cast<float4*>(out + r * kSolvePitch + c) = make_float4(sign * sum.x, sign * sum.y, sign * sum.z, sign * sum.w);
+}
+
+template <int WIDTH>
+__global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 3 : 2) delta_solve_kernel(const DeltaChunkArgs p) {
+    using Tile = SplitTile<kChunk, WIDTH>;
+    using TTile = SplitTile<kChunk, 64>;
+    using VTile = SplitTile<kChunk, 64>;
+    extern __shared__ __align__(128) __nv_bfloat16 tiles[];
+    __shared__ float2 cum_s[kChunk];
+    __shared__ float beta_s[kChunk], start_s[kChunk], end_s[kChunk];
+    chain_release();
+    chain_wait();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
+    const int chunk = blockIdx.y, head = blockIdx.x, dim = p.dim, vdim = p.vdim;
+    const int begin = p.chunk_begin[chunk], count = p.chunk_begin[chunk + 1] - begin;
+    if (count <= 0) return;
+    __nv_bfloat16* k_t = tiles;                              // k, then v
+    __nv_bfloat16* t_t = tiles + Tile::kElements;            // T's planes, at first L
+    float* lower = reinterpret_cast<float*>(t_t);
+    float* inverse = reinterpret_cast<float*>(t_t + TTile::kElements);
+    const float* k_src = p.k + (size_t)begin * p.k_stride + (size_t)(head / (p.heads / p.kv_heads)) * dim;
+    const float* v_src = p.v + (size_t)begin * p.v_stride + (size_t)head * vdim;
+    const bool k_four = by_fours(p.k, p.k_stride, dim), v_four = by_fours(p.v, p.v_stride, vdim);
+    if (tid < kChunk) {
+        const size_t t = begin + min(tid, count - 1);
+        const float2 own = p.cum[t * p.heads + head];
+        cum_s[tid] = own;
+        beta_s[tid] = tid < count ? p.gates[t * 2 * p.heads + head] : 0.0f;
+        start_s[tid] = expf(own.x);
+        end_s[tid] = exp_between(p.cum[(size_t)(begin + count - 1) * p.heads + head], own);
+    }
+    for (int i = tid; i < kChunk * kSolvePitch; i += kSolveThreads) inverse[i] = 0.0f;
+    __syncthreads();
+    const size_t at = ((size_t)chunk * p.heads + head) * 2;
+    __nv_bfloat16* w_out = p.operands + at * Tile::kElements;
+    __nv_bfloat16* k_out = w_out + Tile::kElements;
+    using Part = TileShare<kChunk, 32, kSolveThreads>;
+    Part share;
+#pragma unroll 1
+    for (int e = 0; e < WIDTH; e += 32) {
+        share.load(k_src + e, p.k_stride, count, dim - e, k_four);
+        share.template store<Tile>(k_t, e >> 3, Unscaled());
+        share.template store<Tile>(k_out, e >> 3, [&](int r) { return end_s[r]; });      // G(n, j) k_j: what S is given of u_j
+    }
+    __syncthreads();
+    {
+        float raw[8][4] = {};                                // k.k: the warp's 16 tokens against 8 n + 2 tig, + 1
+#pragma unroll 2
+        for (int e = 0; e < WIDTH; e += 16) {
+            unsigned a[3][4];
+            load_a<Tile>(a, k_t, 16 * warp, e);
+#pragma unroll
+            for (int n = 0; n < 4; n += 2) {
+                if (n > warp) break;
+                unsigned b[4][3][2];
+                load_b<Tile>(b, k_t, 16 * n, e);
+                load_b<Tile>(b + 2, k_t, 16 * n + 16, e);
+                mma_split<4>(raw + 2 * n, a, b);
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int i = 16 * warp + g + 8 * (r >> 1), j = 8 * n + 2 * tig + (r & 1);
+                lower[i * kSolvePitch + j] = j < i && i < count ? raw[n][r] * beta_s[i] * exp_between(cum_s[i], cum_s[j]) : 0.0f;
+            }
+    }
+    __syncwarp();
+    if (lane < 16) {                                         // the warp's own diagonal block
+        const float* l = lower + 16 * warp * kSolvePitch + 16 * warp;
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float sum[4] = {i == lane ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int j = 0; j < i; ++j) sum[j & 3] = fmaf(-l[i * kSolvePitch + j], x[j], sum[j & 3]);
+            x[i] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            inverse[(16 * warp + i) * kSolvePitch + 16 * warp + lane] = x[i];
+        }
+    }
+    __syncthreads();
+    {
+        // two pairs of blocks of 16, 64 threads each; L_10 T_00 goes where the block above the diagonal is (zero at the end)
+        const int o = (tid >> 6) * 32 * (kSolvePitch + 1), slot = tid & 63;
+        float* spare = inverse + o + 16;
+        join_product<16>(lower + o + 16 * kSolvePitch, inverse + o, spare, 1.0f, slot);
+        __syncthreads();
+        join_product<16>(inverse + o + 16 * (kSolvePitch + 1), spare, inverse + o + 16 * kSolvePitch, -1.0f, slot);
+        __syncthreads();
+        const int r = slot >> 2, c = (slot & 3) * 4;
+        *reinterpret_cast<float4*>(spare + r * kSolvePitch + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        __syncthreads();
+        float* corner = inverse + 32;                        // the same with the two blocks of 32
+        join_product<32>(lower + 32 * kSolvePitch, inverse, corner, 1.0f, tid);
+        join_product<32>(lower + 32 * kSolvePitch, inverse, corner, 1.0f, tid + 128);
+        __syncthreads();
+        const float* below = inverse + 32 * (kSolvePitch + 1);
+        join_product<32>(below, corner, inverse + 32 * kSolvePitch, -1.0f, tid);
+        join_product<32>(below, corner, inverse + 32 * kSolvePitch, -1.0f, tid + 128);
+        __syncthreads();                                     // (what is above the diagonal is left out below)
+    }
+    // T with its columns scaled, split: every thread two neighbouring entries a time
+    auto split_inverse = [&](bool with_decay) {
+        for (int i = tid; i < kChunk * kChunk / 2; i += kSolveThreads) {
+            const int r = i >> 5, c = (i & 31) * 2;
+            const float fx = beta_s[c] * (with_decay ? start_s[c] : 1.0f), fy = beta_s[c + 1] * (with_decay ? start_s[c + 1] : 1.0f);
+            const float2 x = *reinterpret_cast<const float2*>(inverse + r * kSolvePitch + c);
+            unsigned plane[3];
+            split_pair(c <= r ? x.x * fx : 0.0f, c + 1 <= r ? x.y * fy : 0.0f, plane[0], plane[1], plane[2]);
+#pragma unroll
+            for (int n = 0; n < 3; ++n)
+                *reinterpret_cast<unsigned*>(t_t + n * TTile::kPlane + TTile::at(r, c >> 3) + (c & 7)) = plane[n];
+        }
+    };
+    float acc[8][4];
+    auto multiply = [&](auto tile, const __nv_bfloat16* from, int n0) {        // T times 64 columns from n0 on
+        using B = decltype(tile);
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acc[n][r] = 0.0f;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            if (t > warp) break;
+            unsigned a[3][4];
+            load_a<TTile>(a, t_t, 16 * warp, 16 * t);
+#pragma unroll
+            for (int n = 0; n < 4; n += 2) {
+                unsigned b[4][3][2];
+                load_b_transposed<B>(b, from, n0 + 16 * n, 16 * t);
+                load_b_transposed<B>(b + 2, from, n0 + 16 * n + 16, 16 * t);
+                mma_split<4>(acc + 2 * n, a, b);
+            }
+        }
+    };
+    split_inverse(true);
+    __syncthreads();
+#pragma unroll 1
+    for (int e = 0; e < WIDTH; e += 64) {                    // -W = -T beta G k
+        multiply(Tile(), k_t, e);
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                unsigned plane[3];
+                split_pair(-acc[n][2 * h], -acc[n][2 * h + 1], plane[0], plane[1], plane[2]);
+                __nv_bfloat16* to = w_out + Tile::at(16 * warp + g + 8 * h, (e >> 3) + n) + 2 * tig;
+#pragma unroll
+                for (int x = 0; x < 3; ++x) *reinterpret_cast<unsigned*>(to + x * Tile::kPlane) = plane[x];
+            }
+    }
+    __syncthreads();
+    split_inverse(false);
+    for (int c0 = 0; c0 < vdim; c0 += 64) {                  // U_0 = T beta v
+        if (c0 > 0) __syncthreads();
+#pragma unroll 1
+        for (int c = 0; c < 64; c += 32) {
+            share.load(v_src + c0 + c, p.v_stride, count, vdim - c0 - c, v_four);
+            share.template store<VTile>(k_t, c >> 3, Unscaled());
+        }
+        __syncthreads();
+        multiply(VTile(), k_t, 0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int t = 16 * warp + g + 8 * h;
+            if (t >= count) continue;
+            float* dst = p.u + (size_t)(begin + t) * p.heads * vdim + (size_t)head * vdim + c0;
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+                const int c = 8 * n + 2 * tig;
+                if ((vdim & 1) == 0) {
+                    if (c0 + c < vdim) *reinterpret_cast<float2*>(dst + c) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+                } else {
+                    if (c0 + c < vdim) dst[c] = acc[n][2 * h];
+                    if (c0 + c + 1 < vdim) dst[c + 1] = acc[n][2 * h + 1];
+                }
+            }
+        }
+    }
+}
+
+// -------------------------------------------------------------------------------------------------------------- walk
+constexpr int kDeltaWalkThreads = 256;
+template <int WIDTH> constexpr int kDeltaStages = WIDTH == 64 ? 2 : 1;
+template <int WIDTH, int COLUMNS> constexpr int delta_walk_bytes() {
+    return (kDeltaStages<WIDTH> * 2 * SplitTile<kChunk, WIDTH>::kElements + SplitTile<WIDTH, COLUMNS>::kElements +
+            SplitTile<kChunk, COLUMNS>::kElements) * (int)sizeof(__nv_bfloat16);
+}
+
+// COLUMNS of S a block: 16, or 32 where that is blocks enough
+template <int WIDTH, int COLUMNS>
+__global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const DeltaChunkArgs p) {
+    using Tile = SplitTile<kChunk, WIDTH>;
+    using STile = SplitTile<WIDTH, COLUMNS>;
+    using UTile = SplitTile<kChunk, COLUMNS>;
+    constexpr int kStages = kDeltaStages<WIDTH>;
+    constexpr int kAlong = WIDTH / 16, kTiles = COLUMNS / 8 * kAlong / 8;      // of S: warps along the keys, tiles of columns
+    constexpr int kUTiles = COLUMNS / 16;                    // of u: tiles of columns a warp
+    extern __shared__ __align__(128) __nv_bfloat16 tiles[];
+    __shared__ __align__(8) unsigned long long full[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
+    const int span = blockIdx.z, head = blockIdx.y, c0 = blockIdx.x * COLUMNS, dim = p.dim, vdim = p.vdim;
+    const int first = p.span_first[span], last = p.span_first[span + 1];
+    if (first >= last) return;
+    const int t_begin = p.chunk_begin[first], t_end = p.chunk_begin[last], chunks = last - first;
+    __nv_bfloat16* s_t = tiles + kStages * 2 * Tile::kElements;
+    __nv_bfloat16* u_t = s_t + STile::kElements;
+    float* s_head = p.state + (long long)p.span_slot[span] * p.slot_stride + (size_t)head * dim * vdim;
+    constexpr unsigned kBytes = 2 * Tile::kElements * (unsigned)sizeof(__nv_bfloat16);
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) mbar_init(smem_u32(&full[s]), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    auto bring = [&](int i) {                                // thread 0: a chunk's two operands, one behind the other
+        if (i >= chunks) return;
+        const unsigned bar = smem_u32(&full[i % kStages]);
+        mbar_expect_tx(bar, kBytes);
+        bulk_load(smem_u32(tiles + (i % kStages) * 2 * Tile::kElements),
+                  p.operands + ((size_t)(first + i) * p.heads + head) * 2 * Tile::kElements, kBytes, bar);
+    };
+    if (tid == 0)
+        for (int s = 0; s < kStages; ++s) bring(s);
+    // the warp's parts. S: rows er + g, er + g + 8, columns sc + 8 n + 2 tig, + 1. u: tokens tr + g, + 8, columns uc + ..
+    const int er = 16 * (warp % kAlong), sc = 8 * kTiles * (warp / kAlong);
+    const int tr = 16 * (warp & 3), uc = 8 * kUTiles * (warp >> 2);
+    const bool two = (vdim & 1) == 0;
+    float s[kTiles][4];
+    auto put = [&](__nv_bfloat16* tile, int at, int plane, float x, float y) {
+        unsigned h, m, l;
+        split_pair(x, y, h, m, l);
+        *reinterpret_cast<unsigned*>(tile + at) = h;
+        *reinterpret_cast<unsigned*>(tile + at + plane) = m;
+        *reinterpret_cast<unsigned*>(tile + at + 2 * plane) = l;
+    };
+    auto put_s = [&] {
+#pragma unroll
+        for (int n = 0; n < kTiles; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                put(s_t, STile::at(er + g + 8 * h, (sc >> 3) + n) + 2 * tig, STile::kPlane, s[n][2 * h], s[n][2 * h + 1]);
+    };
+#pragma unroll
+    for (int n = 0; n < kTiles; ++n)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int e = er + g + 8 * (r >> 1), c = c0 + sc + 8 * n + 2 * tig + (r & 1);
+            s[n][r] = e < dim && c < vdim ? s_head[(size_t)e * vdim + c] : 0.0f;
+        }
+    put_s();
+    float next[kUTiles][4], next_keep = 0.0f;                      // U_0 of the chunk to come, its decay
+    auto ask = [&](int i) {
+        if (i >= chunks) return;
+        const int begin = t_begin + i * kChunk, count = min(kChunk, t_end - begin);
+#pragma unroll
+        for (int n = 0; n < kUTiles; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int t = tr + g + 8 * h, c = c0 + uc + 8 * n + 2 * tig;
+                const float* src = p.u + (size_t)(begin + t) * p.heads * vdim + (size_t)head * vdim + c;
+                float2 x = make_float2(0.0f, 0.0f);
+                if (t < count && two && c < vdim) x = *reinterpret_cast<const float2*>(src);
+                else if (t < count && c < vdim) x = make_float2(src[0], c + 1 < vdim ? src[1] : 0.0f);
+                next[n][2 * h] = x.x;
+                next[n][2 * h + 1] = x.y;
+            }
+        next_keep = p.cum[(size_t)(begin + count - 1) * p.heads + head].x;
+    };
+    auto store = [&](float* dst, int r, int c, float x, float y) {     // dst: the row's columns from c0 on
+        if (c0 + c >= vdim) return;
+        if (two) *reinterpret_cast<float2*>(dst + c) = make_float2(x, y);
+        else {
+            dst[c] = x;
+            if (c0 + c + 1 < vdim) dst[c + 1] = y;
+        }
+    };
+    ask(0);
+    __syncthreads();
+    auto odd_first = [](unsigned (*b)[3][2]) {               // the second tile of eight columns in the first's place
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+            b[0][n][0] = b[1][n][0];
+            b[0][n][1] = b[1][n][1];
+        }
+    };
+    bool ok = true;
+    for (int i = 0; i < chunks; ++i) {
+        const int begin = t_begin + i * kChunk, count = min(kChunk, t_end - begin);
+        const __nv_bfloat16* w_t = tiles + (i % kStages) * 2 * Tile::kElements;
+        const __nv_bfloat16* k_t = w_t + Tile::kElements;
+        float u[kUTiles][4];
+#pragma unroll
+        for (int n = 0; n < kUTiles; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) u[n][r] = next[n][r];
+        const float keep = expf(next_keep);
+        ask(i + 1);
+#pragma unroll
+        for (int n = 0; n < kTiles; ++n)                     // the state before the chunk
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (er + g + 8 * h < dim)
+                    store(p.states + (((size_t)(first + i) * p.heads + head) * dim + er + g + 8 * h) * vdim + c0, 0,
+                          sc + 8 * n + 2 * tig, s[n][2 * h], s[n][2 * h + 1]);
+        ok = __syncthreads_and(mbar_wait(smem_u32(&full[i % kStages]), (i / kStages) & 1));
+        if (!ok) break;
+#pragma unroll
+        for (int e = 0; e < WIDTH; e += 32) {                // u = U_0 - W S
+            float d[2][kUTiles][4] = {};
+            unsigned a[2][3][4], b[2][2][3][2];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                load_a<Tile>(a[x], w_t, tr, e + 16 * x);
+                load_b_transposed<STile>(b[x], s_t, uc & ~15, e + 16 * x);
+                if (kUTiles == 1 && (uc & 8)) odd_first(b[x]);
+            }
+            constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+            for (int k6 = 0; k6 < 6; ++k6)
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int n = 0; n < kUTiles; ++n) mma_step(d[x][n], a[x][kA[k6]], b[x][n][kB[k6]]);
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int n = 0; n < kUTiles; ++n)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) u[n][r] += d[x][n][r];
+        }
+#pragma unroll
+        for (int n = 0; n < kUTiles; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int t = tr + g + 8 * h, c = uc + 8 * n + 2 * tig;
+                put(u_t, UTile::at(t, c >> 3) + 2 * tig, UTile::kPlane, u[n][2 * h], u[n][2 * h + 1]);
+                if (t < count)
+                    store(p.u + (size_t)(begin + t) * p.heads * vdim + (size_t)head * vdim + c0, 0, c, u[n][2 * h], u[n][2 * h + 1]);
+            }
+        __syncthreads();
+        float sum[kTiles][4] = {};
+#pragma unroll
+        for (int t = 0; t < kChunk; t += 32) {               // S = G S + sum_j G k_j u_j^T
+            float d[2][kTiles][4] = {};
+            unsigned a[2][3][4], b[2][(kTiles + 1) & ~1][3][2];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                load_a_transposed<Tile>(a[x], k_t, er, t + 16 * x);
+#pragma unroll
+                for (int n = 0; n < kTiles; n += 2) load_b_transposed<UTile>(b[x] + n, u_t, (sc & ~15) + 8 * n, t + 16 * x);
+                if (kTiles == 1 && (sc & 8)) odd_first(b[x]);
+            }
+            constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+            for (int k6 = 0; k6 < 6; ++k6)
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int n = 0; n < kTiles; ++n) mma_step(d[x][n], a[x][kA[k6]], b[x][n][kB[k6]]);
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int n = 0; n < kTiles; ++n)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) sum[n][r] += d[x][n][r];
+        }
+#pragma unroll
+        for (int n = 0; n < kTiles; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) s[n][r] = fmaf(keep, s[n][r], sum[n][r]);
+        put_s();
+        __syncthreads();                                     // the operands have been used; the state is there
+        if (tid == 0) bring(i + kStages);
+    }
+    if (!ok) {                                               // (a copy that did not come: nothing of the block's is left behind)
+        if (tid == 0) {
+            atomicExch(p.error_flag, 71);
+            for (int s = 0; s < kStages; ++s) mbar_wait(smem_u32(&full[s]), 0);
+        }
+        return;
+    }
+#pragma unroll
+    for (int n = 0; n < kTiles; ++n)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int e = er + g + 8 * (r >> 1), c = c0 + sc + 8 * n + 2 * tig + (r & 1);
+            if (e < dim && c < vdim) s_head[(size_t)e * vdim + c] = s[n][r];
+        }
+}
+
+template <int WIDTH, int COLUMNS>
+static int launch_delta_walk(const DeltaChunkArgs& p, int spans, cudaStream_t stream) {
+    constexpr size_t bytes = (size_t)delta_walk_bytes<WIDTH, COLUMNS>();
+    const int status = allow_shared(delta_walk_kernel<WIDTH, COLUMNS>, bytes, "delta_walk");
+    if (status != 0) return status;
+    // (a plain launch: see the walk of chunk_scan.cuh)
+    delta_walk_kernel<WIDTH, COLUMNS><<<dim3((p.vdim + COLUMNS - 1) / COLUMNS, p.heads, spans), kDeltaWalkThreads, bytes, stream>>>(p);
+    return check_launch("delta_walk");
+}
+
+template <int WIDTH>
+static int launch_delta_chunks(const DeltaChunkArgs& p, int chunks, int spans, cudaStream_t stream) {
+    constexpr size_t bytes = (size_t)solve_bytes<WIDTH>();
+    int status = allow_shared(delta_solve_kernel<WIDTH>, bytes, "delta_solve");
+    if (status != 0) return status;
+    launch_chained(delta_solve_kernel<WIDTH>, dim3(p.heads, chunks), kSolveThreads, bytes, stream, p);
+    if ((status = check_launch("delta_solve")) != 0) return status;
+    // A chunk is two products and two barriers deep however few columns a block has: 16 of them while the blocks are no more
+    // than the SMs (32 heads of 64 x 64, one span of 2,048 tokens: 128 blocks 62 us, 64 blocks of 32 columns 73 us).
+    const long long blocks = (long long)((p.vdim + 15) / 16) * p.heads * spans;
+    return blocks <= 148 ? launch_delta_walk<WIDTH, 16>(p, spans, stream) : launch_delta_walk<WIDTH, 32>(p, spans, stream);
+}
+
+}  // namespace celeg_b200
+
+using namespace celeg_b200;
+
+// Bytes of one (chunk, head)'s operands.
+CELEG_API int celeg_delta_operand_bytes(int dim) {
+    return 2 * 3 * kChunk * (dim <= 64 ? 64 : 128) * (int)sizeof(__nv_bfloat16);
+}
+
+// Over the step's spans from rows that celeg_delta_prepare has convolved and normalised; cum: of the scalar decays' kernel
+// (celeg_decay_sums). plan: of celeg_chunk_plan with the same max_chunks. Scratch: operands [chunks, heads, celeg_delta_
+// operand_bytes], 16-byte aligned; u [tokens, heads * vdim]; states [chunks, heads, dim, vdim]. dim at most 128.
+CELEG_API int celeg_delta_chunk_scan(const float* q, int q_stride, const float* k, int k_stride, const float* v, int v_stride,
+                                     const float* gates, const float2* cum, void* operands, float* u, float* states, float* out,
+                                     float* state, long long slot_stride, const int* span_slot, const int* plan, int max_chunks,
+                                     int spans, int chunks, int heads, int kv_heads, int dim, int vdim, float q_scale,
+                                     int* error_flag, cudaStream_t stream) {
+    CELEG_REQUIRE(spans >= 0 && chunks >= 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && dim <= 128 && vdim > 0,
+                  "delta_chunk_scan: invalid sizes spans=%d heads=%d kv_heads=%d dim=%d (at most 128) vdim=%d", spans, heads, kv_heads,
+                  dim, vdim);
+    CELEG_REQUIRE(chunks <= max_chunks && chunks <= 65535 && spans <= 65535 && heads <= 65535,
+                  "delta_chunk_scan: %d chunks of %d, %d spans or %d heads exceed one launch", chunks, max_chunks, spans, heads);
+    CELEG_REQUIRE(((size_t)operands & 15) == 0 && error_flag, "delta_chunk_scan: unaligned operands or no error flag");
+    if (spans == 0 || chunks == 0) return 0;
+    const int* span_first = plan + max_chunks + 1;
+    const DeltaChunkArgs d = {k, k_stride, v, v_stride, gates, cum, plan, span_first, (__nv_bfloat16*)operands, u, states, state,
+                              slot_stride, span_slot, heads, kv_heads, dim, vdim, error_flag};
+    int status = dim <= 64 ? launch_delta_chunks<64>(d, chunks, spans, stream) : launch_delta_chunks<128>(d, chunks, spans, stream);
+    if (status != 0) return status;
+    ChunkArgs p = {};
+    p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = u; p.v_stride = heads * vdim;
+    p.cum = cum; p.q_scale = q_scale;
+    p.chunk_begin = plan; p.pieces = 1; p.span_first = span_first; p.spans = spans;
+    p.states = states; p.out = out;
+    p.heads = heads; p.groups = kv_heads; p.dim = dim; p.vdim = vdim;
+    return launch_reads<kChunkScalar>(p, chunks, stream);
+}

@@ -179,6 +179,11 @@ _SIGNATURES = {
     "celeg_channel_decay_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    "celeg_decay_sums": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
+    "celeg_delta_operand_bytes": [c_int],
+    "celeg_delta_chunk_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                               c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                               c_int, c_float, c_void_p, c_void_p],
     "celeg_mlstm_chunk_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
                                c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
@@ -915,6 +920,40 @@ def recurrent_scan(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     _check(library().celeg_recurrent_scan(mode, _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0),
                                           _ptr(gates), _ptr(out), _ptr(state), slot_stride, _ptr(span_begin),
                                           _ptr(span_slot), spans, heads, kv_heads, dim, vdim, q_scale, _stream()))
+
+
+DELTA_CHUNK_MAX_DIM = 128      # key size of the chunked delta rule
+
+
+def delta_operand_bytes(dim: int) -> int:
+    """Bytes of scratch that one (chunk, head) of :func:`delta_chunk_scan` takes for its operands."""
+    return int(library().celeg_delta_operand_bytes(dim))
+
+
+def delta_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates: torch.Tensor, pre_a: torch.Tensor,
+                     dt_bias: torch.Tensor, a_log: torch.Tensor, cum: torch.Tensor, dt: torch.Tensor, operands: torch.Tensor,
+                     u: torch.Tensor, states: torch.Tensor, out: torch.Tensor, state: torch.Tensor, slot_stride: int,
+                     span_slot: torch.Tensor, plan: torch.Tensor, max_chunks: int, spans: int, chunks: int, heads: int,
+                     kv_heads: int, dim: int, vdim: int, q_scale: float, error_flag: torch.Tensor) -> None:
+    """The gated delta rule (mode SCAN_DELTA of :func:`recurrent_scan`) over the step's spans in chunks of 64 tokens
+    (csrc/delta_chunks.cu), from :func:`delta_prepare`'s q, k, v and beta (the first half of ``gates``); the decays are made
+    again from ``pre_a``, as sums of logarithms. Scratch: float32 ``cum`` [tokens, 2 heads], ``dt`` [tokens, heads], ``u``
+    [tokens, heads * vdim], ``states`` [chunks * heads * dim * vdim], ``operands`` of chunks * heads *
+    :func:`delta_operand_bytes`."""
+    for tensor in (q, k, v, gates, pre_a, dt_bias, a_log, cum, dt, u, states, out, state):
+        assert tensor.dtype == torch.float32 and tensor.stride(-1) == 1
+    assert gates.is_contiguous() and gates.shape[1] == 2 * heads and cum.is_contiguous() and cum.shape[1] == 2 * heads
+    assert dt.is_contiguous() and u.is_contiguous() and out.is_contiguous() and u.shape[1] == out.shape[1] == heads * vdim
+    assert states.numel() >= chunks * heads * dim * vdim
+    assert operands.numel() * operands.element_size() >= chunks * heads * delta_operand_bytes(dim)
+    _check(library().celeg_decay_sums(_ptr(pre_a), pre_a.stride(0), _ptr(dt_bias), _ptr(a_log), _ptr(cum), _ptr(dt), _ptr(plan),
+                                      chunks, heads, _stream()))
+    _check(library().celeg_delta_chunk_scan(
+        _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(gates), _ptr(cum), _ptr(operands), _ptr(u),
+        _ptr(states), _ptr(out), _ptr(state), slot_stride, _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, kv_heads,
+        dim, vdim, q_scale, _ptr(error_flag), _stream()))
+    global LAUNCHES
+    LAUNCHES += 2          # (two calls counted) the system, the walk, the read-outs
 
 
 def mlstm_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, pre_i: torch.Tensor, pre_f: torch.Tensor,

@@ -1,6 +1,6 @@
-"""The mLSTM in chunks (csrc/chunk_scan.cuh) against a float64 restatement and the token-by-token kernel, at the edges of
-chunks (64 tokens), of the blocks of key channels (32, 64, 128) and of columns (32, 64), and its mixer on a step of single
-tokens and portions."""
+"""The mLSTM and the gated delta rule in chunks (csrc/chunk_scan.cuh, csrc/delta_chunks.cu) against a float64 restatement and
+the token-by-token kernels, at the edges of chunks (64 tokens), of the blocks of key channels (32, 64, 128) and of columns (32,
+64), and the mLSTM's mixer on a step of single tokens and portions."""
 from __future__ import annotations
 
 import pytest
@@ -114,3 +114,64 @@ def test_mlstm_mixer_on_single_tokens_and_portions_together(dtype):
     bound = 2e-5 if dtype == torch.float32 else 2 ** -8
     for a, b in zip(*results):
         assert float((a - b).norm() / b.norm()) <= bound
+
+
+@pytest.mark.parametrize("lengths,heads,kv_heads,dim,vdim,slowest", [
+    ([64, 65, 1, 128, 63], 4, 2, 24, 36, 1e-3),      # whole chunks, one token more and less; shared keys; sizes between tiles
+    ([200], 2, 2, 64, 64, 1e-4),                     # a normal head, almost nothing forgotten
+    ([130, 66], 2, 1, 40, 7, 0.1),                   # odd columns: no access of two or four
+    ([97], 3, 3, 128, 200, 1e-2),                    # wide keys, more right sides than a pass of the solver takes
+    ([70, 150], 2, 1, 66, 32, 3.0),                  # just beyond 64 keys; decays of a twentieth a token
+])
+def test_delta_rule_in_chunks_is_as_near_to_64_bits_as_token_by_token(lengths, heads, kv_heads, dim, vdim, slowest):
+    from celeg_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(12)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g)      # noqa: E731
+    tokens, spans = sum(lengths), len(lengths)
+    rows = rand(tokens, kv_heads * 2 * dim + heads * vdim + 5)                 # as the prepared rows: one stride
+    q, k = rows[:, :kv_heads * dim], rows[:, kv_heads * dim:2 * kv_heads * dim]
+    for part in (q, k):
+        part.copy_(torch.nn.functional.normalize(part.reshape(tokens, kv_heads, dim), dim=-1).reshape(tokens, -1))
+    v = rows[:, 2 * kv_heads * dim:2 * kv_heads * dim + heads * vdim]
+    pre_a, dt_bias, a_log = rand(tokens, heads), rand(heads), torch.full((heads,), slowest, device="cuda").log()
+    decay = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus((pre_a + dt_bias).double(), threshold=100.0))
+    gates = torch.cat([torch.sigmoid(rand(tokens, heads)), decay.float()], dim=1).contiguous()
+    elements = heads * dim * vdim
+    before = rand(spans + 1, elements + 3)
+    begins = [0]
+    for n in lengths:
+        begins.append(begins[-1] + n)
+    slots = list(range(spans, 0, -1))
+    want, want_state = torch.zeros(tokens, heads, vdim, device="cuda", dtype=torch.float64), before.double()
+    share = heads // kv_heads
+    q64, k64 = (x.double().view(tokens, kv_heads, dim).repeat_interleave(share, dim=1) for x in (q, k))
+    v64, beta = v.double().view(tokens, heads, vdim), gates[:, :heads].double()
+    for span, slot in enumerate(slots):
+        s = want_state[slot, :elements].view(heads, dim, vdim).clone()
+        for t in range(begins[span], begins[span + 1]):
+            s = decay[t][:, None, None] * s
+            u = beta[t][:, None] * (v64[t] - (s * k64[t].unsqueeze(-1)).sum(-2))
+            s = s + k64[t].unsqueeze(-1) * u.unsqueeze(-2)
+            want[t] = (s * q64[t].unsqueeze(-1)).sum(-2) * dim ** -0.5
+        want_state[slot, :elements] = s.flatten()
+    want = want.flatten(1)
+
+    out, state = torch.zeros(tokens, heads * vdim, device="cuda"), before.clone()
+    kernels.recurrent_scan(kernels.SCAN_DELTA, q, k, v, gates, out, state, state.stride(0), i32(begins), i32(slots), spans, heads,
+                           kv_heads, dim, vdim, dim ** -0.5)
+    chunks = tokens // 64 + spans
+    full = lambda *shape: torch.full(shape, 5.0, device="cuda")                # noqa: E731
+    plan, got, got_state, flag = torch.zeros(chunks + spans + 8, dtype=torch.int32, device="cuda"), full(tokens, heads * vdim), before.clone(), i32([0])
+    kernels.chunk_plan(i32(begins), spans, chunks + 3, plan)
+    operands = full(chunks * heads * kernels.delta_operand_bytes(dim) // 4)
+    kernels.delta_chunk_scan(q, k, v, gates, pre_a, dt_bias, a_log, full(tokens, 2 * heads), full(tokens, heads), operands,
+                             full(tokens, heads * vdim), full(chunks * elements), got, got_state, got_state.stride(0), i32(slots), plan,
+                             chunks + 3, spans, chunks, heads, kv_heads, dim, vdim, dim ** -0.5, flag)
+    assert int(flag.item()) == 0
+
+    def off(x, y):
+        return float((x.double() - y).norm() / y.norm())
+    # float32 sums of the same products in different orders: errors of the same size, of a few units of 2^-24
+    for name, a, b, c in (("read", got, out, want), ("state", got_state, state, want_state)):
+        assert off(a, c) <= 2 * off(b, c) + 3e-7, (name, off(a, c), off(b, c))
+    assert torch.equal(got_state[:, elements:], before[:, elements:]) and torch.equal(got_state[0], before[0])
