@@ -32,6 +32,7 @@ enum ChunkMode : int {
     kChunkChannel = 1,     // a decay a token and key channel, taken into q and k beforehand (gated linear attention)
     kChunkConstant = 2,    // a decay a head (retention)
     kChunkStable = 3,      // exponential gates in range of a running maximum, with a normaliser (mLSTM)
+    kChunkPair = 4,        // read-outs alone: as channel, with a second set of values and products (generalised delta rule)
 };
 
 struct ChunkArgs {
@@ -40,6 +41,7 @@ struct ChunkArgs {
     const float2* cum; const float* dt;      // scalar: [tokens, heads]: sums of the decays' logarithms, steps (null: ones)
     const float* total;                      // channel: [chunks, heads * dim], the chunk's product of decays
     const float* products;                   // channel: [chunks, heads, 64, 64], zero above the diagonal
+    const float* products_b; const float* v_b; int v_b_stride;         // pair: the same for other values beside v
     const float* direct;                     // scalar: [heads], the values' share of the read-out, or null
     const float* decay; float q_scale;       // constant: [heads], and the keys' factor; stable, scalar: the queries' factor
     const float2* gates;                     // stable: [tokens, 3, heads]: forget sum F, i - F, the largest i - F so far
@@ -633,6 +635,7 @@ static_assert(SplitTile<kChunk, kReadRows>::kElements == SplitTile<kReadRows, kR
 // What the read-outs need of a head's gates over the chunk, twice: a head's are made while warps may still read the last one's.
 template <int MODE> struct ReadGates;
 template <> struct ReadGates<kChunkChannel> {};
+template <> struct ReadGates<kChunkPair> {};
 template <> struct ReadGates<kChunkScalar> { float2 cum[kChunk]; float step[kChunk], from_start[kChunk]; };
 template <> struct ReadGates<kChunkConstant> { float power[kChunk + 1]; };
 template <> struct ReadGates<kChunkStable> { float2 high[kChunk], own[kChunk]; float from_start[kChunk], low[kChunk], norm[256]; };
@@ -643,6 +646,8 @@ template <> struct ReadGates<kChunkStable> { float2 high[kChunk], own[kChunk]; f
 // hides the rest.
 template <int MODE, int WIDTH>
 __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_kernel(const ChunkArgs p, int heads_a_block, int columns) {
+    constexpr int passes = MODE == kChunkPair ? 2 : 1;       // sets of values
+    constexpr bool kPrepared = MODE == kChunkChannel || MODE == kChunkPair;
     using QTile = SplitTile<kChunk, WIDTH>;
     using KTile = SplitTile<kChunk, kReadRows>;
     using STile = SplitTile<kReadRows, kReadColumns>;
@@ -665,7 +670,7 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
     const float* q_src = p.q + (size_t)begin * p.q_stride + (size_t)qk_head * dim;
     const float* k_src = p.k + (size_t)begin * p.k_stride + (size_t)qk_head * dim;
     const bool q_four = by_fours(p.q, p.q_stride, dim), k_four = by_fours(p.k, p.k_stride, dim);
-    const bool v_four = by_fours(p.v, p.v_stride, vdim), s_four = by_fours(p.states, vdim, dim * vdim);
+    const bool v_four = by_fours(p.v, p.v_stride, vdim) && (passes == 1 || by_fours(p.v_b, p.v_b_stride, vdim)), s_four = by_fours(p.states, vdim, dim * vdim);
     const int row0 = 16 * warp + g;                          // this lane's tokens: row0, row0 + 8
     auto take_q = [&](int e0) {                              // (32 columns at a time: 16 registers)
 #pragma unroll 1
@@ -677,7 +682,7 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
         }
     };
     int turn = 0;                                            // the buffer that the next block goes to
-    const int s_blocks = (dim + kReadRows - 1) / kReadRows, a_tile = s_blocks + 2;
+    const int s_blocks = (dim + kReadRows - 1) / kReadRows, a_tile = s_blocks + 2 * passes;
     const int c_begin = blockIdx.z * columns, c_end = min(vdim, c_begin + columns);
     const int v_tiles = (c_end - c_begin + kReadColumns - 1) / kReadColumns;
     const int all_blocks = heads_a_block * v_tiles * a_tile;
@@ -686,12 +691,14 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
     auto ask = [&](int j) {
         if (j < all_blocks) {
             const int tile = j / a_tile, part = j - tile * a_tile, h = tile / v_tiles, c0 = c_begin + (tile - h * v_tiles) * kReadColumns;
-            const int head = head0 + h, r0 = (part < s_blocks ? part : part - s_blocks) * kReadRows;
-            const bool of_state = part < s_blocks;
+            const bool of_state = part < s_blocks, second = passes == 2 && part >= s_blocks + 2;
+            const int head = head0 + h, r0 = (of_state ? part : (part - s_blocks) & 1) * kReadRows;
+            const float* values = second ? p.v_b : p.v;
+            const long long values_stride = second ? p.v_b_stride : p.v_stride;
             const int real = (of_state ? dim : count) - r0;
             const float* from = of_state ? p.states + (((size_t)chunk * p.heads + head) * dim + r0) * vdim + c0
-                                         : p.v + (size_t)(begin + min(r0, count - 1)) * p.v_stride + (size_t)head * vdim + c0;
-            const long long stride = of_state ? vdim : p.v_stride;
+                                         : values + (size_t)(begin + min(r0, count - 1)) * values_stride + (size_t)head * vdim + c0;
+            const long long stride = of_state ? vdim : values_stride;
             const bool four = of_state ? s_four : v_four;
             if (WIDTH == 64) next.load(from, stride, real, vdim - c0, four);
             else share_copy<kReadRows, kReadColumns, kReadThreads>(ring + (j % kReadAhead<WIDTH>) * kReadRows * kReadColumns, from,
@@ -728,9 +735,8 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
 
     // q.k of the warp's tokens: columns 8 n + 2 tig, + 1
     float raw[8][4] = {};
-    if (MODE == kChunkChannel) {
-        if (whole) take_q(0);
-        const float* m = p.products + ((size_t)chunk * p.heads + head0) * kChunk * kChunk;
+    auto load_raw = [&](const float* products) {             // channel
+        const float* m = products + ((size_t)chunk * p.heads + head0) * kChunk * kChunk;
 #pragma unroll
         for (int n = 0; n < 8; ++n) {
             if (n > 2 * warp + 1) break;
@@ -742,6 +748,10 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
                 raw[n][2 * h + 1] = x.y;
             }
         }
+    };
+    if (kPrepared) {
+        if (whole) take_q(0);
+        load_raw(p.products);
     } else {
         TileShare<kChunk, kReadRows, kReadThreads> share;
         share.load(k_src, p.k_stride, count, dim, k_four);
@@ -842,7 +852,7 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
                     }
                 }
             }
-            if constexpr (MODE != kChunkChannel) {
+            if constexpr (!kPrepared) {
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     float f;
@@ -856,6 +866,8 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
                 }
             }
             float sums[2] = {0.0f, 0.0f};
+            for (int pass = 0; pass < passes; ++pass) {
+            if (passes == 2 && (pass == 1 || c0 > c_begin)) load_raw(pass ? p.products_b : p.products);
 #pragma unroll
             for (int part = 0; part < 2; ++part, ++j, turn ^= 1) {                 // the chunk's own tokens, 32 at a time
                 __nv_bfloat16* v_t = buffers + turn * STile::kElements;
@@ -894,6 +906,7 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
                         mma_split<4>(acc + 2 * n, a, b);
                     }
                 }
+            }
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {

@@ -22,6 +22,7 @@
 //
 // Products and their precision: chunk_scan.cuh.
 #include "chunk_scan.cuh"
+#include "general_delta.cuh"
 #include "tcgen05.cuh"
 
 namespace celeg_b200 {
@@ -38,6 +39,8 @@ struct DeltaChunkArgs {
     float* state; long long slot_stride; const int* span_slot;
     int heads, kv_heads, dim, vdim;
     int* error_flag;
+    const float* total;                      // general: [chunks, heads * dim], the channels' decays over a chunk (then cum, gates
+                                             // are null, and `states` holds what the chunk's own values add)
 };
 
 // ------------------------------------------------------------------------------------------------------------- solve
@@ -65,6 +68,42 @@ __device__ __forceinline__ void join_product(const float* a, const float* b, flo
         sum.x = fmaf(x, y.x, sum.x); sum.y = fmaf(x, y.y, sum.y); sum.z = fmaf(x, y.z, sum.z); sum.w = fmaf(x, y.w, sum.w);
     }
     *reinterpret_cast<float4*>(out + r * kSolvePitch + c) = make_float4(sign * sum.x, sign * sum.y, sign * sum.z, sign * sum.w);
+}
+
+// inverse = (1 + L)^-1, kSolvePitch floats a row, `lower` strictly lower triangular, `inverse` zero at first; what is left above
+// its diagonal is not to be used. All threads of a block come here, 128 of them work.
+__device__ __forceinline__ void invert(const float* lower, float* inverse) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool works = tid < 128;
+    __syncthreads();
+    if (works && lane < 16) {                                // a diagonal block a warp
+        const float* l = lower + 16 * warp * kSolvePitch + 16 * warp;
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float sum[4] = {i == lane ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int j = 0; j < i; ++j) sum[j & 3] = fmaf(-l[i * kSolvePitch + j], x[j], sum[j & 3]);
+            x[i] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            inverse[(16 * warp + i) * kSolvePitch + 16 * warp + lane] = x[i];
+        }
+    }
+    __syncthreads();
+    // two pairs of blocks of 16, 64 threads each; L_10 T_00 goes where the block above the diagonal is, zero again at the end
+    const int o = ((tid >> 6) & 1) * 32 * (kSolvePitch + 1), slot = tid & 63;
+    float* spare = inverse + o + 16;
+    if (works) join_product<16>(lower + o + 16 * kSolvePitch, inverse + o, spare, 1.0f, slot);
+    __syncthreads();
+    if (works) join_product<16>(inverse + o + 16 * (kSolvePitch + 1), spare, inverse + o + 16 * kSolvePitch, -1.0f, slot);
+    __syncthreads();
+    if (works) *reinterpret_cast<float4*>(spare + (slot >> 2) * kSolvePitch + (slot & 3) * 4) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    __syncthreads();
+    float* corner = inverse + 32;                            // the same with the two blocks of 32
+    for (int i = tid; i < 256; i += blockDim.x) join_product<32>(lower + 32 * kSolvePitch, inverse, corner, 1.0f, i);
+    __syncthreads();
+    for (int i = tid; i < 256; i += blockDim.x)
+        join_product<32>(inverse + 32 * (kSolvePitch + 1), corner, inverse + 32 * kSolvePitch, -1.0f, i);
+    __syncthreads();
 }
 
 template <int WIDTH>
@@ -133,40 +172,7 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 3 : 2) delta_solv
                 lower[i * kSolvePitch + j] = j < i && i < count ? raw[n][r] * beta_s[i] * exp_between(cum_s[i], cum_s[j]) : 0.0f;
             }
     }
-    __syncwarp();
-    if (lane < 16) {                                         // the warp's own diagonal block
-        const float* l = lower + 16 * warp * kSolvePitch + 16 * warp;
-        float x[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            float sum[4] = {i == lane ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int j = 0; j < i; ++j) sum[j & 3] = fmaf(-l[i * kSolvePitch + j], x[j], sum[j & 3]);
-            x[i] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
-            inverse[(16 * warp + i) * kSolvePitch + 16 * warp + lane] = x[i];
-        }
-    }
-    __syncthreads();
-    {
-        // two pairs of blocks of 16, 64 threads each; L_10 T_00 goes where the block above the diagonal is (zero at the end)
-        const int o = (tid >> 6) * 32 * (kSolvePitch + 1), slot = tid & 63;
-        float* spare = inverse + o + 16;
-        join_product<16>(lower + o + 16 * kSolvePitch, inverse + o, spare, 1.0f, slot);
-        __syncthreads();
-        join_product<16>(inverse + o + 16 * (kSolvePitch + 1), spare, inverse + o + 16 * kSolvePitch, -1.0f, slot);
-        __syncthreads();
-        const int r = slot >> 2, c = (slot & 3) * 4;
-        *reinterpret_cast<float4*>(spare + r * kSolvePitch + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        __syncthreads();
-        float* corner = inverse + 32;                        // the same with the two blocks of 32
-        join_product<32>(lower + 32 * kSolvePitch, inverse, corner, 1.0f, tid);
-        join_product<32>(lower + 32 * kSolvePitch, inverse, corner, 1.0f, tid + 128);
-        __syncthreads();
-        const float* below = inverse + 32 * (kSolvePitch + 1);
-        join_product<32>(below, corner, inverse + 32 * kSolvePitch, -1.0f, tid);
-        join_product<32>(below, corner, inverse + 32 * kSolvePitch, -1.0f, tid + 128);
-        __syncthreads();                                     // (what is above the diagonal is left out below)
-    }
+    invert(lower, inverse);
     // T with its columns scaled, split: every thread two neighbouring entries a time
     auto split_inverse = [&](bool with_decay) {
         for (int i = tid; i < kChunk * kChunk / 2; i += kSolveThreads) {
@@ -255,8 +261,9 @@ template <int WIDTH, int COLUMNS> constexpr int delta_walk_bytes() {
             SplitTile<kChunk, COLUMNS>::kElements) * (int)sizeof(__nv_bfloat16);
 }
 
-// COLUMNS of S a block: 16, or 32 where that is blocks enough
-template <int WIDTH, int COLUMNS>
+// COLUMNS of S a block: 16, or 32 where that is blocks enough. GENERAL: a decay a key channel, and the state is given what lies
+// in `states` of the chunk too.
+template <int WIDTH, int COLUMNS, bool GENERAL>
 __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const DeltaChunkArgs p) {
     using Tile = SplitTile<kChunk, WIDTH>;
     using STile = SplitTile<WIDTH, COLUMNS>;
@@ -316,6 +323,7 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
             s[n][r] = e < dim && c < vdim ? s_head[(size_t)e * vdim + c] : 0.0f;
         }
     put_s();
+    float add[kTiles][4] = {}, keeps[2] = {1.0f, 1.0f};      // general: of the chunk to come
     float next[kUTiles][4], next_keep = 0.0f;                      // U_0 of the chunk to come, its decay
     auto ask = [&](int i) {
         if (i >= chunks) return;
@@ -332,7 +340,20 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
                 next[n][2 * h] = x.x;
                 next[n][2 * h + 1] = x.y;
             }
-        next_keep = p.cum[(size_t)(begin + count - 1) * p.heads + head].x;
+        if (!GENERAL) {
+            next_keep = p.cum[(size_t)(begin + count - 1) * p.heads + head].x;
+            return;
+        }
+        const size_t rows = ((size_t)(first + i) * p.heads + head) * dim;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) keeps[h] = er + g + 8 * h < dim ? p.total[rows + er + g + 8 * h] : 0.0f;
+#pragma unroll
+        for (int n = 0; n < kTiles; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int e = er + g + 8 * (r >> 1), c = c0 + sc + 8 * n + 2 * tig + (r & 1);
+                add[n][r] = e < dim && c < vdim ? p.states[(rows + e) * vdim + c] : 0.0f;
+            }
     };
     auto store = [&](float* dst, int r, int c, float x, float y) {     // dst: the row's columns from c0 on
         if (c0 + c >= vdim) return;
@@ -362,6 +383,11 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
 #pragma unroll
             for (int r = 0; r < 4; ++r) u[n][r] = next[n][r];
         const float keep = expf(next_keep);
+        float given[kTiles][4], kept[2] = {keeps[0], keeps[1]};
+#pragma unroll
+        for (int n = 0; n < kTiles; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) given[n][r] = add[n][r];
         ask(i + 1);
 #pragma unroll
         for (int n = 0; n < kTiles; ++n)                     // the state before the chunk
@@ -435,7 +461,7 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
 #pragma unroll
         for (int n = 0; n < kTiles; ++n)
 #pragma unroll
-            for (int r = 0; r < 4; ++r) s[n][r] = fmaf(keep, s[n][r], sum[n][r]);
+            for (int r = 0; r < 4; ++r) s[n][r] = fmaf(GENERAL ? kept[r >> 1] : keep, s[n][r], GENERAL ? sum[n][r] + given[n][r] : sum[n][r]);
         put_s();
         __syncthreads();                                     // the operands have been used; the state is there
         if (tid == 0) bring(i + kStages);
@@ -456,13 +482,318 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
         }
 }
 
-template <int WIDTH, int COLUMNS>
+// ------------------------------------------------------------------------------------------------- the generalised rule
+// S_t = diag(w_t) S_(t-1) - b_t (u_t^T S_(t-1)) + k_t v_t^T, o_t = S_t^T r_t (general_delta_scan.cu has it in chunks of eight
+// tokens). With P_i the product of the chunk's decays through token i (a decay is at least 0.545, so 64 of them at least 1e-17:
+// quotients of two of them stay within float32, and lose nothing but rounding), u^ = u P_(i-1), r^ = r P_i, k^ = k / P_j, b^ = b /
+// P_j, and s_i = u_i^T S_(i-1),
+//
+//   s_i + sum_(j<i) (u^_i . b^_j) s_j = u^_i^T S_0 + sum_(j<i) (u^_i . k^_j) v_j
+//   o_i = r^_i^T S_0 + sum_(j<=i) [ (r^_i . k^_j) v_j - (r^_i . b^_j) s_j ]
+//   S_n = diag(P_n) [ S_0 + sum_j k^_j v_j^T - sum_j b^_j s_j^T ]
+//
+// the same shape: a system's inverse T, W = T u^ and s_0 = T ((u^ . k^) v), the same walk with s = s_0 + W S_0, and read-outs
+// with two sets of values. One block a (chunk, head) of 64 channels makes everything that does not wait for the state:
+// 140 us at 32 heads of 64 and 2,048 tokens, two blocks an SM (187 us with one); with the walk's 68 and the read-outs' 49 that is
+// 257 us where chunks of eight tokens take 344.
+struct GeneralChunkArgs {
+    const float* proj; int stride; int r_off, k_off, v_off, a_off;     // columns of a token's row: head h at h * dim
+    const float* z; int z_stride;                              // [tokens, heads * dim], before its bias
+    const float* w0; const float* a_bias;
+    float unit_eps;
+    const int* chunk_begin;
+    float* r_out;                                              // [tokens, heads * dim]: r^
+    float* products; float* products_b;                        // [chunks, heads, 64, 64]: r^.k^, -r^.b^, zero above the diagonal
+    __nv_bfloat16* operands;                                   // [chunks, heads, 2]: W, -b^ P_n
+    float* written;                                            // [tokens, heads * dim]: s_0
+    float* states; float* total;                               // diag(P_n) sum_j k^_j v_j^T; P_n
+    int heads, dim;
+};
+
+constexpr int kGeneralThreads = 256;
+constexpr int kGeneralBytes = 4 * SplitTile<kChunk, 64>::kElements * 2;
+
+__global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const GeneralChunkArgs p) {
+    using Tile = SplitTile<kChunk, 64>;
+    using Share = TileShare<kChunk, 64, kGeneralThreads>;
+    constexpr int kUnits = Share::kUnits, kRows = kGeneralThreads / Share::kPieces;
+    extern __shared__ __align__(128) __nv_bfloat16 tiles[];
+    __shared__ float last_s[4][64];
+    chain_release();
+    chain_wait();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
+    const int chunk = blockIdx.y, head = blockIdx.x, dim = p.dim;
+    const int begin = p.chunk_begin[chunk], count = p.chunk_begin[chunk + 1] - begin;
+    if (count <= 0) return;
+    __nv_bfloat16* u_t = tiles;                              // at first P, then u^
+    __nv_bfloat16* r_t = u_t + Tile::kElements;              // r^, then v, then L, then T's planes
+    __nv_bfloat16* k_t = r_t + Tile::kElements;              // k^, then T in float32
+    __nv_bfloat16* b_t = k_t + Tile::kElements;              // b^, then (u^ . k^) v
+    float* prefix = reinterpret_cast<float*>(u_t);           // [token][channel]
+    float* lower = reinterpret_cast<float*>(r_t);
+    float* inverse = reinterpret_cast<float*>(k_t);
+    const size_t inner = (size_t)p.heads * dim, at_head = (size_t)head * dim;
+    const float* rows = p.proj + (size_t)begin * p.stride;
+    const int piece = tid % Share::kPieces, c0 = piece * 8;
+    auto load = [&](Share& share, int offset) {
+        const float* src = rows + offset + at_head;
+        share.load(src, p.stride, count, dim, by_fours(src, p.stride, dim));
+    };
+    Share k, x;
+    load(k, p.k_off);
+    {
+        const float* src = p.z + (size_t)begin * p.z_stride + at_head;
+        x.load(src, p.z_stride, count, dim, by_fours(src, p.z_stride, dim));
+    }
+    float inv[kUnits];
+#pragma unroll
+    for (int n = 0; n < kUnits; ++n) {
+        const int t = tid / Share::kPieces + n * kRows;
+        float squares = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            squares = fmaf(k.x[n][j], k.x[n][j], squares);
+            const float w0 = c0 + j < dim ? p.w0[at_head + c0 + j] : 0.0f;
+            prefix[t * kSolvePitch + c0 + j] = t < count && c0 + j < dim ? channel_decay(x.x[n][j] + w0) : 1.0f;
+        }
+#pragma unroll
+        for (int offset = 1; offset < Share::kPieces; offset <<= 1) squares += __shfl_xor_sync(0xffffffffu, squares, offset);
+        inv[n] = 1.0f / sqrtf(squares + p.unit_eps);
+    }
+    load(x, p.r_off);
+    __syncthreads();
+    {
+        const int e = tid & 63, quarter = tid >> 6;          // products along 16 tokens, then of the quarters before
+        float* column = prefix + quarter * 16 * kSolvePitch + e;
+        float f = 1.0f;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            f *= column[t * kSolvePitch];
+            column[t * kSolvePitch] = f;
+        }
+        last_s[quarter][e] = f;
+        __syncthreads();
+        f = 1.0f;
+        for (int q = 0; q < quarter; ++q) f *= last_s[q][e];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) column[t * kSolvePitch] *= f;
+    }
+    __syncthreads();
+    const size_t at = ((size_t)chunk * p.heads + head);
+    __nv_bfloat16* w_out = p.operands + at * 2 * Tile::kElements;
+    __nv_bfloat16* b_out = w_out + Tile::kElements;
+    Share a;
+    load(a, p.a_off);
+    float through[kUnits][8], before[kUnits][8], whole[8];
+#pragma unroll
+    for (int n = 0; n < kUnits; ++n) {
+        const int t = tid / Share::kPieces + n * kRows;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            through[n][j] = prefix[t * kSolvePitch + c0 + j];
+            before[n][j] = t > 0 ? prefix[(t - 1) * kSolvePitch + c0 + j] : 1.0f;
+            whole[j] = prefix[(kChunk - 1) * kSolvePitch + c0 + j];
+        }
+    }
+    if (tid < 64) last_s[0][tid] = prefix[(kChunk - 1) * kSolvePitch + tid];
+    __syncthreads();                                         // (u^ takes the place of P)
+    auto put = [&](__nv_bfloat16* tile, int t, const float (&y)[8]) {
+        unsigned plane[3][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) split_pair(y[2 * j], y[2 * j + 1], plane[0][j], plane[1][j], plane[2][j]);
+#pragma unroll
+        for (int n = 0; n < 3; ++n)
+            *reinterpret_cast<uint4*>(tile + n * Tile::kPlane + Tile::at(t, piece)) = make_uint4(plane[n][0], plane[n][1], plane[n][2], plane[n][3]);
+    };
+#pragma unroll
+    for (int n = 0; n < kUnits; ++n) {
+        const int t = tid / Share::kPieces + n * kRows;
+        float u[8], r[8], kk[8], b[8], out[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = c0 + j;
+            const bool here = t < count && c < dim;
+            const float unit = k.x[n][j] * inv[n], back = 1.0f / through[n][j];
+            const float bias = c < dim ? p.a_bias[at_head + c] : 0.0f;
+            u[j] = unit * before[n][j];
+            r[j] = x.x[n][j] * through[n][j];
+            kk[j] = k.x[n][j] * back;
+            b[j] = here ? sigmoid_of(a.x[n][j] + bias) * unit * back : 0.0f;
+            out[j] = -b[j] * whole[j];
+            if (here) p.r_out[(size_t)(begin + t) * inner + at_head + c] = r[j];
+            if (t == 0 && c < dim) p.total[(size_t)chunk * inner + at_head + c] = whole[j];
+        }
+        put(u_t, t, u);
+        put(r_t, t, r);
+        put(k_t, t, kk);
+        put(b_t, t, b);
+        put(b_out, t, out);
+    }
+    __syncthreads();
+    // products: warps 0-3 r^.k^ and u^.k^, warps 4-7 r^.b^ and u^.b^, 16 tokens each
+    const int w4 = warp & 3;
+    const bool of_b = warp >= 4;
+    float acc[8][4];
+    auto product = [&](const __nv_bfloat16* left) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acc[n][r] = 0.0f;
+#pragma unroll 2
+        for (int e = 0; e < 64; e += 16) {
+            unsigned l[3][4];
+            load_a<Tile>(l, left, 16 * w4, e);
+#pragma unroll
+            for (int n = 0; n < 4; n += 2) {
+                if (n > w4) break;
+                unsigned b[4][3][2];
+                load_b<Tile>(b, of_b ? b_t : k_t, 16 * n, e);
+                load_b<Tile>(b + 2, of_b ? b_t : k_t, 16 * n + 16, e);
+                mma_split<4>(acc + 2 * n, l, b);
+            }
+        }
+    };
+    product(r_t);
+    {
+        float* dst = (of_b ? p.products_b : p.products) + at * kChunk * kChunk;
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = 16 * w4 + g + 8 * h, j = 8 * n + 2 * tig;
+                const float sign = of_b ? -1.0f : 1.0f;
+                *reinterpret_cast<float2*>(dst + i * kChunk + j) =
+                    make_float2(j <= i ? sign * acc[n][2 * h] : 0.0f, j + 1 <= i ? sign * acc[n][2 * h + 1] : 0.0f);
+            }
+    }
+    product(u_t);
+    __syncthreads();                                         // r^ has been used
+    load(x, p.v_off);
+    x.template store<Tile>(r_t, 0, Unscaled());
+    __syncthreads();
+    if (!of_b) {                                             // (u^ . k^) v
+        float y[8][4] = {};
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            if (m > w4) break;
+            unsigned l[3][4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int n = 2 * m + (q >> 1), i = 16 * w4 + g + 8 * (q & 1), j = 8 * n + 2 * tig;
+                split_pair(j < i ? acc[n][2 * (q & 1)] : 0.0f, j + 1 < i ? acc[n][2 * (q & 1) + 1] : 0.0f, l[0][q], l[1][q], l[2][q]);
+            }
+#pragma unroll
+            for (int n = 0; n < 4; n += 2) {
+                unsigned b[4][3][2];
+                load_b_transposed<Tile>(b, r_t, 16 * n, 16 * m);
+                load_b_transposed<Tile>(b + 2, r_t, 16 * n + 16, 16 * m);
+                mma_split<4>(y + 2 * n, l, b);
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                unsigned plane[3];
+                split_pair(y[n][2 * h], y[n][2 * h + 1], plane[0], plane[1], plane[2]);
+                __nv_bfloat16* to = b_t + Tile::at(16 * w4 + g + 8 * h, n) + 2 * tig;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) *reinterpret_cast<unsigned*>(to + q * Tile::kPlane) = plane[q];
+            }
+    } else {                                                 // diag(P_n) sum_j k^_j v_j^T
+        float y[8][4] = {};
+#pragma unroll 2
+        for (int t = 0; t < kChunk; t += 16) {
+            unsigned l[3][4];
+            load_a_transposed<Tile>(l, k_t, 16 * w4, t);
+#pragma unroll
+            for (int n = 0; n < 4; n += 2) {
+                unsigned b[4][3][2];
+                load_b_transposed<Tile>(b, r_t, 16 * n, t);
+                load_b_transposed<Tile>(b + 2, r_t, 16 * n + 16, t);
+                mma_split<4>(y + 2 * n, l, b);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int e = 16 * w4 + g + 8 * h;
+            if (e >= dim) continue;
+            const float f = last_s[0][e];
+            float* dst = p.states + (at * dim + e) * dim;
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+                    if (8 * n + 2 * tig + r < dim) dst[8 * n + 2 * tig + r] = f * y[n][2 * h + r];
+        }
+    }
+    __syncthreads();                                         // v and k^ have been used
+    if (of_b) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int i = 16 * w4 + g + 8 * (r >> 1), j = 8 * n + 2 * tig + (r & 1);
+                lower[i * kSolvePitch + j] = j < i ? acc[n][r] : 0.0f;
+            }
+    } else {
+        for (int i = tid; i < kChunk * kSolvePitch; i += 128) inverse[i] = 0.0f;
+    }
+    invert(lower, inverse);
+    for (int i = tid; i < kChunk * kChunk / 2; i += kGeneralThreads) {         // T's planes (L has been used)
+        const int r = i >> 5, c = (i & 31) * 2;
+        const float2 y = *reinterpret_cast<const float2*>(inverse + r * kSolvePitch + c);
+        unsigned plane[3];
+        split_pair(c <= r ? y.x : 0.0f, c + 1 <= r ? y.y : 0.0f, plane[0], plane[1], plane[2]);
+#pragma unroll
+        for (int n = 0; n < 3; ++n) *reinterpret_cast<unsigned*>(r_t + n * Tile::kPlane + Tile::at(r, c >> 3) + (c & 7)) = plane[n];
+    }
+    __syncthreads();
+    const __nv_bfloat16* right = of_b ? b_t : u_t;           // s_0 = T (u^ . k^) v, W = T u^
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[n][r] = 0.0f;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        if (t > w4) break;
+        unsigned l[3][4];
+        load_a<Tile>(l, r_t, 16 * w4, 16 * t);
+#pragma unroll
+        for (int n = 0; n < 4; n += 2) {
+            unsigned b[4][3][2];
+            load_b_transposed<Tile>(b, right, 16 * n, 16 * t);
+            load_b_transposed<Tile>(b + 2, right, 16 * n + 16, 16 * t);
+            mma_split<4>(acc + 2 * n, l, b);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int t = 16 * w4 + g + 8 * h, c = 8 * n + 2 * tig;
+            if (of_b) {
+                if (t >= count) continue;
+                float* dst = p.written + (size_t)(begin + t) * inner + at_head + c;
+                if (c < dim) dst[0] = acc[n][2 * h];
+                if (c + 1 < dim) dst[1] = acc[n][2 * h + 1];
+            } else {
+                unsigned plane[3];
+                split_pair(acc[n][2 * h], acc[n][2 * h + 1], plane[0], plane[1], plane[2]);
+                __nv_bfloat16* to = w_out + Tile::at(t, n) + 2 * tig;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) *reinterpret_cast<unsigned*>(to + q * Tile::kPlane) = plane[q];
+            }
+        }
+}
+
+template <int WIDTH, int COLUMNS, bool GENERAL>
 static int launch_delta_walk(const DeltaChunkArgs& p, int spans, cudaStream_t stream) {
     constexpr size_t bytes = (size_t)delta_walk_bytes<WIDTH, COLUMNS>();
-    const int status = allow_shared(delta_walk_kernel<WIDTH, COLUMNS>, bytes, "delta_walk");
+    const int status = allow_shared(delta_walk_kernel<WIDTH, COLUMNS, GENERAL>, bytes, "delta_walk");
     if (status != 0) return status;
     // (a plain launch: see the walk of chunk_scan.cuh)
-    delta_walk_kernel<WIDTH, COLUMNS><<<dim3((p.vdim + COLUMNS - 1) / COLUMNS, p.heads, spans), kDeltaWalkThreads, bytes, stream>>>(p);
+    delta_walk_kernel<WIDTH, COLUMNS, GENERAL><<<dim3((p.vdim + COLUMNS - 1) / COLUMNS, p.heads, spans), kDeltaWalkThreads, bytes, stream>>>(p);
     return check_launch("delta_walk");
 }
 
@@ -476,7 +807,7 @@ static int launch_delta_chunks(const DeltaChunkArgs& p, int chunks, int spans, c
     // A chunk is two products and two barriers deep however few columns a block has: 16 of them while the blocks are no more
     // than the SMs (32 heads of 64 x 64, one span of 2,048 tokens: 128 blocks 62 us, 64 blocks of 32 columns 73 us).
     const long long blocks = (long long)((p.vdim + 15) / 16) * p.heads * spans;
-    return blocks <= 148 ? launch_delta_walk<WIDTH, 16>(p, spans, stream) : launch_delta_walk<WIDTH, 32>(p, spans, stream);
+    return blocks <= 148 ? launch_delta_walk<WIDTH, 16, false>(p, spans, stream) : launch_delta_walk<WIDTH, 32, false>(p, spans, stream);
 }
 
 }  // namespace celeg_b200
@@ -515,4 +846,41 @@ CELEG_API int celeg_delta_chunk_scan(const float* q, int q_stride, const float* 
     p.states = states; p.out = out;
     p.heads = heads; p.groups = kv_heads; p.dim = dim; p.vdim = vdim;
     return launch_reads<kChunkScalar>(p, chunks, stream);
+}
+
+// The generalised rule over the step's spans. Offsets: columns of r, k, v and the removal rate in a row of proj (float32, rows
+// `stride` apart); z: float32 [tokens, heads * dim]. plan: of celeg_chunk_plan with the same max_chunks. Scratch: r_out, written
+// [tokens, heads * dim]; products, products_b [chunks, heads, 64, 64]; operands as above; states [chunks, heads, dim, dim];
+// total [chunks, heads * dim]. dim at most 64.
+CELEG_API int celeg_general_delta_chunk_scan(const float* proj, int stride, int r_off, int k_off, int v_off, int a_off,
+                                             const float* z, int z_stride, const float* w0, const float* a_bias, float unit_eps,
+                                             float* r_out, float* products, float* products_b, void* operands, float* written,
+                                             float* states, float* total, float* out, float* state, long long slot_stride,
+                                             const int* span_slot, const int* plan, int max_chunks, int spans, int chunks, int heads,
+                                             int dim, int* error_flag, cudaStream_t stream) {
+    CELEG_REQUIRE(spans >= 0 && chunks >= 0 && heads > 0 && dim > 0 && dim <= 64 && unit_eps > 0.0f,
+                  "general_delta_chunk_scan: invalid sizes spans=%d heads=%d dim=%d (at most 64)", spans, heads, dim);
+    CELEG_REQUIRE(chunks <= max_chunks && chunks <= 65535 && spans <= 65535 && heads <= 65535,
+                  "general_delta_chunk_scan: %d chunks of %d, %d spans or %d heads exceed one launch", chunks, max_chunks, spans, heads);
+    CELEG_REQUIRE(((size_t)operands & 15) == 0 && error_flag, "general_delta_chunk_scan: unaligned operands or no error flag");
+    if (spans == 0 || chunks == 0) return 0;
+    const int* span_first = plan + max_chunks + 1;
+    const GeneralChunkArgs first = {proj, stride, r_off, k_off, v_off, a_off, z, z_stride, w0, a_bias, unit_eps, plan, r_out, products,
+                                    products_b, (__nv_bfloat16*)operands, written, states, total, heads, dim};
+    int status = allow_shared(general_solve_kernel, kGeneralBytes, "general_solve");
+    if (status != 0) return status;
+    launch_chained(general_solve_kernel, dim3(heads, chunks), kGeneralThreads, kGeneralBytes, stream, first);
+    if ((status = check_launch("general_solve")) != 0) return status;
+    const DeltaChunkArgs d = {nullptr, 0, nullptr, 0, nullptr, nullptr, plan, span_first, (__nv_bfloat16*)operands, written, states, state,
+                              slot_stride, span_slot, heads, heads, dim, dim, error_flag, total};
+    const long long blocks = (long long)((dim + 15) / 16) * heads * spans;       // (see launch_delta_chunks)
+    status = blocks <= 148 ? launch_delta_walk<64, 16, true>(d, spans, stream) : launch_delta_walk<64, 32, true>(d, spans, stream);
+    if (status != 0) return status;
+    ChunkArgs p = {};
+    p.q = r_out; p.q_stride = heads * dim; p.v = proj + v_off; p.v_stride = stride; p.products = products;
+    p.products_b = products_b; p.v_b = written; p.v_b_stride = heads * dim;
+    p.chunk_begin = plan; p.pieces = 1; p.span_first = span_first; p.spans = spans;
+    p.states = states; p.out = out;
+    p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = dim;
+    return launch_reads<kChunkPair>(p, chunks, stream);
 }

@@ -179,6 +179,9 @@ _SIGNATURES = {
     "celeg_channel_decay_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    "celeg_general_delta_chunk_scan": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float,
+                                       c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                       c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "celeg_decay_sums": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "celeg_delta_operand_bytes": [c_int],
     "celeg_delta_chunk_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -954,6 +957,33 @@ def delta_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates: t
         dim, vdim, q_scale, _ptr(error_flag), _stream()))
     global LAUNCHES
     LAUNCHES += 2          # (two calls counted) the system, the walk, the read-outs
+
+
+GENERAL_DELTA_CHUNK_MAX_DIM = 64      # head size of the generalised delta rule in chunks of 64 tokens
+
+
+def general_delta_chunk_scan(proj: torch.Tensor, offsets: Tuple[int, int, int, int], z: torch.Tensor, w0: torch.Tensor,
+                             a_bias: torch.Tensor, unit_eps: float, r_out: torch.Tensor, products: torch.Tensor,
+                             products_b: torch.Tensor, operands: torch.Tensor, written: torch.Tensor, states: torch.Tensor,
+                             total: torch.Tensor, out: torch.Tensor, state: torch.Tensor, slot_stride: int,
+                             span_slot: torch.Tensor, plan: torch.Tensor, max_chunks: int, spans: int, chunks: int, heads: int,
+                             dim: int, error_flag: torch.Tensor) -> None:
+    """:func:`general_delta_scan` in chunks of 64 tokens (csrc/delta_chunks.cu), from a plan of :func:`chunk_plan`. Scratch:
+    float32 ``r_out``, ``written`` [tokens, heads * dim], ``products``, ``products_b`` of chunks * heads * 4096, ``states`` of chunks *
+    heads * dim^2, ``total`` of chunks * heads * dim; ``operands`` of chunks * heads * :func:`delta_operand_bytes`."""
+    for tensor in (proj, z, w0, a_bias, r_out, products, products_b, written, states, total, out, state):
+        assert tensor.dtype == torch.float32 and tensor.stride(-1) == 1
+    assert r_out.is_contiguous() and written.is_contiguous() and out.is_contiguous()
+    assert r_out.shape[1] == written.shape[1] == out.shape[1] == heads * dim
+    assert products.numel() >= chunks * heads * 4096 and products_b.numel() >= chunks * heads * 4096
+    assert states.numel() >= chunks * heads * dim * dim and total.numel() >= chunks * heads * dim
+    assert operands.numel() * operands.element_size() >= chunks * heads * delta_operand_bytes(dim)
+    _check(library().celeg_general_delta_chunk_scan(
+        _ptr(proj), proj.stride(0), *offsets, _ptr(z), z.stride(0), _ptr(w0), _ptr(a_bias), unit_eps, _ptr(r_out), _ptr(products),
+        _ptr(products_b), _ptr(operands), _ptr(written), _ptr(states), _ptr(total), _ptr(out), _ptr(state), slot_stride,
+        _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, dim, _ptr(error_flag), _stream()))
+    global LAUNCHES
+    LAUNCHES += 2          # the systems, the walk, the read-outs
 
 
 def mlstm_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, pre_i: torch.Tensor, pre_f: torch.Tensor,

@@ -175,3 +175,62 @@ def test_delta_rule_in_chunks_is_as_near_to_64_bits_as_token_by_token(lengths, h
     for name, a, b, c in (("read", got, out, want), ("state", got_state, state, want_state)):
         assert off(a, c) <= 2 * off(b, c) + 3e-7, (name, off(a, c), off(b, c))
     assert torch.equal(got_state[:, elements:], before[:, elements:]) and torch.equal(got_state[0], before[0])
+
+
+@pytest.mark.parametrize("lengths,heads,dim,decay", [
+    ([64, 65, 1, 128, 63], 3, 24, 0.0),              # whole chunks, one token more and less; a size between tiles
+    ([300], 2, 64, -8.0),                            # almost nothing forgotten
+    ([130, 66], 2, 7, 0.0),                          # odd columns: no access of two or four
+    ([70, 200], 5, 64, 20.0),                        # every decay at its least: products of 1e-17 over a chunk
+])
+def test_generalised_delta_rule_in_chunks_of_64(lengths, heads, dim, decay):
+    from celeg_b200 import kernels
+    import math
+    g = torch.Generator(device="cuda").manual_seed(13)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g)      # noqa: E731
+    tokens, spans, inner = sum(lengths), len(lengths), heads * dim
+    proj, z = rand(tokens, 4 * inner + 4), rand(tokens, inner) + decay
+    w0, a_bias, eps = rand(inner) * 0.3, rand(inner) * 0.3, 1e-6
+    offsets = (0, inner, 2 * inner, 3 * inner)
+    before = rand(spans + 1, inner * dim + 3)
+    begins = [0]
+    for n in lengths:
+        begins.append(begins[-1] + n)
+    slots = list(range(spans, 0, -1))
+    r, k, v, a = (proj[:, o:o + inner].double().view(tokens, heads, dim) for o in offsets)
+    keep = torch.exp(-math.exp(-0.5) * torch.sigmoid((z + w0).double())).view(tokens, heads, dim)
+    unit = k / torch.sqrt(k.square().sum(-1, keepdim=True) + eps)
+    removal = torch.sigmoid(a + a_bias.double().view(heads, dim)) * unit
+    want, want_state = torch.zeros(tokens, heads, dim, device="cuda", dtype=torch.float64), before.double()
+    for span, slot in enumerate(slots):
+        s = want_state[slot, :inner * dim].view(heads, dim, dim).clone()
+        for t in range(begins[span], begins[span + 1]):
+            taken = (s * unit[t].unsqueeze(-1)).sum(-2)
+            s = keep[t].unsqueeze(-1) * s - removal[t].unsqueeze(-1) * taken.unsqueeze(-2) + k[t].unsqueeze(-1) * v[t].unsqueeze(-2)
+            want[t] = (s * r[t].unsqueeze(-1)).sum(-2)
+        want_state[slot, :inner * dim] = s.flatten()
+    want = want.flatten(1)
+
+    token_span = i32([i for i, n in enumerate(lengths) for _ in range(n)])
+    out, state, flag = torch.zeros(tokens, inner, device="cuda"), before.clone(), i32([0])
+    records = torch.zeros(tokens * kernels.general_delta_scratch(heads, dim), device="cuda")
+    kernels.general_delta_scan(proj, offsets, z, w0, a_bias, eps, token_span, i32(begins), i32(slots), records, out, state,
+                               state.stride(0), tokens, spans, heads, dim, flag)
+    chunks = tokens // 64 + spans
+    full = lambda *shape: torch.full(shape, 5.0, device="cuda")                # noqa: E731
+    plan, got, got_state = torch.zeros(chunks + spans + 8, dtype=torch.int32, device="cuda"), full(tokens, inner), before.clone()
+    kernels.chunk_plan(i32(begins), spans, chunks + 3, plan)
+    operands = full(chunks * heads * kernels.delta_operand_bytes(dim) // 4)
+    kernels.general_delta_chunk_scan(proj, offsets, z, w0, a_bias, eps, full(tokens, inner), full(chunks * heads * 4096),
+                                     full(chunks * heads * 4096), operands, full(tokens, inner), full(chunks * inner * dim),
+                                     full(chunks * inner), got, got_state, got_state.stride(0), i32(slots), plan, chunks + 3, spans,
+                                     chunks, heads, dim, flag)
+    assert int(flag.item()) == 0
+
+    def off(x, y):
+        return float((x.double() - y).norm() / y.norm())
+    # float32 sums of the same products in different orders: errors of the same size, of a few units of 2^-24
+    for name, a, b, c in (("read", got, out, want), ("state", got_state, state, want_state)):
+        print(name, off(a, c), off(b, c))
+        assert off(a, c) <= 2 * off(b, c) + 3e-7, (name, off(a, c), off(b, c))
+    assert torch.equal(got_state[:, inner * dim:], before[:, inner * dim:]) and torch.equal(got_state[0], before[0])
