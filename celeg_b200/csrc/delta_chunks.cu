@@ -45,15 +45,17 @@ struct DeltaChunkArgs {
 
 // ------------------------------------------------------------------------------------------------------------- solve
 // The system's matrix is inverted, T = (1 + L)^-1: its four diagonal blocks of 16 by substitution, a warp a block and a lane a
-// column; then two blocks of 16 and at last two of 32 are joined, T_21 = -T_22 L_21 T_11; and W and U_0 are products of T, its
-// columns scaled, with k and v as they lie. (Substitution over whole right sides, a thread two columns, was one chain of 64
-// steps a block: 138 us for 32 heads of 64 and 2,048 tokens, 69 us like this.)
+// column; then two blocks of 16 and at last two of 32 are joined, T_21 = -T_22 L_21 T_11; and W and U_0 are products of T with
+// the scaled k and v. It is bound by the latency of these steps, so blocks an SM count: T in float32 lies where k did and L where
+// T's planes will, 50 KB a block, four of them an SM; the right sides are scaled, so that T is split once. 57 us for 32 heads of
+// 64 and 2,048 tokens (69 with three blocks and T split twice; 138 by substitution over whole right sides, one chain of 64 steps
+// a block).
 constexpr int kSolveThreads = 128;
 constexpr int kSolvePitch = kChunk + 4;
 template <int WIDTH> constexpr int solve_bytes() {
-    return (SplitTile<kChunk, WIDTH>::kElements + SplitTile<kChunk, 64>::kElements) * 2 + kChunk * kSolvePitch * 4;
+    return (SplitTile<kChunk, WIDTH>::kElements + SplitTile<kChunk, 64>::kElements) * 2;
 }
-static_assert(SplitTile<kChunk, 64>::kElements * 2 >= kChunk * kSolvePitch * 4, "L lies where T's planes will");
+static_assert(SplitTile<kChunk, 64>::kElements * 2 >= kChunk * kSolvePitch * 4, "L lies where T's planes will, T where k did");
 
 // out = sign a b of N x N blocks of matrices with kSolvePitch floats a row, 128 / (N * N / 4) of them side by side; a thread four
 // neighbours of a row. `a`, `b`, `out`: of the thread's block.
@@ -107,7 +109,7 @@ __device__ __forceinline__ void invert(const float* lower, float* inverse) {
 }
 
 template <int WIDTH>
-__global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 3 : 2) delta_solve_kernel(const DeltaChunkArgs p) {
+__global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 4 : 2) delta_solve_kernel(const DeltaChunkArgs p) {
     using Tile = SplitTile<kChunk, WIDTH>;
     using TTile = SplitTile<kChunk, 64>;
     using VTile = SplitTile<kChunk, 64>;
@@ -120,10 +122,10 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 3 : 2) delta_solv
     const int chunk = blockIdx.y, head = blockIdx.x, dim = p.dim, vdim = p.vdim;
     const int begin = p.chunk_begin[chunk], count = p.chunk_begin[chunk + 1] - begin;
     if (count <= 0) return;
-    __nv_bfloat16* k_t = tiles;                              // k, then v
+    __nv_bfloat16* k_t = tiles;                              // k, then T in float32, then the right sides
     __nv_bfloat16* t_t = tiles + Tile::kElements;            // T's planes, at first L
     float* lower = reinterpret_cast<float*>(t_t);
-    float* inverse = reinterpret_cast<float*>(t_t + TTile::kElements);
+    float* inverse = reinterpret_cast<float*>(k_t);
     const float* k_src = p.k + (size_t)begin * p.k_stride + (size_t)(head / (p.heads / p.kv_heads)) * dim;
     const float* v_src = p.v + (size_t)begin * p.v_stride + (size_t)head * vdim;
     const bool k_four = by_fours(p.k, p.k_stride, dim), v_four = by_fours(p.v, p.v_stride, vdim);
@@ -135,7 +137,6 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 3 : 2) delta_solv
         start_s[tid] = expf(own.x);
         end_s[tid] = exp_between(p.cum[(size_t)(begin + count - 1) * p.heads + head], own);
     }
-    for (int i = tid; i < kChunk * kSolvePitch; i += kSolveThreads) inverse[i] = 0.0f;
     __syncthreads();
     const size_t at = ((size_t)chunk * p.heads + head) * 2;
     __nv_bfloat16* w_out = p.operands + at * Tile::kElements;
@@ -172,20 +173,23 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 3 : 2) delta_solv
                 lower[i * kSolvePitch + j] = j < i && i < count ? raw[n][r] * beta_s[i] * exp_between(cum_s[i], cum_s[j]) : 0.0f;
             }
     }
+    __syncthreads();                                         // k has been used
+    for (int i = tid; i < kChunk * kSolvePitch; i += kSolveThreads) inverse[i] = 0.0f;
     invert(lower, inverse);
-    // T with its columns scaled, split: every thread two neighbouring entries a time
-    auto split_inverse = [&](bool with_decay) {
-        for (int i = tid; i < kChunk * kChunk / 2; i += kSolveThreads) {
-            const int r = i >> 5, c = (i & 31) * 2;
-            const float fx = beta_s[c] * (with_decay ? start_s[c] : 1.0f), fy = beta_s[c + 1] * (with_decay ? start_s[c + 1] : 1.0f);
-            const float2 x = *reinterpret_cast<const float2*>(inverse + r * kSolvePitch + c);
-            unsigned plane[3];
-            split_pair(c <= r ? x.x * fx : 0.0f, c + 1 <= r ? x.y * fy : 0.0f, plane[0], plane[1], plane[2]);
+    for (int i = tid; i < kChunk * kChunk / 2; i += kSolveThreads) {           // T's planes in the place of L
+        const int r = i >> 5, c = (i & 31) * 2;
+        const float2 x = *reinterpret_cast<const float2*>(inverse + r * kSolvePitch + c);
+        unsigned plane[3];
+        split_pair(c <= r ? x.x : 0.0f, c + 1 <= r ? x.y : 0.0f, plane[0], plane[1], plane[2]);
 #pragma unroll
-            for (int n = 0; n < 3; ++n)
-                *reinterpret_cast<unsigned*>(t_t + n * TTile::kPlane + TTile::at(r, c >> 3) + (c & 7)) = plane[n];
-        }
-    };
+        for (int n = 0; n < 3; ++n) *reinterpret_cast<unsigned*>(t_t + n * TTile::kPlane + TTile::at(r, c >> 3) + (c & 7)) = plane[n];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int e = 0; e < WIDTH; e += 32) {                    // the right sides beta G k
+        share.load(k_src + e, p.k_stride, count, dim - e, k_four);
+        share.template store<Tile>(k_t, e >> 3, [&](int r) { return beta_s[r] * start_s[r]; });
+    }
     float acc[8][4];
     auto multiply = [&](auto tile, const __nv_bfloat16* from, int n0) {        // T times 64 columns from n0 on
         using B = decltype(tile);
@@ -207,7 +211,6 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 3 : 2) delta_solv
             }
         }
     };
-    split_inverse(true);
     __syncthreads();
 #pragma unroll 1
     for (int e = 0; e < WIDTH; e += 64) {                    // -W = -T beta G k
@@ -223,14 +226,12 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 3 : 2) delta_solv
                 for (int x = 0; x < 3; ++x) *reinterpret_cast<unsigned*>(to + x * Tile::kPlane) = plane[x];
             }
     }
-    __syncthreads();
-    split_inverse(false);
     for (int c0 = 0; c0 < vdim; c0 += 64) {                  // U_0 = T beta v
-        if (c0 > 0) __syncthreads();
+        __syncthreads();
 #pragma unroll 1
         for (int c = 0; c < 64; c += 32) {
             share.load(v_src + c0 + c, p.v_stride, count, vdim - c0 - c, v_four);
-            share.template store<VTile>(k_t, c >> 3, Unscaled());
+            share.template store<VTile>(k_t, c >> 3, [&](int r) { return beta_s[r]; });
         }
         __syncthreads();
         multiply(VTile(), k_t, 0);
