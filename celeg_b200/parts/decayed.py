@@ -34,6 +34,10 @@ class ChunkedSpans:
         self.max_chunks = rt.max_tokens // self.tokens + rt.max_requests + 48
         self.plan = rt.flat_scratch("decay.plan", 2 * self.max_chunks + rt.max_tokens + 64, torch.int32)
 
+    def fits(self, step: StepContext, single: int) -> bool:
+        """Whether the scratch holds the chunks of the spans from ``single`` on."""
+        return (step.tokens - single) // self.tokens + step.spans - single <= self.max_chunks
+
     def of(self, step: StepContext, single: int):
         """(plan, spans, bound of the chunks) of the spans from ``single`` on."""
         spans = step.spans - single

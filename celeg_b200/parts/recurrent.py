@@ -105,7 +105,8 @@ class MlstmMixer:
             rt.linear(self.gated, self.w_out, out, t)
             return
         # long portions in chunks; what lies before them (single tokens), and steps of short spans, token by token
-        one_by_one = step.leading_single_tokens if step.max_span >= self.CHUNKED_FROM else t
+        chunked = step.max_span >= self.CHUNKED_FROM and self.spans.fits(step, step.leading_single_tokens)
+        one_by_one = step.leading_single_tokens if chunked else t
         if one_by_one:
             spans = step.spans if one_by_one == t else one_by_one
             kernels.mlstm_gates(pre_i, pre_f, self.bias_i, self.bias_f, self.cap, self.gates, one_by_one, self.heads)
@@ -222,7 +223,8 @@ class GatedDeltaMixer:
         k = conv[:, self.qk_width:2 * self.qk_width]
         v = conv[:, 2 * self.qk_width:]
         # long portions in chunks; what lies before them (single tokens), and steps of short spans, token by token
-        chunked = step.max_span >= self.CHUNKED_FROM and self.dim <= kernels.DELTA_CHUNK_MAX_DIM
+        chunked = (step.max_span >= self.CHUNKED_FROM and self.dim <= kernels.DELTA_CHUNK_MAX_DIM
+                   and self.spans.fits(step, step.leading_single_tokens))
         one_by_one = step.leading_single_tokens if chunked else t
         if one_by_one:
             kernels.recurrent_scan(kernels.SCAN_DELTA, q, k, v, self.gates, self.read, b.state, b.slot_stride,
@@ -550,7 +552,8 @@ class GeneralDeltaMixer:
         kernels.activation_cast(rows[:, 5 * inner:], self.low, t, kernels.ACT_TANH)
         rt.linear(self.low, self.w_decay, self.z, t)
         # long portions in chunks of 64 tokens; what lies before them (single tokens), and steps of short spans, in chunks of 8
-        chunked = step.max_span >= self.CHUNKED_FROM and self.dim <= kernels.GENERAL_DELTA_CHUNK_MAX_DIM
+        chunked = (step.max_span >= self.CHUNKED_FROM and self.dim <= kernels.GENERAL_DELTA_CHUNK_MAX_DIM
+                   and self.spans.fits(step, step.leading_single_tokens))
         short = step.leading_single_tokens if chunked else t
         columns = (0, inner, 2 * inner, 4 * inner)
         if short:
