@@ -672,4 +672,4 @@ class StepFunction:
 def device_error_text(code: int) -> str:
     return (f"a kernel reported error code {code} (1: cache write without a page, 2: attention read without "
             f"a page, 3: more key splits than the launch has blocks for, 11-24 and 61-65: a bounded wait of "
-            f"a tcgen05 kernel ran out)")
+            f"a tcgen05 kernel ran out, 71: one of the chunked delta rules' walk did)")
