@@ -201,7 +201,8 @@ class KernelTimer:
              "block_diagonal_product", "lru_scan", "lru_decode", "add_layernorm", "qkv_prepare", "rmsnorm_strided",
              "sigmoid_gate", "output_norm", "activation_cast", "general_delta_scan", "general_delta_decode",
              "hyper_connect", "normed_pair", "channel_conv", "chunk_plan", "channel_decay_scan", "scalar_decay_scan",
-             "channel_decay_decode", "scalar_decay_decode")
+             "channel_decay_decode", "scalar_decay_decode", "mlstm_chunk_scan", "delta_chunk_scan",
+             "general_delta_chunk_scan")
 
     def __init__(self):
         self.pairs = []
