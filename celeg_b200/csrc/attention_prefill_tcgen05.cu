@@ -468,9 +468,12 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                                             ? exp2f(p.sinks[h] * 1.4426950408889634f - used_max) : 0.0f;
                 const float inv = run_sum > 0.0f ? 1.0f / (run_sum + sink_part) : 0.0f;
                 __nv_bfloat16* dst = p.out + ((size_t)(t0 + row) * p.q_heads + h) * D;
+                // (a load from tensor memory wants the whole warp: lanes past the span come to every one of them, and the
+                // warp is whole again before each; only the stores are the live lanes' own)
 #pragma unroll
                 for (int c0 = 0; c0 < D; c0 += 32) {
                     unsigned o[32];
+                    __syncwarp();
                     if (blocks > 0) {
                         tmem_load_32_issue(o_taddr + (unsigned)c0, o);
                         tmem_load_wait();
@@ -478,17 +481,19 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 #pragma unroll
                         for (int j = 0; j < 32; ++j) o[j] = 0u;
                     }
-                    if (!live) continue;
+                    if (live) {
 #pragma unroll
-                    for (int c = 0; c < 32; c += 8) {
-                        uint4 packed;
-                        __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&packed);
+                        for (int c = 0; c < 32; c += 8) {
+                            uint4 packed;
+                            __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&packed);
 #pragma unroll
-                        for (int e2 = 0; e2 < 4; ++e2)
-                            h2[e2] = __floats2bfloat162_rn(__uint_as_float(o[c + 2 * e2]) * inv, __uint_as_float(o[c + 2 * e2 + 1]) * inv);
-                        *reinterpret_cast<uint4*>(dst + c0 + c) = packed;
+                            for (int e2 = 0; e2 < 4; ++e2)
+                                h2[e2] = __floats2bfloat162_rn(__uint_as_float(o[c + 2 * e2]) * inv, __uint_as_float(o[c + 2 * e2 + 1]) * inv);
+                            *reinterpret_cast<uint4*>(dst + c0 + c) = packed;
+                        }
                     }
                 }
+                __syncwarp();
             }
         }
         if (error) atomicExch(p.error_flag, error);
