@@ -23,6 +23,7 @@
 // Products and their precision: chunk_scan.cuh.
 #include "chunk_scan.cuh"
 #include "general_delta.cuh"
+#include "ring_drain.h"
 #include "tcgen05.cuh"
 
 namespace celeg_b200 {
@@ -374,7 +375,8 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
         }
     };
     bool ok = true;
-    for (int i = 0; i < chunks; ++i) {
+    int i = 0;
+    for (; i < chunks; ++i) {
         const int begin = t_begin + i * kChunk, count = min(kChunk, t_end - begin);
         const __nv_bfloat16* w_t = tiles + (i % kStages) * 2 * Tile::kElements;
         const __nv_bfloat16* k_t = w_t + Tile::kElements;
@@ -467,10 +469,11 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
         __syncthreads();                                     // the operands have been used; the state is there
         if (tid == 0) bring(i + kStages);
     }
-    if (!ok) {                                               // (a copy that did not come: nothing of the block's is left behind)
+    if (!ok) {                             // a copy did not come: chunk i's and those behind it (nothing of the block's is left behind)
         if (tid == 0) {
             atomicExch(p.error_flag, 71);
-            for (int s = 0; s < kStages; ++s) mbar_wait(smem_u32(&full[s]), 0);
+            drain_ring(i, min(chunks, i + kStages), kStages,
+                       [&](int stage, unsigned parity) { mbar_wait(smem_u32(&full[stage]), parity); });
         }
         return;
     }
