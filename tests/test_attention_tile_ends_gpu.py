@@ -1,5 +1,5 @@
 """Where a query tile of the tcgen05 prompt attention (csrc/attention_prefill_tcgen05.cu) ends before its 128 rows or its last
-block's 64 keys do, at both head sizes: rows that end inside a warp."""
+block's 64 keys do, at both head sizes: rows that end inside a warp, and what lies where no row looks."""
 from __future__ import annotations
 
 import pytest
@@ -53,4 +53,17 @@ def test_rows_that_end_inside_a_warp(dim):
     lengths = (1, 31, 32, 33, 63, 65, 95, 97, 127, 128, 129, 161)
     out, want = attention(dim, 8, 2, 16, None, lengths, tuple(7 * i for i in range(len(lengths))))
     # the weights and the output are rounded to 8 bits once each: two errors of at most 2^-9 of a row's numbers
+    assert float((out - want).norm() / want.norm()) <= 2 ** -8
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("unseen", [float("nan"), float("inf")])
+@pytest.mark.parametrize("page,window,lengths,starts", [
+    (16, None, (5, 130, 200), (0, 3, 1000)), (8, 70, (129, 40), (500, 77)), (64, None, (33, 128), (0, 60)), (32, 150, (300,), (1001,)),
+])
+def test_places_that_no_row_of_a_tile_sees_may_hold_anything(dim, unseen, page, window, lengths, starts):
+    """A weight of zero times a NaN is a NaN: what another request left in page 0, in a page that was used again or before the
+    window does not reach a prompt's rows."""
+    out, want = attention(dim, 4, 2, page, window, lengths, starts, unseen)
+    # (as above)
     assert float((out - want).norm() / want.norm()) <= 2 ** -8
