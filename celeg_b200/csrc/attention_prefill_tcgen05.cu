@@ -33,6 +33,7 @@
 // go to attention_prefill.cu (mma.sync) or attention_generic.cu.
 //
 // Counterparts in celeg: see attention_prefill.cu.
+#include "ring_drain.h"
 #include "tcgen05.cuh"
 
 namespace celeg_b200 {
@@ -210,6 +211,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             const int blocks = block_end - block_begin;
             int page = lookup(block_begin), page_next = L::kTogether ? 0 : lookup(block_begin + 1);
             bool ok = true;
+            int k_brought = 0, v_brought = 0;
             if (L::kTogether) {
                 const CUtensorMap* map = part ? &map_v : &map_k;
                 const unsigned to = part ? v_addr : k_addr;
@@ -217,21 +219,33 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                     const int mine = page;
                     page = lookup(block_begin + i + 1);
                     ok = bring(map, kf, ke, 2 * L::kKvBytes, to, 0, i, mine);
+                    k_brought += ok;
                 }
             } else {
                 const unsigned half = part * L::kKvHalf;
                 ok = bring(&map_k, kf, ke, L::kKvBytes, k_addr + half, part * 64, 0, page);
+                k_brought += ok;
                 for (int i = 0; i < blocks && ok; ++i) {
                     const int page_v = page;
                     if (i + 1 < blocks) {
                         page = page_next;
                         page_next = lookup(block_begin + i + 2);
                         ok = bring(&map_k, kf, ke, L::kKvBytes, k_addr + half, part * 64, i + 1, page);
+                        k_brought += ok;
                     }
                     ok = ok && bring(&map_v, vf, ve, L::kKvBytes, v_addr + half, part * 64, i, page_v);
+                    v_brought += ok;
                 }
             }
-            if (!ok && lane == 0) error = 61;
+            if (lane == 0) {
+                if (!ok) error = 61;
+                // whichever role gives up: the block does not end before its copies have landed
+                mbar_wait_suspended(smem_u32(&q_full), 0);
+                drain_ring(max(0, k_brought - kStages), k_brought, kStages,
+                           [&](int stage, unsigned parity) { mbar_wait_suspended(kf + 8u * stage, parity); });
+                drain_ring(max(0, v_brought - kStages), v_brought, kStages,
+                           [&](int stage, unsigned parity) { mbar_wait_suspended(vf + 8u * stage, parity); });
+            }
         } else if (warp == 1 && lane == 0) {
             // ---------------------------------------------------------------- MMA issuer
             constexpr unsigned idesc_s = instruction_descriptor(kFaM, kFaN);
