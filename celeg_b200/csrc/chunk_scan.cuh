@@ -18,8 +18,17 @@
 // towards zero at every link of a chain: read-outs and states are nearer to 64 bits than float32 multiplications and
 // additions in order (1.1e-7 against 2.4e-7 over 2,000 tokens of 16 heads of 64 x 128). A number is split once a block, on
 // its way into shared memory; split at every use by the warps that load it (two tf32 numbers, m16n8k8), a fragment cost more
-// instructions than its products. An infinite operand gives NaN (its mid is inf - inf).
+// instructions than its products.
+//
+// Numbers that are not finite. An infinite operand gives NaN (its mid is inf - inf). A token's NaN belongs to it and to the
+// tokens behind it, but a weight of zero times a NaN is a NaN, and the tokens before it meet it under a weight of zero in the
+// products with v. So v's tiles take a zero in its place and note the column's first such token (BadTokens), and the read-outs
+// from that token on are NaN; the same for the right sides of the delta rules' systems. It costs the cases of 2,048 tokens
+// between nothing and 1 %, the generalised delta rule 2 % (359 to 365 us with the projections). (A decay a channel that is NaN
+// reaches the tokens of its block of eight: decayed_scan.cu.)
 #pragma once
+
+#include <cfloat>
 
 #include "mma_tiles.cuh"
 
@@ -118,6 +127,29 @@ __device__ __forceinline__ bool by_fours(const float* p, long long stride, int s
     return ((((unsigned long long)p >> 2) | (unsigned long long)stride | (unsigned)sizes) & 3) == 0;
 }
 
+// Of a chunk's 64 columns of values the first token with a number that is not finite, in shared memory; every use lies between
+// barriers that are there for the tile itself.
+struct BadTokens {
+    int first[64];
+    int any;
+    __device__ __forceinline__ void clear() {                // (65 threads at least)
+        if (threadIdx.x < 64) first[threadIdx.x] = kChunk;
+        if (threadIdx.x == 64) any = 0;
+    }
+    __device__ __forceinline__ void note(int column, int token) {
+        atomicMin(&first[column], token);
+        any = 1;
+    }
+    // a warp's results of tokens t, t + 8 and columns c + 8 n, + 1: NaN from `behind` tokens behind the first bad one on
+    __device__ __forceinline__ void mark(float (&acc)[8][4], int t, int c, int behind = 0) const {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (t + 8 * (r >> 1) >= first[c + 8 * n + (r & 1)] + behind) acc[n][r] = NAN;
+    }
+};
+
 // A thread's share of a ROWS x COLUMNS tile of floats: pieces of eight neighbours, THREADS apart. load(): zeros from row
 // `real_rows` and column `real_columns` on; store(): times scale(row), split, into shared memory.
 template <int ROWS, int COLUMNS, int THREADS>
@@ -143,20 +175,44 @@ struct TileShare {
             }
         }
     }
-    template <typename T, typename Scale>                    // T: the tile it is part of, from the row's piece `piece` on
-    __device__ __forceinline__ void store(__nv_bfloat16* tile, int piece, Scale scale) const {
+    // T: the tile it is part of, from the row's piece `piece` on. False where a number is not finite.
+    template <typename T, typename Scale>
+    __device__ __forceinline__ bool store(__nv_bfloat16* tile, int piece, Scale scale) const {
+        unsigned none = 0;                                   // (two zeros, NaN as soon as a number is infinite or NaN)
 #pragma unroll
         for (int u = 0; u < kUnits; ++u) {
             const int r = threadIdx.x / kPieces + u * (THREADS / kPieces);
             const float f = scale(r);
             unsigned plane[3][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) split_pair(x[u][2 * j] * f, x[u][2 * j + 1] * f, plane[0][j], plane[1][j], plane[2][j]);
+            for (int j = 0; j < 4; ++j) {
+                split_pair(x[u][2 * j] * f, x[u][2 * j + 1] * f, plane[0][j], plane[1][j], plane[2][j]);
+                asm("fma.rn.bf16x2 %0, %1, %2, %0;\n" : "+r"(none) : "r"(plane[0][j]), "r"(0));
+            }
             __nv_bfloat16* to = tile + T::at(r, piece + threadIdx.x % kPieces);
 #pragma unroll
             for (int n = 0; n < 3; ++n)
                 *reinterpret_cast<uint4*>(to + n * T::kPlane) = make_uint4(plane[n][0], plane[n][1], plane[n][2], plane[n][3]);
         }
+        return (none & 0x7fff7fffu) == 0;
+    }
+    // Where store() says so: use(row, column, cell of the first plane) of the share's numbers that are not finite
+    template <typename T, typename Use>
+    static __device__ __forceinline__ void each_bad(__nv_bfloat16* tile, int piece, Use use) {
+#pragma unroll 1
+        for (int x = 0; x < 8 * kUnits; ++x) {
+            const int r = threadIdx.x / kPieces + (x >> 3) * (THREADS / kPieces), at = threadIdx.x % kPieces;
+            __nv_bfloat16* cell = tile + T::at(r, piece + at) + (x & 7);
+            if (!(fabsf(__bfloat162float(*cell)) <= FLT_MAX)) use(r, at * 8 + (x & 7), cell);
+        }
+    }
+    // the same: they give way to zeros in the tile and are noted. The share is tokens from `token` on, columns from `column`.
+    template <typename T>
+    static __device__ __forceinline__ void take_out(__nv_bfloat16* tile, int piece, BadTokens& bad, int token, int column) {
+        each_bad<T>(tile, piece, [&](int r, int c, __nv_bfloat16* cell) {
+            bad.note(column + c, token + r);
+            for (int n = 0; n < 3; ++n) cell[n * T::kPlane] = __float2bfloat16_rn(0.0f);
+        });
     }
 };
 // The same share by way of shared memory, where a thread finds its own pieces again: copied asynchronously, read back later.
@@ -653,10 +709,12 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
     using STile = SplitTile<kReadRows, kReadColumns>;
     extern __shared__ __align__(128) __nv_bfloat16 tiles[];
     __shared__ ReadGates<MODE> gates_s[2];
+    __shared__ BadTokens bad;
     chain_release();
     chain_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
     const int chunk = blockIdx.y;
+    bad.clear();
     int begin, count;
     chunk_tokens_of(p, chunk, begin, count);
     if (count <= 0) return;
@@ -872,7 +930,7 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
             for (int part = 0; part < 2; ++part, ++j, turn ^= 1) {                 // the chunk's own tokens, 32 at a time
                 __nv_bfloat16* v_t = buffers + turn * STile::kElements;
                 take(j);
-                next.template store<STile>(v_t, 0, Unscaled());
+                if (!next.template store<STile>(v_t, 0, Unscaled())) next.template take_out<STile>(v_t, 0, bad, part * kReadRows, 0);
                 ask(j + kReadAhead<WIDTH>);
                 __syncthreads();
 #pragma unroll
@@ -907,6 +965,11 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
                     }
                 }
             }
+            }
+            if (bad.any) {                                   // (the same for all threads: it is written before the next barrier only)
+                bad.mark(acc, row0, 2 * tig);
+                __syncthreads();
+                bad.clear();
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {

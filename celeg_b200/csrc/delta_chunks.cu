@@ -109,6 +109,15 @@ __device__ __forceinline__ void invert(const float* lower, float* inverse) {
     __syncthreads();
 }
 
+// a warp's rows t, t + 8 of W: NaN from `good` on
+__device__ __forceinline__ void leave_out(float (&acc)[8][4], int t, int good) {
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (t + 8 * (r >> 1) >= good) acc[n][r] = NAN;
+}
+
 template <int WIDTH>
 __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 4 : 2) delta_solve_kernel(const DeltaChunkArgs p) {
     using Tile = SplitTile<kChunk, WIDTH>;
@@ -117,9 +126,13 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 4 : 2) delta_solv
     extern __shared__ __align__(128) __nv_bfloat16 tiles[];
     __shared__ float2 cum_s[kChunk];
     __shared__ float beta_s[kChunk], start_s[kChunk], end_s[kChunk];
+    __shared__ BadTokens v_bad;
+    __shared__ int k_bad;                                    // the first token with a key, rate or decay that is not finite
     chain_release();
     chain_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
+    v_bad.clear();
+    if (tid == 0) k_bad = kChunk;
     const int chunk = blockIdx.y, head = blockIdx.x, dim = p.dim, vdim = p.vdim;
     const int begin = p.chunk_begin[chunk], count = p.chunk_begin[chunk + 1] - begin;
     if (count <= 0) return;
@@ -139,6 +152,7 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 4 : 2) delta_solv
         end_s[tid] = exp_between(p.cum[(size_t)(begin + count - 1) * p.heads + head], own);
     }
     __syncthreads();
+    if (tid < kChunk && !(fabsf(beta_s[tid]) <= FLT_MAX && fabsf(cum_s[tid].x) <= FLT_MAX)) atomicMin(&k_bad, tid);
     const size_t at = ((size_t)chunk * p.heads + head) * 2;
     __nv_bfloat16* w_out = p.operands + at * Tile::kElements;
     __nv_bfloat16* k_out = w_out + Tile::kElements;
@@ -147,10 +161,14 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 4 : 2) delta_solv
 #pragma unroll 1
     for (int e = 0; e < WIDTH; e += 32) {
         share.load(k_src + e, p.k_stride, count, dim - e, k_four);
-        share.template store<Tile>(k_t, e >> 3, Unscaled());
+        const bool finite = share.template store<Tile>(k_t, e >> 3, Unscaled());
         share.template store<Tile>(k_out, e >> 3, [&](int r) { return end_s[r]; });      // G(n, j) k_j: what S is given of u_j
+        if (!finite) Part::each_bad<Tile>(k_t, e >> 3, [&](int r, int, __nv_bfloat16*) { atomicMin(&k_bad, r); });
     }
     __syncthreads();
+    // The rows of the system from the first bad token on are left out (the tokens before it meet them under weights of zero:
+    // chunk_scan.cuh); their W is NaN in the end, and with it their u.
+    const int good = min(count, k_bad);
     {
         float raw[8][4] = {};                                // k.k: the warp's 16 tokens against 8 n + 2 tig, + 1
 #pragma unroll 2
@@ -171,7 +189,7 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 4 : 2) delta_solv
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int i = 16 * warp + g + 8 * (r >> 1), j = 8 * n + 2 * tig + (r & 1);
-                lower[i * kSolvePitch + j] = j < i && i < count ? raw[n][r] * beta_s[i] * exp_between(cum_s[i], cum_s[j]) : 0.0f;
+                lower[i * kSolvePitch + j] = j < i && i < good ? raw[n][r] * beta_s[i] * exp_between(cum_s[i], cum_s[j]) : 0.0f;
             }
     }
     __syncthreads();                                         // k has been used
@@ -188,8 +206,8 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 4 : 2) delta_solv
     __syncthreads();
 #pragma unroll 1
     for (int e = 0; e < WIDTH; e += 32) {                    // the right sides beta G k
-        share.load(k_src + e, p.k_stride, count, dim - e, k_four);
-        share.template store<Tile>(k_t, e >> 3, [&](int r) { return beta_s[r] * start_s[r]; });
+        share.load(k_src + e, p.k_stride, good, dim - e, k_four);
+        share.template store<Tile>(k_t, e >> 3, [&](int r) { return r < good ? beta_s[r] * start_s[r] : 0.0f; });
     }
     float acc[8][4];
     auto multiply = [&](auto tile, const __nv_bfloat16* from, int n0) {        // T times 64 columns from n0 on
@@ -216,6 +234,7 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 4 : 2) delta_solv
 #pragma unroll 1
     for (int e = 0; e < WIDTH; e += 64) {                    // -W = -T beta G k
         multiply(Tile(), k_t, e);
+        if (good < count) leave_out(acc, 16 * warp + g, good);
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
@@ -231,11 +250,17 @@ __global__ void __launch_bounds__(kSolveThreads, WIDTH == 64 ? 4 : 2) delta_solv
         __syncthreads();
 #pragma unroll 1
         for (int c = 0; c < 64; c += 32) {
-            share.load(v_src + c0 + c, p.v_stride, count, vdim - c0 - c, v_four);
-            share.template store<VTile>(k_t, c >> 3, [&](int r) { return beta_s[r]; });
+            share.load(v_src + c0 + c, p.v_stride, good, vdim - c0 - c, v_four);
+            if (!share.template store<VTile>(k_t, c >> 3, [&](int r) { return r < good ? beta_s[r] : 0.0f; }))
+                Part::take_out<VTile>(k_t, c >> 3, v_bad, 0, c);
         }
         __syncthreads();
         multiply(VTile(), k_t, 0);
+        if (v_bad.any) {                                     // (the same for all threads)
+            v_bad.mark(acc, 16 * warp + g, 2 * tig);
+            __syncthreads();
+            v_bad.clear();
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int t = 16 * warp + g + 8 * h;
@@ -523,10 +548,14 @@ __global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const
     constexpr int kUnits = Share::kUnits, kRows = kGeneralThreads / Share::kPieces;
     extern __shared__ __align__(128) __nv_bfloat16 tiles[];
     __shared__ float last_s[4][64];
+    __shared__ BadTokens v_bad;
+    __shared__ int k_bad;                                    // the first token with a key, removal or decay that is not finite
     chain_release();
     chain_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
     const int chunk = blockIdx.y, head = blockIdx.x, dim = p.dim;
+    v_bad.clear();
+    if (tid == 0) k_bad = kChunk;
     const int begin = p.chunk_begin[chunk], count = p.chunk_begin[chunk + 1] - begin;
     if (count <= 0) return;
     __nv_bfloat16* u_t = tiles;                              // at first P, then u^
@@ -612,7 +641,7 @@ __global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const
 #pragma unroll
     for (int n = 0; n < kUnits; ++n) {
         const int t = tid / Share::kPieces + n * kRows;
-        float u[8], r[8], kk[8], b[8], out[8];
+        float u[8], r[8], kk[8], b[8], out[8], none = 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int c = c0 + j;
@@ -624,8 +653,14 @@ __global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const
             kk[j] = k.x[n][j] * back;
             b[j] = here ? sigmoid_of(a.x[n][j] + bias) * unit * back : 0.0f;
             out[j] = -b[j] * whole[j];
+            none = fmaf(u[j], 0.0f, fmaf(b[j], 0.0f, none));
             if (here) p.r_out[(size_t)(begin + t) * inner + at_head + c] = r[j];
             if (t == 0 && c < dim) p.total[(size_t)chunk * inner + at_head + c] = whole[j];
+        }
+        if (none != 0.0f) {                                  // (NaN: the token's key, removal or decay is not finite)
+            atomicMin(&k_bad, t);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) u[j] = 0.0f;
         }
         put(u_t, t, u);
         put(r_t, t, r);
@@ -634,6 +669,7 @@ __global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const
         put(b_out, t, out);
     }
     __syncthreads();
+    const int good = min(count, k_bad);                      // (what is left out, and why: delta_solve_kernel)
     // products: warps 0-3 r^.k^ and u^.k^, warps 4-7 r^.b^ and u^.b^, 16 tokens each
     const int w4 = warp & 3;
     const bool of_b = warp >= 4;
@@ -673,7 +709,7 @@ __global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const
     product(u_t);
     __syncthreads();                                         // r^ has been used
     load(x, p.v_off);
-    x.template store<Tile>(r_t, 0, Unscaled());
+    if (!x.template store<Tile>(r_t, 0, Unscaled())) Share::take_out<Tile>(r_t, 0, v_bad, 0, 0);
     __syncthreads();
     if (!of_b) {                                             // (u^ . k^) v
         float y[8][4] = {};
@@ -684,7 +720,8 @@ __global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int n = 2 * m + (q >> 1), i = 16 * w4 + g + 8 * (q & 1), j = 8 * n + 2 * tig;
-                split_pair(j < i ? acc[n][2 * (q & 1)] : 0.0f, j + 1 < i ? acc[n][2 * (q & 1) + 1] : 0.0f, l[0][q], l[1][q], l[2][q]);
+                split_pair(j < i && i < good ? acc[n][2 * (q & 1)] : 0.0f, j + 1 < i && i < good ? acc[n][2 * (q & 1) + 1] : 0.0f, l[0][q], l[1][q],
+                           l[2][q]);
             }
 #pragma unroll
             for (int n = 0; n < 4; n += 2) {
@@ -718,6 +755,13 @@ __global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const
                 mma_split<4>(y + 2 * n, l, b);
             }
         }
+        if (v_bad.any) {                                     // (every row of a column with a bad value)
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    if (v_bad.first[8 * n + 2 * tig + (r & 1)] < kChunk) y[n][r] = NAN;
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int e = 16 * w4 + g + 8 * h;
@@ -738,7 +782,7 @@ __global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int i = 16 * w4 + g + 8 * (r >> 1), j = 8 * n + 2 * tig + (r & 1);
-                lower[i * kSolvePitch + j] = j < i ? acc[n][r] : 0.0f;
+                lower[i * kSolvePitch + j] = j < i && i < good ? acc[n][r] : 0.0f;
             }
     } else {
         for (int i = tid; i < kChunk * kSolvePitch; i += 128) inverse[i] = 0.0f;
@@ -771,6 +815,9 @@ __global__ void __launch_bounds__(kGeneralThreads, 2) general_solve_kernel(const
             mma_split<4>(acc + 2 * n, l, b);
         }
     }
+    // (s of a token is of the state before it: NaN behind the first bad value)
+    if (of_b && v_bad.any) v_bad.mark(acc, 16 * w4 + g, 2 * tig, 1);
+    if (!of_b && good < count) leave_out(acc, 16 * w4 + g, good);
 #pragma unroll
     for (int n = 0; n < 8; ++n)
 #pragma unroll
