@@ -52,6 +52,12 @@ __global__ void chunk_plan_kernel(const int* span_begin, int spans, int chunk, i
 }
 
 // ------------------------------------------------------------------------------------------------- prepare, scalar
+// A decay's logarithm, a product of floats. Below -104 the decay is zero in float32 however far below, and a sum with -1e30 in
+// it has lost the tokens behind it (with an infinity in it, everything: inf - inf).
+__device__ __forceinline__ double decay_log(float rate, float step) {
+    const float x = -rate * step;
+    return x < -1e4f ? -1e4f : x;                                // (a NaN stays one)
+}
 // cum[t, h]: the sum of the decays' logarithms from the chunk's first token through t, a float and what it leaves of the double
 // that is summed in; dt[t, h]. A block takes 8 heads of a chunk: a warp a head, two neighbouring tokens a lane, the running
 // sum by shuffles.
@@ -73,7 +79,7 @@ __global__ void __launch_bounds__(256) scalar_decay_kernel(const float* raw, int
     if (h0 + warp < heads) {
         const float rate = expf(a_log[h0 + warp]), b = bias[h0 + warp];
         const float first = softplus_of(raw_s[2 * lane][warp] + b), second = softplus_of(raw_s[2 * lane + 1][warp] + b);
-        const double x = -rate * first, y = -rate * second;      // (products of floats)
+        const double x = decay_log(rate, first), y = decay_log(rate, second);
         double sum = x + y;
 #pragma unroll
         for (int offset = 1; offset < 32; offset <<= 1) {

@@ -1,4 +1,4 @@
-"""What a NaN in one token's rows does in the chunked scans (csrc/chunk_scan.cuh, csrc/delta_chunks.cu): the tokens before it,
+"""Decays of zero, and what a NaN in one token's rows does, in the chunked scans (csrc/chunk_scan.cuh, csrc/delta_chunks.cu): the tokens before it,
 other heads, other requests and, for a value, other columns are bit for bit what they are without it; the head's (or the
 column's) read-outs from that token on and the state afterwards are NaN, as token by token."""
 from __future__ import annotations
@@ -100,3 +100,36 @@ def test_a_nan_reaches_its_own_token_and_those_behind_it(kind, what, at):
     assert bool(same.all()), (~same).nonzero()[:8].tolist()
     same = (got_state == expected_state) | (got_state.isnan() & expected_state.isnan())
     assert bool(same.all()), (~same).nonzero()[:8].tolist()
+
+
+@pytest.mark.parametrize("rate,step", [(85.0, 0.0), (100.0, 0.0), (0.0, 3e30), (0.0, float("inf")), (30.0, 1e20)])
+def test_a_decay_of_zero_leaves_the_decays_behind_it_alone(rate, step):
+    """exp(-exp(a_log) softplus(.)) with logarithms from -1e13 to minus infinity, at some tokens or at all of them: the old state
+    is gone there, and what follows decays as it does without them."""
+    from celeg_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(19)
+    rand = lambda columns: torch.randn(TOKENS, columns, device="cuda", generator=g)      # noqa: E731
+    q, v, pre_a, dim, vdim = rand(HEADS * DIM), rand(HEADS * 24), rand(HEADS), DIM, 24
+    k = torch.nn.functional.normalize(rand(HEADS * DIM).view(TOKENS, HEADS, DIM), dim=-1).view(TOKENS, -1)
+    if step:
+        pre_a[[3, 70, 71, 150], 1] = step
+    a_log, dt_bias = torch.tensor([-2.0, rate], device="cuda"), torch.zeros(HEADS, device="cuda")
+    decay = torch.exp(-torch.exp(a_log) * torch.nn.functional.softplus(pre_a, threshold=30.0))
+    gates = torch.cat([torch.sigmoid(rand(HEADS)), decay], dim=1).contiguous()
+    assert bool(gates.isfinite().all()) and float(decay.min()) == 0.0
+    begins, slots, flag = i32(BEGINS), i32([2, 0, 1]), i32([0])
+    before = torch.full((SPANS, HEADS * dim * vdim), 0.25, device="cuda")
+    want, want_state = full(TOKENS, HEADS * vdim), before.clone()
+    kernels.recurrent_scan(kernels.SCAN_DELTA, q, k, v, gates, want, want_state, before.stride(0), begins, slots, SPANS, HEADS, HEADS,
+                           dim, vdim, 0.2)
+    plan = torch.zeros(2 * (CHUNKS + 3) + 16, dtype=torch.int32, device="cuda")
+    kernels.chunk_plan(begins, SPANS, CHUNKS + 3, plan)
+    got, got_state = full(TOKENS, HEADS * vdim), before.clone()
+    kernels.delta_chunk_scan(q, k, v, gates, pre_a, dt_bias, a_log, full(TOKENS, 2 * HEADS), full(TOKENS, HEADS),
+                             full(CHUNKS * HEADS * kernels.delta_operand_bytes(dim) // 4), full(TOKENS, HEADS * vdim),
+                             full(CHUNKS * HEADS * dim * vdim), got, got_state, before.stride(0), slots, plan, CHUNKS + 3, SPANS, CHUNKS,
+                             HEADS, HEADS, dim, vdim, 0.2, flag)
+    assert int(flag.item()) == 0
+    # float32 sums of the same products in two orders, behind decays that differ in their last bits: a few units of 2^-24
+    for a, b in ((got, want), (got_state, want_state)):
+        assert float((a.double() - b.double()).norm() / b.double().norm()) <= 2e-6
