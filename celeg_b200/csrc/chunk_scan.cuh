@@ -41,7 +41,8 @@ enum ChunkMode : int {
     kChunkChannel = 1,     // a decay a token and key channel, taken into q and k beforehand (gated linear attention)
     kChunkConstant = 2,    // a decay a head (retention)
     kChunkStable = 3,      // exponential gates in range of a running maximum, with a normaliser (mLSTM)
-    kChunkPair = 4,        // read-outs alone: as channel, with a second set of values and products (generalised delta rule)
+    kChunkPair = 4,        // read-outs alone: as channel, with a second set of values and products, at most 64 columns and
+                           // key channels (generalised delta rule)
 };
 
 struct ChunkArgs {
@@ -925,7 +926,7 @@ __global__ void __launch_bounds__(kReadThreads, WIDTH == 64 ? 4 : 2) chunk_read_
             }
             float sums[2] = {0.0f, 0.0f};
             for (int pass = 0; pass < passes; ++pass) {
-            if (passes == 2 && (pass == 1 || c0 > c_begin)) load_raw(pass ? p.products_b : p.products);
+            if (passes == 2 && pass == 1) load_raw(p.products_b);          // (one tile of columns: vdim is at most 64)
 #pragma unroll
             for (int part = 0; part < 2; ++part, ++j, turn ^= 1) {                 // the chunk's own tokens, 32 at a time
                 __nv_bfloat16* v_t = buffers + turn * STile::kElements;

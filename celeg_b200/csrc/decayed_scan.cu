@@ -442,10 +442,10 @@ CELEG_API int celeg_channel_decay_scan(const float* q, int q_stride, const float
 }
 
 // The scalar form: q and k have `groups` heads of dim that heads / groups heads of v share; raw: the steps before bias and
-// softplus, head h in column h. Scratch: cum (two floats each), dt [tokens, heads], products [chunks, groups, 64, 64], states as above.
+// softplus, head h in column h. Scratch: cum (two floats each), dt [tokens, heads], states as above.
 CELEG_API int celeg_scalar_decay_scan(const float* q, int q_stride, const float* k, int k_stride, const float* v, int v_stride,
                                       const float* raw, int raw_stride, const float* dt_bias, const float* a_log,
-                                      const float* direct, float2* cum, float* dt, float* products, float* states, float* out,
+                                      const float* direct, float2* cum, float* dt, float* states, float* out,
                                       float* state, long long slot_stride, const int* span_slot, const int* plan,
                                       int max_chunks, int spans, int chunks, int heads, int groups, int dim, int vdim,
                                       cudaStream_t stream) {

@@ -933,5 +933,5 @@ CELEG_API int celeg_general_delta_chunk_scan(const float* proj, int stride, int 
     p.chunk_begin = plan; p.pieces = 1; p.span_first = span_first; p.spans = spans;
     p.states = states; p.out = out;
     p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = dim;
-    return launch_reads<kChunkPair>(p, chunks, stream);
+    return launch_read<kChunkPair, 64>(p, chunks, 1, stream);
 }

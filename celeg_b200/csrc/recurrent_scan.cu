@@ -871,138 +871,7 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Retention over long spans, cut into segments: of up to 128 tokens by the kernels of chunk_scan.cuh, a state every 64 tokens;
-// longer ones, for which the caller's scratch holds no such states, by the kernels here. With a constant decay d the state after token t of a segment
-// that begins at token b is S_t = d^(t-b+1) S_(b-1) + L_t, L_t the state the segment's own tokens would have built
-// from zero. So the segments of all spans are scanned side by side from zero states (the scan kernel above, one
-// "span" a segment), which also gives the segment's final L and the local read-outs L_t^T q_t; the states at the
-// segments' starts follow from one another by S <- d^len S + L (a handful of steps a span, element by element);
-// and the read-outs get d^(t-b+1) S_(b-1)^T q_t added, a small product per segment. Only rounding differs
-// from the token-by-token order.
-// The segments' scan, built for throughput instead of a short chain per token (many segments run side by side, so
-// no single one is waited for): a lane holds 64 consecutive elements of a column of S (the whole column up to a key
-// size of 64; L = 2 or 4 lanes a column beyond), reads a token's key and query as 16-byte broadcasts from shared
-// memory, and k.q is formed once per token for all columns. Per element and token that is a third of the
-// instructions of the kernel above, which spreads a column over eight lanes to keep ONE long span's chain short.
-template <int L>
-__global__ void __launch_bounds__(kScanThreads) retention_wide_scan_kernel(const ScanParams p) {
-    constexpr int kE = 64;
-    constexpr int kColsWarp = 32 / L;
-    constexpr int kCols = kScanWarps * kColsWarp;
-    constexpr int kDimPad = kE * L;
-    constexpr int kTile = L > 2 ? 8 : 16;
-    __shared__ __align__(16) float k_s[2][kTile][kDimPad];
-    __shared__ __align__(16) float q_s[2][kTile][kDimPad];
-    __shared__ float v_s[2][kTile][kCols];
-    __shared__ float kq_s[2][kTile];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int sub = lane % L, col_in = warp * kColsWarp + lane / L;
-    const int head = blockIdx.y, span = blockIdx.z;
-    const int col = blockIdx.x * kCols + col_in;
-    const bool col_ok = col < p.vdim;
-    const int dim = p.dim, vdim = p.vdim;
-    const int t_begin = p.span_begin[span], t_end = p.span_begin[span + 1];
-    if (t_end <= t_begin) return;
-    for (int i = tid; i < 2 * kTile * kDimPad; i += kScanThreads) {      // keys beyond the head's size stay zero
-        (&k_s[0][0][0])[i] = 0.0f;
-        (&q_s[0][0][0])[i] = 0.0f;
-    }
-    for (int i = tid; i < 2 * kTile * kCols; i += kScanThreads) (&v_s[0][0][0])[i] = 0.0f;
-    __syncthreads();
-    float* s_head = p.state + (long long)p.span_slot[span] * p.slot_stride + (size_t)head * dim * vdim;
-    const float decay = p.gates[head];
-    float s[kE];
-#pragma unroll
-    for (int r = 0; r < kE; ++r) {
-        const int e = sub * kE + r;
-        s[r] = (col_ok && e < dim) ? s_head[(size_t)e * vdim + col] : 0.0f;
-    }
-    const float* k_base = p.k + (size_t)head * dim;
-    const float* q_base = p.q + (size_t)head * dim;
-    auto issue = [&](int t0, int stage) {
-        const int count = min(kTile, t_end - t0);
-        if (p.vector_copies) {
-            const int quads = dim >> 2;
-            for (int i = tid; i < count * quads; i += kScanThreads) {
-                const int tt = i / quads, e = (i - tt * quads) << 2;
-                cp_async_16(&k_s[stage][tt][e], k_base + (size_t)(t0 + tt) * p.k_stride + e);
-                cp_async_16(&q_s[stage][tt][e], q_base + (size_t)(t0 + tt) * p.q_stride + e);
-            }
-        } else {
-            for (int i = tid; i < count * dim; i += kScanThreads) {
-                const int tt = i / dim, e = i - tt * dim;
-                cp_async_4(&k_s[stage][tt][e], k_base + (size_t)(t0 + tt) * p.k_stride + e);
-                cp_async_4(&q_s[stage][tt][e], q_base + (size_t)(t0 + tt) * p.q_stride + e);
-            }
-        }
-        for (int i = tid; i < count * kCols; i += kScanThreads) {
-            const int tt = i / kCols, c = i % kCols;
-            const int gc = blockIdx.x * kCols + c;
-            if (gc < vdim) cp_async_4(&v_s[stage][tt][c], p.v + (size_t)(t0 + tt) * p.v_stride + (size_t)head * vdim + gc);
-        }
-        cp_async_commit_group();
-    };
-    issue(t_begin, 0);
-    int stage = 0;
-    for (int t0 = t_begin; t0 < t_end; t0 += kTile, stage ^= 1) {
-        if (t0 + kTile < t_end) {
-            issue(t0 + kTile, stage ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();                                // every thread's copies of this stage have landed
-        const int count = min(kTile, t_end - t0);
-        for (int tt = warp; tt < count; tt += kScanWarps) {            // k.q of the tile's tokens, a warp a token
-            float sum = 0.0f;
-            for (int e = lane; e < kDimPad; e += 32) sum = fmaf(k_s[stage][tt][e], q_s[stage][tt][e], sum);
-            sum = warp_sum(sum);
-            if (lane == 0) kq_s[stage][tt] = sum * p.q_scale;
-        }
-        __syncthreads();
-        for (int tt = 0; tt < count; ++tt) {
-            const float vj = v_s[stage][tt][col_in];
-            const float vs = vj * p.q_scale;
-            const float4* kp = reinterpret_cast<const float4*>(&k_s[stage][tt][sub * kE]);
-            const float4* qp = reinterpret_cast<const float4*>(&q_s[stage][tt][sub * kE]);
-            float sq[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int r4 = 0; r4 < kE / 4; ++r4) {
-                const float4 kv = kp[r4], qv = qp[r4];
-                sq[0] = fmaf(s[4 * r4], qv.x, sq[0]);
-                sq[1] = fmaf(s[4 * r4 + 1], qv.y, sq[1]);
-                sq[2] = fmaf(s[4 * r4 + 2], qv.z, sq[2]);
-                sq[3] = fmaf(s[4 * r4 + 3], qv.w, sq[3]);
-                s[4 * r4] = fmaf(kv.x, vs, decay * s[4 * r4]);
-                s[4 * r4 + 1] = fmaf(kv.y, vs, decay * s[4 * r4 + 1]);
-                s[4 * r4 + 2] = fmaf(kv.z, vs, decay * s[4 * r4 + 2]);
-                s[4 * r4 + 3] = fmaf(kv.w, vs, decay * s[4 * r4 + 3]);
-            }
-            float d_sq = (sq[0] + sq[1]) + (sq[2] + sq[3]);
-#pragma unroll
-            for (int offset = 1; offset < L; offset <<= 1) d_sq += __shfl_xor_sync(0xffffffffu, d_sq, offset);
-            if (sub == 0 && col_ok)
-                p.out[(size_t)(t0 + tt) * p.heads * vdim + (size_t)head * vdim + col] = fmaf(decay, d_sq, vj * kq_s[stage][tt]);
-        }
-        __syncthreads();                                // the stage is free for the tile after the next
-    }
-#pragma unroll
-    for (int r = 0; r < kE; ++r) {
-        const int e = sub * kE + r;
-        if (col_ok && e < dim) s_head[(size_t)e * vdim + col] = s[r];
-    }
-}
-
-static int launch_wide_scan(const ScanParams& p, int spans, cudaStream_t stream) {
-    const int lanes = p.dim <= 64 ? 1 : p.dim <= 128 ? 2 : 4;
-    const int cols = kScanWarps * (32 / lanes);
-    dim3 grid((p.vdim + cols - 1) / cols, p.heads, spans);
-    if (lanes == 1) retention_wide_scan_kernel<1><<<grid, kScanThreads, 0, stream>>>(p);
-    else if (lanes == 2) retention_wide_scan_kernel<2><<<grid, kScanThreads, 0, stream>>>(p);
-    else retention_wide_scan_kernel<4><<<grid, kScanThreads, 0, stream>>>(p);
-    return check_launch("retention_wide_scan");
-}
-
+// Retention over long spans, cut into segments of 64 or 128 tokens for the kernels of chunk_scan.cuh: their plan.
 __global__ void retention_plan_kernel(const int* span_begin, int spans, int segment, int max_segments, int* seg_begin,
                                       int* span_first) {
     chain_release();
@@ -1015,82 +884,6 @@ __global__ void retention_plan_kernel(const int* span_begin, int spans, int segm
     }
     span_first[spans] = n;
     for (int i = n; i <= max_segments; ++i) seg_begin[i] = span_begin[spans];      // (segments beyond the last are empty)
-}
-
-// one thread a state element: the state at every segment's start, and the span's state after its last token
-__global__ void retention_carry_kernel(float* state, long long slot_stride, const int* span_slot, const int* span_first,
-                                       const int* seg_begin, const float* local, float* carried, const float* decay,
-                                       int elements, int head_elements) {
-    chain_release();
-    chain_wait();
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= elements) return;
-    const int span = blockIdx.y;
-    float* cell = state + (long long)span_slot[span] * slot_stride + e;
-    const float d = decay[e / head_elements];
-    float s = *cell;
-    for (int seg = span_first[span]; seg < span_first[span + 1]; ++seg) {
-        carried[(size_t)seg * elements + e] = s;
-        s = fmaf(powf(d, (float)(seg_begin[seg + 1] - seg_begin[seg])), s, local[(size_t)seg * elements + e]);
-    }
-    *cell = s;
-}
-
-// out[t, head, :] += d^(t - b + 1) (carried[segment of t][head]^T q_t): 64 tokens x 64 columns a block, FFMA
-__global__ void __launch_bounds__(256) retention_add_carried_kernel(const float* q, int q_stride, const float* carried,
-                                                                    const int* seg_begin, const float* decay, float* out,
-                                                                    int heads, int dim, int vdim, int pieces) {
-    __shared__ float qs[16][64 + 4];
-    __shared__ float ss[16][64 + 4];
-    chain_release();
-    chain_wait();
-    const int seg = blockIdx.z / pieces, piece = blockIdx.z % pieces;
-    const int head = blockIdx.y, col0 = blockIdx.x * 64;
-    const int begin = seg_begin[seg], end = seg_begin[seg + 1];
-    const int t0 = begin + piece * 64;
-    if (t0 >= end) return;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const float* state = carried + ((size_t)seg * heads + head) * dim * vdim;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < dim; k0 += 16) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int idx = threadIdx.x + i * 256;
-            const int r = idx >> 4, kk = idx & 15;            // queries: 16 k of a token are neighbours
-            qs[kk][r] = (t0 + r < end && k0 + kk < dim) ? q[(size_t)(t0 + r) * q_stride + (size_t)head * dim + k0 + kk] : 0.0f;
-            const int c = idx & 63, kr = idx >> 6;            // state rows: 64 columns of a k are neighbours
-            ss[kr][c] = (col0 + c < vdim && k0 + kr < dim) ? state[(size_t)(k0 + kr) * vdim + col0 + c] : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = qs[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = ss[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-    const float d = decay[head];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = t0 + ty * 4 + i;
-        if (t >= end) continue;
-        const float factor = powf(d, (float)(t - begin + 1));
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = col0 + tx * 4 + j;
-            if (c < vdim) {
-                float* cell = out + (size_t)t * heads * vdim + (size_t)head * vdim + c;
-                *cell = fmaf(factor, acc[i][j], *cell);
-            }
-        }
-    }
 }
 
 template <int MODE>
@@ -1322,18 +1115,16 @@ CELEG_API int celeg_retention_decode_raw(const float* proj, int stride, int q_of
                                    heads, heads, dim, vdim, q_scale, raw_out, kFloat32, input_act, raw_out, stream);
 }
 
-// Retention over the step's spans in segments of `segment` tokens (a multiple of 64). Scratch: floats
-// [2 * max_segments * heads * dim * vdim] (the segments' own states, then the states at their starts), ints
-// [max_segments + spans + 2] (segment starts, the spans' first segments), with max_segments >= tokens / segment +
-// spans; identity: the numbers 0 .. max_segments - 1. decay: [heads]. Same result as mode 2 of celeg_recurrent_scan
-// but for rounding.
+// Retention over the step's spans in segments of `segment` tokens, 64 or 128: what a segment's tokens leave in the state does
+// not depend on what was carried into it, as the decay is a constant. Scratch: floats [2 * max_segments * heads * dim * vdim] (a
+// state every 64 tokens), ints [max_segments + spans + 2] (segment starts, the spans' first segments), with max_segments >=
+// tokens / segment + spans. decay: [heads]. Same result as mode 2 of celeg_recurrent_scan but for rounding.
 CELEG_API int celeg_retention_segmented(const float* q, int q_stride, const float* k, int k_stride, const float* v,
                                         int v_stride, const float* decay, float* out, float* state, long long slot_stride,
                                         const int* span_begin, const int* span_slot, int spans, int tokens, int heads,
                                         int dim, int vdim, float q_scale, int segment, int max_segments,
-                                        float* float_scratch, int* int_scratch, const int* identity,
-                                        cudaStream_t stream) {
-    CELEG_REQUIRE(spans >= 0 && tokens >= 0 && heads > 0 && dim > 0 && vdim > 0 && segment >= 64 && segment % 64 == 0,
+                                        float* float_scratch, int* int_scratch, cudaStream_t stream) {
+    CELEG_REQUIRE(spans >= 0 && tokens >= 0 && heads > 0 && dim > 0 && vdim > 0 && (segment == 64 || segment == 128),
                   "retention_segmented: invalid sizes spans=%d tokens=%d heads=%d dim=%d vdim=%d segment=%d", spans, tokens,
                   heads, dim, vdim, segment);
     CELEG_REQUIRE(dim <= kScanMaxDim, "retention_segmented: a key size of %d exceeds %d", dim, kScanMaxDim);
@@ -1347,35 +1138,15 @@ CELEG_API int celeg_retention_segmented(const float* q, int q_stride, const floa
     CELEG_REQUIRE((long long)max_segments * pieces <= 65535, "retention_segmented: %d segments of %d pieces exceed one launch",
                   max_segments, pieces);
     launch_chained(retention_plan_kernel, 1, 32, 0, stream, span_begin, spans, segment, max_segments, seg_begin, span_first);
-    int status = check_launch("retention_plan");
+    const int status = check_launch("retention_plan");
     if (status != 0) return status;
-    if (pieces <= 2) {         // the scratch holds a state for every 64 tokens
-        ChunkArgs p = {};
-        p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = v; p.v_stride = v_stride;
-        p.decay = decay; p.q_scale = q_scale;
-        p.chunk_begin = seg_begin; p.pieces = pieces; p.span_first = span_first; p.spans = spans;
-        p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = float_scratch; p.out = out;
-        p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = vdim;
-        return launch_chunk_scan<kChunkConstant>(p, max_segments * pieces, stream);
-    }
-    const long long elements = (long long)heads * dim * vdim;
-    float* local = float_scratch;
-    float* carried = float_scratch + (size_t)max_segments * elements;
-    cudaMemsetAsync(local, 0, (size_t)max_segments * elements * sizeof(float), stream);
-    const int vector_copies = dim % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && (((size_t)q | (size_t)k) & 15) == 0;
-    const ScanParams p = {q, k, v, q_stride, k_stride, v_stride, decay, out, local, elements, seg_begin, identity,
-                          heads, heads, dim, vdim, q_scale, vector_copies};
-    status = launch_wide_scan(p, max_segments, stream);
-    if (status != 0) return status;
-    dim3 carry_grid((unsigned)((elements + 255) / 256), spans);
-    retention_carry_kernel<<<carry_grid, 256, 0, stream>>>(state, slot_stride, span_slot, span_first, seg_begin, local,
-                                                            carried, decay, (int)elements, dim * vdim);
-    status = check_launch("retention_carry");
-    if (status != 0) return status;
-    dim3 add_grid((vdim + 63) / 64, heads, max_segments * pieces);
-    retention_add_carried_kernel<<<add_grid, 256, 0, stream>>>(q, q_stride, carried, seg_begin, decay, out, heads, dim, vdim,
-                                                                pieces);
-    return check_launch("retention_add_carried");
+    ChunkArgs p = {};
+    p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = v; p.v_stride = v_stride;
+    p.decay = decay; p.q_scale = q_scale;
+    p.chunk_begin = seg_begin; p.pieces = pieces; p.span_first = span_first; p.spans = spans;
+    p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = float_scratch; p.out = out;
+    p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = vdim;
+    return launch_chunk_scan<kChunkConstant>(p, max_segments * pieces, stream);
 }
 
 // The mLSTM over the step's spans in chunks of 64 tokens, from the projection's rows to the read-outs. plan: of

@@ -149,7 +149,7 @@ _SIGNATURES = {
                               c_int, c_void_p],
     "celeg_retention_segmented": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_longlong,
                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
-                                  c_void_p, c_void_p, c_void_p],
+                                  c_void_p, c_void_p],
     "celeg_depth_average": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p,
                             c_float, c_int, c_int, c_int, c_void_p],
     "celeg_latent_prepare": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, c_void_p, c_void_p,
@@ -191,7 +191,7 @@ _SIGNATURES = {
                                c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
                                c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
     "celeg_scalar_decay_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p,
+                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "celeg_channel_decay_decode": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_int,
                                    c_void_p, c_float, c_void_p, c_float, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int,
@@ -1011,22 +1011,27 @@ def mlstm_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, pre_i: t
 def retention_segmented(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
                         state: torch.Tensor, slot_stride: int, span_begin: torch.Tensor, span_slot: torch.Tensor, spans: int,
                         tokens: int, heads: int, dim: int, vdim: int, q_scale: float, segment: int, max_segments: int,
-                        float_scratch: torch.Tensor, int_scratch: torch.Tensor, identity: torch.Tensor) -> None:
+                        float_scratch: torch.Tensor, int_scratch: torch.Tensor,
+                        identity: Optional[torch.Tensor] = None) -> None:
     """The retention (mode SCAN_RETENTION of :func:`recurrent_scan`) with every span cut into segments of ``segment``
-    tokens that are scanned side by side, the states at their starts carried from one to the next, and the carried
-    share added to the read-outs (csrc/recurrent_scan.cu). Scratch: float32 [2 * max_segments * heads * dim * vdim],
-    int32 [max_segments + spans + 2], ``identity`` = arange(max_segments) int32."""
+    tokens, 64 or 128, that are worked on side by side (csrc/chunk_scan.cuh). Scratch: float32 [2 * max_segments * heads * dim *
+    vdim], a state every 64 tokens, int32 [max_segments + spans + 2]. Longer segments (a multiple of 64), for which that
+    scratch is too small, are scanned token by token. ``identity`` is not read."""
     for tensor in (q, k, v, decay, out, state, float_scratch):
         assert tensor.dtype == torch.float32 and tensor.stride(-1) == 1
     assert out.is_contiguous() and out.shape[1] == heads * vdim and decay.shape == (heads,)
-    assert max_segments >= tokens // segment + spans and identity.numel() >= max_segments
+    assert max_segments >= tokens // segment + spans
     assert float_scratch.numel() >= 2 * max_segments * heads * dim * vdim and int_scratch.numel() >= max_segments + spans + 2
+    if segment > 128 and segment % 64 == 0:
+        recurrent_scan(SCAN_RETENTION, q, k, v, decay, out, state, slot_stride, span_begin, span_slot, spans, heads, heads, dim,
+                       vdim, q_scale)
+        return
     _check(library().celeg_retention_segmented(_ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay),
                                                _ptr(out), _ptr(state), slot_stride, _ptr(span_begin), _ptr(span_slot), spans,
                                                tokens, heads, dim, vdim, q_scale, segment, max_segments,
-                                               _ptr(float_scratch), _ptr(int_scratch), _ptr(identity), _stream()))
+                                               _ptr(float_scratch), _ptr(int_scratch), _stream()))
     global LAUNCHES
-    LAUNCHES += 2 if segment <= 128 else 3     # the plan, the states, the read-outs; or scan, carried states and their share
+    LAUNCHES += 2          # (a call counts one) the plan, the states (one launch at least), the read-outs
 
 
 def recurrent_decode(mode: int, proj: torch.Tensor, offsets: Tuple[int, int, int, int, int, int],
@@ -1476,20 +1481,19 @@ def channel_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: tor
 
 def scalar_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: torch.Tensor, dt_bias: torch.Tensor,
                       a_log: torch.Tensor, direct: Optional[torch.Tensor], cum: torch.Tensor, dt: torch.Tensor,
-                      products: torch.Tensor, states: torch.Tensor, out: torch.Tensor, state: torch.Tensor, slot_stride: int,
-                      span_slot: torch.Tensor, plan: torch.Tensor, max_chunks: int, spans: int, chunks: int, heads: int,
-                      groups: int, dim: int, vdim: int) -> None:
+                      products: Optional[torch.Tensor], states: torch.Tensor, out: torch.Tensor, state: torch.Tensor,
+                      slot_stride: int, span_slot: torch.Tensor, plan: torch.Tensor, max_chunks: int, spans: int, chunks: int,
+                      heads: int, groups: int, dim: int, vdim: int) -> None:
     """S <- exp(-exp(a_log) dt) S + dt k v^T, o = S^T q + direct v with dt = softplus(raw + dt_bias) along the step's spans;
     heads / groups heads share queries and keys (csrc/decayed_scan.cu). Scratch: ``cum`` [tokens, 2 heads], ``dt`` [tokens,
-    heads]."""
+    heads]. ``products`` is not read."""
     assert cum.is_contiguous() and cum.shape[1] == 2 * heads and dt.is_contiguous() and dt.shape[1] == heads
-    for tensor in (q, k, v, raw, dt_bias, a_log, cum, dt, products, states, out, state):
+    for tensor in (q, k, v, raw, dt_bias, a_log, cum, dt, states, out, state):
         assert tensor.dtype == torch.float32 and tensor.stride(-1) == 1
     assert out.is_contiguous() and out.shape[1] == heads * vdim and states.numel() >= chunks * heads * dim * vdim
-    assert products.numel() >= chunks * groups * 4096
     _check(library().celeg_scalar_decay_scan(
         _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(raw), raw.stride(0), _ptr(dt_bias), _ptr(a_log),
-        _ptr(direct), _ptr(cum), _ptr(dt), _ptr(products), _ptr(states), _ptr(out), _ptr(state), slot_stride, _ptr(span_slot),
+        _ptr(direct), _ptr(cum), _ptr(dt), _ptr(states), _ptr(out), _ptr(state), slot_stride, _ptr(span_slot),
         _ptr(plan), max_chunks, spans, chunks, heads, groups, dim, vdim, _stream()))
     global LAUNCHES
     LAUNCHES += 2          # the decays, then as above

@@ -103,7 +103,6 @@ class Mamba2Mixer:
         self.convolved = rt.scratch("recurrent.conv", self.channels, torch.float32)
         self.cum = rt.scratch("decay.cum", 2 * self.heads, torch.float32)
         self.dt = rt.scratch("decay.dt", self.heads, torch.float32)
-        self.products = rt.flat_scratch("decay.products", chunks * self.groups * self.spans.tokens ** 2, torch.float32)
         self.states = rt.flat_scratch("decay.states", chunks * self.state_elements, torch.float32)
         self.read = rt.scratch("recurrent.read", inner, torch.float32)
         self.gated = rt.scratch("recurrent.gated", inner)
@@ -137,7 +136,7 @@ class Mamba2Mixer:
                                         step.span_slot, single, self.heads, self.groups, self.state, self.vdim, self.read)
         if single < t:
             plan, spans, chunks = self.spans.of(step, single)
-            kernels.scalar_decay_scan(q, k, v, raw, self.dt_bias, self.a_log, self.direct, self.cum, self.dt, self.products,
+            kernels.scalar_decay_scan(q, k, v, raw, self.dt_bias, self.a_log, self.direct, self.cum, self.dt, None,
                                       self.states, self.read, b.state, b.slot_stride, step.span_slot[single:], plan,
                                       self.spans.max_chunks, spans, chunks, self.heads, self.groups, self.state, self.vdim)
         kernels.gated_head_norm(self.read, rows[:, :inner], self.norm, True, self.gated, t, self.norm_groups,

@@ -277,7 +277,6 @@ class RetentionMixer:
         elements = self.heads * self.dim * self.vdim
         self.segment_states = rt.flat_scratch("retention.segments", 2 * self.max_segments * elements, torch.float32)
         self.segment_plan = rt.flat_scratch("retention.plan", 2 * self.max_segments + 8, torch.int32, zero=True)
-        self.segment_numbers = torch.arange(self.max_segments, dtype=torch.int32, device=rt.device)
 
     SEGMENT = 128               # tokens a segment
     # Steps of at least this many tokens are scanned in segments. Measured for one portion at 16 heads of 64 x 128, the mixer
@@ -302,7 +301,7 @@ class RetentionMixer:
             # (span_begin counts the step's tokens: the rows stay where they are)
             kernels.retention_segmented(q, k, v, self.decay, self.read, b.state, b.slot_stride, step.span_begin[single:],
                                         step.span_slot[single:], spans, t - single, self.heads, self.dim, self.vdim, scale,
-                                        self.SEGMENT, segments, self.segment_states, self.segment_plan, self.segment_numbers)
+                                        self.SEGMENT, segments, self.segment_states, self.segment_plan)
 
     def cache_need(self):
         return StateNeed(elements=self.heads * self.dim * self.vdim)
