@@ -375,7 +375,9 @@ class StepFunction:
                 or single_rows - singles > PADDING_TOKENS - PROMPT_TOKEN_STEP
                 or spare > spare_room):
             return None
-        key = ("padded prompt", single_rows, len(portions), padded_tokens, logit_rows, _context_bucket(max_ctx))
+        # (parts whose launches follow from the portions' lengths: their choices are part of the shape)
+        routes = self.rt.portion_routes(portions + [spare] if spare else portions)
+        key = ("padded prompt", single_rows, len(portions), padded_tokens, logit_rows, _context_bucket(max_ctx)) + routes
         if key not in self._graphs:
             if len(self._prompt_seen) > 4096:
                 self._prompt_seen.clear()

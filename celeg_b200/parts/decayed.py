@@ -27,24 +27,33 @@ from .runtime import Runtime, StepContext
 
 class ChunkedSpans:
     """The chunks that a step's portions are cut into: how many at most, and their plan on the device, which the first mixer
-    of a run makes for all of them."""
+    of a run makes for all of them. ``tokens_a_chunk``: the mixer cuts only steps that bring at least so many tokens a chunk
+    (:class:`~.recurrent.PortionsInChunks`); without it any step is cut whose chunks the scratch holds."""
 
-    def __init__(self, rt: Runtime):
+    LEAST_TOKENS_A_CHUNK = 20
+
+    def __init__(self, rt: Runtime, tokens_a_chunk: Optional[int] = None):
         self.tokens = kernels.chunk_tokens()
-        self.max_chunks = rt.max_tokens // self.tokens + rt.max_requests + 48
+        self.tokens_a_chunk = tokens_a_chunk
+        # (of the plan; mixers with different needs share one, and size their scratch by `chunks_held`)
+        self.max_chunks = (rt.max_tokens // self.tokens + rt.max_requests + 48 if tokens_a_chunk is None else
+                           max(1, rt.max_tokens // self.LEAST_TOKENS_A_CHUNK))
+        self.chunks_held = self.max_chunks if tokens_a_chunk is None else max(1, rt.max_tokens // tokens_a_chunk)
         self.plan = rt.flat_scratch("decay.plan", 2 * self.max_chunks + rt.max_tokens + 64, torch.int32)
 
     def fits(self, step: StepContext, single: int) -> bool:
         """Whether the scratch holds the chunks of the spans from ``single`` on."""
-        return (step.tokens - single) // self.tokens + step.spans - single <= self.max_chunks
+        return (step.tokens - single) // self.tokens + step.spans - single <= self.chunks_held
 
     def of(self, step: StepContext, single: int):
         """(plan, spans, bound of the chunks) of the spans from ``single`` on."""
         spans = step.spans - single
         chunks = (step.tokens - single) // self.tokens + spans
-        if chunks > self.max_chunks:
-            raise ValueError(f"{chunks} chunks of a step exceed the {self.max_chunks} that the scratch holds")
-        key = ("decay.plan", single)
+        if self.tokens_a_chunk is not None:
+            chunks = min(chunks, (step.tokens - single) // self.tokens_a_chunk)
+        if chunks > self.chunks_held:
+            raise ValueError(f"{chunks} chunks of a step exceed the {self.chunks_held} that the scratch holds")
+        key = ("decay.plan", single, self.max_chunks)
         if key not in step.extras:
             kernels.chunk_plan(step.span_begin[single:], spans, self.max_chunks, self.plan)
             step.extras[key] = True

@@ -30,8 +30,46 @@ from .registry import register_part
 from .runtime import Runtime, StepContext
 
 
+class PortionsInChunks:
+    """The rule by which a step's portions (what lies behind its leading single tokens) are scanned in chunks of 64 tokens
+    instead of token by token (the generalised delta rule: in chunks of eight).
+
+    Token by token a step takes as long as its longest portion's chain of tokens, or as all its tokens take on the GPU's lanes.
+    In chunks it takes a 64th of the steps, each many times the work, and a chunk that is mostly empty costs as much as a full
+    one. So the longest portion has to have CHUNKED_FROM tokens, and the step TOKENS_A_CHUNK tokens a chunk. Measured beside
+    each mixer: microseconds in chunks and token by token, the mixer between its projections included, "8 x 20" for eight
+    portions of 20 tokens."""
+
+    CHUNKED_FROM: int
+    TOKENS_A_CHUNK: int
+
+    def plan_chunks(self, rt: Runtime, possible: bool = True) -> None:
+        """``spans``, or None where no step of the runtime can be long enough (no scratch then)."""
+        self.spans = ChunkedSpans(rt, self.TOKENS_A_CHUNK) if possible and rt.max_tokens >= self.CHUNKED_FROM else None
+        if self.spans is not None:
+            rt.portion_rules[type(self).__name__, self.CHUNKED_FROM, self.TOKENS_A_CHUNK] = self.in_chunks
+
+    def in_chunks(self, lengths) -> bool:
+        """Whether portions of these lengths go in chunks. A launch shape that several steps share holds for one answer
+        only (engine/step.py)."""
+        return (self.spans is not None and bool(lengths) and max(lengths) >= self.CHUNKED_FROM
+                and self.TOKENS_A_CHUNK * sum(-(-n // 64) for n in lengths) <= sum(lengths))
+
+    def leading(self, step: StepContext) -> int:
+        """How many of the step's tokens go token by token: its leading single tokens, or all of them."""
+        single = step.leading_single_tokens
+        lengths = step.host_span_lengths
+        if lengths is None:        # (every bound that the lengths may reach)
+            tokens, spans = step.tokens - single, step.spans - single
+            chunked = (self.spans is not None and step.max_span >= self.CHUNKED_FROM
+                       and self.TOKENS_A_CHUNK * (tokens // 64 + spans) <= tokens)
+        else:
+            chunked = self.in_chunks(lengths[single:])
+        return single if chunked else step.tokens
+
+
 @register_part("mixer", "mlstm")
-class MlstmMixer:
+class MlstmMixer(PortionsInChunks):
     """q = W_q x / sqrt(dim), k = W_k x (heads x dim), v = W_v x (heads x vdim); per head a log input gate
     cap tanh((W_i x + b_i) / cap) and a log forget gate logsigmoid(cap tanh((W_f x + b_f) / cap)). Each head's
     read-out is divided by its root mean square, scaled by ``norm`` (all heads' width), gated by sigmoid(W_g x)
@@ -62,17 +100,19 @@ class MlstmMixer:
         self.gates = rt.scratch("recurrent.gates", 2 * self.heads, torch.float32)
         self.read = rt.scratch("recurrent.read", self.v_width, torch.float32)
         self.gated = rt.scratch("recurrent.gated", self.v_width)
-        self.spans = ChunkedSpans(rt)
-        chunks = self.spans.max_chunks
-        self.chunk_gates = rt.scratch("recurrent.chunk_gates", 6 * self.heads, torch.float32)
-        self.peaks = rt.flat_scratch("recurrent.peaks", chunks * self.heads, torch.float64)
-        self.norms = rt.flat_scratch("recurrent.norms", chunks * self.qk_width, torch.float32)
-        self.states = rt.flat_scratch("recurrent.states", chunks * self.qk_width * self.vdim, torch.float32)
+        self.plan_chunks(rt)
+        if self.spans is not None:
+            chunks = self.spans.chunks_held
+            self.chunk_gates = rt.scratch("recurrent.chunk_gates", 6 * self.heads, torch.float32)
+            self.peaks = rt.flat_scratch("recurrent.peaks", chunks * self.heads, torch.float64)
+            self.norms = rt.flat_scratch("recurrent.norms", chunks * self.qk_width, torch.float32)
+            self.states = rt.flat_scratch("recurrent.states", chunks * self.qk_width * self.vdim, torch.float32)
 
-    # Steps whose longest portion has at least this many tokens are scanned in chunks. Measured for one portion at 16 heads of
-    # 64 x 128, the mixer between its projections included: 128 tokens 53 us in chunks, 51 token by token; 192: 57 and 70;
-    # 2,048: 171 and 564.
+    # Measured at 16 heads of 64 x 128: 1 x 128 53 in chunks, 51 token by token; 1 x 150 53, 59; 1 x 2,048 171, 564; 8 x 20 60,
+    # 43; 48 x 20 168, 152; 48 x 150 557, 921; 200 and 8 x 10 (23 tokens a chunk) 70, 88; 160 and 40 x 8 (11) 142, 96; 600 and
+    # 40 x 20 (28) 187, 272.
     CHUNKED_FROM = 144
+    TOKENS_A_CHUNK = 20
 
     def cache_need(self):
         return StateNeed(elements=self.heads * self.dim * self.vdim + self.heads * self.dim + self.heads)
@@ -105,8 +145,7 @@ class MlstmMixer:
             rt.linear(self.gated, self.w_out, out, t)
             return
         # long portions in chunks; what lies before them (single tokens), and steps of short spans, token by token
-        chunked = step.max_span >= self.CHUNKED_FROM and self.spans.fits(step, step.leading_single_tokens)
-        one_by_one = step.leading_single_tokens if chunked else t
+        one_by_one = self.leading(step)
         if one_by_one:
             spans = step.spans if one_by_one == t else one_by_one
             kernels.mlstm_gates(pre_i, pre_f, self.bias_i, self.bias_f, self.cap, self.gates, one_by_one, self.heads)
@@ -125,7 +164,7 @@ class MlstmMixer:
 
 
 @register_part("mixer", "gated_delta")
-class GatedDeltaMixer:
+class GatedDeltaMixer(PortionsInChunks):
     """q = W_q x, k = W_k x (kv_heads x dim), v = W_v x (heads x vdim), each through a depthwise causal
     convolution of ``taps`` taps and SiLU; q and k per head divided by sqrt(sum of squares + 1e-6), q also by
     sqrt(dim); beta = sigmoid(W_b x) and decay g = exp(-exp(A_log) softplus(W_a x + dt_bias)) per head. Head h
@@ -171,9 +210,11 @@ class GatedDeltaMixer:
         self.gates = rt.scratch("recurrent.gates", 2 * self.heads, torch.float32)
         self.read = rt.scratch("recurrent.read", self.v_width, torch.float32)
         self.gated = rt.scratch("recurrent.gated", self.v_width)
-        if self.dim <= kernels.DELTA_CHUNK_MAX_DIM:
-            self.spans = ChunkedSpans(rt)
-            chunks = self.spans.max_chunks
+        if self.dim > 64:
+            self.CHUNKED_FROM = 288
+        self.plan_chunks(rt, self.dim <= kernels.DELTA_CHUNK_MAX_DIM)
+        if self.spans is not None:
+            chunks = self.spans.chunks_held
             self.cum = rt.scratch("decay.cum", 2 * self.heads, torch.float32)
             self.dt = rt.scratch("decay.dt", self.heads, torch.float32)
             self.written = rt.scratch("recurrent.written", self.v_width, torch.float32)
@@ -181,10 +222,12 @@ class GatedDeltaMixer:
             self.operands = rt.flat_scratch("delta.operands", chunks * self.heads * kernels.delta_operand_bytes(self.dim) // 2,
                                             torch.bfloat16)
 
-    # Steps whose longest portion has at least this many tokens are scanned in chunks. Measured at 32 heads of 64 x 64, the
-    # mixer between its projections included, in chunks and token by token: one portion of 256 tokens 82 and 79 us, 384: 96
-    # and 111, 2,048: 291 and 496; six portions of together 2,048 (the longest 530): 282 and 302.
-    CHUNKED_FROM = 288
+    # Measured at 32 heads of 64 x 64: 1 x 300 98 in chunks, 93 token by token; 1 x 384 96, 111; 1 x 500 110, 133; 1 x 2,048 291,
+    # 496; 8 x 300 334, 306; 16 x 500 866, 904; 48 x 150 944, 835; 600 and 40 x 20 (28 tokens a chunk) 321, 256; 1,500 and 16 x
+    # 30 (49) 303, 461. At 32 heads of 128 x 128, where token by token is twice the work: 1 x 150 107, 102; 1 x 300 140, 169; 8 x
+    # 300 722, 960; 600 and 40 x 20 733, 643.
+    CHUNKED_FROM = 384
+    TOKENS_A_CHUNK = 40
 
     def cache_need(self):
         return StateNeed(elements=self.state_elements + (self.taps - 1) * self.channels)
@@ -223,9 +266,7 @@ class GatedDeltaMixer:
         k = conv[:, self.qk_width:2 * self.qk_width]
         v = conv[:, 2 * self.qk_width:]
         # long portions in chunks; what lies before them (single tokens), and steps of short spans, token by token
-        chunked = (step.max_span >= self.CHUNKED_FROM and self.dim <= kernels.DELTA_CHUNK_MAX_DIM
-                   and self.spans.fits(step, step.leading_single_tokens))
-        one_by_one = step.leading_single_tokens if chunked else t
+        one_by_one = self.leading(step)
         if one_by_one:
             kernels.recurrent_scan(kernels.SCAN_DELTA, q, k, v, self.gates, self.read, b.state, b.slot_stride,
                                    step.span_begin, step.span_slot, step.spans if one_by_one == t else one_by_one, self.heads,
@@ -242,7 +283,7 @@ class GatedDeltaMixer:
 
 
 @register_part("mixer", "retention")
-class RetentionMixer:
+class RetentionMixer(PortionsInChunks):
     """q = W_q x, k = W_k x / sqrt(dim) (heads x dim), v = W_v x (heads x vdim); per head S <- decay_h S + k v^T
     and the read-out S^T q, with ``decay`` one constant a head. Each head's read-out is divided by its root mean
     square (no weight), the heads are gated by SiLU(W_g x) and projected by W_o. Per-request state: S per head,
@@ -272,32 +313,35 @@ class RetentionMixer:
         self.read = rt.scratch("recurrent.read", self.v_width, torch.float32)
         self.gated = rt.scratch("recurrent.gated", self.v_width)
         # long prompts: segments of SEGMENT tokens side by side (the decay is a constant, so what a segment's tokens leave
-        # in the state does not depend on what was carried into it)
-        self.max_segments = rt.max_tokens // self.SEGMENT + rt.max_requests + 16
-        elements = self.heads * self.dim * self.vdim
-        self.segment_states = rt.flat_scratch("retention.segments", 2 * self.max_segments * elements, torch.float32)
-        self.segment_plan = rt.flat_scratch("retention.plan", 2 * self.max_segments + 8, torch.int32, zero=True)
+        # in the state does not depend on what was carried into it), each a chunk or two
+        self.plan_chunks(rt)
+        if self.spans is not None:
+            self.max_segments = rt.max_tokens // self.SEGMENT + min(rt.max_requests + 16, rt.max_tokens // self.TOKENS_A_CHUNK)
+            elements = self.heads * self.dim * self.vdim
+            self.segment_states = rt.flat_scratch("retention.segments", 2 * self.max_segments * elements, torch.float32)
+            self.segment_plan = rt.flat_scratch("retention.plan", 2 * self.max_segments + 8, torch.int32, zero=True)
 
     SEGMENT = 128               # tokens a segment
-    # Steps of at least this many tokens are scanned in segments. Measured for one portion at 16 heads of 64 x 128, the mixer
-    # between its projections included: 128 tokens 39 us in segments, 41 token by token; 192: 43 and 53; 384: 51 and 91.
-    SEGMENTED_FROM = 160
+    # Measured at 16 heads of 64 x 128: 1 x 128 39 in segments, 41 token by token; 1 x 150 41, 47; 2 x 150 55, 55; 1 x 500 55,
+    # 115; 8 x 20 51, 31; 48 x 20 150, 110; 48 x 150 469, 596; 200 and 8 x 10 (23 tokens a chunk) 60, 68; 160 and 40 x 8 (11) 127,
+    # 78; 600 and 40 x 20 (28) 161, 198.
+    CHUNKED_FROM = 144
+    TOKENS_A_CHUNK = 20
 
     def _scan(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, step: StepContext, scale: float) -> None:
         """The recurrence over the step's spans into ``read``: single tokens at the step's head token by token, long
         portions behind them in segments."""
         b, t = self.binding, step.tokens
-        single = step.leading_single_tokens
-        spans = step.spans - single
-        segments = (t - single) // self.SEGMENT + spans
-        if not (t - single >= self.SEGMENTED_FROM and segments <= self.max_segments
-                and segments + spans + 2 <= self.segment_plan.numel()):
-            single, spans = t, step.spans
+        single = self.leading(step)
+        segments = (t - single) // self.SEGMENT + step.spans - single
+        if single < t and segments > self.max_segments:
+            single = t
         if single:
             kernels.recurrent_scan(kernels.SCAN_RETENTION, q, k, v, self.decay, self.read, b.state, b.slot_stride,
-                                   step.span_begin, step.span_slot, spans if single == t else single, self.heads, self.heads,
+                                   step.span_begin, step.span_slot, step.spans if single == t else single, self.heads, self.heads,
                                    self.dim, self.vdim, scale)
         if single < t:
+            spans = step.spans - single
             # (span_begin counts the step's tokens: the rows stay where they are)
             kernels.retention_segmented(q, k, v, self.decay, self.read, b.state, b.slot_stride, step.span_begin[single:],
                                         step.span_slot[single:], spans, t - single, self.heads, self.dim, self.vdim, scale,
@@ -467,7 +511,7 @@ class GatedLinearRecurrenceMixer:
 
 
 @register_part("mixer", "general_delta")
-class GeneralDeltaMixer:
+class GeneralDeltaMixer(PortionsInChunks):
     """r = W_r x, k = W_k x, v = W_v x (heads x dim each). Per key channel a decay w = exp(-e^(-1/2) sigmoid(W_2 tanh(W_1 x)
     + w0)) and a removal rate a = sigmoid(W_a x + b_a); with the unit key u = k / sqrt(sum(k^2) + 1e-6) of each head
     S <- diag(w) S - (a u)(u^T S) + k v^T, both terms of the old state, and the read-out S^T r of the new one. Each head's
@@ -513,9 +557,9 @@ class GeneralDeltaMixer:
                                        rt.max_tokens * kernels.general_delta_scratch(self.heads, self.dim), torch.float32)
         self.read = rt.scratch("recurrent.read", inner, torch.float32)
         self.gated = rt.scratch("recurrent.gated", inner)
-        if self.dim <= kernels.GENERAL_DELTA_CHUNK_MAX_DIM:
-            self.spans = ChunkedSpans(rt)
-            chunks = self.spans.max_chunks
+        self.plan_chunks(rt, self.dim <= kernels.GENERAL_DELTA_CHUNK_MAX_DIM)
+        if self.spans is not None:
+            chunks = self.spans.chunks_held
             self.r_taken = rt.scratch("general_delta.r", inner, torch.float32)
             self.written = rt.scratch("recurrent.written", inner, torch.float32)
             self.products = rt.flat_scratch("general_delta.products", 2 * chunks * self.heads * self.spans.tokens ** 2, torch.float32)
@@ -524,10 +568,10 @@ class GeneralDeltaMixer:
             self.operands = rt.flat_scratch("delta.operands", chunks * self.heads * kernels.delta_operand_bytes(self.dim) // 2,
                                             torch.bfloat16)
 
-    # Steps whose longest portion has at least this many tokens are scanned in chunks of 64 tokens, others in chunks of 8.
-    # Measured at 32 heads of 64, the mixer between its projections included, in chunks of 64 and of 8: one portion of 384 tokens
-    # 109 and 105 us, 512: 125 and 135, 2,048: 361 and 448; six portions of together 2,048 (the longest 530): 365 and 393.
+    # Measured at 32 heads of 64, in chunks of 64 and of 8: 1 x 300 102, 92; 1 x 500 121, 132; 1 x 2,048 361, 448; 16 x 500 1,200,
+    # 1,224; 48 x 150 1,302, 1,118; 600 and 40 x 20 (28 tokens a chunk) 441, 284; 1,500 and 16 x 30 (49) 395, 505.
     CHUNKED_FROM = 480
+    TOKENS_A_CHUNK = 40
 
     def cache_need(self):
         return StateNeed(elements=self.heads * self.dim * self.dim)
@@ -551,9 +595,7 @@ class GeneralDeltaMixer:
         kernels.activation_cast(rows[:, 5 * inner:], self.low, t, kernels.ACT_TANH)
         rt.linear(self.low, self.w_decay, self.z, t)
         # long portions in chunks of 64 tokens; what lies before them (single tokens), and steps of short spans, in chunks of 8
-        chunked = (step.max_span >= self.CHUNKED_FROM and self.dim <= kernels.GENERAL_DELTA_CHUNK_MAX_DIM
-                   and self.spans.fits(step, step.leading_single_tokens))
-        short = step.leading_single_tokens if chunked else t
+        short = self.leading(step)
         columns = (0, inner, 2 * inner, 4 * inner)
         if short:
             kernels.general_delta_scan(rows, columns, self.z, self.decay_bias, self.removal_bias, self.UNIT_EPS,

@@ -3,7 +3,7 @@ matrix product, and the description of the step being run."""
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from typing import Dict, List, Optional, Tuple
+from typing import Callable, Dict, List, Optional, Tuple
 
 import torch
 
@@ -225,6 +225,9 @@ class Runtime:
         self.tcgen05_attention = options.tcgen05_attention
         self.side_by_side_branches = options.side_by_side_branches
         self._side_stream: Optional[torch.cuda.Stream] = None
+        # rules by which parts choose a launch from the lengths of a step's portions: a graph that steps of several lengths
+        # share is captured for one answer of each (``portion_routes``)
+        self.portion_rules: Dict[tuple, Callable[[list], bool]] = {}
         # Decode steps are a chain of short weight-streaming kernels, the same chain every step. Each of them
         # asks the first megabytes of its successor's weights into the L2, so that memory works across the
         # kernel boundary; the successor of a weight is learnt from the order of the calls (the first step of
@@ -255,6 +258,10 @@ class Runtime:
         if key not in self._scratch:
             self._scratch[key] = torch.empty((self.max_tokens, columns), dtype=dtype, device=self.device)
         return self._scratch[key]
+
+    def portion_routes(self, lengths: list) -> Tuple[bool, ...]:
+        """The answers of the parts' rules for portions of these lengths."""
+        return tuple(rule(lengths) for rule in self.portion_rules.values())
 
     def flat_scratch(self, tag: str, elements: int, dtype: torch.dtype, zero: bool = False) -> torch.Tensor:
         """A persistent 1-D buffer shared by parts that ask with the same tag, size and type."""
