@@ -1067,14 +1067,17 @@ inline int launch_reads(const ChunkArgs& p, int chunks, cudaStream_t stream) {
                        : launch_read<MODE, 128>(p, chunks, heads_a_block, stream);
 }
 
+// The walk moves a third of the bytes but needs a block and a half an SM to keep them busy: at 64 heads of 128 x 64 (256 blocks) a
+// span of 2,048 tokens takes 88 us, sums and carry 107 (62 + 45); at 16 heads of 64 x 128 (64 blocks) 46 us and 26 (17 + 9; the
+// mLSTM's carry, with its maxima, 21).
+inline bool walks(int heads, int dim, int vdim, int spans) {
+    return (long long)((vdim + kWalkColumns - 1) / kWalkColumns) * ((dim + kWalkRows - 1) / kWalkRows) * heads * spans >= 222;
+}
+
 // `chunks` bounds the chunks of all spans; p.chunk_begin has chunks / p.pieces + 1 entries
 template <int MODE>
 inline int launch_chunk_scan(const ChunkArgs& p, int chunks, cudaStream_t stream) {
-    // The walk moves a third of the bytes but needs a block and a half an SM to keep them busy: at 64 heads of 128 x 64 (256
-    // blocks) a span of 2,048 tokens takes 88 us, sums and carry 107 (62 + 45); at 16 heads of 64 x 128 (64 blocks) 46 us and
-    // 26 (17 + 9; the mLSTM's carry, with its maxima, 21).
-    const long long blocks = (long long)((p.vdim + kWalkColumns - 1) / kWalkColumns) * ((p.dim + 63) / 64) * p.heads * p.spans;
-    const int status = blocks >= 222 ? launch_walk<MODE>(p, stream) : launch_sums<MODE>(p, chunks, stream);
+    const int status = walks(p.heads, p.dim, p.vdim, p.spans) ? launch_walk<MODE>(p, stream) : launch_sums<MODE>(p, chunks, stream);
     return status != 0 ? status : launch_reads<MODE>(p, chunks, stream);
 }
 

@@ -8,6 +8,7 @@ Kernels run on torch's current CUDA stream.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional, Tuple
 
@@ -184,6 +185,7 @@ _SIGNATURES = {
                                        c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "celeg_decay_sums": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "celeg_delta_operand_bytes": [c_int],
+    "celeg_chunk_state_launches": [c_int, c_int, c_int, c_int],
     "celeg_delta_chunk_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                c_int, c_float, c_void_p, c_void_p],
@@ -1005,7 +1007,7 @@ def mlstm_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, pre_i: t
         _ptr(bias_i), _ptr(bias_f), cap, _ptr(gates), _ptr(peaks), _ptr(norms), _ptr(states), _ptr(out), _ptr(state), slot_stride,
         _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, dim, vdim, q_scale, _stream()))
     global LAUNCHES
-    LAUNCHES += 2          # the gates, the states (one launch or two), the read-outs
+    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans)      # (a call counts one) the gates, the states, the read-outs
 
 
 def retention_segmented(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
@@ -1031,7 +1033,7 @@ def retention_segmented(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay
                                                tokens, heads, dim, vdim, q_scale, segment, max_segments,
                                                _ptr(float_scratch), _ptr(int_scratch), _stream()))
     global LAUNCHES
-    LAUNCHES += 2          # (a call counts one) the plan, the states (one launch at least), the read-outs
+    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans)      # (a call counts one) the plan, the states, the read-outs
 
 
 def recurrent_decode(mode: int, proj: torch.Tensor, offsets: Tuple[int, int, int, int, int, int],
@@ -1452,6 +1454,12 @@ def chunk_tokens() -> int:
     return int(library().celeg_chunk_tokens())
 
 
+@functools.lru_cache(maxsize=256)
+def chunk_state_launches(heads: int, dim: int, vdim: int, spans: int) -> int:
+    """Launches that a chunked scan makes its states with (:data:`LAUNCHES` counts them)."""
+    return int(library().celeg_chunk_state_launches(heads, dim, vdim, spans))
+
+
 def chunk_plan(span_begin: torch.Tensor, spans: int, max_chunks: int, plan: torch.Tensor) -> None:
     """The chunks that the step's spans are cut into (plan: int32 [max_chunks + 1 + spans + 1])."""
     _need(plan, torch.int32, "plan")
@@ -1476,7 +1484,7 @@ def channel_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: tor
         _ptr(q_out), _ptr(k_out), _ptr(total), _ptr(products), _ptr(states), _ptr(out), _ptr(state), slot_stride,
         _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, dim, vdim, _stream()))
     global LAUNCHES
-    LAUNCHES += 2          # the chunks' own products, the states (one launch or two), the read-outs
+    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans)      # the chunks' own products, the states, the read-outs
 
 
 def scalar_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: torch.Tensor, dt_bias: torch.Tensor,
@@ -1496,7 +1504,7 @@ def scalar_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: to
         _ptr(direct), _ptr(cum), _ptr(dt), _ptr(states), _ptr(out), _ptr(state), slot_stride, _ptr(span_slot),
         _ptr(plan), max_chunks, spans, chunks, heads, groups, dim, vdim, _stream()))
     global LAUNCHES
-    LAUNCHES += 2          # the decays, then as above
+    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans)      # the decays, then as above
 
 
 def channel_decay_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_scale: float, low: torch.Tensor,
