@@ -4,8 +4,9 @@
 //   grid = (query heads, query tiles); a query tile is up to 128 consecutive tokens of one span; tiles with
 //   many keys come first in launch order, so that the grid drains with short ones.
 //   Six warps. Warp 0 brings Q (boxes of 128 rows x 64) and, per block of 64 keys, the K and V
-//   rows page by page through the request's block table into a ring each by TMA (128-byte
-//   swizzle; a page is D / 64 boxes of page_tokens rows x 64, a lane each; K a block ahead of V). Warp 1 issues the MMAs:
+//   rows page by page through the request's block table by TMA (128-byte swizzle; a page is D / 64 boxes of
+//   page_tokens rows x 64 of K and of V, a lane each): at a head size of 64 into one ring, at 128 into a ring
+//   each, K a block ahead of V. Warp 1 issues the MMAs:
 //       S[128 x 64] = Q K^T           (tcgen05.mma M128 N64 K16 x D / 16, both operands K-major)
 //       O[128 x D] += P V             (M128 N64 K16 x 4 D / 64, P from tensor memory as the A operand, V as it lies
 //                                      in the cache, keys x 64: the MN-major form of the B operand)
@@ -15,7 +16,8 @@
 //   Warps 2-5 are the softmax: a thread owns one query row (its TMEM lane), reads S with tcgen05.ld, masks
 //   (causal, window, rows past the span; blocks that every row sees whole skip the mask), takes the maximum,
 //   writes P = exp2(scaled S - maximum) as bfloat16 pairs into tensor memory with tcgen05.st and adds to its
-//   denominator, all in float32 (packed f32x2 arithmetic, three-input maxima). O stays in tensor memory: the
+//   denominator, all in float32 (packed f32x2 arithmetic, three-input maxima). Values of keys that no row of the
+//   tile sees (page 0's, a page's tail, before the window) become zeros before P V. O stays in tensor memory: the
 //   maximum that P is relative to follows the true running maximum only when that has grown by more than 2^8,
 //   and only then the warp rescales its rows of O (tcgen05.ld, multiply, tcgen05.st); at the end a thread
 //   divides its row by the denominator and writes it. No shuffles: a row is one thread. Every tensor-memory
