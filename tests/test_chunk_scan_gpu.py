@@ -231,6 +231,5 @@ def test_generalised_delta_rule_in_chunks_of_64(lengths, heads, dim, decay):
         return float((x.double() - y).norm() / y.norm())
     # float32 sums of the same products in different orders: errors of the same size, of a few units of 2^-24
     for name, a, b, c in (("read", got, out, want), ("state", got_state, state, want_state)):
-        print(name, off(a, c), off(b, c))
         assert off(a, c) <= 2 * off(b, c) + 3e-7, (name, off(a, c), off(b, c))
     assert torch.equal(got_state[:, inner * dim:], before[:, inner * dim:]) and torch.equal(got_state[0], before[0])

@@ -271,8 +271,8 @@ def run_attention(kind, paged, queries, heads, groups, dim, scale, window, bias,
 @pytest.mark.parametrize("heads,groups,dim,window,last,with_sinks", [(4, 2, 64, None, 100, False), (2, 1, 64, 70, 30, True),
                                                                     (8, 1, 128, None, 300, False), (3, 3, 24, None, 9, True)])
 def test_score_biases_by_distance_in_every_attention_kernel(kind, heads, groups, dim, window, last, with_sinks):
-    if kind == "tcgen05" and dim != 64:
-        pytest.skip("the tcgen05 kernel takes heads of 64")
+    if kind == "tcgen05" and dim not in (64, 128):
+        pytest.skip("the tcgen05 kernel takes heads of 64 and 128")
     decoding = kind == "decode"
     spans = [(450, 1), (0, 1), (129, 1), (63, 1)] if decoding else [(0, 200), (310, 3), (100, 129), (5, 1)]
     queries, keys, values, bias = attention_case(heads, groups, dim, spans, last, dim + heads)
