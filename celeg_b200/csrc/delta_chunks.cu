@@ -48,8 +48,8 @@ struct DeltaChunkArgs {
 // The system's matrix is inverted, T = (1 + L)^-1: its four diagonal blocks of 16 by substitution, a warp a block and a lane a
 // column; then two blocks of 16 and at last two of 32 are joined, T_21 = -T_22 L_21 T_11; and W and U_0 are products of T with
 // the scaled k and v. It is bound by the latency of these steps, so blocks an SM count: T in float32 lies where k did and L where
-// T's planes will, 50 KB a block, four of them an SM; the right sides are scaled, so that T is split once. 57 us for 32 heads of
-// 64 and 2,048 tokens (69 with three blocks and T split twice; 138 by substitution over whole right sides, one chain of 64 steps
+// T's planes will, 50 KB a block, four of them an SM; the right sides are scaled, so that T is split once. 60 us for 32 heads of
+// 64 and 2,048 tokens (57 before it left out tokens that are not finite; 69 with three blocks and T split twice; 138 by substitution over whole right sides, one chain of 64 steps
 // a block).
 constexpr int kSolveThreads = 128;
 constexpr int kSolvePitch = kChunk + 4;
@@ -523,8 +523,8 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
 //
 // the same shape: a system's inverse T, W = T u^ and s_0 = T ((u^ . k^) v), the same walk with s = s_0 + W S_0, and read-outs
 // with two sets of values. One block a (chunk, head) of 64 channels makes everything that does not wait for the state:
-// 140 us at 32 heads of 64 and 2,048 tokens, two blocks an SM (187 us with one); with the walk's 68 and the read-outs' 49 that is
-// 257 us where chunks of eight tokens take 344.
+// 146 us at 32 heads of 64 and 2,048 tokens, two blocks an SM (139 before it left out tokens that are not finite, 187 with one
+// block an SM); with the walk's 67 and the read-outs' 47 that is 260 us where chunks of eight tokens take 344.
 struct GeneralChunkArgs {
     const float* proj; int stride; int r_off, k_off, v_off, a_off;     // columns of a token's row: head h at h * dim
     const float* z; int z_stride;                              // [tokens, heads * dim], before its bias
