@@ -134,6 +134,160 @@ __device__ __forceinline__ void decode_norm_rope_head(At at, Out out, const floa
     }
 }
 
+// Copies of a warp's tile of 32 keys: row r of [K tile | V tile] from `mine` of lane r (the offset of its key in a head's pages, or
+// -1: zeros). `k_lane`, `v_lane`: the head's caches from this lane's columns on.
+template <int D_PAD>
+__device__ __forceinline__ void decode_copy_tile(__nv_bfloat16* k_dst, __nv_bfloat16* v_dst, const __nv_bfloat16* k_lane,
+                                                 const __nv_bfloat16* v_lane, const long long mine, const bool column, const int lane) {
+    constexpr int kChunks = D_PAD / 8;
+    static_assert(32 % kChunks == 0, "a lane copies the same columns of all its rows");
+    const int ch = lane % kChunks;
+    const unsigned k_to = (unsigned)__cvta_generic_to_shared(k_dst), v_to = (unsigned)__cvta_generic_to_shared(v_dst);
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) {
+        const int r = i * (32 / kChunks) + lane / kChunks;
+        const long long off = __shfl_sync(0xffffffffu, mine, r);
+        const bool there = off >= 0 && column;
+        const long long from = there ? off : 0;
+        const unsigned to = 2 * tile_offset<D_PAD>(r, ch), bytes = there ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(k_to + to), "l"(k_lane + from), "r"(bytes));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(v_to + to), "l"(v_lane + from), "r"(bytes));
+    }
+}
+
+__device__ __forceinline__ float exp2_of(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// A warp's running result over its tiles: rows g and g + 8 of the 16 query heads; maxima in units of log2.
+template <int D_PAD>
+struct DecodeRows {
+    float o[D_PAD / 8][4], run_max[2], run_sum[2];
+    unsigned q[D_PAD == 64 ? 4 : 1][4];                     // the queries' fragments, where the registers allow
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int i = 0; i < D_PAD / 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[i][e] = 0.0f;
+        run_max[0] = run_max[1] = -INFINITY;
+        run_sum[0] = run_sum[1] = 0.0f;
+    }
+    __device__ __forceinline__ void load_q(unsigned (&a)[4], const __nv_bfloat16* q_s, int kt, int lane) const {
+        ldmatrix_x4(a, q_s + tile_offset<D_PAD>(((lane >> 3) & 1) * 8 + (lane & 7), kt * 2 + (lane >> 4)));
+    }
+    __device__ __forceinline__ void hold_q(const __nv_bfloat16* q_s, int lane) {
+        if constexpr (D_PAD == 64) {
+#pragma unroll
+            for (int kt = 0; kt < 4; ++kt) load_q(q[kt], q_s, kt, lane);
+        }
+    }
+    // The tile of keys tile_begin .. tile_begin + 31, those from `end` on do not count. What bounded this kernel over long contexts
+    // was the instructions of a tile, a warp's chain of them and all warps' on the SM, 2 us a tile even with an empty GPU (three
+    // stages of copies instead of two gained nothing). So rows 8 to 15 are left out of the exponentials for groups of at most
+    // eight heads, a tile that needs no mask, cap or bias goes straight from the products into the exponentials, the outputs are
+    // rescaled only when a maximum has grown, the queries' fragments stay in registers, and a copy that has nothing to bring is one
+    // of no bytes instead of a branch. 32 heads on 8 of 64, before and now, us: 8 requests of 16 k keys 72 and 60 (268 MB: 41 at
+    // 6.5 TB/s, and about 10 around the loop), 16 of 6 k 74 and 50, 1 of 130 k 75 and 69, 1 of 16 k 26 and 22, 8 of 578 14.5 and
+    // 12.8.
+    __device__ __forceinline__ void take(const DecodeParams& p, const __nv_bfloat16* q_s, const __nv_bfloat16* k_t,
+                                         const __nv_bfloat16* v_t, const int tile_begin, const int end, const int pos,
+                                         const int kvh, const int group, const int lane) {
+        const int g = lane >> 2, c2 = (lane & 3) * 2, mi = lane >> 3, lr = lane & 7;
+        float s[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[i][e] = 0.0f;
+#pragma unroll
+        for (int kt = 0; kt < D_PAD / 16; ++kt) {
+            unsigned a[4];
+            if constexpr (D_PAD == 64) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = q[kt][i];
+            } else {
+                load_q(a, q_s, kt, lane);
+            }
+#pragma unroll
+            for (int np = 0; np < 2; ++np) {
+                unsigned b[4];
+                ldmatrix_x4(b, k_t + tile_offset<D_PAD>(np * 16 + (mi >> 1) * 8 + lr, kt * 2 + (mi & 1)));
+                mma_bf16(s[2 * np], a, b[0], b[1]);
+                mma_bf16(s[2 * np + 1], a, b[2], b[3]);
+            }
+        }
+        const int halves = group > 8 ? 2 : 1;               // (the rows past the group are never stored)
+        const float scale_log2 = p.scale * 1.4426950408889634f;
+        const bool plain = tile_begin + 32 <= end && p.cap_log2 == 0.0f && !p.distance_bias && scale_log2 > 0.0f;
+        unsigned a[2][4] = {};                               // the weights as the next product's operand
+        float factor = 1.0f;                                 // of s, to units of log2
+        if (plain) {
+            factor = scale_log2;
+        } else {
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int key = tile_begin + nt * 8 + c2 + (e & 1);
+                    float v = key < end ? (p.cap_log2 > 0.0f ? p.cap_log2 * quick_tanh(s[nt][e] * p.cap_in) : s[nt][e] * scale_log2)
+                                        : -INFINITY;
+                    if (p.distance_bias && key < end) {
+                        // a learned number per (head, distance back to the key) joins the scaled score, in units of log2
+                        const int row = min(g + (e >> 1) * 8, group - 1);
+                        v += __ldg(p.distance_bias + (size_t)(kvh * group + row) * (p.distance_last + 1) +
+                                   max(0, min(pos - key, p.distance_last))) * 1.4426950408889634f;
+                    }
+                    s[nt][e] = v;
+                }
+        }
+        bool grown = false;
+        float correction[2] = {1.0f, 1.0f};
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            if (half >= halves) continue;
+            float m = -INFINITY;
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) m = fmaxf(m, fmaxf(s[nt][2 * half], s[nt][2 * half + 1]));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            const float new_max = fmaxf(run_max[half], m * factor);
+            if (new_max != run_max[half]) {
+                grown = true;
+                correction[half] = exp2_of(run_max[half] - new_max);
+            }
+            const float base = new_max == -INFINITY ? 0.0f : new_max;
+            run_max[half] = new_max;
+            float sum = 0.0f;
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const float x = exp2_of(fmaf(s[nt][2 * half], factor, -base)), y = exp2_of(fmaf(s[nt][2 * half + 1], factor, -base));
+                sum += x + y;
+                a[nt >> 1][half + 2 * (nt & 1)] = pack_bf16(x, y);
+            }
+            run_sum[half] = fmaf(run_sum[half], correction[half], sum);
+        }
+        if (__any_sync(0xffffffffu, grown)) {
+#pragma unroll
+            for (int i = 0; i < D_PAD / 8; ++i) {
+                o[i][0] *= correction[0];
+                o[i][1] *= correction[0];
+                o[i][2] *= correction[1];
+                o[i][3] *= correction[1];
+            }
+        }
+#pragma unroll
+        for (int kt = 0; kt < 2; ++kt)
+#pragma unroll
+            for (int np = 0; np < D_PAD / 16; ++np) {
+                unsigned b[4];
+                ldmatrix_x4_trans(b, v_t + tile_offset<D_PAD>(kt * 16 + (mi & 1) * 8 + lr, np * 2 + (mi >> 1)));
+                mma_bf16(o[2 * np], a[kt], b[0], b[1]);
+                mma_bf16(o[2 * np + 1], a[kt], b[2], b[3]);
+            }
+    }
+};
+
 template <int D_PAD, int BN>
 __host__ __device__ constexpr size_t decode_item_bytes() {
     return decode_smem_bytes<D_PAD, BN>() + sizeof(DecodeShared);
@@ -149,12 +303,10 @@ template <int D_PAD, int BN, typename Sync>
 __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, const int split, const int kvh, const int t,
                                                       unsigned char* smem_raw, const int tid, Sync sync) {
     constexpr int kChunks = D_PAD / 8;
-    constexpr int kKTiles = D_PAD / 16;
     constexpr int kOTiles = D_PAD / 8;
-    constexpr int kStages = (D_PAD <= 128 && BN >= 64) ? 2 : 1;     // stages per warp
+    constexpr int kStages = (D_PAD <= 128 && BN >= 64) ? BN / 32 : 1;      // stages per warp
     constexpr int TN = BN / kStages;                       // keys per stage (the warp's shared memory is BN keys of K and of V)
-    constexpr int kKeysPerLane = TN / 32;
-    static_assert(TN % 32 == 0, "a stage holds a multiple of 32 keys");
+    static_assert(TN == 32, "a stage holds a key a lane");
     const int lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, c2 = (lane & 3) * 2;
     const int group = p.q_heads / p.kv_heads;
@@ -187,50 +339,44 @@ __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, con
     // The first tile of keys and values is asked for before anything else (the query's own preparation below
     // takes as long as the tile needs to arrive). The token's own key and value may not be in the cache yet:
     // their row is put right in shared memory when the tile is there (see the loop).
-    // A warp's part of the shared memory is kStages stages of [K tile | V tile] of TN keys: with two
-    // stages the next tile is on its way (page lookups included) while this one is in the tensor cores.
-    auto issue = [&](const int tile_begin, const int stage) {
+    // A warp's part of the shared memory is kStages stages of [K tile | V tile] of TN keys: all but one are on their way while
+    // that one is in the tensor cores. The page of a lane's key is looked up a tile before its copies are issued: a lookup in
+    // the issue itself is a round trip to the L2 a tile in which the warp has one tile less on its way.
+    const bool column = (lane % kChunks) * 8 < d;
+    const __nv_bfloat16* k_lane = p.k_cache + (lane % kChunks) * 8;
+    const __nv_bfloat16* v_lane = p.v_cache + (lane % kChunks) * 8;
+    const int shift = (p.page_tokens & (p.page_tokens - 1)) == 0 ? 31 - __clz(p.page_tokens) : -1;
+    auto page_of = [&](const int key) { return shift >= 0 ? key >> shift : key / p.page_tokens; };
+    auto look_up = [&](const int tile_begin) {
+        const int key = tile_begin + lane;
+        return key < end ? table[page_of(key)] : 0;
+    };
+    auto issue = [&](const int tile_begin, const int stage, const int page) {
+        const int key = tile_begin + lane;
+        long long mine = -1;                                 // the offset of this lane's key
+        if (key < end) {
+            if (page < 0)
+                atomicExch(p.error_flag, 2);
+            else
+                mine = (long long)page * p.page_stride + ((long long)kvh * p.page_tokens + (key - page_of(key) * p.page_tokens)) * d;
+        }
         __nv_bfloat16* k_dst = k_s + (size_t)stage * 2 * TN * D_PAD;
-        __nv_bfloat16* v_dst = k_dst + TN * D_PAD;
-        // page offsets of this lane's keys, then the copies of the whole tile in one go
-        long long offs[kKeysPerLane];
-#pragma unroll
-        for (int i = 0; i < kKeysPerLane; ++i) {
-            const int key = tile_begin + lane + 32 * i;
-            offs[i] = -1;
-            if (key < end) {
-                const int page = table[key / p.page_tokens];
-                if (page < 0)
-                    atomicExch(p.error_flag, 2);
-                else
-                    offs[i] = (long long)page * p.page_stride + ((long long)kvh * p.page_tokens + key % p.page_tokens) * d;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < TN * kChunks / 32; ++i) {
-            const int idx = lane + 32 * i;
-            const int r = idx / kChunks, ch = idx % kChunks;
-            long long off = -1;
-#pragma unroll
-            for (int j = 0; j < kKeysPerLane; ++j) {
-                const long long candidate = __shfl_sync(0xffffffffu, offs[j], r & 31);
-                if ((r >> 5) == j) off = candidate;
-            }
-            __nv_bfloat16* kd = k_dst + tile_offset<D_PAD>(r, ch);
-            __nv_bfloat16* vd = v_dst + tile_offset<D_PAD>(r, ch);
-            if (off >= 0 && ch * 8 < d) {
-                cp_async_16(kd, p.k_cache + off + ch * 8);
-                cp_async_16(vd, p.v_cache + off + ch * 8);
-            } else {
-                *reinterpret_cast<uint4*>(kd) = zero;
-                *reinterpret_cast<uint4*>(vd) = zero;
-            }
-        }
-        cp_async_commit();
+        decode_copy_tile<D_PAD>(k_dst, k_dst + TN * D_PAD, k_lane, v_lane, mine, column, lane);
     };
     constexpr int kTileStride = kDecodeWarps * TN;
-    int tile_begin = begin + warp * TN;
-    if (kStages == 2 && tile_begin < end) issue(tile_begin, 0);
+    constexpr int kAhead = kStages > 1 ? kStages - 1 : 1;      // tiles issued before the loop
+    int tile_begin = begin + warp * TN, next_page;
+    {
+        int pages[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) pages[i] = look_up(tile_begin + i * kTileStride);
+        next_page = look_up(tile_begin + kAhead * kTileStride);
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            if (tile_begin + i * kTileStride < end) issue(tile_begin + i * kTileStride, i, pages[i]);
+            cp_async_commit();
+        }
+    }
     for (int idx = tid; idx < 16 * kChunks; idx += kDecodeThreads) {
         const int r = idx / kChunks, ch = idx % kChunks;
         __nv_bfloat16* dst = q_s + tile_offset<D_PAD>(r, ch);
@@ -279,29 +425,20 @@ __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, con
         sync();
     }
 
-    float o[kOTiles][4];
-#pragma unroll
-    for (int i = 0; i < kOTiles; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[i][e] = 0.0f;
-    float run_max[2] = {-INFINITY, -INFINITY};
-    float run_sum[2] = {0.0f, 0.0f};
-    const float scale_log2 = p.scale * 1.4426950408889634f;
-    const int mi = lane >> 3, lr = lane & 7;
+    DecodeRows<D_PAD> rows;
+    rows.clear();
+    rows.hold_q(q_s, lane);
 
-    for (int iteration = 0; tile_begin < end; ++iteration, tile_begin += kTileStride) {
-        const int stage = kStages == 2 ? (iteration & 1) : 0;
-        if (kStages == 2) {
-            if (tile_begin + kTileStride < end) {
-                issue(tile_begin + kTileStride, stage ^ 1);
-                cp_async_wait_group<1>();
-            } else {
-                cp_async_wait_group<0>();
-            }
-        } else {
-            issue(tile_begin, 0);
-            cp_async_wait_group<0>();
+    auto next_tile = [&](const int at, const int stage) {       // the tile at `at` into a stage that has been used
+        if (at < end) {
+            issue(at, stage, next_page);
+            next_page = look_up(at + kTileStride);
         }
+        cp_async_commit();
+    };
+    for (int stage = 0; tile_begin < end; tile_begin += kTileStride, stage = stage + 1 < kStages ? stage + 1 : 0) {
+        if (kStages > 1) next_tile(tile_begin + kAhead * kTileStride, stage > 0 ? stage - 1 : kStages - 1);
+        cp_async_wait_group<kStages - 1>();
         __syncwarp();
         __nv_bfloat16* k_t = k_s + (size_t)stage * 2 * TN * D_PAD;
         __nv_bfloat16* v_t = k_t + TN * D_PAD;
@@ -315,100 +452,24 @@ __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, con
             __syncwarp();
         }
 
-        float s[TN / 8][4];
-#pragma unroll
-        for (int i = 0; i < TN / 8; ++i)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s[i][e] = 0.0f;
-#pragma unroll
-        for (int kt = 0; kt < kKTiles; ++kt) {
-            unsigned a[4];
-            ldmatrix_x4(a, q_s + tile_offset<D_PAD>((mi & 1) * 8 + lr, kt * 2 + (mi >> 1)));
-#pragma unroll
-            for (int np = 0; np < TN / 16; ++np) {
-                unsigned b[4];
-                ldmatrix_x4(b, k_t + tile_offset<D_PAD>(np * 16 + (mi >> 1) * 8 + lr, kt * 2 + (mi & 1)));
-                mma_bf16(s[2 * np], a, b[0], b[1]);
-                mma_bf16(s[2 * np + 1], a, b[2], b[3]);
-            }
-        }
-        float tile_max[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-        for (int nt = 0; nt < TN / 8; ++nt) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int key = tile_begin + nt * 8 + c2 + (e & 1);
-                float v = key < end ? (p.cap_log2 > 0.0f ? p.cap_log2 * quick_tanh(s[nt][e] * p.cap_in) : s[nt][e] * scale_log2)
-                                    : -INFINITY;
-                if (p.distance_bias && key < end) {
-                    // a learned number per (head, distance back to the key) joins the scaled score, in units of log2
-                    const int row = min(g + (e >> 1) * 8, group - 1);      // (rows past the group are never stored)
-                    v += __ldg(p.distance_bias + (size_t)(kvh * group + row) * (p.distance_last + 1) +
-                               max(0, min(pos - key, p.distance_last))) * 1.4426950408889634f;
-                }
-                s[nt][e] = v;
-                tile_max[e >> 1] = fmaxf(tile_max[e >> 1], v);
-            }
-        }
-        float correction[2], safe_max[2];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float m = tile_max[half];
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-            const float new_max = fmaxf(run_max[half], m);
-            correction[half] = new_max == -INFINITY ? 1.0f : exp2f(run_max[half] - new_max);
-            safe_max[half] = new_max == -INFINITY ? 0.0f : new_max;
-            run_max[half] = new_max;
-            run_sum[half] *= correction[half];
-        }
-#pragma unroll
-        for (int nt = 0; nt < TN / 8; ++nt) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float pv = exp2f(s[nt][e] - safe_max[e >> 1]);
-                s[nt][e] = pv;
-                run_sum[e >> 1] += pv;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kOTiles; ++i) {
-            o[i][0] *= correction[0];
-            o[i][1] *= correction[0];
-            o[i][2] *= correction[1];
-            o[i][3] *= correction[1];
-        }
-#pragma unroll
-        for (int kt = 0; kt < TN / 16; ++kt) {
-            unsigned a[4];
-            a[0] = pack_bf16(s[2 * kt][0], s[2 * kt][1]);
-            a[1] = pack_bf16(s[2 * kt][2], s[2 * kt][3]);
-            a[2] = pack_bf16(s[2 * kt + 1][0], s[2 * kt + 1][1]);
-            a[3] = pack_bf16(s[2 * kt + 1][2], s[2 * kt + 1][3]);
-#pragma unroll
-            for (int np = 0; np < kOTiles / 2; ++np) {
-                unsigned b[4];
-                ldmatrix_x4_trans(b, v_t + tile_offset<D_PAD>(kt * 16 + (mi & 1) * 8 + lr, np * 2 + (mi >> 1)));
-                mma_bf16(o[2 * np], a, b[0], b[1]);
-                mma_bf16(o[2 * np + 1], a, b[2], b[3]);
-            }
-        }
-            __syncwarp();                               // every lane is done with the stage before it is refilled
+        rows.take(p, q_s, k_t, v_t, tile_begin, end, pos, kvh, group, lane);
+        __syncwarp();                                   // every lane is done with the stage before it is refilled
+        if (kStages == 1) next_tile(tile_begin + kTileStride, 0);
     }
 
     // row sums over the four lanes that share a row; then the warps' results meet in shared memory
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-        run_sum[half] += __shfl_xor_sync(0xffffffffu, run_sum[half], 1);
-        run_sum[half] += __shfl_xor_sync(0xffffffffu, run_sum[half], 2);
+        rows.run_sum[half] += __shfl_xor_sync(0xffffffffu, rows.run_sum[half], 1);
+        rows.run_sum[half] += __shfl_xor_sync(0xffffffffu, rows.run_sum[half], 2);
     }
     sync();                                // every warp is done with its K/V tiles
     float* o_s = reinterpret_cast<float*>(smem_raw + 16 * D_PAD * sizeof(__nv_bfloat16));   // [warps][group][D_PAD]
     if ((lane & 3) == 0) {
-        warp_max_s[warp][g] = run_max[0];
-        warp_max_s[warp][g + 8] = run_max[1];
-        warp_sum_s[warp][g] = run_sum[0];
-        warp_sum_s[warp][g + 8] = run_sum[1];
+        warp_max_s[warp][g] = rows.run_max[0];
+        warp_max_s[warp][g + 8] = rows.run_max[1];
+        warp_sum_s[warp][g] = rows.run_sum[0];
+        warp_sum_s[warp][g + 8] = rows.run_sum[1];
     }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
@@ -417,8 +478,8 @@ __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, con
 #pragma unroll
             for (int i = 0; i < kOTiles; ++i) {
                 float* dst = o_s + ((size_t)warp * group + r) * D_PAD + i * 8 + c2;
-                dst[0] = o[i][half * 2];
-                dst[1] = o[i][half * 2 + 1];
+                dst[0] = rows.o[i][half * 2];
+                dst[1] = rows.o[i][half * 2 + 1];
             }
         }
     }
@@ -593,7 +654,6 @@ __device__ __forceinline__ void attention_decode_item_solo(const DecodeParams& p
                                                            unsigned char* warp_smem, const int lane) {
     constexpr int TN = 32;
     constexpr int kChunks = D_PAD / 8;
-    constexpr int kKTiles = D_PAD / 16;
     constexpr int kOTiles = D_PAD / 8;
     const int g = lane >> 2, c2 = (lane & 3) * 2;
     const int group = p.q_heads / p.kv_heads;
@@ -614,6 +674,9 @@ __device__ __forceinline__ void attention_decode_item_solo(const DecodeParams& p
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     const int* table = p.block_table + (size_t)p.token_span[t] * p.table_stride;
 
+    const bool column = (lane % kChunks) * 8 < d;
+    const __nv_bfloat16* k_lane = p.k_cache + (lane % kChunks) * 8;
+    const __nv_bfloat16* v_lane = p.v_cache + (lane % kChunks) * 8;
     auto issue = [&](const int tile_begin) {
         const int key = tile_begin + lane;
         long long mine = -1;
@@ -624,21 +687,7 @@ __device__ __forceinline__ void attention_decode_item_solo(const DecodeParams& p
             else
                 mine = (long long)page * p.page_stride + ((long long)kvh * p.page_tokens + key % p.page_tokens) * d;
         }
-#pragma unroll
-        for (int i = 0; i < TN * kChunks / 32; ++i) {
-            const int idx = lane + 32 * i;
-            const int r = idx / kChunks, ch = idx % kChunks;
-            const long long off = __shfl_sync(0xffffffffu, mine, r);
-            __nv_bfloat16* kd = k_t + tile_offset<D_PAD>(r, ch);
-            __nv_bfloat16* vd = v_t + tile_offset<D_PAD>(r, ch);
-            if (off >= 0 && ch * 8 < d) {
-                cp_async_16(kd, p.k_cache + off + ch * 8);
-                cp_async_16(vd, p.v_cache + off + ch * 8);
-            } else {
-                *reinterpret_cast<uint4*>(kd) = zero;
-                *reinterpret_cast<uint4*>(vd) = zero;
-            }
-        }
+        decode_copy_tile<D_PAD>(k_t, v_t, k_lane, v_lane, mine, column, lane);
         cp_async_commit();
     };
     issue(first);                                     // the first tile is on its way while the query is prepared
@@ -683,15 +732,9 @@ __device__ __forceinline__ void attention_decode_item_solo(const DecodeParams& p
         __syncwarp();
     }
 
-    float o[kOTiles][4];
-#pragma unroll
-    for (int i = 0; i < kOTiles; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[i][e] = 0.0f;
-    float run_max[2] = {-INFINITY, -INFINITY};
-    float run_sum[2] = {0.0f, 0.0f};
-    const float scale_log2 = p.scale * 1.4426950408889634f;
-    const int mi = lane >> 3, lr = lane & 7;
+    DecodeRows<D_PAD> rows;
+    rows.clear();
+    rows.hold_q(q_s, lane);
 
     for (int tile_begin = first; tile_begin < end; tile_begin += TN) {
         if (tile_begin > first) issue(tile_begin);
@@ -705,107 +748,30 @@ __device__ __forceinline__ void attention_decode_item_solo(const DecodeParams& p
             }
             __syncwarp();
         }
-        float s[TN / 8][4];
-#pragma unroll
-        for (int i = 0; i < TN / 8; ++i)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s[i][e] = 0.0f;
-#pragma unroll
-        for (int kt = 0; kt < kKTiles; ++kt) {
-            unsigned a[4];
-            ldmatrix_x4(a, q_s + tile_offset<D_PAD>((mi & 1) * 8 + lr, kt * 2 + (mi >> 1)));
-#pragma unroll
-            for (int np = 0; np < TN / 16; ++np) {
-                unsigned b[4];
-                ldmatrix_x4(b, k_t + tile_offset<D_PAD>(np * 16 + (mi >> 1) * 8 + lr, kt * 2 + (mi & 1)));
-                mma_bf16(s[2 * np], a, b[0], b[1]);
-                mma_bf16(s[2 * np + 1], a, b[2], b[3]);
-            }
-        }
-        float tile_max[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-        for (int nt = 0; nt < TN / 8; ++nt) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int key = tile_begin + nt * 8 + c2 + (e & 1);
-                float v = key < end ? (p.cap_log2 > 0.0f ? p.cap_log2 * quick_tanh(s[nt][e] * p.cap_in) : s[nt][e] * scale_log2)
-                                    : -INFINITY;
-                if (p.distance_bias && key < end) {
-                    // a learned number per (head, distance back to the key) joins the scaled score, in units of log2
-                    const int row = min(g + (e >> 1) * 8, group - 1);      // (rows past the group are never stored)
-                    v += __ldg(p.distance_bias + (size_t)(kvh * group + row) * (p.distance_last + 1) +
-                               max(0, min(pos - key, p.distance_last))) * 1.4426950408889634f;
-                }
-                s[nt][e] = v;
-                tile_max[e >> 1] = fmaxf(tile_max[e >> 1], v);
-            }
-        }
-        float correction[2], safe_max[2];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float m = tile_max[half];
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-            const float new_max = fmaxf(run_max[half], m);
-            correction[half] = new_max == -INFINITY ? 1.0f : exp2f(run_max[half] - new_max);
-            safe_max[half] = new_max == -INFINITY ? 0.0f : new_max;
-            run_max[half] = new_max;
-            run_sum[half] *= correction[half];
-        }
-#pragma unroll
-        for (int nt = 0; nt < TN / 8; ++nt) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float pv = exp2f(s[nt][e] - safe_max[e >> 1]);
-                s[nt][e] = pv;
-                run_sum[e >> 1] += pv;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kOTiles; ++i) {
-            o[i][0] *= correction[0];
-            o[i][1] *= correction[0];
-            o[i][2] *= correction[1];
-            o[i][3] *= correction[1];
-        }
-#pragma unroll
-        for (int kt = 0; kt < TN / 16; ++kt) {
-            unsigned a[4];
-            a[0] = pack_bf16(s[2 * kt][0], s[2 * kt][1]);
-            a[1] = pack_bf16(s[2 * kt][2], s[2 * kt][3]);
-            a[2] = pack_bf16(s[2 * kt + 1][0], s[2 * kt + 1][1]);
-            a[3] = pack_bf16(s[2 * kt + 1][2], s[2 * kt + 1][3]);
-#pragma unroll
-            for (int np = 0; np < kOTiles / 2; ++np) {
-                unsigned b[4];
-                ldmatrix_x4_trans(b, v_t + tile_offset<D_PAD>(kt * 16 + (mi & 1) * 8 + lr, np * 2 + (mi >> 1)));
-                mma_bf16(o[2 * np], a, b[0], b[1]);
-                mma_bf16(o[2 * np + 1], a, b[2], b[3]);
-            }
-        }
+        rows.take(p, q_s, k_t, v_t, tile_begin, end, pos, kvh, group, lane);
         __syncwarp();                                  // every lane is done with the tile before it is refilled
     }
     // a row's sum over the four lanes that share it; the warp's accumulators are the item's result
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-        run_sum[half] += __shfl_xor_sync(0xffffffffu, run_sum[half], 1);
-        run_sum[half] += __shfl_xor_sync(0xffffffffu, run_sum[half], 2);
+        rows.run_sum[half] += __shfl_xor_sync(0xffffffffu, rows.run_sum[half], 1);
+        rows.run_sum[half] += __shfl_xor_sync(0xffffffffu, rows.run_sum[half], 2);
     }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int r = g + half * 8;
         if (r >= group) continue;
         // (a sink adds its weight relative to the row's maximum to the denominator)
-        const float sink_part = p.sinks ? exp2f(p.sinks[kvh * group + r] * 1.4426950408889634f - run_max[half]) : 0.0f;
-        const float inv = 1.0f / (run_sum[half] + sink_part);
+        const float sink_part = p.sinks ? exp2f(p.sinks[kvh * group + r] * 1.4426950408889634f - rows.run_max[half]) : 0.0f;
+        const float inv = 1.0f / (rows.run_sum[half] + sink_part);
         __nv_bfloat16* dst = p.out + ((size_t)t * p.q_heads + kvh * group + r) * d;
 #pragma unroll
         for (int i = 0; i < kOTiles; ++i) {
             const int col = i * 8 + c2;
             if (col + 1 < d) {
-                *reinterpret_cast<__nv_bfloat162*>(dst + col) = __floats2bfloat162_rn(o[i][half * 2] * inv, o[i][half * 2 + 1] * inv);
+                *reinterpret_cast<__nv_bfloat162*>(dst + col) = __floats2bfloat162_rn(rows.o[i][half * 2] * inv, rows.o[i][half * 2 + 1] * inv);
             } else if (col < d) {
-                dst[col] = __float2bfloat16_rn(o[i][half * 2] * inv);
+                dst[col] = __float2bfloat16_rn(rows.o[i][half * 2] * inv);
             }
         }
     }
