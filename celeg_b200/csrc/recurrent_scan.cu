@@ -386,6 +386,92 @@ __global__ void delta_prepare_kernel(const DeltaPrepareArgs a) {
     }
 }
 
+// The same over portions of many tokens with four taps: a thread four channels of kTile tokens in a row. Their kernels stay in
+// registers and a row is loaded once, plus three before the tile (a block a token reads a row four times and 64 bytes of kernels
+// a thread for every token); the lanes of a head add up its squares among themselves, so nothing goes through shared memory.
+// DIM / 4 lanes are a head of q or k, so a head's lanes are neighbours of one warp.
+constexpr int kPrepareThreads = 128;
+constexpr int kPrepareTile = 8, kPrepareTileTokens = 64;
+template <int DIM, int kTile>
+__global__ void __launch_bounds__(kPrepareThreads) delta_prepare_tile_kernel(const DeltaPrepareArgs a) {
+    chain_release();
+    chain_wait();
+    const int c = (blockIdx.x * kPrepareThreads + threadIdx.x) * 4;
+    const int t0 = blockIdx.y * kTile, t1 = min(t0 + kTile, a.tokens);
+    const bool mine = c < a.channels, of_head = c < 2 * a.qk_heads * DIM;
+    float4 x[kTile + 3], w[4];
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // (the rows before the tile before it is known whether they are of its first token's span)
+#pragma unroll
+    for (int i = 0; i < kTile + 3; ++i) {
+        const int t = t0 - 3 + i;
+        x[i] = mine && t >= 0 && t < t1 ? *reinterpret_cast<const float4*>(a.proj + (size_t)t * a.stride + c) : zero;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = mine ? __ldg(reinterpret_cast<const float4*>(a.kernel + (size_t)(c + j) * 4)) : zero;
+    int span = a.token_span[t0];
+    const int last_span = a.token_span[t1 - 1];
+    float4 history[3];
+    auto begin_span = [&](int t) {                           // the three inputs before token t, its span's or carried
+        const int begin = a.span_begin[span];
+        const float* carried = a.carried + (long long)a.span_slot[span] * a.slot_stride;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int s = t - begin - 3 + j;
+            if (mine)
+                history[j] = *reinterpret_cast<const float4*>(s >= 0 ? a.proj + (size_t)(begin + s) * a.stride + c
+                                                                     : carried + (size_t)(3 + s) * a.channels + c);
+        }
+    };
+#pragma unroll
+    for (int j = 0; j < 3; ++j) history[j] = x[j];
+    if (t0 - a.span_begin[span] < 3) begin_span(t0);
+#pragma unroll
+    for (int i = 0; i < kTile; ++i) {
+        const int t = t0 + i;
+        if (t >= t1) break;
+        if (i > 0 && span != last_span && a.token_span[t] != span) {
+            span = a.token_span[t];
+            begin_span(t);
+        }
+        const float4 own = x[i + 3];
+        float4 sum;
+        // (the same order of additions as the kernel of a token a block: tap 0 first)
+        sum.x = fmaf(w[0].w, own.x, fmaf(w[0].z, history[2].x, fmaf(w[0].y, history[1].x, w[0].x * history[0].x)));
+        sum.y = fmaf(w[1].w, own.y, fmaf(w[1].z, history[2].y, fmaf(w[1].y, history[1].y, w[1].x * history[0].y)));
+        sum.z = fmaf(w[2].w, own.z, fmaf(w[2].z, history[2].z, fmaf(w[2].y, history[1].z, w[2].x * history[0].z)));
+        sum.w = fmaf(w[3].w, own.w, fmaf(w[3].z, history[2].w, fmaf(w[3].y, history[1].w, w[3].x * history[0].w)));
+        history[0] = history[1];
+        history[1] = history[2];
+        history[2] = own;
+        sum.x = sum.x / (1.0f + expf(-sum.x));
+        sum.y = sum.y / (1.0f + expf(-sum.y));
+        sum.z = sum.z / (1.0f + expf(-sum.z));
+        sum.w = sum.w / (1.0f + expf(-sum.w));
+        if ((int)(blockIdx.x * kPrepareThreads) * 4 < 2 * a.qk_heads * DIM) {      // (the same for a block's threads)
+            float squares = of_head ? sum.x * sum.x + sum.y * sum.y + sum.z * sum.z + sum.w * sum.w : 0.0f;
+#pragma unroll
+            for (int o = DIM / 8; o > 0; o >>= 1) squares += __shfl_xor_sync(0xffffffffu, squares, o);
+            if (of_head) {
+                const float inv = 1.0f / sqrtf(squares + a.unit_eps);
+                sum.x *= inv; sum.y *= inv; sum.z *= inv; sum.w *= inv;
+            }
+        }
+        if (mine) *reinterpret_cast<float4*>(a.conv_out + (size_t)t * a.channels + c) = sum;
+    }
+    if (blockIdx.x == gridDim.x - 1) {                       // (the last block along the channels may have few of them)
+        for (int i = threadIdx.x; i < (t1 - t0) * a.heads; i += kPrepareThreads) {
+            const size_t t = t0 + i / a.heads;
+            const int h = i % a.heads;
+            const float b = a.pre_beta[t * a.gate_stride + h];
+            const float z = a.pre_a[t * a.gate_stride + h] + a.dt_bias[h];
+            const float soft = fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z)));
+            a.gates[t * 2 * a.heads + h] = 1.0f / (1.0f + expf(-b));
+            a.gates[t * 2 * a.heads + a.heads + h] = expf(-expf(a.a_log[h]) * soft);
+        }
+    }
+}
+
 // The carried inputs after a step: the last taps - 1 inputs of each request's sequence. One thread per
 // (span, channel) reads everything it needs before it writes, so the update is in place.
 __global__ void carried_inputs_update_kernel(const float* proj, int stride, float* carried, long long slot_stride,
@@ -963,7 +1049,14 @@ CELEG_API int celeg_delta_prepare(const float* proj, int stride, const float* ke
     args.vector_loads =
         channels % 4 == 0 && stride % 4 == 0 && slot_stride % 4 == 0 &&
         (((size_t)proj | (size_t)carried | (size_t)conv_out) & 15) == 0;
-    launch_chained(delta_prepare_kernel, tokens, 256, (size_t)channels * sizeof(float), stream, args);
+    // Tiles of tokens where a step has enough of them to fill the GPU and every access is one of 16 bytes.
+    const bool tiles = taps == 4 && args.vector_loads && ((size_t)kernel & 15) == 0 && (dim == 32 || dim == 64 || dim == 128) &&
+                       tokens >= kPrepareTileTokens;
+    const dim3 grid((channels + 4 * kPrepareThreads - 1) / (4 * kPrepareThreads), (tokens + kPrepareTile - 1) / kPrepareTile);
+    if (tiles && dim == 32) launch_chained(delta_prepare_tile_kernel<32, kPrepareTile>, grid, kPrepareThreads, 0, stream, args);
+    else if (tiles && dim == 64) launch_chained(delta_prepare_tile_kernel<64, kPrepareTile>, grid, kPrepareThreads, 0, stream, args);
+    else if (tiles) launch_chained(delta_prepare_tile_kernel<128, kPrepareTile>, grid, kPrepareThreads, 0, stream, args);
+    else launch_chained(delta_prepare_kernel, tokens, 256, (size_t)channels * sizeof(float), stream, args);
     int status = check_launch("delta_prepare");
     if (status != 0 || taps == 1) return status;
     const long long units = (long long)spans * channels;
