@@ -68,7 +68,10 @@ __global__ void __launch_bounds__(128) channel_conv_kernel(const ChannelConvArgs
 #pragma unroll
     for (int i = 0; i < V; ++i) bias.v[i] = a.bias ? __ldg(a.bias + c + i) : 0.0f;
     auto finish = [&](int t, ConvPack<V> sum) {
-        if (a.act >= 0) {
+        if (a.act == kSilu) {                                // (as a rule; activate()'s other branches cost each number five)
+#pragma unroll
+            for (int i = 0; i < V; ++i) sum.v[i] = sum.v[i] / (1.0f + expf(-sum.v[i]));
+        } else if (a.act >= 0) {
 #pragma unroll
             for (int i = 0; i < V; ++i) sum.v[i] = activate(sum.v[i], a.act);
         }
@@ -81,23 +84,33 @@ __global__ void __launch_bounds__(128) channel_conv_kernel(const ChannelConvArgs
 #pragma unroll
         for (int i = 0; i < TILE; ++i)
             if (t0 + i < t1) ahead[i] = conv_load<V>(a.in + (size_t)(t0 + i) * a.in_stride + c);
-        int span = -1;
+        // The inputs before the tile are asked for with the tile's own, before it is known whether they belong to its first
+        // token's span; where they do not, the carried ones take their place.
+#pragma unroll
+        for (int j = 0; j < TAPS - 1; ++j)
+            if (!a.single && t0 - (TAPS - 1) + j >= 0) history[j] = conv_load<V>(a.in + (size_t)(t0 - (TAPS - 1) + j) * a.in_stride + c);
+        int span = TAPS > 1 ? a.token_span[t0] : 0;
         const int last_span = TAPS > 1 ? a.token_span[t1 - 1] : 0;
+        auto begin_span = [&](int t, bool all) {
+            const int begin = a.span_begin[span];
+            if (!all && t - begin >= TAPS - 1) return;
+            const float* carried = a.carried + (long long)a.span_slot[span] * a.slot_stride;
+#pragma unroll
+            for (int j = 0; j < TAPS - 1; ++j) {
+                const int s = t - begin - (TAPS - 1) + j;
+                if (s < 0) history[j] = conv_load<V>(carried + (size_t)(TAPS - 1 + s) * a.channels + c);
+                else if (all) history[j] = conv_load<V>(a.in + (size_t)(begin + s) * a.in_stride + c);
+            }
+        };
+        if (TAPS > 1) begin_span(t0, false);
 #pragma unroll
         for (int i = 0; i < TILE; ++i) {
             const int t = t0 + i;
             if (t >= t1) continue;
-            // the tile's first token, or a span that begins here (only where the tile's last token is of a later span)
-            if (TAPS > 1 && (i == 0 || (span != last_span && a.token_span[t] != span))) {
+            // a span that begins here (only where the tile's last token is of a later span)
+            if (TAPS > 1 && i > 0 && span != last_span && a.token_span[t] != span) {
                 span = a.token_span[t];
-                const int begin = a.span_begin[span];
-                const float* carried = a.carried + (long long)a.span_slot[span] * a.slot_stride;
-#pragma unroll
-                for (int j = 0; j < TAPS - 1; ++j) {
-                    const int s = t - begin - (TAPS - 1) + j;
-                    history[j] = conv_load<V>(s >= 0 ? a.in + (size_t)(begin + s) * a.in_stride + c
-                                                     : carried + (size_t)(TAPS - 1 + s) * a.channels + c);
-                }
+                begin_span(t, true);
             }
             ConvPack<V> sum;
 #pragma unroll
