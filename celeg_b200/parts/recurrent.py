@@ -126,13 +126,6 @@ class MlstmMixer(PortionsInChunks):
         rt, t, b = self.rt, step.tokens, self.binding
         rt.linear(x, self.w_in, self.projected, t)
         rows = self.projected
-        at = 0
-        q = rows[:, at:at + self.qk_width]; at += self.qk_width
-        k = rows[:, at:at + self.qk_width]; at += self.qk_width
-        v = rows[:, at:at + self.v_width]; at += self.v_width
-        gate = rows[:, at:at + self.v_width]; at += self.v_width
-        pre_i = rows[:, at:at + self.heads]; at += self.heads
-        pre_f = rows[:, at:at + self.heads]
         if step.max_span == 1 and step.spans == t:
             # every request brings one token: gates, state update, read-out, norm and output gate in one launch
             width = self.qk_width
@@ -144,6 +137,13 @@ class MlstmMixer(PortionsInChunks):
                                      self.gated)
             rt.linear(self.gated, self.w_out, out, t)
             return
+        at = 0
+        q = rows[:, at:at + self.qk_width]; at += self.qk_width
+        k = rows[:, at:at + self.qk_width]; at += self.qk_width
+        v = rows[:, at:at + self.v_width]; at += self.v_width
+        gate = rows[:, at:at + self.v_width]; at += self.v_width
+        pre_i = rows[:, at:at + self.heads]; at += self.heads
+        pre_f = rows[:, at:at + self.heads]
         # long portions in chunks; what lies before them (single tokens), and steps of short spans, token by token
         one_by_one = self.leading(step)
         if one_by_one:
@@ -243,9 +243,6 @@ class GatedDeltaMixer(PortionsInChunks):
         rt.linear(x, self.w_in, self.projected, t)
         rows = self.projected
         at = self.channels
-        gate = rows[:, at:at + self.v_width]; at += self.v_width
-        pre_beta = rows[:, at:at + self.heads]; at += self.heads
-        pre_a = rows[:, at:at + self.heads]
         if step.max_span == 1 and step.spans == t:
             # every request brings one token: convolutions, unit norms, gates, state update, read-out, norm and
             # output gate in one launch, the carried inputs in a second
@@ -257,6 +254,9 @@ class GatedDeltaMixer(PortionsInChunks):
                                      self.heads, self.kv_heads, self.dim, self.vdim, self.dim ** -0.5, self.gated)
             rt.linear(self.gated, self.w_out, out, t)
             return
+        gate = rows[:, at:at + self.v_width]; at += self.v_width
+        pre_beta = rows[:, at:at + self.heads]; at += self.heads
+        pre_a = rows[:, at:at + self.heads]
         kernels.delta_prepare(rows, self.kernel, self.carried, b.slot_stride, step.token_span, step.span_begin,
                               step.span_slot, self.convolved, pre_beta, pre_a, self.a_log, self.dt_bias, self.gates,
                               t, step.spans, self.channels, self.taps, self.kv_heads, self.dim, self.heads,
