@@ -248,30 +248,39 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                 drain_ring(max(0, v_brought - kStages), v_brought, kStages,
                            [&](int stage, unsigned parity) { mbar_wait_suspended(vf + 8u * stage, parity); });
             }
-        } else if (warp == 1 && lane == 0) {
+        } else if (warp == 1) {
             // ---------------------------------------------------------------- MMA issuer
+            // The whole warp waits, one elected lane issues: what the instructions are given is the same in all lanes then, and
+            // is made once in uniform registers. (Issued under `lane == 0` every one of a block's eight products moved its
+            // descriptors there again, 700 cycles a block.)
             constexpr unsigned idesc_s = instruction_descriptor(kFaM, kFaN);
             constexpr unsigned idesc_o = instruction_descriptor_b_mn(kFaM, 64);      // (64 columns of O at a time)
             const int blocks = block_end - block_begin;
             const unsigned long long desc_q = smem_descriptor(q_addr);
+            auto wait = [&](unsigned long long& bar, int parity) {
+                return __all_sync(0xffffffffu, mbar_wait_suspended(smem_u32(&bar), (unsigned)parity)) != 0;
+            };
             // S of block i into its buffer, as soon as its keys are there
             auto scores = [&](int i) -> bool {
                 const int s = i % kStages;
-                if (!mbar_wait_suspended(smem_u32(&k_full[s]), (i / kStages) & 1)) return false;
-                if (L::kOverScores && i >= 2 && !mbar_wait_suspended(smem_u32(&o_full[i & 1]), ((i - 2) >> 1) & 1)) return false;
+                if (!wait(k_full[s], (i / kStages) & 1)) return false;
+                if (L::kOverScores && i >= 2 && !wait(o_full[i & 1], ((i - 2) >> 1) & 1)) return false;
                 tcgen05_fence_after();
                 const unsigned long long desc_k = smem_descriptor(k_addr + s * L::kKvBytes);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < D / kUmmaK; ++kk) {
-                    const unsigned long long half = kk >> 2, part = 2 * (kk & 3);
-                    umma_bf16(tmem_base + (unsigned)((i & 1) * kFaN), desc_q + half * (L::kQHalf >> 4) + part,
-                              desc_k + half * (L::kKvHalf >> 4) + part, idesc_s, kk > 0 ? 1u : 0u);
+                    for (int kk = 0; kk < D / kUmmaK; ++kk) {
+                        const unsigned long long half = kk >> 2, part = 2 * (kk & 3);
+                        umma_bf16(tmem_base + (unsigned)((i & 1) * kFaN), desc_q + half * (L::kQHalf >> 4) + part,
+                                  desc_k + half * (L::kKvHalf >> 4) + part, idesc_s, kk > 0 ? 1u : 0u);
+                    }
+                    umma_commit(smem_u32(&s_full[i & 1]));
+                    if (!L::kTogether) umma_commit(smem_u32(&k_empty[s]));
                 }
-                umma_commit(smem_u32(&s_full[i & 1]));
-                if (!L::kTogether) umma_commit(smem_u32(&k_empty[s]));
+                __syncwarp();
                 return true;
             };
-            if (!mbar_wait_suspended(smem_u32(&q_full), 0)) error = 62;
+            if (!wait(q_full, 0)) error = 62;
             if (!error && !scores(0)) error = 63;
             for (int i = 0; i < blocks && !error; ++i) {
                 // the scores of the next block run while the softmax threads are busy with this one (they
@@ -281,25 +290,27 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                     break;
                 }
                 const int s = i % kStages;
-                if (!mbar_wait_suspended(smem_u32(&p_full[i & 1]), (i >> 1) & 1) ||
-                    (!L::kTogether && !mbar_wait_suspended(smem_u32(&v_full[s]), (i / kStages) & 1))) {
+                if (!wait(p_full[i & 1], (i >> 1) & 1) || (!L::kTogether && !wait(v_full[s], (i / kStages) & 1))) {
                     error = 64;
                     break;
                 }
                 tcgen05_fence_after();
                 const unsigned long long desc_v = smem_descriptor(v_addr + s * L::kKvBytes);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < kFaN / kUmmaK; ++kk) {
+                    for (int kk = 0; kk < kFaN / kUmmaK; ++kk) {
 #pragma unroll
-                    for (int half = 0; half < L::kHalves; ++half) {
-                        // P: 16 keys = 8 columns of tensor memory; V: 16 keys further = 16 rows of 128 bytes = 2 KiB
-                        umma_bf16_a_tmem(tmem_base + L::kOColumn + half * 64, tmem_base + L::p_column(i) + (unsigned)(kk * 8),
-                                         desc_v + (unsigned long long)(half * (L::kKvHalf >> 4) + kk * 128), idesc_o,
-                                         (i > 0 || kk > 0) ? 1u : 0u);
+                        for (int half = 0; half < L::kHalves; ++half) {
+                            // P: 16 keys = 8 columns of tensor memory; V: 16 keys further = 16 rows of 128 bytes = 2 KiB
+                            umma_bf16_a_tmem(tmem_base + L::kOColumn + half * 64, tmem_base + L::p_column(i) + (unsigned)(kk * 8),
+                                             desc_v + (unsigned long long)(half * (L::kKvHalf >> 4) + kk * 128), idesc_o,
+                                             (i > 0 || kk > 0) ? 1u : 0u);
+                        }
                     }
+                    umma_commit(smem_u32(L::kTogether ? &k_empty[s] : &v_empty[s]));
+                    umma_commit(smem_u32(&o_full[i & 1]));
                 }
-                umma_commit(smem_u32(L::kTogether ? &k_empty[s] : &v_empty[s]));
-                umma_commit(smem_u32(&o_full[i & 1]));
+                __syncwarp();
             }
         } else if (warp >= 2) {
             // -------------------------------------------------------------------- softmax

@@ -89,6 +89,13 @@ __device__ __forceinline__ void tmem_dealloc(unsigned taddr, unsigned columns) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(columns) : "memory");
 }
 
+// One lane of a whole warp, always the same.
+__device__ __forceinline__ bool elect_one() {
+    unsigned elected;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(elected));
+    return elected != 0;
+}
+
 __device__ __forceinline__ void umma_bf16(unsigned tmem_d, unsigned long long desc_a, unsigned long long desc_b,
                                           unsigned idesc, unsigned accumulate) {
     asm volatile(
