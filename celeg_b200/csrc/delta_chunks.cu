@@ -288,6 +288,31 @@ template <int WIDTH, int COLUMNS> constexpr int delta_walk_bytes() {
             SplitTile<kChunk, COLUMNS>::kElements) * (int)sizeof(__nv_bfloat16);
 }
 
+// The B operands of columns n0 .. n0 + 7 of a tile that lies [k][n], depths k0 .. k0 + 15 and k0 + 16 .. k0 + 31
+template <typename T>
+__device__ __forceinline__ void load_b_two_deep(unsigned (*b)[3][2], const __nv_bfloat16* tile, int n0, int k0) {
+    const __nv_bfloat16* from = tile + T::at(k0 + (threadIdx.x & 31), n0 >> 3);
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+        unsigned r[4];
+        ldmatrix_x4_trans(r, from + n * T::kPlane);
+        b[0][n][0] = r[0]; b[0][n][1] = r[1]; b[1][n][0] = r[2]; b[1][n][1] = r[3];
+    }
+}
+// acc += a b over four depths of 16, the four chains of six side by side
+__device__ __forceinline__ void mma_four_deep(float (&acc)[4], const unsigned (&a)[4][3][4], const unsigned (&b)[4][3][2]) {
+    constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
+    float d[4][4] = {};
+#pragma unroll
+    for (int k6 = 0; k6 < 6; ++k6)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) mma_step(d[x], a[x][kA[k6]], b[x][kB[k6]]);
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[r] += d[x][r];
+}
+
 // COLUMNS of S a block: 16, or 32 where that is blocks enough. GENERAL: a decay a key channel, and the state is given what lies
 // in `states` of the chunk too.
 template <int WIDTH, int COLUMNS, bool GENERAL>
@@ -314,8 +339,10 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
+    int brought = 0;
     auto bring = [&](int i) {                                // thread 0: a chunk's two operands, one behind the other
         if (i >= chunks) return;
+        brought = i + 1;
         const unsigned bar = smem_u32(&full[i % kStages]);
         mbar_expect_tx(bar, kBytes);
         bulk_load(smem_u32(tiles + (i % kStages) * 2 * Tile::kElements),
@@ -352,23 +379,39 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
     put_s();
     float add[kTiles][4] = {}, keeps[2] = {1.0f, 1.0f};      // general: of the chunk to come
     float next[kUTiles][4], next_keep = 0.0f;                      // U_0 of the chunk to come, its decay
-    auto ask = [&](int i) {
+    // Where the thread's rows of S and u of a chunk lie: from one chunk to the next by a constant step. (Made anew from the chunk's
+    // number for every access they cost the walk a twentieth, the generalised rule's a tenth.)
+    const size_t s_step = (size_t)p.heads * dim * vdim, u_step = (size_t)kChunk * p.heads * vdim;
+    float* s_rows = p.states + (((size_t)first * p.heads + head) * dim + er + g) * vdim + c0 + sc + 2 * tig;
+    float* u_rows = p.u + (size_t)(t_begin + tr + g) * p.heads * vdim + (size_t)head * vdim + c0 + uc + 2 * tig;
+    const size_t s_eight = (size_t)8 * vdim, u_eight = (size_t)8 * p.heads * vdim;
+    const int s_left = vdim - (c0 + sc + 2 * tig), u_left = vdim - (c0 + uc + 2 * tig);      // columns from the thread's first on
+    auto fetch = [&](const float* src, bool row, int left) {
+        if (!row || left <= 0) return make_float2(0.0f, 0.0f);
+        if (two) return *reinterpret_cast<const float2*>(src);
+        return make_float2(src[0], left > 1 ? src[1] : 0.0f);
+    };
+    auto store = [&](float* dst, bool row, int left, float x, float y) {
+        if (!row || left <= 0) return;
+        if (two) *reinterpret_cast<float2*>(dst) = make_float2(x, y);
+        else {
+            dst[0] = x;
+            if (left > 1) dst[1] = y;
+        }
+    };
+    auto ask = [&](int i, const float* u_src, const float* s_src) {      // (the rows of chunk i)
         if (i >= chunks) return;
-        const int begin = t_begin + i * kChunk, count = min(kChunk, t_end - begin);
+        const int count = min(kChunk, t_end - (t_begin + i * kChunk));
 #pragma unroll
         for (int n = 0; n < kUTiles; ++n)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int t = tr + g + 8 * h, c = c0 + uc + 8 * n + 2 * tig;
-                const float* src = p.u + (size_t)(begin + t) * p.heads * vdim + (size_t)head * vdim + c;
-                float2 x = make_float2(0.0f, 0.0f);
-                if (t < count && two && c < vdim) x = *reinterpret_cast<const float2*>(src);
-                else if (t < count && c < vdim) x = make_float2(src[0], c + 1 < vdim ? src[1] : 0.0f);
+                const float2 x = fetch(u_src + h * u_eight + 8 * n, tr + g + 8 * h < count, u_left - 8 * n);
                 next[n][2 * h] = x.x;
                 next[n][2 * h + 1] = x.y;
             }
         if (!GENERAL) {
-            next_keep = p.cum[(size_t)(begin + count - 1) * p.heads + head].x;
+            next_keep = p.cum[(size_t)(t_begin + i * kChunk + count - 1) * p.heads + head].x;
             return;
         }
         const size_t rows = ((size_t)(first + i) * p.heads + head) * dim;
@@ -377,21 +420,13 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
 #pragma unroll
         for (int n = 0; n < kTiles; ++n)
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int e = er + g + 8 * (r >> 1), c = c0 + sc + 8 * n + 2 * tig + (r & 1);
-                add[n][r] = e < dim && c < vdim ? p.states[(rows + e) * vdim + c] : 0.0f;
+            for (int h = 0; h < 2; ++h) {
+                const float2 x = fetch(s_src + h * s_eight + 8 * n, er + g + 8 * h < dim, s_left - 8 * n);
+                add[n][2 * h] = x.x;
+                add[n][2 * h + 1] = x.y;
             }
     };
-    auto store = [&](float* dst, int r, int c, float x, float y) {     // dst: the row's columns from c0 on
-        if (c0 + c >= vdim) return;
-        if (two) *reinterpret_cast<float2*>(dst + c) = make_float2(x, y);
-        else {
-            dst[c] = x;
-            if (c0 + c + 1 < vdim) dst[c + 1] = y;
-        }
-    };
-    ask(0);
-    __syncthreads();
+    ask(0, u_rows, s_rows);
     auto odd_first = [](unsigned (*b)[3][2]) {               // the second tile of eight columns in the first's place
 #pragma unroll
         for (int n = 0; n < 3; ++n) {
@@ -399,10 +434,27 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
             b[0][n][1] = b[1][n][1];
         }
     };
+    // Key channels up to 64 and 16 columns: the chain of a chunk is two products deep, and what a warp multiplies S and u with
+    // does not wait for them. -W of the next chunk and G k of this one are in registers before the barriers that S and u come
+    // through, and the four depths of a product are four chains side by side. 32 heads of 64 x 64, 2,048 tokens: 62.4 us before,
+    // 54.5 with it and the constant steps (the generalised rule 67.6 and 58.6); of a chunk's 1.7 us the products are 0.5, what is
+    // left without products, loads and stores 0.5.
+    constexpr bool kHeld = WIDTH == 64 && COLUMNS == 16;
+    static_assert(!kHeld || (kTiles == 1 && kUTiles == 1 && kStages == 2), "");
+    unsigned held[kHeld ? 4 : 1][3][4];
     bool ok = true;
+    auto hold_w = [&](int i) {                               // (chunk i's operands, once they are there)
+        if constexpr (kHeld) {
+            ok = mbar_wait(smem_u32(&full[i % kStages]), (i / kStages) & 1);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) load_a<Tile>(held[x], tiles + (i % kStages) * 2 * Tile::kElements, tr, 16 * x);
+        }
+    };
+    hold_w(0);
+    ok = __syncthreads_and(ok);
     int i = 0;
-    for (; i < chunks; ++i) {
-        const int begin = t_begin + i * kChunk, count = min(kChunk, t_end - begin);
+    for (; i < chunks && ok; ++i, s_rows += s_step, u_rows += u_step) {
+        const int count = min(kChunk, t_end - (t_begin + i * kChunk));
         const __nv_bfloat16* w_t = tiles + (i % kStages) * 2 * Tile::kElements;
         const __nv_bfloat16* k_t = w_t + Tile::kElements;
         float u[kUTiles][4];
@@ -416,14 +468,20 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
         for (int n = 0; n < kTiles; ++n)
 #pragma unroll
             for (int r = 0; r < 4; ++r) given[n][r] = add[n][r];
-        ask(i + 1);
+        ask(i + 1, u_rows + u_step, s_rows + s_step);
 #pragma unroll
         for (int n = 0; n < kTiles; ++n)                     // the state before the chunk
 #pragma unroll
             for (int h = 0; h < 2; ++h)
-                if (er + g + 8 * h < dim)
-                    store(p.states + (((size_t)(first + i) * p.heads + head) * dim + er + g + 8 * h) * vdim + c0, 0,
-                          sc + 8 * n + 2 * tig, s[n][2 * h], s[n][2 * h + 1]);
+                store(s_rows + h * s_eight + 8 * n, er + g + 8 * h < dim, s_left - 8 * n, s[n][2 * h], s[n][2 * h + 1]);
+        if constexpr (kHeld) {
+            unsigned b[4][3][2];
+            load_b_two_deep<STile>(b, s_t, uc, 0);
+            load_b_two_deep<STile>(b + 2, s_t, uc, 32);
+            mma_four_deep(u[0], held, b);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) load_a_transposed<Tile>(held[x], k_t, er, 16 * x);
+        } else {
         ok = __syncthreads_and(mbar_wait(smem_u32(&full[i % kStages]), (i / kStages) & 1));
         if (!ok) break;
 #pragma unroll
@@ -450,17 +508,28 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
 #pragma unroll
                     for (int r = 0; r < 4; ++r) u[n][r] += d[x][n][r];
         }
+        }
 #pragma unroll
         for (int n = 0; n < kUTiles; ++n)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int t = tr + g + 8 * h, c = uc + 8 * n + 2 * tig;
                 put(u_t, UTile::at(t, c >> 3) + 2 * tig, UTile::kPlane, u[n][2 * h], u[n][2 * h + 1]);
-                if (t < count)
-                    store(p.u + (size_t)(begin + t) * p.heads * vdim + (size_t)head * vdim + c0, 0, c, u[n][2 * h], u[n][2 * h + 1]);
             }
         __syncthreads();
+#pragma unroll
+        for (int n = 0; n < kUTiles; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                store(u_rows + h * u_eight + 8 * n, tr + g + 8 * h < count, u_left - 8 * n, u[n][2 * h], u[n][2 * h + 1]);
         float sum[kTiles][4] = {};
+        if constexpr (kHeld) {
+            unsigned b[4][3][2];
+            load_b_two_deep<UTile>(b, u_t, sc, 0);
+            load_b_two_deep<UTile>(b + 2, u_t, sc, 32);
+            mma_four_deep(sum[0], held, b);
+            if (i + 1 < chunks) hold_w(i + 1);
+        } else {
 #pragma unroll
         for (int t = 0; t < kChunk; t += 32) {               // S = G S + sum_j G k_j u_j^T
             float d[2][kTiles][4] = {};
@@ -486,18 +555,21 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
 #pragma unroll
                     for (int r = 0; r < 4; ++r) sum[n][r] += d[x][n][r];
         }
+        }
 #pragma unroll
         for (int n = 0; n < kTiles; ++n)
 #pragma unroll
             for (int r = 0; r < 4; ++r) s[n][r] = fmaf(GENERAL ? kept[r >> 1] : keep, s[n][r], GENERAL ? sum[n][r] + given[n][r] : sum[n][r]);
         put_s();
-        __syncthreads();                                     // the operands have been used; the state is there
-        if (tid == 0) bring(i + kStages);
+        // the operands have been used; the state is there
+        if constexpr (kHeld) ok = __syncthreads_and(ok);
+        else __syncthreads();
+        if (tid == 0 && ok) bring(i + kStages);
     }
     if (!ok) {                             // a copy did not come: chunk i's and those behind it (nothing of the block's is left behind)
         if (tid == 0) {
             atomicExch(p.error_flag, 71);
-            drain_ring(i, min(chunks, i + kStages), kStages,
+            drain_ring(i, brought, kStages,
                        [&](int stage, unsigned parity) { mbar_wait(smem_u32(&full[stage]), parity); });
         }
         return;
@@ -856,7 +928,7 @@ static int launch_delta_chunks(const DeltaChunkArgs& p, int chunks, int spans, c
     launch_chained(delta_solve_kernel<WIDTH>, dim3(p.heads, chunks), kSolveThreads, bytes, stream, p);
     if ((status = check_launch("delta_solve")) != 0) return status;
     // A chunk is two products and two barriers deep however few columns a block has: 16 of them while the blocks are no more
-    // than the SMs (32 heads of 64 x 64, one span of 2,048 tokens: 128 blocks 62 us, 64 blocks of 32 columns 73 us).
+    // than the SMs (32 heads of 64 x 64, one span of 2,048 tokens: 128 blocks 54 us, 64 blocks of 32 columns 73 us).
     const long long blocks = (long long)((p.vdim + 15) / 16) * p.heads * spans;
     return blocks <= 148 ? launch_delta_walk<WIDTH, 16, false>(p, spans, stream) : launch_delta_walk<WIDTH, 32, false>(p, spans, stream);
 }
