@@ -41,14 +41,7 @@ __global__ void chunk_plan_kernel(const int* span_begin, int spans, int chunk, i
                                   int* span_first) {
     chain_release();
     chain_wait();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int n = 0;
-    for (int s = 0; s < spans; ++s) {
-        span_first[s] = n;
-        for (int b = span_begin[s]; b < span_begin[s + 1] && n < max_chunks; b += chunk) chunk_begin[n++] = b;
-    }
-    span_first[spans] = n;
-    for (int i = n; i <= max_chunks; ++i) chunk_begin[i] = span_begin[spans];      // (chunks beyond the last are empty)
+    plan_runs(span_begin, spans, chunk, max_chunks, chunk_begin, span_first);
 }
 
 // ------------------------------------------------------------------------------------------------- prepare, scalar
@@ -399,7 +392,7 @@ CELEG_API int celeg_chunk_state_launches(int heads, int dim, int vdim, int spans
 // plan: ints [max_chunks + 1 | spans + 1]: the chunks' first tokens (the last chunk's end at the end), the spans' first chunks
 CELEG_API int celeg_chunk_plan(const int* span_begin, int spans, int max_chunks, int* plan, cudaStream_t stream) {
     CELEG_REQUIRE(spans >= 0 && max_chunks > 0, "chunk_plan: %d spans, %d chunks", spans, max_chunks);
-    launch_chained(chunk_plan_kernel, 1, 32, 0, stream, span_begin, spans, kChunk, max_chunks, plan, plan + max_chunks + 1);
+    launch_chained(chunk_plan_kernel, 1, 128, 0, stream, span_begin, spans, kChunk, max_chunks, plan, plan + max_chunks + 1);
     return check_launch("chunk_plan");
 }
 

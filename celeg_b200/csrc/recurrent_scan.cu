@@ -585,10 +585,11 @@ __global__ void __launch_bounds__(128) gated_head_norm_quads_kernel(const float*
     chain_release();
     chain_wait();
     const int lane = threadIdx.x % LANES;
-    const long long units = (long long)tokens * heads, unit = (long long)blockIdx.x * (128 / LANES) + threadIdx.x / LANES;
+    // (32 bits: a quotient of 64 costs more instructions than all the rest)
+    const unsigned units = (unsigned)tokens * (unsigned)heads, unit = blockIdx.x * (128 / LANES) + threadIdx.x / LANES;
     const bool real = unit < units;                          // (every lane of a warp comes to the shuffles)
-    const long long mine = real ? unit : units - 1;
-    const int t = (int)(mine / heads), h = (int)(mine % heads);
+    const size_t mine = real ? unit : units - 1;
+    const int t = (int)((unsigned)mine / (unsigned)heads), h = (int)((unsigned)mine - (unsigned)t * (unsigned)heads);
     float4 x = reinterpret_cast<const float4*>(o)[mine * LANES + lane];
     const float4 g = *reinterpret_cast<const float4*>(gate + (size_t)t * gate_stride + (size_t)(h * LANES + lane) * 4);
     const float4 w = weight ? __ldg(reinterpret_cast<const float4*>(weight) + (weight_per_head ? h * LANES : 0) + lane)
@@ -634,10 +635,10 @@ __global__ void __launch_bounds__(128) gated_unit_norm_kernel(const float* o, co
                                                               int heads, int vdim, float eps, int gate_kind) {
     chain_release();
     chain_wait();
-    const long long unit = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (unit >= (long long)tokens * heads) return;
+    const unsigned unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (unit >= (unsigned)tokens * (unsigned)heads) return;
     const int lane = threadIdx.x & 31;
-    const int t = (int)(unit / heads), h = (int)(unit % heads);
+    const int t = (int)(unit / (unsigned)heads), h = (int)(unit - (unsigned)t * (unsigned)heads);
     const float4* src = reinterpret_cast<const float4*>(o + ((size_t)t * heads + h) * vdim);
     const float4* g = reinterpret_cast<const float4*>(gate + (size_t)t * gate_stride + (size_t)h * vdim);
     const float4* w = reinterpret_cast<const float4*>(weight ? weight + (weight_per_head ? (size_t)h * vdim : 0) : nullptr);
@@ -962,14 +963,7 @@ __global__ void retention_plan_kernel(const int* span_begin, int spans, int segm
                                       int* span_first) {
     chain_release();
     chain_wait();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int n = 0;
-    for (int s = 0; s < spans; ++s) {
-        span_first[s] = n;
-        for (int b = span_begin[s]; b < span_begin[s + 1] && n < max_segments; b += segment) seg_begin[n++] = b;
-    }
-    span_first[spans] = n;
-    for (int i = n; i <= max_segments; ++i) seg_begin[i] = span_begin[spans];      // (segments beyond the last are empty)
+    plan_runs(span_begin, spans, segment, max_segments, seg_begin, span_first);
 }
 
 template <int MODE>
@@ -1073,7 +1067,7 @@ CELEG_API int celeg_gated_head_norm(const float* o, const float* gate, int gate_
                   gate_kind);
     if (tokens == 0) return 0;
     const long long units = (long long)tokens * heads;
-    if (vdim > 128 && vdim <= 1024 && units >= 2048 && vdim % 4 == 0 && gate_stride % 4 == 0 &&
+    if (vdim > 128 && vdim <= 1024 && units >= 2048 && units <= 0x7fffffffLL && vdim % 4 == 0 && gate_stride % 4 == 0 &&
         (act_dtype == kFloat32 || act_dtype == kBFloat16) &&
         (((uintptr_t)o | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out) & 15) == 0) {
         if (act_dtype == kFloat32)
@@ -1096,7 +1090,7 @@ CELEG_API int celeg_gated_head_norm(const float* o, const float* gate, int gate_
             CELEG_REQUIRE(false, "gated_head_norm: unknown dtype code %d", act_dtype);
         return check_launch("gated_head_norm");
     }
-    if ((vdim == 16 || vdim == 32 || vdim == 64 || vdim == 128) && gate_stride % 4 == 0 &&
+    if ((vdim == 16 || vdim == 32 || vdim == 64 || vdim == 128) && units <= 0x7fffffffLL && gate_stride % 4 == 0 &&
         (act_dtype == kFloat32 || act_dtype == kBFloat16) && (((uintptr_t)o | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out) & 15) == 0) {
         if (act_dtype == kFloat32)
             launch_quads_norm<float>(o, gate, gate_stride, weight, weight_per_head, (float*)out, tokens, heads, vdim, eps, gate_kind, stream);
@@ -1230,7 +1224,7 @@ CELEG_API int celeg_retention_segmented(const float* q, int q_stride, const floa
     const int pieces = segment / 64;
     CELEG_REQUIRE((long long)max_segments * pieces <= 65535, "retention_segmented: %d segments of %d pieces exceed one launch",
                   max_segments, pieces);
-    launch_chained(retention_plan_kernel, 1, 32, 0, stream, span_begin, spans, segment, max_segments, seg_begin, span_first);
+    launch_chained(retention_plan_kernel, 1, 128, 0, stream, span_begin, spans, segment, max_segments, seg_begin, span_first);
     const int status = check_launch("retention_plan");
     if (status != 0) return status;
     ChunkArgs p = {};
