@@ -26,7 +26,18 @@ namespace celeg_b200 {
 
 constexpr int kAccRegs = 16;     // value_dim <= 32 * kAccRegs
 
-template <typename A>
+__device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_four(const __nv_bfloat16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
+// REGS: registers of the weighted sum, value_dim <= 32 * REGS (a loop over all that a value may need costs one that needs few
+// more instructions than its products). FOUR: a key is read four numbers at a time, added in the same order. 480 tokens of 16
+// heads of 128 in float32: 349 us, 1,145 number by number and with 16 registers.
+template <typename A, int REGS, bool FOUR>
 __global__ void attention_generic_kernel(const A* __restrict__ q, int q_row_stride, A* __restrict__ out,
                                          const A* __restrict__ k_cache, const A* __restrict__ v_cache,
                                          long long page_stride, long long value_page_stride,
@@ -53,9 +64,9 @@ __global__ void attention_generic_kernel(const A* __restrict__ q, int q_row_stri
     for (int i = lane; i < head_dim; i += 32) qs[i] = to_float(qv[i]) * scale;
     __syncwarp();
 
-    float acc[kAccRegs];
+    float acc[REGS];
 #pragma unroll
-    for (int r = 0; r < kAccRegs; ++r) acc[r] = 0.0f;
+    for (int r = 0; r < REGS; ++r) acc[r] = 0.0f;
     // a sink is a score without key or value: the softmax starts from it (weight 1 at the maximum so far)
     float running_max = sinks ? sinks[h] : -INFINITY;
     float denom = sinks ? 1.0f : 0.0f;
@@ -75,7 +86,18 @@ __global__ void attention_generic_kernel(const A* __restrict__ q, int q_row_stri
                 offset = (long long)page * value_page_stride + place * value_dim;
                 const A* kv = k_cache + (long long)page * page_stride + place * head_dim;
                 float s = 0.0f;
-                for (int i = 0; i < head_dim; ++i) s += qs[i] * to_float(kv[i]);
+                if (FOUR) {
+#pragma unroll 4
+                    for (int i = 0; i < head_dim; i += 4) {
+                        const float4 x = load_four(kv + i);
+                        s += qs[i] * x.x;
+                        s += qs[i + 1] * x.y;
+                        s += qs[i + 2] * x.z;
+                        s += qs[i + 3] * x.w;
+                    }
+                } else {
+                    for (int i = 0; i < head_dim; ++i) s += qs[i] * to_float(kv[i]);
+                }
                 if (softcap > 0.0f) s = softcap * tanhf(s / softcap);
                 // a learned number per (head, distance back to the key), added to the scaled score as it is
                 if (distance_bias) s += distance_bias[(size_t)h * (distance_last + 1) + min(pos - key, distance_last)];
@@ -89,15 +111,16 @@ __global__ void attention_generic_kernel(const A* __restrict__ q, int q_row_stri
         const float p = score == -INFINITY ? 0.0f : expf(score - new_max);
         denom = denom * correction + warp_sum(p);
 #pragma unroll
-        for (int r = 0; r < kAccRegs; ++r) acc[r] *= correction;
+        for (int r = 0; r < REGS; ++r) acc[r] *= correction;
         running_max = new_max;
         const int count = min(32, pos - base + 1);
+#pragma unroll 4
         for (int j = 0; j < count; ++j) {
             const float pj = __shfl_sync(0xffffffffu, p, j);
             const long long oj = __shfl_sync(0xffffffffu, offset, j);
             const A* vv = v_cache + oj;
 #pragma unroll
-            for (int r = 0; r < kAccRegs; ++r) {
+            for (int r = 0; r < REGS; ++r) {
                 const int i = lane + 32 * r;
                 if (i < value_dim) acc[r] += pj * to_float(vv[i]);
             }
@@ -106,10 +129,32 @@ __global__ void attention_generic_kernel(const A* __restrict__ q, int q_row_stri
     const float inv = denom > 0.0f ? 1.0f / denom : 0.0f;
     A* ov = out + ((size_t)t * q_heads + h) * value_dim;
 #pragma unroll
-    for (int r = 0; r < kAccRegs; ++r) {
+    for (int r = 0; r < REGS; ++r) {
         const int i = lane + 32 * r;
         if (i < value_dim) ov[i] = from_float<A>(acc[r] * inv);
     }
+}
+
+template <typename A>
+static void launch_generic(const A* q, int q_row_stride, A* out, const A* k_cache, const A* v_cache, long long page_stride,
+                           long long value_page_stride, const int* positions, const int* token_span, const int* block_table,
+                           int table_stride, int tokens, int q_heads, int kv_heads, int head_dim, int value_dim, int page_tokens,
+                           int window, int chunk, float scale, const float* sinks, const float* distance_bias, int distance_last,
+                           float softcap, int* error_flag, cudaStream_t stream) {
+    const int warps = 4;
+    const long long units = (long long)tokens * q_heads;
+    const unsigned blocks = (unsigned)((units + warps - 1) / warps);
+    const size_t smem = (size_t)warps * head_dim * sizeof(float);
+    const bool four = head_dim % 4 == 0 && page_stride % 4 == 0 && ((size_t)k_cache & (4 * sizeof(A) - 1)) == 0;
+    auto kernel = attention_generic_kernel<A, 16, false>;
+    if (value_dim <= 64) kernel = four ? attention_generic_kernel<A, 2, true> : attention_generic_kernel<A, 2, false>;
+    else if (value_dim <= 128) kernel = four ? attention_generic_kernel<A, 4, true> : attention_generic_kernel<A, 4, false>;
+    else if (value_dim <= 256) kernel = four ? attention_generic_kernel<A, 8, true> : attention_generic_kernel<A, 8, false>;
+    else if (four) kernel = attention_generic_kernel<A, 16, true>;
+    kernel<<<blocks, warps * 32, smem, stream>>>(q, q_row_stride, out, k_cache, v_cache, page_stride, value_page_stride, positions,
+                                                 token_span, block_table, table_stride, tokens, q_heads, kv_heads, head_dim, value_dim,
+                                                 page_tokens, window, chunk, scale, sinks, distance_bias, distance_last, softcap,
+                                                 error_flag);
 }
 
 }  // namespace celeg_b200
@@ -139,22 +184,16 @@ CELEG_API int celeg_attention_generic(const void* q, int q_row_stride, void* out
     CELEG_REQUIRE(value_dim <= 32 * kAccRegs, "attention: a value size of %d exceeds %d", value_dim, 32 * kAccRegs);
     CELEG_REQUIRE(chunk >= 0 && (chunk == 0 || window == 0), "attention: a chunk of %d beside a window of %d", chunk, window);
     if (tokens == 0) return 0;
-    const int warps = 4;
-    const long long units = (long long)tokens * q_heads;
-    const unsigned blocks = (unsigned)((units + warps - 1) / warps);
-    const size_t smem = (size_t)warps * head_dim * sizeof(float);
     if (act_dtype == kFloat32)
-        attention_generic_kernel<float><<<blocks, warps * 32, smem, stream>>>(
-            (const float*)q, q_row_stride, (float*)out, (const float*)k_cache, (const float*)v_cache, page_stride,
-            value_page_stride, positions, token_span, block_table, table_stride, tokens, q_heads, kv_heads, head_dim,
-            value_dim, page_tokens, window, chunk, scale, sinks, distance_bias, distance_last, softcap,
-            error_flag);
+        launch_generic<float>((const float*)q, q_row_stride, (float*)out, (const float*)k_cache, (const float*)v_cache, page_stride,
+                              value_page_stride, positions, token_span, block_table, table_stride, tokens, q_heads, kv_heads, head_dim,
+                              value_dim, page_tokens, window, chunk, scale, sinks, distance_bias, distance_last, softcap, error_flag,
+                              stream);
     else if (act_dtype == kBFloat16)
-        attention_generic_kernel<__nv_bfloat16><<<blocks, warps * 32, smem, stream>>>(
-            (const __nv_bfloat16*)q, q_row_stride, (__nv_bfloat16*)out, (const __nv_bfloat16*)k_cache,
-            (const __nv_bfloat16*)v_cache, page_stride, value_page_stride, positions, token_span, block_table,
-            table_stride, tokens, q_heads, kv_heads, head_dim, value_dim, page_tokens, window, chunk, scale, sinks,
-            distance_bias, distance_last, softcap, error_flag);
+        launch_generic<__nv_bfloat16>((const __nv_bfloat16*)q, q_row_stride, (__nv_bfloat16*)out, (const __nv_bfloat16*)k_cache,
+                                      (const __nv_bfloat16*)v_cache, page_stride, value_page_stride, positions, token_span, block_table,
+                                      table_stride, tokens, q_heads, kv_heads, head_dim, value_dim, page_tokens, window, chunk, scale,
+                                      sinks, distance_bias, distance_last, softcap, error_flag, stream);
     else
         CELEG_REQUIRE(false, "attention: unknown dtype code %d", act_dtype);
     return check_launch("attention_generic");
