@@ -1166,12 +1166,23 @@ inline int launch_read(const ChunkArgs& p, int chunks, int heads_a_block, cudaSt
 
 template <int MODE>
 inline int launch_reads(const ChunkArgs& p, int chunks, cudaStream_t stream) {
-    // heads that share queries and keys share a block's products of them, as long as the blocks fill the GPU
+    // Heads that share queries and keys share a block's products of them: as many as make the launch shortest, in rounds of the
+    // blocks that the GPU holds (four an SM, two with wide queries) times a block's steps (products of keys, then of the state's rows
+    // and of the values of every head). 64 heads on 8 of 128 x 64, 2,048 tokens: 96.8 us with
+    // eight heads a block (264 blocks, one round), 110 with four (528, two); 300 tokens 30.6 and 39.4 with one.
     int heads_a_block = 1;
-    if (MODE == kChunkScalar)
-        while (heads_a_block < 4 && (p.heads / p.groups) % (2 * heads_a_block) == 0 &&
-               (long long)chunks * p.heads / (2 * heads_a_block) >= 296)
-            heads_a_block *= 2;
+    if (MODE == kChunkScalar) {
+        const int per_head = ((p.dim + kReadRows - 1) / kReadRows + 2) * ((p.vdim + kReadColumns - 1) / kReadColumns);
+        const int shared = (p.dim + kReadRows - 1) / kReadRows + 2, slots = p.dim <= 64 ? 592 : 296;
+        long long best = 0;
+        for (int n = 1; n <= 8 && (p.heads / p.groups) % n == 0; n *= 2) {
+            const long long blocks = (long long)chunks * p.heads / n, cost = (blocks + slots - 1) / slots * (n * per_head + shared);
+            if (n == 1 || cost < best) {
+                best = cost;
+                heads_a_block = n;
+            }
+        }
+    }
     return p.dim <= 64 ? launch_read<MODE, 64>(p, chunks, heads_a_block, stream)
                        : launch_read<MODE, 128>(p, chunks, heads_a_block, stream);
 }
