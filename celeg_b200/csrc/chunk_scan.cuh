@@ -309,13 +309,14 @@ __device__ __forceinline__ void load_b_transposed(unsigned (*b)[3][2], const __n
 
 // -------------------------------------------------------------------------------------------------------------- walk
 constexpr int kWalkThreads = 256;
-constexpr int kWalkColumns = 32;                             // columns of S a block
+constexpr int kWalkColumns = 64;                             // columns of S a block: half the keys are split twice over for 32 of
+                                                             // them (64 heads of 128 x 64, 2,048 tokens: 81 us, with 32 88)
 constexpr int kWalkRows = 64;                                // and key channels
 constexpr int kWalkBuffer = SplitTile<kChunk, kWalkRows>::kElements + SplitTile<kChunk, kWalkColumns>::kElements;
 
 template <int MODE>
-__global__ void __launch_bounds__(kWalkThreads, 2) chunk_walk_kernel(const ChunkArgs p) {
-    constexpr int kTiles = 2;                                // tiles of eight columns a warp: four warps along the key
+__global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const ChunkArgs p) {
+    constexpr int kTiles = 4;                                // tiles of eight columns a warp: four warps along the key
     using KTile = SplitTile<kChunk, kWalkRows>;              // channels, two along the columns
     using VTile = SplitTile<kChunk, kWalkColumns>;
     extern __shared__ __align__(128) __nv_bfloat16 tiles[];  // two buffers of a chunk's k and v
@@ -457,12 +458,13 @@ __global__ void __launch_bounds__(kWalkThreads, 2) chunk_walk_kernel(const Chunk
         float sum[kTiles][4] = {}, ones[4] = {};
 #pragma unroll
         for (int t = 0; t < kChunk; t += 32) {               // two depths of 16 at a time: their chains take turns
-            unsigned a[2][3][4], b[2][2][3][2];
+            unsigned a[2][3][4], b[2][kTiles][3][2];
             float d[2][kTiles][4] = {}, n_d[2][4] = {};
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 load_a_transposed<KTile>(a[u], k_t, 16 * along, t + 16 * u);
-                load_b_transposed<VTile>(b[u], v_t, 16 * across, t + 16 * u);
+                load_b_transposed<VTile>(b[u], v_t, 32 * across, t + 16 * u);
+                load_b_transposed<VTile>(b[u] + 2, v_t, 32 * across + 16, t + 16 * u);
             }
             constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
@@ -1187,17 +1189,21 @@ inline int launch_reads(const ChunkArgs& p, int chunks, cudaStream_t stream) {
                        : launch_read<MODE, 128>(p, chunks, heads_a_block, stream);
 }
 
-// The walk moves a third of the bytes but needs a block and a half an SM to keep them busy: at 64 heads of 128 x 64 (256 blocks) a
-// span of 2,048 tokens takes 88 us, sums and carry 107 (62 + 45); at 16 heads of 64 x 128 (64 blocks) 46 us and 26 (17 + 9; the
-// mLSTM's carry, with its maxima, 21).
-inline bool walks(int heads, int dim, int vdim, int spans) {
-    return (long long)((vdim + kWalkColumns - 1) / kWalkColumns) * ((dim + kWalkRows - 1) / kWalkRows) * heads * spans >= 222;
+// The walk moves a third of the bytes, but a span's chunks come one after another: 2.5 us each, of the longest span (taken as 1.4
+// times the mean of several) or of all blocks over the SMs, whichever is more. Sums take 0.0148 us a chunk and 64 x 64 of S, the carry
+// its bytes at 3.5 TB/s. Walk / sums and carry, us: 64 heads of 128 x 64, 2,048 tokens 81 / 104, 300 15.1 / 19.5, 4,096 in six spans
+// 166 / 269; 16 heads of 64 x 128, 1,999 in four 34 / 26, 2,048 in one (mLSTM) 80 / 29.
+inline bool walks(int heads, int dim, int vdim, int spans, int chunks) {
+    const double tiles = (double)((vdim + 63) / 64) * ((dim + 63) / 64) * heads, mean = (double)chunks / spans;
+    const double longest = spans > 1 && 1.4 * mean < chunks ? 1.4 * mean : chunks, together = tiles * chunks / 148.0;
+    const double walk = 2.5 * (longest > together ? longest : together);
+    return walk < 0.0148 * tiles * chunks + (double)chunks * heads * dim * vdim * 8.0 / 3.5e6;
 }
 
 // `chunks` bounds the chunks of all spans; p.chunk_begin has chunks / p.pieces + 1 entries
 template <int MODE>
 inline int launch_chunk_scan(const ChunkArgs& p, int chunks, cudaStream_t stream) {
-    const int status = walks(p.heads, p.dim, p.vdim, p.spans) ? launch_walk<MODE>(p, stream) : launch_sums<MODE>(p, chunks, stream);
+    const int status = walks(p.heads, p.dim, p.vdim, p.spans, chunks) ? launch_walk<MODE>(p, stream) : launch_sums<MODE>(p, chunks, stream);
     return status != 0 ? status : launch_reads<MODE>(p, chunks, stream);
 }
 

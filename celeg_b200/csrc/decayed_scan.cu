@@ -387,7 +387,9 @@ using namespace celeg_b200;
 CELEG_API int celeg_chunk_tokens() { return kChunk; }
 
 // Launches that a chunked scan makes its states with: the walk, or sums and carry.
-CELEG_API int celeg_chunk_state_launches(int heads, int dim, int vdim, int spans) { return walks(heads, dim, vdim, spans) ? 1 : 2; }
+CELEG_API int celeg_chunk_state_launches(int heads, int dim, int vdim, int spans, int chunks) {
+    return walks(heads, dim, vdim, spans, chunks) ? 1 : 2;
+}
 
 // plan: ints [max_chunks + 1 | spans + 1]: the chunks' first tokens (the last chunk's end at the end), the spans' first chunks
 CELEG_API int celeg_chunk_plan(const int* span_begin, int spans, int max_chunks, int* plan, cudaStream_t stream) {

@@ -185,7 +185,7 @@ _SIGNATURES = {
                                        c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "celeg_decay_sums": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "celeg_delta_operand_bytes": [c_int],
-    "celeg_chunk_state_launches": [c_int, c_int, c_int, c_int],
+    "celeg_chunk_state_launches": [c_int, c_int, c_int, c_int, c_int],
     "celeg_delta_chunk_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                c_int, c_float, c_void_p, c_void_p],
@@ -1008,7 +1008,7 @@ def mlstm_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, pre_i: t
         _ptr(bias_i), _ptr(bias_f), cap, _ptr(gates), _ptr(peaks), _ptr(norms), _ptr(states), _ptr(out), _ptr(state), slot_stride,
         _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, dim, vdim, q_scale, _stream()))
     global LAUNCHES
-    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans)      # (a call counts one) the gates, the states, the read-outs
+    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans, chunks)      # (a call counts one) the gates, the states, the read-outs
 
 
 def retention_segmented(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
@@ -1034,7 +1034,7 @@ def retention_segmented(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay
                                                tokens, heads, dim, vdim, q_scale, segment, max_segments,
                                                _ptr(float_scratch), _ptr(int_scratch), _stream()))
     global LAUNCHES
-    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans)      # (a call counts one) the plan, the states, the read-outs
+    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans, max_segments * (segment // 64))      # (a call counts one) the plan, the states, the read-outs
 
 
 def recurrent_decode(mode: int, proj: torch.Tensor, offsets: Tuple[int, int, int, int, int, int],
@@ -1456,9 +1456,9 @@ def chunk_tokens() -> int:
 
 
 @functools.lru_cache(maxsize=256)
-def chunk_state_launches(heads: int, dim: int, vdim: int, spans: int) -> int:
+def chunk_state_launches(heads: int, dim: int, vdim: int, spans: int, chunks: int) -> int:
     """Launches that a chunked scan makes its states with (:data:`LAUNCHES` counts them)."""
-    return int(library().celeg_chunk_state_launches(heads, dim, vdim, spans))
+    return int(library().celeg_chunk_state_launches(heads, dim, vdim, spans, chunks))
 
 
 def chunk_plan(span_begin: torch.Tensor, spans: int, max_chunks: int, plan: torch.Tensor) -> None:
@@ -1485,7 +1485,7 @@ def channel_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: tor
         _ptr(q_out), _ptr(k_out), _ptr(total), _ptr(products), _ptr(states), _ptr(out), _ptr(state), slot_stride,
         _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, dim, vdim, _stream()))
     global LAUNCHES
-    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans)      # the chunks' own products, the states, the read-outs
+    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans, chunks)      # the chunks' own products, the states, the read-outs
 
 
 def scalar_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: torch.Tensor, dt_bias: torch.Tensor,
@@ -1505,7 +1505,7 @@ def scalar_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: to
         _ptr(direct), _ptr(cum), _ptr(dt), _ptr(states), _ptr(out), _ptr(state), slot_stride, _ptr(span_slot),
         _ptr(plan), max_chunks, spans, chunks, heads, groups, dim, vdim, _stream()))
     global LAUNCHES
-    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans)      # the decays, then as above
+    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans, chunks)      # the decays, then as above
 
 
 def channel_decay_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_scale: float, low: torch.Tensor,
