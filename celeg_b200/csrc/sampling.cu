@@ -655,6 +655,8 @@ __global__ void argmax_final_kernel(const float* partial_score, const int* parti
 __global__ void mark_seen_kernel(uint8_t* seen_base, int vocab, const int* tokens,
                                  const int* token_span, const int* span_slot,
                                  int count) {
+    chain_release();
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const int token = tokens[i];
@@ -729,6 +731,6 @@ CELEG_API int celeg_mark_seen(uint8_t* seen, int vocab, const int* tokens, const
                               const int* span_slot, int count, cudaStream_t stream) {
     CELEG_REQUIRE(count >= 0 && vocab > 0, "mark_seen: invalid sizes count=%d vocab=%d", count, vocab);
     if (count == 0) return 0;
-    mark_seen_kernel<<<(count + 255) / 256, 256, 0, stream>>>(seen, vocab, tokens, token_span, span_slot, count);
+    launch_chained(mark_seen_kernel, (count + 255) / 256, 256, 0, stream, seen, vocab, tokens, token_span, span_slot, count);
     return check_launch("mark_seen");
 }
