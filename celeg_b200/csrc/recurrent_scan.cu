@@ -751,7 +751,8 @@ __global__ void __launch_bounds__(256) gated_row_norm_kernel(const float* o, con
 struct DecodeStepParams {
     const float* proj; int stride;                 // [tokens, stride] rows of the input projection
     int q_off, k_off, v_off, gate_off, g0_off, g1_off;
-    const float* conv_kernel; const float* carried; int taps, channels;      // delta only
+    const float* conv_kernel; float* carried; int taps, channels;            // delta only
+    int group;                                     // delta: heads a key head where this launch moves the carried inputs on, or 0
     const float* bias0; const float* bias1; float cap;   // mLSTM: gate biases and cap; delta: A_log and dt_bias
     const float* norm_w; int norm_per_head; float eps, unit_eps;
     float* state; long long slot_stride;
@@ -780,7 +781,33 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
     float* part_s = o_s + vdim;
     const float* row = p.proj + (size_t)t * p.stride;
     const long long slot_at = (long long)p.span_slot[t] * p.slot_stride;
-    const float* carried = MODE == kScanDelta ? p.carried + slot_at : nullptr;
+    float* carried = MODE == kScanDelta ? p.carried + slot_at : nullptr;
+    float* slot = p.state + slot_at;
+    float* s_head = slot + (size_t)head * dim * vdim;
+    float* n_head = slot + (size_t)heads * dim * vdim + (size_t)head * dim;
+    float* m_head = slot + (size_t)heads * dim * vdim + (size_t)heads * dim + head;
+    // The state: a warp takes 32 neighbouring columns and every ``split``-th row of them, so that a block's warps
+    // cover the head's columns with `split` warps each; a thread's rows stay in registers between the sums and
+    // the update (up to 32 of them; beyond that they are read again), all of its loads are in flight at once (the first
+    // columns' before anything else: nothing that comes before their use needs the state), and the partial sums of a
+    // column meet in shared memory.
+    constexpr int kKeep = 32;
+    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int groups = (vdim + 31) >> 5;
+    const int split = max(1, warps / groups);
+    const int groups_at_once = warps / split, part = warp % split;
+    const bool kept = dim <= kKeep * split;
+    float cells[kKeep];
+    auto load_cells = [&](int j) {
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i) {
+            const int e = part + i * split;
+            cells[i] = e < dim ? s_head[(size_t)e * vdim + j] : 0.0f;
+        }
+    };
+    const int first_column = (warp / split) * 32 + lane;
+    const bool loaded = kept && warp < groups_at_once * split && warp / split < groups && first_column < vdim;
+    if (loaded) load_cells(first_column);
 
     // a convolved channel of the delta rule: taps - 1 carried inputs (oldest first), then the token's own
     auto convolved = [&](int c) {
@@ -810,6 +837,7 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
         q2 += qv * qv;
     }
     if (MODE == kScanDelta) {
+        if (p.group > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // q's and k's carried inputs: read
         k2 = block_sum(k2, scratch);
         q2 = block_sum(q2, scratch);
         const float k_inv = 1.0f / sqrtf(k2 + p.unit_eps), q_inv = 1.0f / sqrtf(q2 + p.unit_eps);
@@ -819,10 +847,6 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
         }
     }
     __syncthreads();
-    float* slot = p.state + slot_at;
-    float* s_head = slot + (size_t)head * dim * vdim;
-    float* n_head = slot + (size_t)heads * dim * vdim + (size_t)head * dim;
-    float* m_head = slot + (size_t)heads * dim * vdim + (size_t)heads * dim + head;
     float kq = 0.0f, nq = 0.0f;
     for (int e = threadIdx.x; e < dim; e += blockDim.x) {
         kq = fmaf(k_s[e], q_s[e], kq);
@@ -849,30 +873,15 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
         write = expf(g0 - m_new);
         lower = fmaxf(fabsf(keep * nq + write * kq), expf(-m_new)) + 1e-6f;
     }
-    // The state: a warp takes 32 neighbouring columns and every ``split``-th row of them, so that a block's warps
-    // cover the head's columns with `split` warps each; a thread's rows stay in registers between the sums and
-    // the update (up to 32 of them; beyond that they are read again), all of its loads are in flight at once, and
-    // the partial sums of a column meet in shared memory.
-    constexpr int kKeep = 32;
-    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int groups = (vdim + 31) >> 5;
-    const int split = max(1, warps / groups);
-    const int groups_at_once = warps / split;
-    const bool kept = dim <= kKeep * split;
     float squares = 0.0f;
     for (int first_group = 0; first_group < groups; first_group += groups_at_once) {
-        const int g = first_group + warp / split, part = warp % split;
+        const int g = first_group + warp / split;
         const int j = g * 32 + lane;
         const bool active = warp < groups_at_once * split && g < groups && j < vdim;
-        float cells[kKeep];
         float sk = 0.0f, sq = 0.0f;
         if (active) {
             if (kept) {
-#pragma unroll
-                for (int i = 0; i < kKeep; ++i) {
-                    const int e = part + i * split;
-                    cells[i] = e < dim ? s_head[(size_t)e * vdim + j] : 0.0f;
-                }
+                if (first_group > 0) load_cells(j);
 #pragma unroll
                 for (int i = 0; i < kKeep; ++i) {
                     const int e = part + i * split;
@@ -947,6 +956,23 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
         return;
     }
     squares = block_sum(squares, scratch);
+    if (MODE == kScanDelta && p.group > 0) {
+        // The carried inputs move on by the token: v's are this block's alone (and the sum above comes after its threads' reads),
+        // q's and k's are read by every head of the group, a cluster, whose first block writes them once all have.
+        if (p.group > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        const int mine = vdim + (head % (heads / p.kv_heads) == 0 ? 2 * dim : 0);
+        for (int x = threadIdx.x; x < mine; x += blockDim.x) {
+            const int c = x < vdim ? p.v_off + head * vdim + x
+                        : x < vdim + dim ? p.q_off + qk_head * dim + (x - vdim) : p.k_off + qk_head * dim + (x - vdim - dim);
+            float keep_inputs[15];
+#pragma unroll
+            for (int r = 0; r < 15; ++r)
+                if (r < p.taps - 1) keep_inputs[r] = r < p.taps - 2 ? carried[(size_t)(r + 1) * p.channels + c] : row[c];
+#pragma unroll
+            for (int r = 0; r < 15; ++r)
+                if (r < p.taps - 1) carried[(size_t)r * p.channels + c] = keep_inputs[r];
+        }
+    }
     const float inv = 1.0f / sqrtf(squares / (float)vdim + p.eps);
     const float* w = p.norm_w ? p.norm_w + (p.norm_per_head ? (size_t)head * vdim : 0) : nullptr;   // (null: no weight)
     A* dst = static_cast<A*>(p.out) + ((size_t)t * heads + head) * vdim;
@@ -1124,7 +1150,7 @@ CELEG_API int celeg_gated_head_norm(const float* o, const float* gate, int gate_
 // One token per request (row i of ``proj`` is request i's token, its slot span_slot[i]): everything between the
 // two projections of a matrix-state mixer in one launch. mode 0 (delta): the convolved channels [q | k | v] are
 // the first ``channels`` columns of a row, bias0 = A_log, bias1 = dt_bias, the output gate is SiLU; the carried
-// inputs are moved on by a second launch. mode 1 (mLSTM): bias0 / bias1 = the gates' biases, the gate is a sigmoid.
+// inputs are moved on by the same launch where it can (below), else by a second. mode 1 (mLSTM): bias0 / bias1 = the gates' biases, the gate is a sigmoid.
 // mode 2 (retention): bias0 = the heads' decays, the output gate is SiLU, norm_w may be null (no weight).
 static int recurrent_decode_launch(int mode, const float* proj, int stride, int q_off, int k_off, int v_off,
                                    int gate_off, int g0_off, int g1_off, const float* conv_kernel, float* carried,
@@ -1145,17 +1171,36 @@ static int recurrent_decode_launch(int mode, const float* proj, int stride, int 
     const size_t smem = (size_t)(2 * dim + vdim + 2 * kDecodeStepThreads) * sizeof(float);
     CELEG_REQUIRE(smem <= 40 * 1024, "recurrent_decode: head sizes %d and %d exceed a block's shared memory", dim, vdim);
     if (tokens == 0) return 0;
+    // The launch moves the carried inputs on itself where q, k and v are all of them, one after another, and a key head's heads fit
+    // a cluster of portable size: 2 requests of 16 heads of 64 on 8 key heads, 9.8 us of one kernel against 9.1 and 2.5 of two, a whole call of the
+    // mixer 36.2 us against 37.9; elsewhere a second launch does.
+    const int group = heads / kv_heads, qk_width = kv_heads * dim;
+    const bool moves = mode == kScanDelta && taps > 1 && !raw_out && group <= 8 && q_off == 0 && k_off == qk_width && v_off == 2 * qk_width &&
+                       channels == 2 * qk_width + heads * vdim;
     const DecodeStepParams p = {proj, stride, q_off, k_off, v_off, gate_off, g0_off, g1_off, conv_kernel, carried, taps,
-                                channels, bias0, bias1, cap, norm_w, norm_per_head, eps, unit_eps, state, slot_stride,
+                                channels, moves ? group : 0, bias0, bias1, cap, norm_w, norm_per_head, eps, unit_eps, state, slot_stride,
                                 span_slot, heads, kv_heads, dim, vdim, q_scale, out, input_act, raw_out};
     dim3 grid(heads, tokens);
     if (mode == kScanDelta) {
+        cudaLaunchConfig_t config = {};
+        config.gridDim = grid;
+        config.blockDim = kDecodeStepThreads;
+        config.dynamicSmemBytes = smem;
+        config.stream = stream;
+        cudaLaunchAttribute attributes[2];
+        attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attributes[0].val.programmaticStreamSerializationAllowed = chaining_enabled() ? 1 : 0;
+        attributes[1].id = cudaLaunchAttributeClusterDimension;
+        attributes[1].val.clusterDim.x = moves ? group : 1;
+        attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
+        config.attrs = attributes;
+        config.numAttrs = moves && group > 1 ? 2 : 1;
         if (act_dtype == kFloat32)
-            launch_chained(recurrent_decode_kernel<kScanDelta, float>, grid, kDecodeStepThreads, smem, stream, p);
+            cudaLaunchKernelEx(&config, recurrent_decode_kernel<kScanDelta, float>, p);
         else
-            launch_chained(recurrent_decode_kernel<kScanDelta, __nv_bfloat16>, grid, kDecodeStepThreads, smem, stream, p);
+            cudaLaunchKernelEx(&config, recurrent_decode_kernel<kScanDelta, __nv_bfloat16>, p);
         int status = check_launch("recurrent_decode");
-        if (status != 0 || taps == 1) return status;
+        if (status != 0 || taps == 1 || moves) return status;
         const long long units = (long long)tokens * channels;
         launch_chained(carried_inputs_update_kernel, (unsigned)((units + 127) / 128), 128, 0, stream, proj, stride,
                        carried, slot_stride, span_begin, span_slot, tokens, channels, taps);

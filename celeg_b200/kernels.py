@@ -1044,7 +1044,7 @@ def recurrent_decode(mode: int, proj: torch.Tensor, offsets: Tuple[int, int, int
                      span_begin: torch.Tensor, span_slot: torch.Tensor, tokens: int, heads: int, kv_heads: int,
                      dim: int, vdim: int, q_scale: float, out: torch.Tensor) -> None:
     """A decoding step of a matrix-state mixer between its two projections, one launch (the delta rule's carried
-    inputs: a second): row i of ``proj`` (float32) is the one token of request i. ``offsets``: columns of
+    inputs: a second where q, k and v are not all of the channels in this order or a key head has more than 8 heads): row i of ``proj`` (float32) is the one token of request i. ``offsets``: columns of
     (q, k, v, output gate, first gate, second gate) in a row. See csrc/recurrent_scan.cu."""
     assert proj.dtype == torch.float32 and proj.stride(-1) == 1 and out.is_contiguous() and out.shape[1] == heads * vdim
     _check(library().celeg_recurrent_decode(
@@ -1053,7 +1053,9 @@ def recurrent_decode(mode: int, proj: torch.Tensor, offsets: Tuple[int, int, int
         _ptr(span_begin), _ptr(span_slot), tokens, heads, kv_heads, dim, vdim, q_scale, _ptr(out),
         dtype_code(out.dtype), _stream()))
     global LAUNCHES
-    LAUNCHES += 1 if (mode == SCAN_DELTA and taps > 1) else 0
+    if mode == SCAN_DELTA and taps > 1:
+        qk = kv_heads * dim
+        LAUNCHES += heads > 8 * kv_heads or tuple(offsets[:3]) != (0, qk, 2 * qk) or channels != 2 * qk + heads * vdim
 
 
 def mlstm_gates(pre_i: torch.Tensor, pre_f: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float,
