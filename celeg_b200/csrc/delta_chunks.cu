@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(kDeltaWalkThreads) delta_walk_kernel(const Del
 // the same shape: a system's inverse T, W = T u^ and s_0 = T ((u^ . k^) v), the same walk with s = s_0 + W S_0, and read-outs
 // with two sets of values. One block a (chunk, head) of 64 channels makes everything that does not wait for the state:
 // 146 us at 32 heads of 64 and 2,048 tokens, two blocks an SM (139 before it left out tokens that are not finite, 187 with one
-// block an SM); with the walk's 67 and the read-outs' 47 that is 260 us where chunks of eight tokens take 344.
+// block an SM); with the walk's 59 and the read-outs' 47 that is 252 us where chunks of eight tokens take 344.
 struct GeneralChunkArgs {
     const float* proj; int stride; int r_off, k_off, v_off, a_off;     // columns of a token's row: head h at h * dim
     const float* z; int z_stride;                              // [tokens, heads * dim], before its bias

@@ -389,7 +389,8 @@ __global__ void delta_prepare_kernel(const DeltaPrepareArgs a) {
 // The same over portions of many tokens with four taps: a thread four channels of kTile tokens in a row. Their kernels stay in
 // registers and a row is loaded once, plus three before the tile (a block a token reads a row four times and 64 bytes of kernels
 // a thread for every token); the lanes of a head add up its squares among themselves, so nothing goes through shared memory.
-// DIM / 4 lanes are a head of q or k, so a head's lanes are neighbours of one warp.
+// DIM / 4 lanes are a head of q or k, so a head's lanes are neighbours of one warp. 2,048 tokens of 4,096 channels: 19.6 us, a block
+// a token 37.6. Memory bounds it (67 MB, 3.4 TB/s).
 constexpr int kPrepareThreads = 128;
 constexpr int kPrepareTile = 8, kPrepareTileTokens = 64;
 template <int DIM, int kTile>
@@ -576,7 +577,7 @@ __global__ void gated_head_norm_pairs_kernel(const float* o, const float* gate, 
 }
 
 // The same for heads of 16, 32, 64 or 128 entries: LANES lanes a head, four neighbours a lane and access, so that a warp of heads
-// of 64 takes two of them and every load is 16 bytes. It is bound by the loads in flight, then by memory: 10.4 us for 2,048 tokens of
+// of 64 takes two of them and every load is 16 bytes. It is bound by its instructions, then by memory: 10.2 us for 2,048 tokens of
 // 32 heads of 64 (42 MB, 4.0 TB/s, some of it from L2), 18.8 with two neighbours a lane; 10.7 for 16 heads of 128, 18.9 then.
 template <typename A, int LANES>
 __global__ void __launch_bounds__(128) gated_head_norm_quads_kernel(const float* o, const float* gate, int gate_stride,
@@ -1069,7 +1070,8 @@ CELEG_API int celeg_delta_prepare(const float* proj, int stride, const float* ke
     args.vector_loads =
         channels % 4 == 0 && stride % 4 == 0 && slot_stride % 4 == 0 &&
         (((size_t)proj | (size_t)carried | (size_t)conv_out) & 15) == 0;
-    // Tiles of tokens where a step has enough of them to fill the GPU and every access is one of 16 bytes.
+    // Tiles of tokens where every access is one of 16 bytes and a step has tokens enough for eight rows of blocks: below that a block
+    // a token is the one with more blocks (a thread of a tile walks eight tokens in turn). 2,048 tokens: 19.6 us against 37.6.
     const bool tiles = taps == 4 && args.vector_loads && ((size_t)kernel & 15) == 0 && (dim == 32 || dim == 64 || dim == 128) &&
                        tokens >= kPrepareTileTokens;
     const dim3 grid((channels + 4 * kPrepareThreads - 1) / (4 * kPrepareThreads), (tokens + kPrepareTile - 1) / kPrepareTile);
@@ -1172,8 +1174,8 @@ static int recurrent_decode_launch(int mode, const float* proj, int stride, int 
     CELEG_REQUIRE(smem <= 40 * 1024, "recurrent_decode: head sizes %d and %d exceed a block's shared memory", dim, vdim);
     if (tokens == 0) return 0;
     // The launch moves the carried inputs on itself where q, k and v are all of them, one after another, and a key head's heads fit
-    // a cluster of portable size: 2 requests of 16 heads of 64 on 8 key heads, 9.8 us of one kernel against 9.1 and 2.5 of two, a whole call of the
-    // mixer 36.2 us against 37.9; elsewhere a second launch does.
+    // a cluster of portable size: 2 requests of 16 heads of 64 on 8 key heads, 9.8 us of one kernel against 9.1 and 2.5 of two, a
+    // whole call of the mixer 36.2 us against 37.9; elsewhere a second launch does.
     const int group = heads / kv_heads, qk_width = kv_heads * dim;
     const bool moves = mode == kScanDelta && taps > 1 && !raw_out && group <= 8 && q_off == 0 && k_off == qk_width && v_off == 2 * qk_width &&
                        channels == 2 * qk_width + heads * vdim;

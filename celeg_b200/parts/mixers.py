@@ -67,13 +67,13 @@ def decode_split(tokens: int, kv_heads: int, context_bucket: int, window: Option
     1,024 keys. Where that limit binds (many requests or long contexts) the chunk grows up to 4,096 keys: fewer
     blocks start and fewer partial results are merged. The launch's blocks (requests x kv heads x splits) run
     in rounds of ``resident_blocks``. If one round can hold them, about half a round is asked for: the
-    times fall off sharply just above a whole round (2 requests at 65 k keys: 60 us with 720 blocks, 75 us with
-    816) and are flat or a little better towards half of one (1 request at 130 k: 70 us with 712 blocks, 63 us
-    with 368; at 65 k 41 us with 360 to 408). Otherwise, of 1,024 / 2,048 / 4,096 keys the largest chunk within a
+    times fall off sharply just above a whole round (2 requests at 65 k keys: 63 us with 368 blocks, 75 us with
+    1,024) and are flat or a little better towards half of one (1 request at 130 k: 69 us with 368 blocks, 87 us
+    with 1,016; at 65 k 42 to 44 us with 256 to 360). Otherwise, of 1,024 / 2,048 / 4,096 keys the largest chunk within a
     twentieth of the most even filling of the rounds is taken (a count like 1,024 blocks, 1.4 rounds, was the
     slowest choice wherever it was measured). Measured on B200, 32 query heads on 8 kv heads of 64, microseconds
-    a layer at chunks of 1,024 / 2,048 / 4,096 keys: 64 requests at 8 k keys 173 / 168 / 196, 16 at 32 k
-    179 / 171 / 194, 8 at 65 k 188 / 175 / 200, 32 at 65 k 654 / 636 / 631, 8 at 130 k 360 / 337 / 326."""
+    a layer at chunks of 1,024 / 2,048 / 4,096 keys: 64 requests at 8 k keys 156 / 153 / 170, 16 at 32 k
+    181 / 174 / 185, 8 at 65 k 187 / 174 / 187, 32 at 65 k 659 / 639 / 629, 8 at 130 k 362 / 338 / 326."""
     bucket = context_bucket
     if window:
         bucket = min(bucket, 1 << max(8, (window - 1).bit_length()))

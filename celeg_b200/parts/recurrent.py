@@ -108,9 +108,9 @@ class MlstmMixer(PortionsInChunks):
             self.norms = rt.flat_scratch("recurrent.norms", chunks * self.qk_width, torch.float32)
             self.states = rt.flat_scratch("recurrent.states", chunks * self.qk_width * self.vdim, torch.float32)
 
-    # Measured at 16 heads of 64 x 128: 1 x 128 53 in chunks, 51 token by token; 1 x 150 53, 59; 1 x 2,048 171, 564; 8 x 20 60,
-    # 43; 48 x 20 168, 152; 48 x 150 557, 921; 200 and 8 x 10 (23 tokens a chunk) 70, 88; 160 and 40 x 8 (11) 142, 96; 600 and
-    # 40 x 20 (28) 187, 272.
+    # Measured at 16 heads of 64 x 128: 1 x 128 48 in chunks, 51 token by token; 1 x 150 51, 58; 1 x 2,048 149, 556; 48 x 150 560,
+    # 925; 200 and 8 x 10 (23 tokens a chunk) 70, 88; 600 and 40 x 20 (28) 189, 273; with a carry half as fast 8 x 20 60, 43; 48 x
+    # 20 168, 152; 160 and 40 x 8 (11) 142, 96.
     CHUNKED_FROM = 144
     TOKENS_A_CHUNK = 20
 
@@ -222,10 +222,10 @@ class GatedDeltaMixer(PortionsInChunks):
             self.operands = rt.flat_scratch("delta.operands", chunks * self.heads * kernels.delta_operand_bytes(self.dim) // 2,
                                             torch.bfloat16)
 
-    # Measured at 32 heads of 64 x 64: 1 x 300 98 in chunks, 93 token by token; 1 x 384 96, 111; 1 x 500 110, 133; 1 x 2,048 291,
-    # 496; 8 x 300 334, 306; 16 x 500 866, 904; 48 x 150 944, 835; 600 and 40 x 20 (28 tokens a chunk) 321, 256; 1,500 and 16 x
-    # 30 (49) 303, 461. At 32 heads of 128 x 128, where token by token is twice the work: 1 x 150 107, 102; 1 x 300 140, 169; 8 x
-    # 300 722, 960; 600 and 40 x 20 733, 643.
+    # Measured at 32 heads of 64 x 64: 1 x 256 76 in chunks, 76 token by token; 1 x 300 82, 88; 1 x 384 88, 105; 1 x 500 100, 129;
+    # 1 x 2,048 248, 470; 8 x 300 308, 283; 16 x 500 797, 839; 48 x 150 880, 776; 600 and 40 x 20 (28 tokens a chunk) 311, 245;
+    # 1,500 and 16 x 30 (49) 286, 445. At 32 heads of 128 x 128, where token by token is twice the work: 1 x 300 135, 160; 8 x 300
+    # 690, 923; 600 and 40 x 20 718, 626. (One portion alone is level from 256 tokens on; several of 300 are not.)
     CHUNKED_FROM = 384
     TOKENS_A_CHUNK = 40
 
@@ -322,9 +322,9 @@ class RetentionMixer(PortionsInChunks):
             self.segment_plan = rt.flat_scratch("retention.plan", 2 * self.max_segments + 8, torch.int32, zero=True)
 
     SEGMENT = 128               # tokens a segment
-    # Measured at 16 heads of 64 x 128: 1 x 128 39 in segments, 41 token by token; 1 x 150 41, 47; 2 x 150 55, 55; 1 x 500 55,
-    # 115; 8 x 20 51, 31; 48 x 20 150, 110; 48 x 150 469, 596; 200 and 8 x 10 (23 tokens a chunk) 60, 68; 160 and 40 x 8 (11) 127,
-    # 78; 600 and 40 x 20 (28) 161, 198.
+    # Measured at 16 heads of 64 x 128: 1 x 128 38 in segments, 41 token by token; 1 x 150 39, 45; 2 x 150 55, 55; 1 x 500 55,
+    # 115; 8 x 20 51, 31; 48 x 20 152, 110; 48 x 150 471, 599; 200 and 8 x 10 (23 tokens a chunk) 59, 69; 160 and 40 x 8 (11) 129,
+    # 78; 600 and 40 x 20 (28) 162, 198.
     CHUNKED_FROM = 144
     TOKENS_A_CHUNK = 20
 
@@ -568,8 +568,8 @@ class GeneralDeltaMixer(PortionsInChunks):
             self.operands = rt.flat_scratch("delta.operands", chunks * self.heads * kernels.delta_operand_bytes(self.dim) // 2,
                                             torch.bfloat16)
 
-    # Measured at 32 heads of 64, in chunks of 64 and of 8: 1 x 300 102, 92; 1 x 500 121, 132; 1 x 2,048 361, 448; 16 x 500 1,200,
-    # 1,224; 48 x 150 1,302, 1,118; 600 and 40 x 20 (28 tokens a chunk) 441, 284; 1,500 and 16 x 30 (49) 395, 505.
+    # Measured at 32 heads of 64, in chunks of 64 and of 8: 1 x 300 96, 90; 1 x 400 113, 114; 1 x 500 117, 131; 1 x 2,048 347, 440;
+    # 16 x 500 1,190, 1,226; 48 x 150 1,294, 1,121; 600 and 40 x 20 (28 tokens a chunk) 438, 284; 1,500 and 16 x 30 (49) 389, 506.
     CHUNKED_FROM = 480
     TOKENS_A_CHUNK = 40
 
