@@ -155,12 +155,6 @@ __device__ __forceinline__ void decode_copy_tile(__nv_bfloat16* k_dst, __nv_bflo
     }
 }
 
-__device__ __forceinline__ float exp2_of(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // A warp's running result over its tiles: rows g and g + 8 of the 16 query heads; maxima in units of log2.
 template <int D_PAD>
 struct DecodeRows {
@@ -186,7 +180,7 @@ struct DecodeRows {
     // The tile of keys tile_begin .. tile_begin + 31, those from `end` on do not count. What bounded this kernel over long contexts
     // was the instructions of a tile, a warp's chain of them and all warps' on the SM, 2 us a tile even with an empty GPU (three
     // stages of copies instead of two gained nothing). So rows 8 to 15 are left out of the exponentials for groups of at most
-    // eight heads, a tile that needs no mask, cap or bias goes straight from the products into the exponentials, the outputs are
+    // eight heads, a tile that needs no mask, cap or bias has its scores scaled in place, the outputs are
     // rescaled only when a maximum has grown, the queries' fragments stay in registers, and a copy that has nothing to bring is one
     // of no bytes instead of a branch. 32 heads on 8 of 64, before and now, us: 8 requests of 16 k keys 72 and 60 (268 MB: 41 at
     // 6.5 TB/s, and about 10 around the loop), 16 of 6 k 74 and 50, 1 of 130 k 75 and 69, 1 of 16 k 26 and 22, 8 of 578 14.5 and
@@ -219,12 +213,9 @@ struct DecodeRows {
         }
         const int halves = group > 8 ? 2 : 1;               // (the rows past the group are never stored)
         const float scale_log2 = p.scale * 1.4426950408889634f;
-        const bool plain = tile_begin + 32 <= end && p.cap_log2 == 0.0f && !p.distance_bias && scale_log2 > 0.0f;
+        const bool plain = tile_begin + 32 <= end && p.cap_log2 == 0.0f && !p.distance_bias;
         unsigned a[2][4] = {};                               // the weights as the next product's operand
-        float factor = 1.0f;                                 // of s, to units of log2
-        if (plain) {
-            factor = scale_log2;
-        } else {
+        if (!plain) {
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -248,24 +239,32 @@ struct DecodeRows {
             if (half >= halves) continue;
             float m = -INFINITY;
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) m = fmaxf(m, fmaxf(s[nt][2 * half], s[nt][2 * half + 1]));
+            for (int nt = 0; nt < 4; ++nt) {
+                float& x = s[nt][2 * half];
+                float& y = s[nt][2 * half + 1];
+                if (plain) {                                 // (a score is rounded once scaled, as in a tile with a mask)
+                    x = __fmul_rn(x, scale_log2);
+                    y = __fmul_rn(y, scale_log2);
+                }
+                m = fmaxf(m, fmaxf(x, y));
+            }
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-            const float new_max = fmaxf(run_max[half], m * factor);
+            const float new_max = fmaxf(run_max[half], m);
             if (new_max != run_max[half]) {
                 grown = true;
-                correction[half] = exp2_of(run_max[half] - new_max);
+                correction[half] = exp2f(run_max[half] - new_max);
             }
             const float base = new_max == -INFINITY ? 0.0f : new_max;
             run_max[half] = new_max;
-            float sum = 0.0f;
+            run_sum[half] *= correction[half];
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
-                const float x = exp2_of(fmaf(s[nt][2 * half], factor, -base)), y = exp2_of(fmaf(s[nt][2 * half + 1], factor, -base));
-                sum += x + y;
+                const float x = exp2f(s[nt][2 * half] - base), y = exp2f(s[nt][2 * half + 1] - base);
+                run_sum[half] += x;
+                run_sum[half] += y;
                 a[nt >> 1][half + 2 * (nt & 1)] = pack_bf16(x, y);
             }
-            run_sum[half] = fmaf(run_sum[half], correction[half], sum);
         }
         if (__any_sync(0xffffffffu, grown)) {
 #pragma unroll

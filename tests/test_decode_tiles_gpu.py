@@ -49,3 +49,27 @@ def test_decode_attention_at_the_ends_of_tiles(heads, kv_heads, dim, page, chunk
     # the weights are rounded to 8 bits before their product with values of order one, the output once more
     error = np.abs(out.double().cpu().numpy().reshape(tokens, heads, dim) - want)
     assert (error <= 2.0 ** -8 * (np.abs(want) + np.abs(v.double().numpy()).max() * 0.5)).all(), error.max()
+
+
+@pytest.mark.parametrize("chunk", [256, 640])                  # one stage a warp, two
+@pytest.mark.parametrize("heads,dim", [(1, 64), (16, 64), (4, 128)])
+@pytest.mark.parametrize("n", [32, 160])                       # one warp's first tile, and its second
+def test_weights_below_the_smallest_normal_number_count(n, heads, dim, chunk):
+    """The first key's value is zero, the others' are 2^118 under weights of about 2^-130: bfloat16 holds such weights with three
+    bits (2^-133), so an output is off by a sixteenth of itself at most, and by its own rounding."""
+    from celeg_b200 import kernels
+    page = 16
+    pages = -(-n // page)
+    k, v = torch.zeros((pages, 1, page, dim), dtype=torch.bfloat16), torch.full((pages, 1, page, dim), 2.0 ** 118, dtype=torch.bfloat16)
+    k[..., 0], k[0, 0, 0, 0], v[0, 0, 0] = -90.0, 0.0, 0.0
+    q = torch.zeros((1, heads, dim), dtype=torch.bfloat16)
+    q[..., 0] = 1.0
+    i32 = lambda x: torch.tensor(list(x), dtype=torch.int32, device="cuda")                   # noqa: E731
+    splits = -(-n // chunk)
+    scratch = torch.empty(heads * splits * dim, device="cuda"), torch.empty(heads * splits * 2, device="cuda")
+    flag, out = i32([0]), torch.zeros((1, heads * dim), dtype=torch.bfloat16, device="cuda")
+    kernels.attention_decode(q.cuda().view(1, -1), heads * dim, out, k.cuda(), v.cuda(), i32([n - 1]), i32([0]), i32(range(pages)).view(1, -1),
+                             1, heads, 1, dim, page, 0, 1.0, chunk, splits, *scratch, i32([0]), flag)
+    want = (n - 1) * np.exp(-90.0) * 2.0 ** 118
+    assert int(flag.item()) == 0
+    assert bool(((out.double() / want - 1.0).abs() <= 2.0 ** -4 + 2.0 ** -8).all()), float((out.double() / want).min())
