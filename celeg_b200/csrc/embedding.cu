@@ -25,15 +25,30 @@ __global__ void embedding_kernel(const W* __restrict__ table, const int* tokens,
     const W* src = table + (size_t)(valid ? token : 0) * hidden;
     float squares = 0.0f;
     const float place = frequencies ? (float)positions[row] : 0.0f;
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        float v = valid ? to_float(src[i]) * multiplier : 0.0f;
-        if (frequencies) {
-            const float angle = place * frequencies[i >> 1];
-            v += (i & 1) ? cosf(angle) : sinf(angle);
+    constexpr int kAhead = 8;
+    for (int first = threadIdx.x; first < hidden; first += kAhead * blockDim.x) {
+        W x[kAhead];
+        float w[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int i = first + u * blockDim.x;
+            if (i >= hidden) continue;
+            x[u] = src[i];
+            if (next_w) w[u] = next_w[i];
         }
-        dst[i] = v;
-        if (xw_out) xw_out[(size_t)row * hidden + i] = __float2bfloat16_rn(next_w ? v * next_w[i] : v);
-        if (next_w) squares += v * v;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int i = first + u * blockDim.x;
+            if (i >= hidden) continue;
+            float v = valid ? to_float(x[u]) * multiplier : 0.0f;
+            if (frequencies) {
+                const float angle = place * frequencies[i >> 1];
+                v += (i & 1) ? cosf(angle) : sinf(angle);
+            }
+            dst[i] = v;
+            if (xw_out) xw_out[(size_t)row * hidden + i] = __float2bfloat16_rn(next_w ? v * w[u] : v);
+            if (next_w) squares += v * v;
+        }
     }
     if (next_w) {
         squares = block_sum(squares, scratch);
@@ -41,24 +56,20 @@ __global__ void embedding_kernel(const W* __restrict__ table, const int* tokens,
     }
 }
 
-// The same, eight neighbours a thread and access, where rows are multiples of that and there are no positions to add. A row of the
-// table is a miss in every cache, and element by element the loads of one turn wait for the stores of the one before: 8 rows of
-// 2,048, 6.5 us so, 2.3 us with a row's loads all under way at once.
+// The same, eight neighbours a thread and access, where rows are multiples of that and there are neither positions to add nor
+// squares to add up (whose order the kernel above gives).
 template <typename W>
 __global__ void __launch_bounds__(256) embedding_eights_kernel(const W* __restrict__ table, const int* tokens, float* __restrict__ out,
                                                                int hidden, int vocab, float multiplier,
-                                                               const float* __restrict__ next_w, __nv_bfloat16* __restrict__ xw_out,
-                                                               float* sumsq_out, int sumsq_stride) {
-    __shared__ float scratch[33];
+                                                               __nv_bfloat16* __restrict__ xw_out) {
     chain_release();
     chain_wait();
     const int row = blockIdx.x, token = tokens[row];
     const bool valid = token >= 0 && token < vocab;          // the host refuses other ids before launch
     const W* src = table + (size_t)(valid ? token : 0) * hidden;
     float* dst = out + (size_t)row * hidden;
-    float squares = 0.0f;
     for (int i = threadIdx.x * 8; i < hidden; i += blockDim.x * 8) {
-        float v[8], w[8];
+        float v[8];
         if (sizeof(W) == 2) {
             const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src + i));
             const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -75,33 +86,17 @@ __global__ void __launch_bounds__(256) embedding_eights_kernel(const W* __restri
                 v[j] = x.x; v[j + 1] = x.y; v[j + 2] = x.z; v[j + 3] = x.w;
             }
         }
-        if (next_w) {
 #pragma unroll
-            for (int j = 0; j < 8; j += 4) {
-                const float4 x = *reinterpret_cast<const float4*>(next_w + i + j);
-                w[j] = x.x; w[j + 1] = x.y; w[j + 2] = x.z; w[j + 3] = x.w;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            v[j] = valid ? v[j] * multiplier : 0.0f;
-            if (next_w) squares += v[j] * v[j];
-        }
+        for (int j = 0; j < 8; ++j) v[j] = valid ? v[j] * multiplier : 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; j += 4) *reinterpret_cast<float4*>(dst + i + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
         if (xw_out) {
             uint4 raw;
             __nv_bfloat162* pairs = reinterpret_cast<__nv_bfloat162*>(&raw);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                pairs[j] = next_w ? __floats2bfloat162_rn(v[2 * j] * w[2 * j], v[2 * j + 1] * w[2 * j + 1])
-                                  : __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+            for (int j = 0; j < 4; ++j) pairs[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
             *reinterpret_cast<uint4*>(xw_out + (size_t)row * hidden + i) = raw;
         }
-    }
-    if (next_w) {
-        squares = block_sum(squares, scratch);
-        if (threadIdx.x == 0) sumsq_out[(size_t)row * sumsq_stride] = squares;
     }
 }
 
@@ -118,17 +113,17 @@ static int embedding_checked(const void* table, int table_dtype, const int* toke
     CELEG_REQUIRE(!next_w || (xw_out && sumsq_out && sumsq_stride >= 1),
                   "embedding: preparing the norm that follows needs its two outputs");
     if (rows == 0) return 0;
-    // Every such row takes the wide kernel: at 8 rows of 2,048 2.3 us against 6.5, and its loads need 16-byte addresses, which the
-    // row's start has when its length is a multiple of eight (bfloat16) and the buffers' starts have them.
-    if (hidden % 8 == 0 && !frequencies && (table_dtype == kFloat32 || table_dtype == kBFloat16) &&
-        (((size_t)table | (size_t)out | (size_t)next_w | (size_t)xw_out) & 15) == 0) {
+    // Its loads need 16-byte addresses, which the row's start has when its length is a multiple of eight (bfloat16) and the
+    // buffers' starts have them.
+    if (hidden % 8 == 0 && !frequencies && !next_w && (table_dtype == kFloat32 || table_dtype == kBFloat16) &&
+        (((size_t)table | (size_t)out | (size_t)xw_out) & 15) == 0) {
         const int eights = hidden / 8, block = eights >= 256 ? 256 : (eights + 31) / 32 * 32;
         if (table_dtype == kFloat32)
             launch_chained(embedding_eights_kernel<float>, rows, block, 0, stream, (const float*)table, tokens, out, hidden, vocab,
-                           multiplier, next_w, (__nv_bfloat16*)xw_out, sumsq_out, sumsq_stride);
+                           multiplier, (__nv_bfloat16*)xw_out);
         else
             launch_chained(embedding_eights_kernel<__nv_bfloat16>, rows, block, 0, stream, (const __nv_bfloat16*)table, tokens, out,
-                           hidden, vocab, multiplier, next_w, (__nv_bfloat16*)xw_out, sumsq_out, sumsq_stride);
+                           hidden, vocab, multiplier, (__nv_bfloat16*)xw_out);
         return check_launch("embedding");
     }
     const int threads = hidden >= 1024 ? 256 : 128;

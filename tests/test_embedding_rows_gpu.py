@@ -32,3 +32,21 @@ def test_rows(dtype, hidden, shift):
     assert torch.equal(out, expected) and torch.equal(first.xw, (expected * weight).bfloat16())
     exact = expected.double().square().sum(1)
     assert bool(((first.sumsq[:, 0].double() - exact).abs() <= exact * hidden * 2 ** -24).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hidden", [64, 1000, 2048, 2056, 5000])
+def test_squares_are_added_in_one_order(dtype, hidden):
+    """A row's sum of squares has the same bits wherever the table and the outputs lie."""
+    torch.manual_seed(hidden)
+    vocab, rows = 11, 7
+    tokens, weight = torch.randint(0, vocab, (rows,), dtype=torch.int32, device="cuda"), torch.randn(hidden, device="cuda")
+    values = torch.randn(vocab, hidden, device="cuda").to(dtype)
+    sums = []
+    for shift in (0, 1):
+        table = torch.empty(vocab * hidden + shift, device="cuda", dtype=dtype)[shift:].view(vocab, hidden)
+        table.copy_(values)
+        first = kernels.SplitNorm(torch.empty(rows, hidden, device="cuda", dtype=torch.bfloat16), torch.empty(rows, 1, device="cuda"), 1, 1e-5, hidden)
+        kernels.embedding(table, tokens, torch.empty(rows, hidden, device="cuda"), 1.3, prepare=first, next_weight=weight)
+        sums.append(first.sumsq.clone())
+    assert torch.equal(*sums)
