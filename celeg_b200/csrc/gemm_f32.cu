@@ -144,13 +144,13 @@ CELEG_API int celeg_gemm_f32(const float* x, const float* w, float* y, int m, in
     CELEG_REQUIRE(m >= 0 && n > 0 && k > 0 && ldx >= k && ldw >= k && ldy >= n,
                   "gemm_f32: invalid sizes m=%d n=%d k=%d ldx=%d ldw=%d ldy=%d", m, n, k, ldx, ldw, ldy);
     if (m == 0) return 0;
-    CELEG_REQUIRE((m + 31) / 32 <= 65535, "gemm_f32: %d rows exceed one launch", m);
     // Tiles of 64 x 64 where they give every SM work; few rows and narrow matrices in tiles of 32 x 32 (k is never cut: an element
     // is one thread's sum in ascending k). In 64 and in 32, us: 500 x 10,304, k 2,048 673 and 1,012; 400 x 2,048, k 2,048 (224 tiles)
     // 163 and 176; 300 x 1,024, k 1,024 (80) 52 and 52; 200 x 768, k 768 (48) 39 and 30; 490 x 64, k 2,048 (8) 99 and 68; 8 x 6,144,
     // k 2,048 (96) 97 and 76. Patches of 8 x 8 in tiles of 64 x 128 are level with the first where they fill the GPU and slower
     // elsewhere.
     const long long tiles = (long long)((m + 63) / 64) * ((n + 63) / 64);
+    CELEG_REQUIRE((m + 63) / 64 <= 65535, "gemm_f32: %d rows exceed one launch", m);      // (so many take the larger tiles)
     if (tiles >= 148) launch_gemm_f32<64, 64, 4, 8>(x, w, y, m, n, k, ldx, ldw, ldy, accumulate, stream);
     else launch_gemm_f32<32, 32, 4, 4>(x, w, y, m, n, k, ldx, ldw, ldy, accumulate, stream);
     return check_launch("gemm_f32");

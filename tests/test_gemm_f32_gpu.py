@@ -31,3 +31,15 @@ def test_a_row_does_not_depend_on_the_rows_beside_it():
     kernels.gemm_f32(x, w, many, 700)                     # tiles of 64 x 64
     kernels.gemm_f32(x[200:203], w, few, 3)               # of 32 x 32
     assert torch.equal(many[200:203], few)
+
+
+def test_as_many_rows_as_a_launch_has_tiles_of_64():
+    from celeg_b200 import kernels
+    w = torch.full((1, 1), 3.0, device="cuda")
+    for rows in (32 * 65535, 32 * 65535 + 1, 64 * 65535):
+        x = torch.arange(rows, device="cuda").float()[:, None]
+        y = torch.empty_like(x)
+        kernels.gemm_f32(x, w, y, rows)
+        assert torch.equal(y, x * 3.0)
+    with pytest.raises(kernels.KernelLibraryError, match="exceed one launch"):
+        kernels.gemm_f32(x, w, y, 64 * 65535 + 1)
