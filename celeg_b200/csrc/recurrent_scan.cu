@@ -1073,7 +1073,7 @@ CELEG_API int celeg_delta_prepare(const float* proj, int stride, const float* ke
     // Tiles of tokens where every access is one of 16 bytes and a step has tokens enough for eight rows of blocks: below that a block
     // a token is the one with more blocks (a thread of a tile walks eight tokens in turn). 2,048 tokens: 19.6 us against 37.6.
     const bool tiles = taps == 4 && args.vector_loads && ((size_t)kernel & 15) == 0 && (dim == 32 || dim == 64 || dim == 128) &&
-                       tokens >= kPrepareTileTokens;
+                       tokens >= kPrepareTileTokens && tokens <= kPrepareTile * 65535;       // (the grid's second extent)
     const dim3 grid((channels + 4 * kPrepareThreads - 1) / (4 * kPrepareThreads), (tokens + kPrepareTile - 1) / kPrepareTile);
     if (tiles && dim == 32) launch_chained(delta_prepare_tile_kernel<32, kPrepareTile>, grid, kPrepareThreads, 0, stream, args);
     else if (tiles && dim == 64) launch_chained(delta_prepare_tile_kernel<64, kPrepareTile>, grid, kPrepareThreads, 0, stream, args);

@@ -70,6 +70,28 @@ def test_delta_prepare_in_tiles(lengths, dim, kv_heads, vw):
         assert np.array_equal(state[slot, :3 * channels].cpu().numpy().reshape(3, channels), rows.astype(np.float32))
 
 
+def test_delta_prepare_of_more_tokens_than_a_launch_has_rows_of_tiles():
+    """524,281 tokens of one span: one more than 65,535 tiles of eight hold."""
+    from celeg_b200 import kernels
+    tokens, dim, vw = 8 * 65535 + 1, 32, 4
+    channels, stride = 2 * dim + vw, 2 * dim + vw + 4
+    g = torch.Generator(device="cuda").manual_seed(8)
+    proj, kernel = torch.randn(tokens, stride, device="cuda", generator=g), torch.randn(channels, 4, device="cuda", generator=g)
+    state = torch.randn(1, 3 * channels, device="cuda", generator=g)
+    rows = torch.cat([state.view(3, channels), proj[:, :channels]]).double()
+    conv, gates = torch.zeros(tokens, channels, device="cuda"), torch.zeros(tokens, 2, device="cuda")
+    span, begins = torch.zeros(tokens, dtype=torch.int32, device="cuda"), dev(np.array([0, tokens], dtype=np.int32))
+    kernels.delta_prepare(proj, kernel, state, state.stride(0), span, begins, span[:1], conv, proj[:, channels:], proj[:, channels + 1:],
+                          torch.zeros(1, device="cuda"), torch.zeros(1, device="cuda"), gates, tokens, 1, channels, 4, 1, dim, 1, 1e-6)
+    sums = sum(rows[j:j + tokens] * kernel[:, j].double() for j in range(4))
+    want = sums * torch.sigmoid(sums)
+    units = want[:, :2 * dim].view(tokens, 2, dim)
+    units /= torch.sqrt(units.square().sum(-1, keepdim=True) + 1e-6)
+    assert float((conv - want).abs().max()) < 10 * 2.0 ** -24 * float(sums.abs().max())      # (as above)
+    assert float((gates[:, 0] - torch.sigmoid(proj[:, channels].double())).abs().max()) < 2e-6
+    assert torch.equal(state.view(3, channels), rows[-3:].float())
+
+
 @pytest.mark.parametrize("lengths", LENGTHS[2:])
 @pytest.mark.parametrize("taps,channels,act", [(4, 516, 2), (3, 64, -1), (2, 33, 2)])
 def test_channel_conv_in_tiles(lengths, taps, channels, act):
