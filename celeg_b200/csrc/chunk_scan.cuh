@@ -309,14 +309,16 @@ __device__ __forceinline__ void load_b_transposed(unsigned (*b)[3][2], const __n
 
 // -------------------------------------------------------------------------------------------------------------- walk
 constexpr int kWalkThreads = 256;
-constexpr int kWalkColumns = 64;                             // columns of S a block: half the keys are split twice over for 32 of
-                                                             // them (64 heads of 128 x 64, 2,048 tokens: 81 us, with 32 88)
-constexpr int kWalkRows = 64;                                // and key channels
-constexpr int kWalkBuffer = SplitTile<kChunk, kWalkRows>::kElements + SplitTile<kChunk, kWalkColumns>::kElements;
+constexpr int kWalkRows = 64;                                // key channels of S a block
+template <int COLUMNS> constexpr int walk_buffer() {
+    return SplitTile<kChunk, kWalkRows>::kElements + SplitTile<kChunk, COLUMNS>::kElements;
+}
 
-template <int MODE>
-__global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const ChunkArgs p) {
-    constexpr int kTiles = 4;                                // tiles of eight columns a warp: four warps along the key
+// COLUMNS of S a block: 32, two blocks an SM, or 64 and one (walk_columns() below says which and why).
+template <int MODE, int COLUMNS>
+__global__ void __launch_bounds__(kWalkThreads, 64 / COLUMNS) chunk_walk_kernel(const ChunkArgs p) {
+    constexpr int kWalkColumns = COLUMNS, kWalkBuffer = walk_buffer<COLUMNS>();
+    constexpr int kTiles = COLUMNS / 16;                     // tiles of eight columns a warp: four warps along the key
     using KTile = SplitTile<kChunk, kWalkRows>;              // channels, two along the columns
     using VTile = SplitTile<kChunk, kWalkColumns>;
     extern __shared__ __align__(128) __nv_bfloat16 tiles[];  // two buffers of a chunk's k and v
@@ -463,8 +465,8 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const Chunk
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 load_a_transposed<KTile>(a[u], k_t, 16 * along, t + 16 * u);
-                load_b_transposed<VTile>(b[u], v_t, 32 * across, t + 16 * u);
-                load_b_transposed<VTile>(b[u] + 2, v_t, 32 * across + 16, t + 16 * u);
+#pragma unroll
+                for (int n = 0; n < kTiles; n += 2) load_b_transposed<VTile>(b[u] + n, v_t, 8 * (kTiles * across + n), t + 16 * u);
             }
             constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
@@ -1120,14 +1122,14 @@ inline int allow_shared(Kernel kernel, size_t bytes, const char* what) {
     return -2;
 }
 
-template <int MODE>
+template <int MODE, int COLUMNS>
 inline int launch_walk(const ChunkArgs& p, cudaStream_t stream) {
-    constexpr size_t bytes = (size_t)2 * kWalkBuffer * sizeof(__nv_bfloat16);
-    const int status = allow_shared(chunk_walk_kernel<MODE>, bytes, "chunk_walk");
+    constexpr size_t bytes = (size_t)2 * walk_buffer<COLUMNS>() * sizeof(__nv_bfloat16);
+    const int status = allow_shared(chunk_walk_kernel<MODE, COLUMNS>, bytes, "chunk_walk");
     if (status != 0) return status;
-    const int v_tiles = (p.vdim + kWalkColumns - 1) / kWalkColumns;
+    const int v_tiles = (p.vdim + COLUMNS - 1) / COLUMNS;
     // A plain launch: blocks of a chained launch that walks for long end up on the few SMs that had room for them.
-    chunk_walk_kernel<MODE><<<dim3(v_tiles * ((p.dim + kWalkRows - 1) / kWalkRows), p.heads, p.spans), kWalkThreads, bytes, stream>>>(p);
+    chunk_walk_kernel<MODE, COLUMNS><<<dim3(v_tiles * ((p.dim + kWalkRows - 1) / kWalkRows), p.heads, p.spans), kWalkThreads, bytes, stream>>>(p);
     return check_launch("chunk_walk");
 }
 
@@ -1166,44 +1168,65 @@ inline int launch_read(const ChunkArgs& p, int chunks, int heads_a_block, cudaSt
     return check_launch("chunk_read");
 }
 
-template <int MODE>
-inline int launch_reads(const ChunkArgs& p, int chunks, cudaStream_t stream) {
-    // Heads that share queries and keys share a block's products of them: as many as make the launch shortest, in rounds of the
-    // blocks that the GPU holds (four an SM, two with wide queries) times a block's steps (products of keys, then of the state's rows
-    // and of the values of every head). 64 heads on 8 of 128 x 64, 2,048 tokens: 96.8 us with
-    // eight heads a block (264 blocks, one round), 110 with four (528, two); 300 tokens 30.6 and 39.4 with one.
+// Heads that share queries and keys share a read-out block's products of them: as many as make the launch shortest, in rounds of the
+// blocks that the GPU holds (four an SM, two with wide queries) times a block's steps (products of keys, then of the state's rows
+// and of the values of every head). 64 heads on 8 of 128 x 64, 2,048 tokens: 96.8 us with eight heads a block (264 blocks, one
+// round), 110 with four (528, two); 300 tokens 30.6 and 39.4 with one.
+inline int heads_of_a_read(int heads, int groups, int dim, int vdim, int chunks) {
+    const int shared = (dim + kReadRows - 1) / kReadRows + 2, slots = dim <= 64 ? 592 : 296;
+    const int per_head = shared * ((vdim + kReadColumns - 1) / kReadColumns);
     int heads_a_block = 1;
-    if (MODE == kChunkScalar) {
-        const int per_head = ((p.dim + kReadRows - 1) / kReadRows + 2) * ((p.vdim + kReadColumns - 1) / kReadColumns);
-        const int shared = (p.dim + kReadRows - 1) / kReadRows + 2, slots = p.dim <= 64 ? 592 : 296;
-        long long best = 0;
-        for (int n = 1; n <= 8 && (p.heads / p.groups) % n == 0; n *= 2) {
-            const long long blocks = (long long)chunks * p.heads / n, cost = (blocks + slots - 1) / slots * (n * per_head + shared);
-            if (n == 1 || cost < best) {
-                best = cost;
-                heads_a_block = n;
-            }
+    long long best = 0;
+    for (int n = 1; n <= 8 && (heads / groups) % n == 0; n *= 2) {
+        const long long blocks = (long long)chunks * heads / n, cost = (blocks + slots - 1) / slots * (n * per_head + shared);
+        if (n == 1 || cost < best) {
+            best = cost;
+            heads_a_block = n;
         }
     }
+    return heads_a_block;
+}
+
+template <int MODE>
+inline int launch_reads(const ChunkArgs& p, int chunks, cudaStream_t stream) {
+    const int heads_a_block = MODE == kChunkScalar ? heads_of_a_read(p.heads, p.groups, p.dim, p.vdim, chunks) : 1;
     return p.dim <= 64 ? launch_read<MODE, 64>(p, chunks, heads_a_block, stream)
                        : launch_read<MODE, 128>(p, chunks, heads_a_block, stream);
 }
 
-// The walk moves a third of the bytes, but a span's chunks come one after another: 2.5 us each, of the longest span (taken as 1.4
-// times the mean of several) or of all blocks over the SMs, whichever is more. Sums take 0.0148 us a chunk and 64 x 64 of S, the carry
-// its bytes at 3.5 TB/s. Walk / sums and carry, us: 64 heads of 128 x 64, 2,048 tokens 81 / 104, 300 15.1 / 19.5, 4,096 in six spans
-// 166 / 269; 16 heads of 64 x 128, 1,999 in four 34 / 26, 2,048 in one (mLSTM) 80 / 29.
-inline bool walks(int heads, int dim, int vdim, int spans, int chunks) {
-    const double tiles = (double)((vdim + 63) / 64) * ((dim + 63) / 64) * heads, mean = (double)chunks / spans;
-    const double longest = spans > 1 && 1.4 * mean < chunks ? 1.4 * mean : chunks, together = tiles * chunks / 148.0;
-    const double walk = 2.5 * (longest > together ? longest : together);
-    return walk < 0.0148 * tiles * chunks + (double)chunks * heads * dim * vdim * 8.0 / 3.5e6;
+// How the states are made: by the walk with 32 or 64 columns a block, or (0) by sums and carry. `longest`: chunks of the longest
+// span, as many as the others leave where it is not known (0).
+//
+// The walk moves a third of the bytes, but a span's chunks come one after another: of the longest span, 1.6 us each with a block of
+// 32 columns an SM (the mLSTM 2.1), 2.6 with two blocks, more by what is above two; 2.4 (2.8) with 64 columns. So it is 64 columns
+// where the blocks of 32, as many as walk at a time on the whole, would share the SMs and those of 64 do not: 64 heads of 128 x 64,
+// 4,096 tokens 158 us, with 32 columns 171; 16 heads of 64 x 128 (64 blocks of 32) 153 and 102, two fifths of a block zeros at values
+// of 96. Sums and carry are bound by their work and bytes: 4.5 us, 11 ns a chunk and 64 x 64 of S, the states' bytes at 4.8 TB/s and
+// those beyond the L2 twice over, and what a span's beginning and end cost, to the mLSTM most. Walk (by its rule) and sums, us: 64
+// heads of 128 x 64, 2,048 tokens 81 / 104, 300 tokens 15.1 / 19.4; 16 of 64 x 128 2,048 tokens 52 / 25, six spans of 512 40 / 34,
+// sixteen of 150 34 / 41, one of 4,096 beside seven of 64 104 / 52 (mLSTM 140 / 69).
+inline int walk_columns(bool stable, int heads, int dim, int vdim, int spans, int chunks, int longest) {
+    const double key_tiles = (double)((dim + kWalkRows - 1) / kWalkRows) * heads;
+    const double narrow = key_tiles * ((vdim + 31) / 32), wide = key_tiles * ((vdim + 63) / 64);
+    const int most = chunks - spans + 1 > 1 ? chunks - spans + 1 : 1;
+    const double chain = longest > 0 && longest < most ? longest : most, at_once = chunks / chain;
+    const bool is_wide = narrow * at_once > 148.0 && wide * at_once <= 148.0 && wide < narrow;
+    double each = stable ? 2.05 : 1.57;
+    if (is_wide) each = stable ? 2.75 : 2.4;
+    else if (narrow * at_once > 148.0) each = (stable ? 3.2 : 2.63) * (narrow * at_once > 296.0 ? narrow * at_once / 296.0 : 1.0);
+    const double elements = (double)heads * dim * vdim, bytes = elements * chunks * 8.0;
+    const double sums = 4.5 + 0.011 * wide * chunks + bytes / 4.8e6 + (bytes > 1e8 ? (bytes - 1e8) / 4e6 : 0.0) +
+                        elements / 131072.0 * spans * (stable ? 2.0 : 0.3);
+    return 2.8 + chain * each < sums ? (is_wide ? 64 : 32) : 0;
 }
 
-// `chunks` bounds the chunks of all spans; p.chunk_begin has chunks / p.pieces + 1 entries
+// `chunks` bounds the chunks of all spans, `longest` those of the longest (0: not known); p.chunk_begin has chunks / p.pieces + 1
+// entries
 template <int MODE>
-inline int launch_chunk_scan(const ChunkArgs& p, int chunks, cudaStream_t stream) {
-    const int status = walks(p.heads, p.dim, p.vdim, p.spans, chunks) ? launch_walk<MODE>(p, stream) : launch_sums<MODE>(p, chunks, stream);
+inline int launch_chunk_scan(const ChunkArgs& p, int chunks, int longest, cudaStream_t stream) {
+    const int columns = walk_columns(MODE == kChunkStable, p.heads, p.dim, p.vdim, p.spans, chunks, longest);
+    const int status = columns == 64 ? launch_walk<MODE, 64>(p, stream) : columns == 32 ? launch_walk<MODE, 32>(p, stream)
+                                                                                        : launch_sums<MODE>(p, chunks, stream);
     return status != 0 ? status : launch_reads<MODE>(p, chunks, stream);
 }
 

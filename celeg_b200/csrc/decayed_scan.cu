@@ -386,9 +386,15 @@ using namespace celeg_b200;
 
 CELEG_API int celeg_chunk_tokens() { return kChunk; }
 
-// Launches that a chunked scan makes its states with: the walk, or sums and carry.
-CELEG_API int celeg_chunk_state_launches(int heads, int dim, int vdim, int spans, int chunks) {
-    return walks(heads, dim, vdim, spans, chunks) ? 1 : 2;
+// How a chunked scan (stable: the mLSTM's) makes its states: columns a block of the walk, or 0 for sums and carry. longest: tokens
+// of the longest span, 0 where they are not known.
+CELEG_API int celeg_chunk_walk_columns(int stable, int heads, int dim, int vdim, int spans, int chunks, int longest) {
+    return spans > 0 && chunks > 0 ? walk_columns(stable != 0, heads, dim, vdim, spans, chunks, (longest + kChunk - 1) / kChunk) : 0;
+}
+
+// Heads that a block of the scalar form's (and the delta rule's) read-outs takes.
+CELEG_API int celeg_chunk_read_heads(int heads, int groups, int dim, int vdim, int chunks) {
+    return heads > 0 && groups > 0 && chunks > 0 ? heads_of_a_read(heads, groups, dim, vdim, chunks) : 0;
 }
 
 // plan: ints [max_chunks + 1 | spans + 1]: the chunks' first tokens (the last chunk's end at the end), the spans' first chunks
@@ -415,7 +421,8 @@ CELEG_API int celeg_channel_decay_scan(const float* q, int q_stride, const float
                                        const float* z, int z_stride, const float* bias, float inv_tau, float q_scale,
                                        float* q_out, float* k_out, float* total, float* products, float* states, float* out,
                                        float* state, long long slot_stride, const int* span_slot, const int* plan,
-                                       int max_chunks, int spans, int chunks, int heads, int dim, int vdim, cudaStream_t stream) {
+                                       int max_chunks, int spans, int chunks, int longest, int heads, int dim, int vdim,
+                                       cudaStream_t stream) {
     CELEG_REQUIRE(spans >= 0 && chunks >= 0 && heads > 0 && dim > 0 && dim <= kDecayMaxDim && vdim > 0,
                   "channel_decay_scan: invalid sizes spans=%d heads=%d dim=%d (at most %d) vdim=%d", spans, heads, dim,
                   kDecayMaxDim, vdim);
@@ -436,7 +443,7 @@ CELEG_API int celeg_channel_decay_scan(const float* q, int q_stride, const float
     p.chunk_begin = plan; p.pieces = 1; p.span_first = span_first; p.spans = spans;
     p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = states; p.out = out;
     p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = vdim;
-    return launch_chunk_scan<kChunkChannel>(p, chunks, stream);
+    return launch_chunk_scan<kChunkChannel>(p, chunks, (longest + kChunk - 1) / kChunk, stream);
 }
 
 // The scalar form: q and k have `groups` heads of dim that heads / groups heads of v share; raw: the steps before bias and
@@ -445,7 +452,7 @@ CELEG_API int celeg_scalar_decay_scan(const float* q, int q_stride, const float*
                                       const float* raw, int raw_stride, const float* dt_bias, const float* a_log,
                                       const float* direct, float2* cum, float* dt, float* states, float* out,
                                       float* state, long long slot_stride, const int* span_slot, const int* plan,
-                                      int max_chunks, int spans, int chunks, int heads, int groups, int dim, int vdim,
+                                      int max_chunks, int spans, int chunks, int longest, int heads, int groups, int dim, int vdim,
                                       cudaStream_t stream) {
     CELEG_REQUIRE(spans >= 0 && chunks >= 0 && heads > 0 && groups > 0 && heads % groups == 0 && dim > 0 && vdim > 0,
                   "scalar_decay_scan: invalid sizes spans=%d heads=%d groups=%d dim=%d vdim=%d", spans, heads, groups, dim, vdim);
@@ -463,7 +470,7 @@ CELEG_API int celeg_scalar_decay_scan(const float* q, int q_stride, const float*
     p.chunk_begin = plan; p.pieces = 1; p.span_first = span_first; p.spans = spans;
     p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = states; p.out = out;
     p.heads = heads; p.groups = groups; p.dim = dim; p.vdim = vdim;
-    return launch_chunk_scan<kChunkScalar>(p, chunks, stream);
+    return launch_chunk_scan<kChunkScalar>(p, chunks, (longest + kChunk - 1) / kChunk, stream);
 }
 
 // A token a request (row i of the inputs is request i's token, its slot span_slot[i]): state update, read-out, and for the

@@ -1256,7 +1256,7 @@ CELEG_API int celeg_retention_decode_raw(const float* proj, int stride, int q_of
 CELEG_API int celeg_retention_segmented(const float* q, int q_stride, const float* k, int k_stride, const float* v,
                                         int v_stride, const float* decay, float* out, float* state, long long slot_stride,
                                         const int* span_begin, const int* span_slot, int spans, int tokens, int heads,
-                                        int dim, int vdim, float q_scale, int segment, int max_segments,
+                                        int dim, int vdim, float q_scale, int segment, int max_segments, int longest,
                                         float* float_scratch, int* int_scratch, cudaStream_t stream) {
     CELEG_REQUIRE(spans >= 0 && tokens >= 0 && heads > 0 && dim > 0 && vdim > 0 && (segment == 64 || segment == 128),
                   "retention_segmented: invalid sizes spans=%d tokens=%d heads=%d dim=%d vdim=%d segment=%d", spans, tokens,
@@ -1280,7 +1280,7 @@ CELEG_API int celeg_retention_segmented(const float* q, int q_stride, const floa
     p.chunk_begin = seg_begin; p.pieces = pieces; p.span_first = span_first; p.spans = spans;
     p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = float_scratch; p.out = out;
     p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = vdim;
-    return launch_chunk_scan<kChunkConstant>(p, max_segments * pieces, stream);
+    return launch_chunk_scan<kChunkConstant>(p, max_segments * pieces, (longest + kChunk - 1) / kChunk, stream);
 }
 
 // The mLSTM over the step's spans in chunks of 64 tokens, from the projection's rows to the read-outs. plan: of
@@ -1291,7 +1291,7 @@ CELEG_API int celeg_mlstm_chunk_scan(const float* q, int q_stride, const float* 
                                      const float* pre_i, const float* pre_f, int pre_stride, const float* bias_i,
                                      const float* bias_f, float cap, float2* gates, double* peaks, float* norms, float* states,
                                      float* out, float* state, long long slot_stride, const int* span_slot, const int* plan,
-                                     int max_chunks, int spans, int chunks, int heads, int dim, int vdim, float q_scale,
+                                     int max_chunks, int spans, int chunks, int longest, int heads, int dim, int vdim, float q_scale,
                                      cudaStream_t stream) {
     CELEG_REQUIRE(spans >= 0 && chunks >= 0 && heads > 0 && dim > 0 && vdim > 0 && cap > 0.0f,
                   "mlstm_chunk_scan: invalid sizes spans=%d chunks=%d heads=%d dim=%d vdim=%d cap=%g", spans, chunks, heads, dim,
@@ -1310,5 +1310,5 @@ CELEG_API int celeg_mlstm_chunk_scan(const float* q, int q_stride, const float* 
     p.chunk_begin = plan; p.pieces = 1; p.span_first = plan + max_chunks + 1; p.spans = spans;
     p.state = state; p.slot_stride = slot_stride; p.span_slot = span_slot; p.states = states; p.out = out;
     p.heads = heads; p.groups = heads; p.dim = dim; p.vdim = vdim;
-    return launch_chunk_scan<kChunkStable>(p, chunks, stream);
+    return launch_chunk_scan<kChunkStable>(p, chunks, (longest + kChunk - 1) / kChunk, stream);
 }

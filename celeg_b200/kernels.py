@@ -149,7 +149,7 @@ _SIGNATURES = {
     "celeg_gated_head_norm": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_int,
                               c_int, c_void_p],
     "celeg_retention_segmented": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_longlong,
-                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
+                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p,
                                   c_void_p, c_void_p],
     "celeg_depth_average": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p,
                             c_float, c_int, c_int, c_int, c_void_p],
@@ -179,22 +179,23 @@ _SIGNATURES = {
     "celeg_chunk_plan": [c_void_p, c_int, c_int, c_void_p, c_void_p],
     "celeg_channel_decay_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
-                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "celeg_general_delta_chunk_scan": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "celeg_decay_sums": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "celeg_delta_operand_bytes": [c_int],
-    "celeg_chunk_state_launches": [c_int, c_int, c_int, c_int, c_int],
+    "celeg_chunk_walk_columns": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
+    "celeg_chunk_read_heads": [c_int, c_int, c_int, c_int, c_int],
     "celeg_delta_chunk_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                c_int, c_float, c_void_p, c_void_p],
     "celeg_mlstm_chunk_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
-                               c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
+                               c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
     "celeg_scalar_decay_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p,
-                                c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "celeg_channel_decay_decode": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_int,
                                    c_void_p, c_float, c_void_p, c_float, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int,
                                    c_int, c_int, c_int, c_void_p, c_int, c_void_p],
@@ -993,10 +994,11 @@ def mlstm_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, pre_i: t
                      bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float, gates: torch.Tensor, peaks: torch.Tensor,
                      norms: torch.Tensor, states: torch.Tensor, out: torch.Tensor, state: torch.Tensor, slot_stride: int,
                      span_slot: torch.Tensor, plan: torch.Tensor, max_chunks: int, spans: int, chunks: int, heads: int,
-                     dim: int, vdim: int, q_scale: float) -> None:
+                     dim: int, vdim: int, q_scale: float, longest: int = 0) -> None:
     """The mLSTM (:func:`mlstm_gates`, then mode SCAN_MLSTM of :func:`recurrent_scan`) over the step's spans in chunks of
     64 tokens (csrc/chunk_scan.cuh), from a plan of :func:`chunk_plan`. Scratch: float32 ``gates`` [tokens, 6 heads],
-    float64 ``peaks`` [chunks * heads], float32 ``norms`` [chunks * heads * dim], ``states`` [chunks * heads * dim * vdim]."""
+    float64 ``peaks`` [chunks * heads], float32 ``norms`` [chunks * heads * dim], ``states`` [chunks * heads * dim * vdim].
+    ``longest``: tokens of the longest span, for :func:`chunk_walk_columns` (0: not known)."""
     for tensor in (q, k, v, pre_i, pre_f, bias_i, bias_f, gates, norms, states, out, state):
         assert tensor.dtype == torch.float32 and tensor.stride(-1) == 1
     assert gates.is_contiguous() and gates.shape[1] == 6 * heads and pre_i.stride(0) == pre_f.stride(0)
@@ -1006,20 +1008,21 @@ def mlstm_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, pre_i: t
     _check(library().celeg_mlstm_chunk_scan(
         _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(pre_i), _ptr(pre_f), pre_i.stride(0),
         _ptr(bias_i), _ptr(bias_f), cap, _ptr(gates), _ptr(peaks), _ptr(norms), _ptr(states), _ptr(out), _ptr(state), slot_stride,
-        _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, dim, vdim, q_scale, _stream()))
+        _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, longest, heads, dim, vdim, q_scale, _stream()))
     global LAUNCHES
-    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans, chunks)      # (a call counts one) the gates, the states, the read-outs
+    LAUNCHES += 1 + _state_launches(True, heads, dim, vdim, spans, chunks, longest)      # (a call counts one) the gates, the states, the read-outs
 
 
 def retention_segmented(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
                         state: torch.Tensor, slot_stride: int, span_begin: torch.Tensor, span_slot: torch.Tensor, spans: int,
                         tokens: int, heads: int, dim: int, vdim: int, q_scale: float, segment: int, max_segments: int,
                         float_scratch: torch.Tensor, int_scratch: torch.Tensor,
-                        identity: Optional[torch.Tensor] = None) -> None:
+                        identity: Optional[torch.Tensor] = None, longest: int = 0) -> None:
     """The retention (mode SCAN_RETENTION of :func:`recurrent_scan`) with every span cut into segments of ``segment``
     tokens, 64 or 128, that are worked on side by side (csrc/chunk_scan.cuh). Scratch: float32 [2 * max_segments * heads * dim *
     vdim], a state every 64 tokens, int32 [max_segments + spans + 2]. Longer segments (a multiple of 64), for which that
-    scratch is too small, are scanned token by token. ``identity`` is not read."""
+    scratch is too small, are scanned token by token. ``identity`` is not read. ``longest``: tokens of the longest span, for
+    :func:`chunk_walk_columns` (0: not known)."""
     for tensor in (q, k, v, decay, out, state, float_scratch):
         assert tensor.dtype == torch.float32 and tensor.stride(-1) == 1
     assert out.is_contiguous() and out.shape[1] == heads * vdim and decay.shape == (heads,)
@@ -1031,10 +1034,11 @@ def retention_segmented(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay
         return
     _check(library().celeg_retention_segmented(_ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay),
                                                _ptr(out), _ptr(state), slot_stride, _ptr(span_begin), _ptr(span_slot), spans,
-                                               tokens, heads, dim, vdim, q_scale, segment, max_segments,
+                                               tokens, heads, dim, vdim, q_scale, segment, max_segments, longest,
                                                _ptr(float_scratch), _ptr(int_scratch), _stream()))
     global LAUNCHES
-    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans, max_segments * (segment // 64))      # (a call counts one) the plan, the states, the read-outs
+    # (a call counts one) the plan, the states, the read-outs
+    LAUNCHES += 1 + _state_launches(False, heads, dim, vdim, spans, max_segments * (segment // 64), longest)
 
 
 def recurrent_decode(mode: int, proj: torch.Tensor, offsets: Tuple[int, int, int, int, int, int],
@@ -1458,9 +1462,19 @@ def chunk_tokens() -> int:
 
 
 @functools.lru_cache(maxsize=256)
-def chunk_state_launches(heads: int, dim: int, vdim: int, spans: int, chunks: int) -> int:
-    """Launches that a chunked scan makes its states with (:data:`LAUNCHES` counts them)."""
-    return int(library().celeg_chunk_state_launches(heads, dim, vdim, spans, chunks))
+def chunk_walk_columns(stable: bool, heads: int, dim: int, vdim: int, spans: int, chunks: int, longest: int = 0) -> int:
+    """How a chunked scan (``stable``: the mLSTM's) makes the states before its ``chunks`` chunks: columns a block of the walk
+    along them, or 0 for sums side by side and their carry. ``longest``: tokens of the longest span (0: not known)."""
+    return int(library().celeg_chunk_walk_columns(int(stable), heads, dim, vdim, spans, chunks, longest))
+
+
+def chunk_read_heads(heads: int, groups: int, dim: int, vdim: int, chunks: int) -> int:
+    """Heads that a block of the read-outs takes in the scans whose heads share queries and keys."""
+    return int(library().celeg_chunk_read_heads(heads, groups, dim, vdim, chunks))
+
+
+def _state_launches(*rule) -> int:
+    return 1 if chunk_walk_columns(*rule) else 2
 
 
 def chunk_plan(span_begin: torch.Tensor, spans: int, max_chunks: int, plan: torch.Tensor) -> None:
@@ -1474,9 +1488,10 @@ def channel_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: tor
                        q_scale: float, q_out: torch.Tensor, k_out: torch.Tensor, total: torch.Tensor, products: torch.Tensor,
                        states: torch.Tensor, out: torch.Tensor, state: torch.Tensor, slot_stride: int,
                        span_slot: torch.Tensor, plan: torch.Tensor, max_chunks: int, spans: int, chunks: int, heads: int,
-                       dim: int, vdim: int) -> None:
+                       dim: int, vdim: int, longest: int = 0) -> None:
     """S <- diag(sigmoid(z + bias)^(1 / tau)) S + k v^T, o = q_scale S^T q along the step's spans (csrc/decayed_scan.cu).
-    ``chunks`` bounds the chunks that the spans make; the scratch holds that many."""
+    ``chunks`` bounds the chunks that the spans make; the scratch holds that many. ``longest``: tokens of the longest span, for
+    :func:`chunk_walk_columns` (0: not known)."""
     for tensor in (q, k, v, z, bias, q_out, k_out, total, products, states, out, state):
         assert tensor.dtype == torch.float32 and tensor.stride(-1) == 1
     assert q_out.shape[1] == k_out.shape[1] == heads * dim and out.is_contiguous() and out.shape[1] == heads * vdim
@@ -1485,19 +1500,19 @@ def channel_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: tor
     _check(library().celeg_channel_decay_scan(
         _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(z), z.stride(0), _ptr(bias), 1.0 / tau, q_scale,
         _ptr(q_out), _ptr(k_out), _ptr(total), _ptr(products), _ptr(states), _ptr(out), _ptr(state), slot_stride,
-        _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, heads, dim, vdim, _stream()))
+        _ptr(span_slot), _ptr(plan), max_chunks, spans, chunks, longest, heads, dim, vdim, _stream()))
     global LAUNCHES
-    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans, chunks)      # the chunks' own products, the states, the read-outs
+    LAUNCHES += 1 + _state_launches(False, heads, dim, vdim, spans, chunks, longest)      # the chunks' own products, the states, the read-outs
 
 
 def scalar_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: torch.Tensor, dt_bias: torch.Tensor,
                       a_log: torch.Tensor, direct: Optional[torch.Tensor], cum: torch.Tensor, dt: torch.Tensor,
                       products: Optional[torch.Tensor], states: torch.Tensor, out: torch.Tensor, state: torch.Tensor,
                       slot_stride: int, span_slot: torch.Tensor, plan: torch.Tensor, max_chunks: int, spans: int, chunks: int,
-                      heads: int, groups: int, dim: int, vdim: int) -> None:
+                      heads: int, groups: int, dim: int, vdim: int, longest: int = 0) -> None:
     """S <- exp(-exp(a_log) dt) S + dt k v^T, o = S^T q + direct v with dt = softplus(raw + dt_bias) along the step's spans;
     heads / groups heads share queries and keys (csrc/decayed_scan.cu). Scratch: ``cum`` [tokens, 2 heads], ``dt`` [tokens,
-    heads]. ``products`` is not read."""
+    heads]. ``products`` is not read. ``longest`` as above."""
     assert cum.is_contiguous() and cum.shape[1] == 2 * heads and dt.is_contiguous() and dt.shape[1] == heads
     for tensor in (q, k, v, raw, dt_bias, a_log, cum, dt, states, out, state):
         assert tensor.dtype == torch.float32 and tensor.stride(-1) == 1
@@ -1505,9 +1520,9 @@ def scalar_decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: to
     _check(library().celeg_scalar_decay_scan(
         _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(raw), raw.stride(0), _ptr(dt_bias), _ptr(a_log),
         _ptr(direct), _ptr(cum), _ptr(dt), _ptr(states), _ptr(out), _ptr(state), slot_stride, _ptr(span_slot),
-        _ptr(plan), max_chunks, spans, chunks, heads, groups, dim, vdim, _stream()))
+        _ptr(plan), max_chunks, spans, chunks, longest, heads, groups, dim, vdim, _stream()))
     global LAUNCHES
-    LAUNCHES += 1 + chunk_state_launches(heads, dim, vdim, spans, chunks)      # the decays, then as above
+    LAUNCHES += 1 + _state_launches(False, heads, dim, vdim, spans, chunks, longest)      # the decays, then as above
 
 
 def channel_decay_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_scale: float, low: torch.Tensor,

@@ -45,12 +45,15 @@ class ChunkedSpans:
         """Whether the scratch holds the chunks of the spans from ``single`` on."""
         return (step.tokens - single) // self.tokens + step.spans - single <= self.chunks_held
 
+    def bound(self, tokens: int, spans: int) -> int:
+        """The chunks that as many tokens in as many spans make at most."""
+        chunks = tokens // self.tokens + spans
+        return chunks if self.tokens_a_chunk is None else min(chunks, tokens // self.tokens_a_chunk)
+
     def of(self, step: StepContext, single: int):
         """(plan, spans, bound of the chunks) of the spans from ``single`` on."""
         spans = step.spans - single
-        chunks = (step.tokens - single) // self.tokens + spans
-        if self.tokens_a_chunk is not None:
-            chunks = min(chunks, (step.tokens - single) // self.tokens_a_chunk)
+        chunks = self.bound(step.tokens - single, spans)
         if chunks > self.chunks_held:
             raise ValueError(f"{chunks} chunks of a step exceed the {self.chunks_held} that the scratch holds")
         key = ("decay.plan", single, self.max_chunks)
@@ -58,6 +61,12 @@ class ChunkedSpans:
             kernels.chunk_plan(step.span_begin[single:], spans, self.max_chunks, self.plan)
             step.extras[key] = True
         return self.plan, spans, chunks
+
+
+def longest_of(step: StepContext, single: int) -> int:
+    """Tokens of the longest span from ``single`` on; a launch shape that several steps share is captured for one answer of
+    each rule that reads this (``Runtime.portion_rules``)."""
+    return max(step.host_span_lengths[single:]) if step.host_span_lengths is not None else step.max_span
 
 
 def _padded_rows(matrix: torch.Tensor, multiple: int = 8) -> torch.Tensor:
@@ -107,6 +116,7 @@ class Mamba2Mixer:
         self.binding: Optional[StateBinding] = None
         self.carried: Optional[torch.Tensor] = None
         self.spans = ChunkedSpans(rt)
+        rt.portion_rules[type(self).__name__, self.heads, self.state, self.vdim] = self.walk_columns
         chunks = self.spans.max_chunks
         self.projected = rt.scratch("recurrent.proj", int(self.w_in.shape[0]), torch.float32)
         self.convolved = rt.scratch("recurrent.conv", self.channels, torch.float32)
@@ -118,6 +128,11 @@ class Mamba2Mixer:
 
     def cache_need(self):
         return StateNeed(elements=self.state_elements + (self.taps - 1) * self.channels)
+
+    def walk_columns(self, lengths) -> int:
+        """How portions of these lengths make their states (:func:`kernels.chunk_walk_columns`)."""
+        return kernels.chunk_walk_columns(False, self.heads, self.state, self.vdim, len(lengths),
+                                          self.spans.bound(sum(lengths), len(lengths)), max(lengths)) if lengths else 0
 
     def bind_cache(self, binding: StateBinding) -> None:
         self.binding = binding
@@ -147,7 +162,8 @@ class Mamba2Mixer:
             plan, spans, chunks = self.spans.of(step, single)
             kernels.scalar_decay_scan(q, k, v, raw, self.dt_bias, self.a_log, self.direct, self.cum, self.dt, None,
                                       self.states, self.read, b.state, b.slot_stride, step.span_slot[single:], plan,
-                                      self.spans.max_chunks, spans, chunks, self.heads, self.groups, self.state, self.vdim)
+                                      self.spans.max_chunks, spans, chunks, self.heads, self.groups, self.state, self.vdim,
+                                      longest_of(step, single))
         kernels.gated_head_norm(self.read, rows[:, :inner], self.norm, True, self.gated, t, self.norm_groups,
                                 inner // self.norm_groups, self.eps, kernels.GATE_SILU + kernels.GATE_BEFORE_NORM)
         rt.linear(self.gated, self.w_out, out, t)
@@ -188,6 +204,7 @@ class GatedLinearAttentionMixer:
                              f"{tuple(self.norm.shape)}, expected ({qk},) and ({self.vdim},)")
         self.binding: Optional[StateBinding] = None
         self.spans = ChunkedSpans(rt)
+        rt.portion_rules[type(self).__name__, self.heads, self.dim, self.vdim] = self.walk_columns
         chunks = self.spans.max_chunks
         self.projected = rt.scratch("linear_attention.proj", int(self.w_in.shape[0]), torch.float32)
         self.low = rt.scratch("linear_attention.low", self.rank)
@@ -202,6 +219,11 @@ class GatedLinearAttentionMixer:
 
     def cache_need(self):
         return StateNeed(elements=self.heads * self.dim * self.vdim)
+
+    def walk_columns(self, lengths) -> int:
+        """How portions of these lengths make their states (:func:`kernels.chunk_walk_columns`)."""
+        return kernels.chunk_walk_columns(False, self.heads, self.dim, self.vdim, len(lengths),
+                                          self.spans.bound(sum(lengths), len(lengths)), max(lengths)) if lengths else 0
 
     def bind_cache(self, binding: StateBinding) -> None:
         self.binding = binding
@@ -230,7 +252,7 @@ class GatedLinearAttentionMixer:
             kernels.channel_decay_scan(q, k, v, self.z, self.decay_bias, self.tau, scale, self.q_taken, self.k_taken,
                                        self.total, self.products, self.states, self.read, b.state, b.slot_stride,
                                        step.span_slot[single:], plan, self.spans.max_chunks, spans, chunks, self.heads,
-                                       self.dim, self.vdim)
+                                       self.dim, self.vdim, longest_of(step, single))
             kernels.gated_head_norm(self.read[single:], gate[single:], self.norm, False, self.gated[single:], t - single,
                                     self.heads, self.vdim, self.eps, kernels.GATE_SILU)
         rt.linear(self.gated, self.w_out, out, t)

@@ -24,7 +24,7 @@ import torch
 
 from .. import kernels
 from ..cache.manager import StateNeed
-from .decayed import ChunkedSpans
+from .decayed import ChunkedSpans, longest_of
 from .mixers import StateBinding
 from .registry import register_part
 from .runtime import Runtime, StepContext
@@ -102,6 +102,7 @@ class MlstmMixer(PortionsInChunks):
         self.gated = rt.scratch("recurrent.gated", self.v_width)
         self.plan_chunks(rt)
         if self.spans is not None:
+            rt.portion_rules[type(self).__name__, self.heads, self.dim, self.vdim] = self.walk_columns
             chunks = self.spans.chunks_held
             self.chunk_gates = rt.scratch("recurrent.chunk_gates", 6 * self.heads, torch.float32)
             self.peaks = rt.flat_scratch("recurrent.peaks", chunks * self.heads, torch.float64)
@@ -113,6 +114,11 @@ class MlstmMixer(PortionsInChunks):
     # 20 168, 152; 160 and 40 x 8 (11) 142, 96.
     CHUNKED_FROM = 144
     TOKENS_A_CHUNK = 20
+
+    def walk_columns(self, lengths) -> int:
+        """How portions of these lengths make their states (:func:`kernels.chunk_walk_columns`)."""
+        return kernels.chunk_walk_columns(True, self.heads, self.dim, self.vdim, len(lengths),
+                                          self.spans.bound(sum(lengths), len(lengths)), max(lengths)) if self.in_chunks(lengths) else 0
 
     def cache_need(self):
         return StateNeed(elements=self.heads * self.dim * self.vdim + self.heads * self.dim + self.heads)
@@ -157,7 +163,7 @@ class MlstmMixer(PortionsInChunks):
             kernels.mlstm_chunk_scan(q, k, v, pre_i, pre_f, self.bias_i, self.bias_f, self.cap, self.chunk_gates, self.peaks,
                                      self.norms, self.states, self.read, b.state, b.slot_stride, step.span_slot[one_by_one:],
                                      plan, self.spans.max_chunks, spans, chunks, self.heads, self.dim, self.vdim,
-                                     self.dim ** -0.5)
+                                     self.dim ** -0.5, longest_of(step, one_by_one))
         kernels.gated_head_norm(self.read, gate, self.norm, True, self.gated, t, self.heads, self.vdim, self.eps,
                                 kernels.GATE_SIGMOID)
         rt.linear(self.gated, self.w_out, out, t)
@@ -316,6 +322,7 @@ class RetentionMixer(PortionsInChunks):
         # in the state does not depend on what was carried into it), each a chunk or two
         self.plan_chunks(rt)
         if self.spans is not None:
+            rt.portion_rules[type(self).__name__, self.heads, self.dim, self.vdim] = self.walk_columns
             self.max_segments = rt.max_tokens // self.SEGMENT + min(rt.max_requests + 16, rt.max_tokens // self.TOKENS_A_CHUNK)
             elements = self.heads * self.dim * self.vdim
             self.segment_states = rt.flat_scratch("retention.segments", 2 * self.max_segments * elements, torch.float32)
@@ -327,6 +334,12 @@ class RetentionMixer(PortionsInChunks):
     # 78; 600 and 40 x 20 (28) 162, 198.
     CHUNKED_FROM = 144
     TOKENS_A_CHUNK = 20
+
+    def walk_columns(self, lengths) -> int:
+        """How portions of these lengths make their states (:func:`kernels.chunk_walk_columns`)."""
+        chunks = 2 * (sum(lengths) // self.SEGMENT + len(lengths))
+        return kernels.chunk_walk_columns(False, self.heads, self.dim, self.vdim, len(lengths), chunks,
+                                          max(lengths)) if self.in_chunks(lengths) else 0
 
     def _scan(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, step: StepContext, scale: float) -> None:
         """The recurrence over the step's spans into ``read``: single tokens at the step's head token by token, long
@@ -345,7 +358,7 @@ class RetentionMixer(PortionsInChunks):
             # (span_begin counts the step's tokens: the rows stay where they are)
             kernels.retention_segmented(q, k, v, self.decay, self.read, b.state, b.slot_stride, step.span_begin[single:],
                                         step.span_slot[single:], spans, t - single, self.heads, self.dim, self.vdim, scale,
-                                        self.SEGMENT, segments, self.segment_states, self.segment_plan)
+                                        self.SEGMENT, segments, self.segment_states, self.segment_plan, longest=longest_of(step, single))
 
     def cache_need(self):
         return StateNeed(elements=self.heads * self.dim * self.vdim)

@@ -227,7 +227,7 @@ class Runtime:
         self._side_stream: Optional[torch.cuda.Stream] = None
         # rules by which parts choose a launch from the lengths of a step's portions: a graph that steps of several lengths
         # share is captured for one answer of each (``portion_routes``)
-        self.portion_rules: Dict[tuple, Callable[[list], bool]] = {}
+        self.portion_rules: Dict[tuple, Callable[[list], int]] = {}
         # Decode steps are a chain of short weight-streaming kernels, the same chain every step. Each of them
         # asks the first megabytes of its successor's weights into the L2, so that memory works across the
         # kernel boundary; the successor of a weight is learnt from the order of the calls (the first step of
@@ -259,7 +259,7 @@ class Runtime:
             self._scratch[key] = torch.empty((self.max_tokens, columns), dtype=dtype, device=self.device)
         return self._scratch[key]
 
-    def portion_routes(self, lengths: list) -> Tuple[bool, ...]:
+    def portion_routes(self, lengths: list) -> Tuple[int, ...]:
         """The answers of the parts' rules for portions of these lengths."""
         return tuple(rule(lengths) for rule in self.portion_rules.values())
 

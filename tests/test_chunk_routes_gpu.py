@@ -1,6 +1,6 @@
-"""The forms of the chunked scans that large sizes select, each against float64: the walk over the chunks (from 222 blocks on)
-where smaller ones sum the chunks side by side, the delta rules' walk with 32 columns a block (from 149 blocks of 16 on),
-read-outs of two and four heads a block; and the delta rules' mixers on single tokens and portions in one step."""
+"""The forms of the chunked scans that their rules select, each against float64: the walk over the chunks with 32 and with 64 columns
+a block, sums of the chunks side by side, the delta rules' walk with 32 columns a block (from 149 blocks of 16 on), read-outs of one
+to eight heads a block; and the delta rules' mixers on single tokens and portions in one step."""
 from __future__ import annotations
 
 import pytest
@@ -39,16 +39,20 @@ def linear(begins, q, k, v, decay, before):
     return out.flatten(1), after
 
 
-@pytest.mark.parametrize("kind,lengths,heads,groups,dim,vdim,walks", [
-    ("scalar", [65, 130], 64, 8, 128, 64, True),
-    ("scalar", [64 * 9 + 1, 63], 64, 8, 64, 33, True),       # two heads a block of the read-outs
-    ("scalar", [64 * 19 + 5], 64, 8, 72, 20, False),         # four
-    ("channel", [65, 130], 56, 56, 64, 64, True), ("channel", [100, 64], 56, 56, 40, 50, True), ("channel", [70], 60, 60, 136, 33, True),
-    ("constant", [65, 130], 56, 56, 64, 64, True), ("constant", [100, 64], 56, 56, 40, 50, True),
-    ("constant", [70, 193, 128], 2, 2, 136, 70, False),      # queries in two passes
-    ("constant", [70], 60, 60, 136, 33, True),
+@pytest.mark.parametrize("kind,lengths,heads,groups,dim,vdim,columns,share", [
+    ("scalar", [130], 100, 100, 64, 64, 64, 1),              # (no heads share keys)
+    ("scalar", [64 * 9 + 1, 63], 64, 8, 64, 33, 0, 2),
+    ("scalar", [64 * 19 + 5], 64, 8, 72, 20, 32, 2),
+    ("scalar", [900], 64, 8, 72, 20, 32, 4),
+    ("scalar", [2048], 64, 8, 128, 64, 64, 8),
+    ("scalar", [100, 64], 64, 8, 64, 33, 64, 1),             # one column in the second half of a block's 64
+    ("channel", [63, 64, 65], 40, 40, 40, 50, 64, 1), ("channel", [70], 60, 60, 136, 33, 32, 1), ("channel", [130, 64], 2, 2, 40, 33, 0, 1),
+    ("constant", [100, 64], 120, 120, 40, 70, 32, 1),
+    ("constant", [65, 130], 64, 64, 64, 33, 64, 1), ("constant", [70], 60, 60, 136, 33, 32, 1),
+    ("constant", [70, 193, 128], 2, 2, 136, 70, 0, 1),       # queries in two passes
+    ("constant", [577, 1, 1, 64], 16, 16, 40, 66, 0, 1),     # one long span beside short ones
 ])
-def test_walk_and_shared_read_outs(kind, lengths, heads, groups, dim, vdim, walks):
+def test_walk_and_shared_read_outs(kind, lengths, heads, groups, dim, vdim, columns, share):
     from celeg_b200 import kernels
     g = torch.Generator(device="cuda").manual_seed(23)
     rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g)      # noqa: E731
@@ -58,7 +62,9 @@ def test_walk_and_shared_read_outs(kind, lengths, heads, groups, dim, vdim, walk
     for n in lengths:
         begins.append(begins[-1] + n)
     chunks = tokens // 64 + spans
-    assert (-(-vdim // 32) * -(-dim // 64) * heads * spans >= 222) == walks
+    cut = 2 * (tokens // 128 + spans) if kind == "constant" else chunks
+    assert kernels.chunk_walk_columns(False, heads, dim, vdim, spans, cut, max(lengths)) == columns
+    assert kind != "scalar" or kernels.chunk_read_heads(heads, groups, dim, vdim, chunks) == share
     q, k, v = rand(tokens, groups * dim), rand(tokens, groups * dim), rand(tokens, wide)
     before, out = rand(spans, elements), full(tokens, wide)
     state = before.clone()
@@ -70,7 +76,7 @@ def test_walk_and_shared_read_outs(kind, lengths, heads, groups, dim, vdim, walk
     if kind == "scalar":
         raw, a_log, direct, bias = rand(tokens, heads), rand(heads) - 2, rand(heads), rand(heads) - 2
         kernels.scalar_decay_scan(q, k, v, raw, bias, a_log, direct, full(tokens, 2 * heads), full(tokens, heads), None,
-                                  full(chunks * elements), out, *where, heads, groups, dim, vdim)
+                                  full(chunks * elements), out, *where, heads, groups, dim, vdim, max(lengths))
         dt = torch.nn.functional.softplus((raw + bias).double(), threshold=100.0)
         share = heads // groups
         want, want_state = linear(begins, q64.repeat_interleave(share, 1), k64.repeat_interleave(share, 1) * dt.unsqueeze(-1), v64,
@@ -80,7 +86,7 @@ def test_walk_and_shared_read_outs(kind, lengths, heads, groups, dim, vdim, walk
         z, bias = rand(tokens, heads * dim), rand(heads * dim)
         kernels.channel_decay_scan(q, k, v, z, bias, 16.0, 0.3, full(tokens, heads * dim), full(tokens, heads * dim),
                                    full(chunks * heads * dim), full(chunks * heads * 4096), full(chunks * elements), out, *where, heads,
-                                   dim, vdim)
+                                   dim, vdim, max(lengths))
         decay = torch.exp(torch.nn.functional.logsigmoid((z + bias).double()) / 16.0).view(tokens, heads, dim)
         want, want_state = linear(begins, q64 * 0.3, k64, v64, decay, before.view(spans, heads, dim, vdim))
     else:
@@ -88,13 +94,40 @@ def test_walk_and_shared_read_outs(kind, lengths, heads, groups, dim, vdim, walk
         segments = tokens // 128 + spans
         kernels.retention_segmented(q, k, v, decay, out, state, state.stride(0), i32(begins), slots, spans, tokens, heads, dim, vdim,
                                     0.3, 128, segments, full(2 * segments * elements),
-                                    torch.zeros(segments + spans + 2, dtype=torch.int32, device="cuda"))
+                                    torch.zeros(segments + spans + 2, dtype=torch.int32, device="cuda"), longest=max(lengths))
         each = decay.double().view(1, heads, 1).expand(tokens, heads, 1)
         want, want_state = linear(begins, q64, k64 * 0.3, v64, each, before.view(spans, heads, dim, vdim))
     # a weight is a product of up to 64 decays with a rounding each: 64 units of 2^-24 at most
     for name, a, b in (("read", out, want), ("state", state, want_state.flatten(1))):
         off = float((a.double() - b).norm() / b.norm())
         assert off <= 64 * 2 ** -24, (name, off)
+
+
+@pytest.mark.parametrize("lengths,heads,dim,vdim,forget,columns", [
+    ([70, 300], 40, 64, 96, -3.0, 64),               # a decay of a twentieth a token
+    ([100, 64], 64, 64, 128, 2.0, 32),               # two spans of two chunks, whole blocks
+    ([63, 64, 65], 40, 40, 33, 3.0, 64),             # odd columns
+    ([70, 65, 64, 1], 40, 136, 33, 1.0, 32),         # three blocks of key channels, the last one almost empty
+    ([130], 100, 72, 20, 4.0, 32),                   # a head in less than half of a block
+    ([577, 1, 64], 6, 32, 48, 3.0, 0),               # one long span beside short ones
+])
+def test_mlstm_by_either_route(lengths, heads, dim, vdim, forget, columns):
+    from celeg_b200 import kernels
+    chunks = sum(lengths) // 64 + len(lengths)
+    assert kernels.chunk_walk_columns(True, heads, dim, vdim, len(lengths), chunks, max(lengths)) == columns
+    chunk_scan.test_mlstm_in_chunks_is_as_near_to_64_bits_as_token_by_token(lengths, heads, dim, vdim, forget)
+
+
+@pytest.mark.parametrize("stable", [False, True])
+def test_one_long_span_beside_short_ones_is_not_walked(stable):
+    """The walk takes a span's chunks one after another: with a span of 4,096 tokens beside seven of 64, or of 3,500 beside fifteen
+    of 40, it takes two to three times what the sums do."""
+    from celeg_b200 import kernels
+    for lengths in ([4096] + [64] * 7, [3500] + [40] * 15):
+        chunks = sum(lengths) // 64 + len(lengths)
+        for heads, dim, vdim in ((16, 64, 128), (16, 128, 64), (8, 96, 96)):
+            assert kernels.chunk_walk_columns(stable, heads, dim, vdim, len(lengths), chunks, max(lengths)) == 0
+    assert kernels.chunk_walk_columns(stable, 16, 64, 128, 16, 53, 150) != 0        # sixteen of 150
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

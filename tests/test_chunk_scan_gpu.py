@@ -36,7 +36,7 @@ def plain_mlstm(q, k, v, gate_i, gate_f, state, begins, slots, heads, dim, vdim)
     ([200], 2, 64, 128, 5.0),                        # a normal head, almost nothing forgotten
     ([130, 66], 2, 40, 7, 2.0),                      # odd columns: no access of two or four
     ([97], 1, 130, 64, 3.0),                         # two blocks of key channels, one almost empty
-    ([70, 300], 40, 64, 96, -3.0),                   # enough blocks for the walk; a decay of a twentieth a token
+    ([70, 300], 40, 64, 96, -3.0),                   # blocks of many heads; a decay of a twentieth a token
 ])
 def test_mlstm_in_chunks_is_as_near_to_64_bits_as_token_by_token(lengths, heads, dim, vdim, forget):
     from celeg_b200 import kernels
@@ -69,7 +69,7 @@ def test_mlstm_in_chunks_is_as_near_to_64_bits_as_token_by_token(lengths, heads,
     kernels.mlstm_chunk_scan(q, k, v, pre_i, pre_f, bias_i, bias_f, cap, full(tokens, 6 * heads),
                              torch.zeros(chunks * heads, dtype=torch.float64, device="cuda"), full(chunks * heads * dim),
                              full(chunks * heads * dim * vdim), got, got_state, got_state.stride(0), i32(slots), plan, chunks + 3,
-                             spans, chunks, heads, dim, vdim, dim ** -0.5)
+                             spans, chunks, heads, dim, vdim, dim ** -0.5, max(lengths))
 
     def off(x, y):
         return float((x.double() - y).norm() / y.norm())
