@@ -392,7 +392,7 @@ __global__ void delta_prepare_kernel(const DeltaPrepareArgs a) {
 // DIM / 4 lanes are a head of q or k, so a head's lanes are neighbours of one warp. 2,048 tokens of 4,096 channels: 19.6 us, a block
 // a token 37.6. Memory bounds it (67 MB, 3.4 TB/s).
 constexpr int kPrepareThreads = 128;
-constexpr int kPrepareTile = 8, kPrepareTileTokens = 64;
+constexpr int kPrepareTile = 8;
 template <int DIM, int kTile>
 __global__ void __launch_bounds__(kPrepareThreads) delta_prepare_tile_kernel(const DeltaPrepareArgs a) {
     chain_release();
@@ -401,15 +401,16 @@ __global__ void __launch_bounds__(kPrepareThreads) delta_prepare_tile_kernel(con
     const int t0 = blockIdx.y * kTile, t1 = min(t0 + kTile, a.tokens);
     const bool mine = c < a.channels, of_head = c < 2 * a.qk_heads * DIM;
     float4 x[kTile + 3], w[4];
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // (ones where a thread has no channels: a quotient of zeros would take its slow path, 2 us for eight tokens)
+    const float4 none = mine ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
     // (the rows before the tile before it is known whether they are of its first token's span)
 #pragma unroll
     for (int i = 0; i < kTile + 3; ++i) {
         const int t = t0 - 3 + i;
-        x[i] = mine && t >= 0 && t < t1 ? *reinterpret_cast<const float4*>(a.proj + (size_t)t * a.stride + c) : zero;
+        x[i] = mine && t >= 0 && t < t1 ? *reinterpret_cast<const float4*>(a.proj + (size_t)t * a.stride + c) : none;
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w[j] = mine ? __ldg(reinterpret_cast<const float4*>(a.kernel + (size_t)(c + j) * 4)) : zero;
+    for (int j = 0; j < 4; ++j) w[j] = mine ? __ldg(reinterpret_cast<const float4*>(a.kernel + (size_t)(c + j) * 4)) : none;
     int span = a.token_span[t0];
     const int last_span = a.token_span[t1 - 1];
     float4 history[3];
@@ -1070,10 +1071,14 @@ CELEG_API int celeg_delta_prepare(const float* proj, int stride, const float* ke
     args.vector_loads =
         channels % 4 == 0 && stride % 4 == 0 && slot_stride % 4 == 0 &&
         (((size_t)proj | (size_t)carried | (size_t)conv_out) & 15) == 0;
-    // Tiles of tokens where every access is one of 16 bytes and a step has tokens enough for eight rows of blocks: below that a block
-    // a token is the one with more blocks (a thread of a tile walks eight tokens in turn). 2,048 tokens: 19.6 us against 37.6.
+    // Tiles of tokens where every access is one of 16 bytes and the step has work enough. A thread of a tile walks eight tokens in
+    // turn: 6 us however few there are. A block a token takes 2.6 us and one for every 900 channels, then 2.8 ns a thousand numbers,
+    // and twice that as soon as the blocks are more than five an SM. By tokens, us, tiles / a block a token: 4,096 channels 64 tokens
+    // 6.0 / 7.5, 512 7.6 / 12.5, 2,000 18.4 / 34.9; 2,048 channels 64 tokens 6.0 / 4.8, 512 6.4 / 7.7; 1,280 channels 512 tokens 6.6 /
+    // 5.8, 800 6.9 / 9.5.
     const bool tiles = taps == 4 && args.vector_loads && ((size_t)kernel & 15) == 0 && (dim == 32 || dim == 64 || dim == 128) &&
-                       tokens >= kPrepareTileTokens && tokens <= kPrepareTile * 65535;       // (the grid's second extent)
+                       tokens >= 64 && (tokens > 740 || (long long)channels * (tokens + 600) >= 2100000) &&
+                       tokens <= kPrepareTile * 65535;       // (the grid's second extent)
     const dim3 grid((channels + 4 * kPrepareThreads - 1) / (4 * kPrepareThreads), (tokens + kPrepareTile - 1) / kPrepareTile);
     if (tiles && dim == 32) launch_chained(delta_prepare_tile_kernel<32, kPrepareTile>, grid, kPrepareThreads, 0, stream, args);
     else if (tiles && dim == 64) launch_chained(delta_prepare_tile_kernel<64, kPrepareTile>, grid, kPrepareThreads, 0, stream, args);

@@ -32,12 +32,13 @@ def spans_of(lengths):
     return dev(np.repeat(np.arange(len(lengths)), lengths).astype(np.int32)), dev(begins)
 
 
-# 63 and 64 tokens: the kernel of a token a block and the first step of tiles; spans of 1 to 3 tokens begin inside tiles
 LENGTHS = [[63], [64], [61, 1, 2, 3, 1, 9], [1, 1, 1, 70], [7, 8, 9, 40, 17], [200]]
 
 
-@pytest.mark.parametrize("lengths", LENGTHS)
-@pytest.mark.parametrize("dim,kv_heads,vw", [(32, 3, 100), (64, 2, 64), (128, 5, 36)])
+# Tiles from 741 tokens on, with 4,132 channels from 64: the last step without them and the first with; spans of 1 to 3 tokens begin
+# inside tiles, and a block along the channels may have few of them
+@pytest.mark.parametrize("lengths", LENGTHS + [[740], [741], [725, 1, 2, 3, 1, 9], [1, 1, 1, 740]])
+@pytest.mark.parametrize("dim,kv_heads,vw", [(32, 3, 100), (64, 2, 64), (128, 5, 36), (128, 16, 36)])
 def test_delta_prepare_in_tiles(lengths, dim, kv_heads, vw):
     from celeg_b200 import kernels
     rng = np.random.default_rng(len(lengths) + dim)
