@@ -754,7 +754,7 @@ struct DecodeStepParams {
     const float* proj; int stride;                 // [tokens, stride] rows of the input projection
     int q_off, k_off, v_off, gate_off, g0_off, g1_off;
     const float* conv_kernel; float* carried; int taps, channels;            // delta only
-    int group;                                     // delta: heads a key head where this launch moves the carried inputs on, or 0
+    int group;                                     // delta, where the launch moves the carried inputs on: heads a key head
     const float* bias0; const float* bias1; float cap;   // mLSTM: gate biases and cap; delta: A_log and dt_bias
     const float* norm_w; int norm_per_head; float eps, unit_eps;
     float* state; long long slot_stride;
@@ -767,7 +767,10 @@ struct DecodeStepParams {
                                                    // heads * vdim], and norm and gate are the caller's (one over all heads)
 };
 
-template <int MODE, typename A>
+// EARLY: the state's first columns are asked for before anything else. Not so in the delta rule's launches whose blocks come in
+// rounds, where the convolutions' loads would queue behind them (64 requests of 32 heads of 64: 110 us, 105 without); the others
+// of the delta rule move the carried inputs on too.
+template <int MODE, typename A, bool EARLY>
 __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepParams p) {
     extern __shared__ float decode_smem[];          // k [dim] | q [dim] | o [vdim] | partial sums [2 * warps * 32]
     __shared__ float scratch[33];
@@ -783,7 +786,7 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
     float* part_s = o_s + vdim;
     const float* row = p.proj + (size_t)t * p.stride;
     const long long slot_at = (long long)p.span_slot[t] * p.slot_stride;
-    float* carried = MODE == kScanDelta ? p.carried + slot_at : nullptr;
+    const float* carried = MODE == kScanDelta ? p.carried + slot_at : nullptr;
     float* slot = p.state + slot_at;
     float* s_head = slot + (size_t)head * dim * vdim;
     float* n_head = slot + (size_t)heads * dim * vdim + (size_t)head * dim;
@@ -795,10 +798,15 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
     // column meet in shared memory.
     constexpr int kKeep = 32;
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int groups = (vdim + 31) >> 5;
-    const int split = max(1, warps / groups);
-    const int groups_at_once = warps / split, part = warp % split;
-    const bool kept = dim <= kKeep * split;
+    int groups, split, groups_at_once, part;
+    bool kept;
+    auto cut = [&] {                                         // (not EARLY: behind the convolutions; ahead of them 2 % slower)
+        groups = (vdim + 31) >> 5;
+        split = max(1, warps / groups);
+        groups_at_once = warps / split;
+        part = warp % split;
+        kept = dim <= kKeep * split;
+    };
     float cells[kKeep];
     auto load_cells = [&](int j) {
 #pragma unroll
@@ -807,9 +815,11 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
             cells[i] = e < dim ? s_head[(size_t)e * vdim + j] : 0.0f;
         }
     };
-    const int first_column = (warp / split) * 32 + lane;
-    const bool loaded = kept && warp < groups_at_once * split && warp / split < groups && first_column < vdim;
-    if (loaded) load_cells(first_column);
+    if constexpr (EARLY) {
+        cut();
+        const int first_column = (warp / split) * 32 + lane;
+        if (kept && warp < groups_at_once * split && warp / split < groups && first_column < vdim) load_cells(first_column);
+    }
 
     // a convolved channel of the delta rule: taps - 1 carried inputs (oldest first), then the token's own
     auto convolved = [&](int c) {
@@ -839,7 +849,7 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
         q2 += qv * qv;
     }
     if (MODE == kScanDelta) {
-        if (p.group > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // q's and k's carried inputs: read
+        if (EARLY && p.group > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // q's and k's carried inputs: read
         k2 = block_sum(k2, scratch);
         q2 = block_sum(q2, scratch);
         const float k_inv = 1.0f / sqrtf(k2 + p.unit_eps), q_inv = 1.0f / sqrtf(q2 + p.unit_eps);
@@ -875,6 +885,7 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
         write = expf(g0 - m_new);
         lower = fmaxf(fabsf(keep * nq + write * kq), expf(-m_new)) + 1e-6f;
     }
+    if constexpr (!EARLY) cut();
     float squares = 0.0f;
     for (int first_group = 0; first_group < groups; first_group += groups_at_once) {
         const int g = first_group + warp / split;
@@ -883,7 +894,7 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
         float sk = 0.0f, sq = 0.0f;
         if (active) {
             if (kept) {
-                if (first_group > 0) load_cells(j);
+                if (!EARLY || first_group > 0) load_cells(j);
 #pragma unroll
                 for (int i = 0; i < kKeep; ++i) {
                     const int e = part + i * split;
@@ -958,7 +969,7 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
         return;
     }
     squares = block_sum(squares, scratch);
-    if (MODE == kScanDelta && p.group > 0) {
+    if (MODE == kScanDelta && EARLY) {
         // The carried inputs move on by the token: v's are this block's alone (and the sum above comes after its threads' reads),
         // q's and k's are read by every head of the group, a cluster, whose first block writes them once all have.
         if (p.group > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
@@ -972,7 +983,7 @@ __global__ void __launch_bounds__(256) recurrent_decode_kernel(const DecodeStepP
                 if (r < p.taps - 1) keep_inputs[r] = r < p.taps - 2 ? carried[(size_t)(r + 1) * p.channels + c] : row[c];
 #pragma unroll
             for (int r = 0; r < 15; ++r)
-                if (r < p.taps - 1) carried[(size_t)r * p.channels + c] = keep_inputs[r];
+                if (r < p.taps - 1) p.carried[slot_at + (size_t)r * p.channels + c] = keep_inputs[r];
         }
     }
     const float inv = 1.0f / sqrtf(squares / (float)vdim + p.eps);
@@ -1154,6 +1165,19 @@ CELEG_API int celeg_gated_head_norm(const float* o, const float* gate, int gate_
     return check_launch("gated_head_norm");
 }
 
+// Whether a decoding launch of the delta rule moves the carried inputs on itself (q, k and v being all of them, one after another).
+// A key head's heads are a cluster then, so they have to fit one of portable size, and all clusters the GPU at once: a block takes
+// an SM, of the clusters of more than two blocks some SMs are left over, and blocks that wait for a cluster's room wait for all of
+// it. Beyond that a second launch costs less. One launch / two, 64 x 64, us: 2 requests of 32 heads on 16 9.0 / 10.9; 32 on 4, 3
+// requests 9.2 / 10.8, 4 16.7 / 11.0, 64 155 / 109; 32 on 16, 4 9.3 / 11.1, 24 53 / 47; a key head a head, 8 17.1 / 18.4, 16 32.5 / 32.2.
+static bool moves_carried(int taps, int tokens, int heads, int kv_heads) {
+    const int group = heads / kv_heads;
+    return taps > 1 && group <= 8 && (long long)tokens * heads <= (group == 1 ? 296 : group == 2 ? 148 : group <= 4 ? 128 : 96);
+}
+CELEG_API int celeg_recurrent_decode_moves_carried(int taps, int tokens, int heads, int kv_heads) {
+    return moves_carried(taps, tokens, heads, kv_heads) ? 1 : 0;
+}
+
 // One token per request (row i of ``proj`` is request i's token, its slot span_slot[i]): everything between the
 // two projections of a matrix-state mixer in one launch. mode 0 (delta): the convolved channels [q | k | v] are
 // the first ``channels`` columns of a row, bias0 = A_log, bias1 = dt_bias, the output gate is SiLU; the carried
@@ -1178,14 +1202,11 @@ static int recurrent_decode_launch(int mode, const float* proj, int stride, int 
     const size_t smem = (size_t)(2 * dim + vdim + 2 * kDecodeStepThreads) * sizeof(float);
     CELEG_REQUIRE(smem <= 40 * 1024, "recurrent_decode: head sizes %d and %d exceed a block's shared memory", dim, vdim);
     if (tokens == 0) return 0;
-    // The launch moves the carried inputs on itself where q, k and v are all of them, one after another, and a key head's heads fit
-    // a cluster of portable size: 2 requests of 16 heads of 64 on 8 key heads, 9.8 us of one kernel against 9.1 and 2.5 of two, a
-    // whole call of the mixer 36.2 us against 37.9; elsewhere a second launch does.
-    const int group = heads / kv_heads, qk_width = kv_heads * dim;
-    const bool moves = mode == kScanDelta && taps > 1 && !raw_out && group <= 8 && q_off == 0 && k_off == qk_width && v_off == 2 * qk_width &&
-                       channels == 2 * qk_width + heads * vdim;
+    const int qk_width = kv_heads * dim;
+    const bool moves = mode == kScanDelta && !raw_out && q_off == 0 && k_off == qk_width && v_off == 2 * qk_width &&
+                       channels == 2 * qk_width + heads * vdim && moves_carried(taps, tokens, heads, kv_heads);
     const DecodeStepParams p = {proj, stride, q_off, k_off, v_off, gate_off, g0_off, g1_off, conv_kernel, carried, taps,
-                                channels, moves ? group : 0, bias0, bias1, cap, norm_w, norm_per_head, eps, unit_eps, state, slot_stride,
+                                channels, heads / kv_heads, bias0, bias1, cap, norm_w, norm_per_head, eps, unit_eps, state, slot_stride,
                                 span_slot, heads, kv_heads, dim, vdim, q_scale, out, input_act, raw_out};
     dim3 grid(heads, tokens);
     if (mode == kScanDelta) {
@@ -1198,14 +1219,15 @@ static int recurrent_decode_launch(int mode, const float* proj, int stride, int 
         attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attributes[0].val.programmaticStreamSerializationAllowed = chaining_enabled() ? 1 : 0;
         attributes[1].id = cudaLaunchAttributeClusterDimension;
-        attributes[1].val.clusterDim.x = moves ? group : 1;
+        attributes[1].val.clusterDim.x = moves ? heads / kv_heads : 1;
         attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
         config.attrs = attributes;
-        config.numAttrs = moves && group > 1 ? 2 : 1;
+        config.numAttrs = moves && heads > kv_heads ? 2 : 1;
         if (act_dtype == kFloat32)
-            cudaLaunchKernelEx(&config, recurrent_decode_kernel<kScanDelta, float>, p);
+            cudaLaunchKernelEx(&config, moves ? recurrent_decode_kernel<kScanDelta, float, true> : recurrent_decode_kernel<kScanDelta, float, false>, p);
         else
-            cudaLaunchKernelEx(&config, recurrent_decode_kernel<kScanDelta, __nv_bfloat16>, p);
+            cudaLaunchKernelEx(&config, moves ? recurrent_decode_kernel<kScanDelta, __nv_bfloat16, true>
+                                              : recurrent_decode_kernel<kScanDelta, __nv_bfloat16, false>, p);
         int status = check_launch("recurrent_decode");
         if (status != 0 || taps == 1 || moves) return status;
         const long long units = (long long)tokens * channels;
@@ -1215,15 +1237,15 @@ static int recurrent_decode_launch(int mode, const float* proj, int stride, int 
     }
     if (mode == kScanRetention) {
         if (act_dtype == kFloat32)
-            launch_chained(recurrent_decode_kernel<kScanRetention, float>, grid, kDecodeStepThreads, smem, stream, p);
+            launch_chained(recurrent_decode_kernel<kScanRetention, float, true>, grid, kDecodeStepThreads, smem, stream, p);
         else
-            launch_chained(recurrent_decode_kernel<kScanRetention, __nv_bfloat16>, grid, kDecodeStepThreads, smem, stream, p);
+            launch_chained(recurrent_decode_kernel<kScanRetention, __nv_bfloat16, true>, grid, kDecodeStepThreads, smem, stream, p);
         return check_launch("recurrent_decode");
     }
     if (act_dtype == kFloat32)
-        launch_chained(recurrent_decode_kernel<kScanMlstm, float>, grid, kDecodeStepThreads, smem, stream, p);
+        launch_chained(recurrent_decode_kernel<kScanMlstm, float, true>, grid, kDecodeStepThreads, smem, stream, p);
     else
-        launch_chained(recurrent_decode_kernel<kScanMlstm, __nv_bfloat16>, grid, kDecodeStepThreads, smem, stream, p);
+        launch_chained(recurrent_decode_kernel<kScanMlstm, __nv_bfloat16, true>, grid, kDecodeStepThreads, smem, stream, p);
     return check_launch("recurrent_decode");
 }
 

@@ -187,6 +187,7 @@ _SIGNATURES = {
     "celeg_delta_operand_bytes": [c_int],
     "celeg_chunk_walk_columns": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
     "celeg_chunk_read_heads": [c_int, c_int, c_int, c_int, c_int],
+    "celeg_recurrent_decode_moves_carried": [c_int, c_int, c_int, c_int],
     "celeg_delta_chunk_scan": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                c_int, c_float, c_void_p, c_void_p],
@@ -1048,8 +1049,9 @@ def recurrent_decode(mode: int, proj: torch.Tensor, offsets: Tuple[int, int, int
                      span_begin: torch.Tensor, span_slot: torch.Tensor, tokens: int, heads: int, kv_heads: int,
                      dim: int, vdim: int, q_scale: float, out: torch.Tensor) -> None:
     """A decoding step of a matrix-state mixer between its two projections, one launch (the delta rule's carried
-    inputs: a second where q, k and v are not all of the channels in this order or a key head has more than 8 heads): row i of ``proj`` (float32) is the one token of request i. ``offsets``: columns of
-    (q, k, v, output gate, first gate, second gate) in a row. See csrc/recurrent_scan.cu."""
+    inputs: a second where q, k and v are not all of the channels in this order, or for many heads,
+    :func:`decode_moves_carried`): row i of ``proj`` (float32) is the one token of request i. ``offsets``: columns of (q, k, v,
+    output gate, first gate, second gate) in a row. See csrc/recurrent_scan.cu."""
     assert proj.dtype == torch.float32 and proj.stride(-1) == 1 and out.is_contiguous() and out.shape[1] == heads * vdim
     _check(library().celeg_recurrent_decode(
         mode, _ptr(proj), proj.stride(0), *offsets, _ptr(conv_kernel), _ptr(carried), taps, channels, _ptr(bias0),
@@ -1059,7 +1061,14 @@ def recurrent_decode(mode: int, proj: torch.Tensor, offsets: Tuple[int, int, int
     global LAUNCHES
     if mode == SCAN_DELTA and taps > 1:
         qk = kv_heads * dim
-        LAUNCHES += heads > 8 * kv_heads or tuple(offsets[:3]) != (0, qk, 2 * qk) or channels != 2 * qk + heads * vdim
+        LAUNCHES += (tuple(offsets[:3]) != (0, qk, 2 * qk) or channels != 2 * qk + heads * vdim
+                     or not decode_moves_carried(taps, tokens, heads, kv_heads))
+
+
+@functools.lru_cache(maxsize=256)
+def decode_moves_carried(taps: int, tokens: int, heads: int, kv_heads: int) -> bool:
+    """Whether the delta rule's decoding launch moves the carried inputs on itself."""
+    return bool(library().celeg_recurrent_decode_moves_carried(taps, tokens, heads, kv_heads))
 
 
 def mlstm_gates(pre_i: torch.Tensor, pre_f: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float,

@@ -251,7 +251,7 @@ class GatedDeltaMixer(PortionsInChunks):
         at = self.channels
         if step.max_span == 1 and step.spans == t:
             # every request brings one token: convolutions, unit norms, gates, state update, read-out, norm, output gate
-            # and the carried inputs' move in one launch (the last in a second at more than 8 heads a key head)
+            # and, of few requests, the carried inputs' move in one launch
             offsets = (0, self.qk_width, 2 * self.qk_width, self.channels, self.channels + self.v_width,
                        self.channels + self.v_width + self.heads)
             kernels.recurrent_decode(kernels.SCAN_DELTA, rows, offsets, self.kernel, self.carried, self.taps,

@@ -12,9 +12,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps", [(4, 4, 64, 64, 4), (4, 2, 64, 64, 4), (8, 1, 32, 40, 2), (9, 1, 16, 24, 3),
                                                             (6, 2, 200, 300, 3), (3, 1, 40, 520, 16), (16, 2, 128, 128, 4),
                                                             (2, 1, 8, 8, 1)])
-def test_carried_inputs_move_on(heads, kv_heads, dim, vdim, taps):
+def test_carried_inputs_move_on(heads, kv_heads, dim, vdim, taps, tokens=3):
     torch.manual_seed(heads)
-    tokens, qk, vw = 3, kv_heads * dim, heads * vdim
+    qk, vw = kv_heads * dim, heads * vdim
     channels = 2 * qk + vw
     kernel = torch.randn(channels, taps, device="cuda") * 0.5
     a_log, dt_bias = torch.randn(heads, device="cuda") - 1.0, torch.randn(heads, device="cuda")
@@ -24,7 +24,7 @@ def test_carried_inputs_move_on(heads, kv_heads, dim, vdim, taps):
     state = torch.randn(tokens, stride, device="cuda") * 0.3
     whole = state.clone()
     begins = torch.arange(tokens + 1, dtype=torch.int32, device="cuda")
-    slots = torch.tensor([2, 0, 1], dtype=torch.int32, device="cuda")
+    slots = (torch.arange(tokens, dtype=torch.int32, device="cuda") + 2) % tokens
     spans = torch.arange(tokens, dtype=torch.int32, device="cuda")
     gates, conv = torch.zeros(tokens, 2 * heads, device="cuda"), torch.zeros(tokens, channels, device="cuda")
     read, want, got = (torch.zeros(tokens, vw, device="cuda") for _ in range(3))
@@ -50,3 +50,11 @@ def test_carried_inputs_move_on(heads, kv_heads, dim, vdim, taps):
         bound = 8 * dim * 2 ** -24
         assert float((got - want).abs().max()) <= bound * float(want.abs().max()) + 1e-5
         assert float((whole - state).abs().max()) <= bound * float(state.abs().max()) + 1e-5
+
+
+@pytest.mark.parametrize("heads,kv_heads,most", [(4, 4, 74), (4, 2, 37), (8, 2, 16), (8, 1, 12)])
+def test_carried_inputs_of_many_requests(heads, kv_heads, most):
+    """The most requests whose launch moves the inputs on itself, and one more."""
+    for tokens in (most, most + 1):
+        assert kernels.decode_moves_carried(4, tokens, heads, kv_heads) == (tokens == most)
+        test_carried_inputs_move_on(heads, kv_heads, 32, 40, 4, tokens)
