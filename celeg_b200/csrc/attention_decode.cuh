@@ -156,10 +156,11 @@ __device__ __forceinline__ void decode_copy_tile(__nv_bfloat16* k_dst, __nv_bflo
 }
 
 // A warp's running result over its tiles: rows g and g + 8 of the 16 query heads; maxima in units of log2.
-template <int D_PAD>
+// HELD: the queries' fragments stay in registers.
+template <int D_PAD, bool HELD>
 struct DecodeRows {
     float o[D_PAD / 8][4], run_max[2], run_sum[2];
-    unsigned q[D_PAD == 64 ? 4 : 1][4];                     // the queries' fragments, where the registers allow
+    unsigned q[HELD ? D_PAD / 16 : 1][4];
     __device__ __forceinline__ void clear() {
 #pragma unroll
         for (int i = 0; i < D_PAD / 8; ++i)
@@ -172,19 +173,19 @@ struct DecodeRows {
         ldmatrix_x4(a, q_s + tile_offset<D_PAD>(((lane >> 3) & 1) * 8 + (lane & 7), kt * 2 + (lane >> 4)));
     }
     __device__ __forceinline__ void hold_q(const __nv_bfloat16* q_s, int lane) {
-        if constexpr (D_PAD == 64) {
+        if constexpr (HELD) {
 #pragma unroll
-            for (int kt = 0; kt < 4; ++kt) load_q(q[kt], q_s, kt, lane);
+            for (int kt = 0; kt < D_PAD / 16; ++kt) load_q(q[kt], q_s, kt, lane);
         }
     }
     // The tile of keys tile_begin .. tile_begin + 31, those from `end` on do not count. What bounded this kernel over long contexts
     // was the instructions of a tile, a warp's chain of them and all warps' on the SM, 2 us a tile even with an empty GPU (three
     // stages of copies instead of two gained nothing). So rows 8 to 15 are left out of the exponentials for groups of at most
-    // eight heads, a tile that needs no mask, cap or bias has its scores scaled in place, the outputs are
-    // rescaled only when a maximum has grown, the queries' fragments stay in registers, and a copy that has nothing to bring is one
-    // of no bytes instead of a branch. 32 heads on 8 of 64, before and now, us: 8 requests of 16 k keys 72 and 60 (268 MB: 41 at
-    // 6.5 TB/s, and about 10 around the loop), 16 of 6 k 74 and 50, 1 of 130 k 75 and 69, 1 of 16 k 26 and 22, 8 of 578 14.5 and
-    // 12.8.
+    // eight heads, a tile that needs no mask, cap or bias has its scores scaled in place, the outputs are rescaled only when a
+    // maximum has grown, the queries' fragments stay in registers where blocks have two stages (at one, five blocks an SM, they
+    // spilled), and a copy that has nothing to bring is one of no bytes instead of a branch. 32 heads on 8 of 64, before and now, us:
+    // 8 requests of 16,384 keys 71 and 49 (268 MB: 41 at 6.5 TB/s), 16 of 6,000 77 and 44, 1 of 130,000 72 and 56, 1 of 16,384 23
+    // and 18, 8 of 578 12.8 and 11.7.
     __device__ __forceinline__ void take(const DecodeParams& p, const __nv_bfloat16* q_s, const __nv_bfloat16* k_t,
                                          const __nv_bfloat16* v_t, const int tile_begin, const int end, const int pos,
                                          const int kvh, const int group, const int lane) {
@@ -197,7 +198,7 @@ struct DecodeRows {
 #pragma unroll
         for (int kt = 0; kt < D_PAD / 16; ++kt) {
             unsigned a[4];
-            if constexpr (D_PAD == 64) {
+            if constexpr (HELD) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) a[i] = q[kt][i];
             } else {
@@ -424,14 +425,14 @@ __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, con
         sync();
     }
 
-    DecodeRows<D_PAD> rows;
+    DecodeRows<D_PAD, D_PAD == 64 && kStages == 2> rows;
     rows.clear();
     rows.hold_q(q_s, lane);
 
     auto next_tile = [&](const int at, const int stage) {       // the tile at `at` into a stage that has been used
         if (at < end) {
-            issue(at, stage, next_page);
-            next_page = look_up(at + kTileStride);
+            issue(at, stage, kStages > 1 || D_PAD > 64 ? next_page : look_up(at));
+            if (kStages > 1 || D_PAD > 64) next_page = look_up(at + kTileStride);
         }
         cp_async_commit();
     };
@@ -731,7 +732,7 @@ __device__ __forceinline__ void attention_decode_item_solo(const DecodeParams& p
         __syncwarp();
     }
 
-    DecodeRows<D_PAD> rows;
+    DecodeRows<D_PAD, D_PAD == 64> rows;
     rows.clear();
     rows.hold_q(q_s, lane);
 
