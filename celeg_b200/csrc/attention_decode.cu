@@ -11,7 +11,7 @@ struct BlockSync {
 // (the forms are laid out for five blocks per SM at head size 64 with one stage, three with two stages or at head
 // size 128: the registers must allow them too)
 template <int D_PAD, int BN>
-__global__ void __launch_bounds__(kDecodeThreads, (D_PAD == 64 && BN == 32) ? 5 : D_PAD * BN <= 4096 ? 3 : D_PAD * BN <= 6144 ? 2 : 1)
+__global__ void __launch_bounds__(kDecodeThreads, (D_PAD == 64 && BN == 32) ? 5 : D_PAD * BN <= 4096 ? 3 : 1)
 attention_decode_kernel(const DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     chain_release();

@@ -304,7 +304,7 @@ __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, con
                                                       unsigned char* smem_raw, const int tid, Sync sync) {
     constexpr int kChunks = D_PAD / 8;
     constexpr int kOTiles = D_PAD / 8;
-    constexpr int kStages = (D_PAD <= 128 && BN >= 64) ? BN / 32 : 1;      // stages per warp
+    constexpr int kStages = (D_PAD <= 128 && BN == 64) ? 2 : 1;      // stages per warp
     constexpr int TN = BN / kStages;                       // keys per stage (the warp's shared memory is BN keys of K and of V)
     static_assert(TN == 32, "a stage holds a key a lane");
     const int lane = tid & 31, warp = tid >> 5;
@@ -339,9 +339,9 @@ __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, con
     // The first tile of keys and values is asked for before anything else (the query's own preparation below
     // takes as long as the tile needs to arrive). The token's own key and value may not be in the cache yet:
     // their row is put right in shared memory when the tile is there (see the loop).
-    // A warp's part of the shared memory is kStages stages of [K tile | V tile] of TN keys: all but one are on their way while
-    // that one is in the tensor cores. The page of a lane's key is looked up a tile before its copies are issued: a lookup in
-    // the issue itself is a round trip to the L2 a tile in which the warp has one tile less on its way.
+    // A warp's part of the shared memory is kStages stages of [K tile | V tile] of TN keys: with two, one is on its way while the
+    // other is in the tensor cores. The page of a lane's key is looked up a tile before its copies are issued, where the registers
+    // allow (kAhead): a lookup in the issue itself is a round trip to the L2 a tile in which the warp has one tile less on its way.
     const bool column = (lane % kChunks) * 8 < d;
     const __nv_bfloat16* k_lane = p.k_cache + (lane % kChunks) * 8;
     const __nv_bfloat16* v_lane = p.v_cache + (lane % kChunks) * 8;
@@ -364,18 +364,13 @@ __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, con
         decode_copy_tile<D_PAD>(k_dst, k_dst + TN * D_PAD, k_lane, v_lane, mine, column, lane);
     };
     constexpr int kTileStride = kDecodeWarps * TN;
-    constexpr int kAhead = kStages > 1 ? kStages - 1 : 1;      // tiles issued before the loop
-    int tile_begin = begin + warp * TN, next_page;
+    constexpr bool kAhead = kStages > 1 || D_PAD > 64;
+    int tile_begin = begin + warp * TN, next_page = 0;
     {
-        int pages[kAhead];
-#pragma unroll
-        for (int i = 0; i < kAhead; ++i) pages[i] = look_up(tile_begin + i * kTileStride);
-        next_page = look_up(tile_begin + kAhead * kTileStride);
-#pragma unroll
-        for (int i = 0; i < kAhead; ++i) {
-            if (tile_begin + i * kTileStride < end) issue(tile_begin + i * kTileStride, i, pages[i]);
-            cp_async_commit();
-        }
+        const int page = look_up(tile_begin);
+        if (kAhead) next_page = look_up(tile_begin + kTileStride);
+        if (tile_begin < end) issue(tile_begin, 0, page);
+        cp_async_commit();
     }
     for (int idx = tid; idx < 16 * kChunks; idx += kDecodeThreads) {
         const int r = idx / kChunks, ch = idx % kChunks;
@@ -431,13 +426,13 @@ __device__ __forceinline__ void attention_decode_item(const DecodeParams& p, con
 
     auto next_tile = [&](const int at, const int stage) {       // the tile at `at` into a stage that has been used
         if (at < end) {
-            issue(at, stage, kStages > 1 || D_PAD > 64 ? next_page : look_up(at));
-            if (kStages > 1 || D_PAD > 64) next_page = look_up(at + kTileStride);
+            issue(at, stage, kAhead ? next_page : look_up(at));
+            if (kAhead) next_page = look_up(at + kTileStride);
         }
         cp_async_commit();
     };
-    for (int stage = 0; tile_begin < end; tile_begin += kTileStride, stage = stage + 1 < kStages ? stage + 1 : 0) {
-        if (kStages > 1) next_tile(tile_begin + kAhead * kTileStride, stage > 0 ? stage - 1 : kStages - 1);
+    for (int stage = 0; tile_begin < end; tile_begin += kTileStride, stage ^= kStages - 1) {
+        if (kStages > 1) next_tile(tile_begin + kTileStride, stage ^ 1);
         cp_async_wait_group<kStages - 1>();
         __syncwarp();
         __nv_bfloat16* k_t = k_s + (size_t)stage * 2 * TN * D_PAD;
