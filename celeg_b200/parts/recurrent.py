@@ -109,9 +109,9 @@ class MlstmMixer(PortionsInChunks):
             self.norms = rt.flat_scratch("recurrent.norms", chunks * self.qk_width, torch.float32)
             self.states = rt.flat_scratch("recurrent.states", chunks * self.qk_width * self.vdim, torch.float32)
 
-    # Measured at 16 heads of 64 x 128: 1 x 128 48 in chunks, 51 token by token; 1 x 150 51, 58; 1 x 2,048 149, 556; 48 x 150 560,
-    # 925; 200 and 8 x 10 (23 tokens a chunk) 70, 88; 600 and 40 x 20 (28) 189, 273; with a carry half as fast 8 x 20 60, 43; 48 x
-    # 20 168, 152; 160 and 40 x 8 (11) 142, 96.
+    # Measured at 16 heads of 64 x 128: 1 x 128 43 in chunks, 49 token by token; 1 x 150 49, 57; 2 x 150 53, 72; 1 x 2,048 148, 555; 8
+    # x 20 57, 41; 48 x 20 163, 148; 48 x 150 549, 917; 200 and 8 x 10 (23 tokens a chunk) 70, 88; 160 and 40 x 8 (11) 139, 92; 600 and
+    # 40 x 20 (28) 183, 270.
     CHUNKED_FROM = 144
     TOKENS_A_CHUNK = 20
 
@@ -329,9 +329,9 @@ class RetentionMixer(PortionsInChunks):
             self.segment_plan = rt.flat_scratch("retention.plan", 2 * self.max_segments + 8, torch.int32, zero=True)
 
     SEGMENT = 128               # tokens a segment
-    # Measured at 16 heads of 64 x 128: 1 x 128 38 in segments, 41 token by token; 1 x 150 39, 45; 2 x 150 55, 55; 1 x 500 55,
-    # 115; 8 x 20 51, 31; 48 x 20 152, 110; 48 x 150 471, 599; 200 and 8 x 10 (23 tokens a chunk) 59, 69; 160 and 40 x 8 (11) 129,
-    # 78; 600 and 40 x 20 (28) 162, 198.
+    # Measured at 16 heads of 64 x 128: 1 x 128 33 in segments, 39 token by token; 1 x 150 39, 45; 2 x 150 53, 53; 1 x 500 53,
+    # 113; 8 x 20 49, 30; 48 x 20 148, 105; 48 x 150 463, 592; 200 and 8 x 10 (23 tokens a chunk) 59, 66; 160 and 40 x 8 (11) 127,
+    # 74; 600 and 40 x 20 (28) 157, 194.
     CHUNKED_FROM = 144
     TOKENS_A_CHUNK = 20
 
